@@ -1,0 +1,123 @@
+// Device memory and stream sets of the interpreters of one GPU.
+//
+// An interpreter owns a few hundred device buffers (every tensor of the module stays resident) and two streams. With
+// cudaMalloc / cudaFree each of them costs a driver call that also waits for the whole device, and
+// cudaGetDeviceProperties and the stream and event calls cost milliseconds more: the auto-tuner, which loads one small
+// module per tuned op, spent 95% of its time there (102 ms for 17 modules of a few ops; 5 ms per module).
+// Buffers therefore come from a stream-ordered memory pool of this library's own (cudaMallocFromPoolAsync), and the
+// streams and events of a destroyed interpreter are handed to the next one.
+//
+// Both are bounded and given back: when a module goes, free memory above kPoolKeepBytes returns to the driver, at most
+// kPoolKeepStreams idle stream sets are kept, and when the last interpreter of a GPU goes, everything goes.
+// Several threads may use it at once (one mutex around the lists; the pool calls are thread-safe themselves). A buffer is
+// allocated and freed on its interpreter's stream, which is idle when the interpreter is destroyed.
+#pragma once
+#include "host_common.h"
+
+#include <mutex>
+
+namespace tpucb {
+
+constexpr size_t kPoolKeepBytes = 256u << 20;
+constexpr size_t kPoolKeepStreams = 8;
+
+struct StreamSet {
+  cudaStream_t stream = nullptr, copy_stream = nullptr;
+  cudaEvent_t upload_done[2] = {nullptr, nullptr}, staging_free[2] = {nullptr, nullptr};
+  int *d_err = nullptr; // the interpreter's device error word
+};
+
+class DevicePool {
+public:
+  // The pools live until the process ends (no CUDA call from a static destructor).
+  static DevicePool &of(int device) {
+    static std::mutex m;
+    static std::map<int, DevicePool *> *pools = new std::map<int, DevicePool *>();
+    std::lock_guard<std::mutex> lock(m);
+    DevicePool *&p = (*pools)[device];
+    if (!p) p = new DevicePool(device);
+    return *p;
+  }
+
+  int sm_count = 148;
+
+  // One interpreter more on this device (current on the calling thread): its streams, events and error word (zero).
+  StreamSet acquire() {
+    std::lock_guard<std::mutex> lock(m_);
+    StreamSet s;
+    if (!idle_.empty()) {
+      s = idle_.back();
+      idle_.pop_back();
+    } else {
+      TPUCB_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+      TPUCB_CUDA(cudaStreamCreateWithFlags(&s.copy_stream, cudaStreamNonBlocking));
+      for (int i = 0; i < 2; ++i) {
+        TPUCB_CUDA(cudaEventCreateWithFlags(&s.upload_done[i], cudaEventDisableTiming));
+        TPUCB_CUDA(cudaEventCreateWithFlags(&s.staging_free[i], cudaEventDisableTiming));
+      }
+      TPUCB_CUDA(cudaMallocFromPoolAsync((void **)&s.d_err, sizeof(int), mem_, s.stream));
+    }
+    ++live_;
+    TPUCB_CUDA(cudaMemsetAsync(s.d_err, 0, sizeof(int), s.stream));
+    return s;
+  }
+  // ... and one less. Nothing may still run on its streams and all of its buffers are freed.
+  void release(const StreamSet &s) {
+    cudaStreamSynchronize(s.stream);
+    trim();
+    std::lock_guard<std::mutex> lock(m_);
+    idle_.push_back(s);
+    if (--live_ > 0 && idle_.size() <= kPoolKeepStreams) return;
+    while (!idle_.empty() && (live_ == 0 || idle_.size() > kPoolKeepStreams)) {
+      StreamSet &d = idle_.back();
+      cudaFreeAsync(d.d_err, d.stream);
+      cudaStreamSynchronize(d.stream);
+      for (int i = 0; i < 2; ++i) {
+        cudaEventDestroy(d.upload_done[i]);
+        cudaEventDestroy(d.staging_free[i]);
+      }
+      cudaStreamDestroy(d.copy_stream);
+      cudaStreamDestroy(d.stream);
+      idle_.pop_back();
+    }
+    if (live_ == 0) cudaMemPoolTrimTo(mem_, 0);
+  }
+
+  void *alloc(size_t bytes, cudaStream_t stream) {
+    void *p = nullptr;
+    TPUCB_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, mem_, stream));
+    return p;
+  }
+
+  // Gives the driver back what lies free above kPoolKeepBytes. Called where a module's buffers have been freed; in between
+  // the pool holds on to what it has (its release threshold counts the memory in use too, so with any finite threshold
+  // a process that holds a large module would unmap and map again at every synchronisation: 40 ms spikes).
+  void trim() {
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(mem_, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+      cudaMemPoolTrimTo(mem_, used + kPoolKeepBytes);
+  }
+
+private:
+  explicit DevicePool(int device) {
+    int major = 0, minor = 0;
+    TPUCB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    TPUCB_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    TPUCB_CHECK(major == 10, "this backend is written for sm_100a (B200); device %d is sm_%d%d", device, major, minor);
+    TPUCB_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    TPUCB_CUDA(cudaMemPoolCreate(&mem_, &props));
+    uint64_t keep = UINT64_MAX; // see trim()
+    TPUCB_CUDA(cudaMemPoolSetAttribute(mem_, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
+
+  std::mutex m_;
+  cudaMemPool_t mem_ = nullptr;
+  std::vector<StreamSet> idle_;
+  int live_ = 0;
+};
+
+} // namespace tpucb

@@ -7,6 +7,7 @@
 // get_tensor / get_all_tensor work as in the reference.
 #pragma once
 #include "conv_plan.cuh"
+#include "device_pool.h"
 #include "f32_kernels.cuh"
 #include "calib_kernels.cuh"
 #include "extra_kernels.cuh"
@@ -85,37 +86,36 @@ class Interpreter {
 public:
   explicit Interpreter(int device) : device_(device) {
     TPUCB_CUDA(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    TPUCB_CUDA(cudaGetDeviceProperties(&prop, device));
-    TPUCB_CHECK(prop.major == 10, "this backend is written for sm_100a (B200); device %d is sm_%d%d",
-                device, prop.major, prop.minor);
-    sm_count = prop.multiProcessorCount;
-    TPUCB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    TPUCB_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
+    pool = &DevicePool::of(device);
+    sm_count = pool->sm_count;
+    const StreamSet s = pool->acquire();
+    stream = s.stream;
+    copy_stream = s.copy_stream;
     for (int i = 0; i < 2; ++i) {
-      TPUCB_CUDA(cudaEventCreateWithFlags(&upload_done[i], cudaEventDisableTiming));
-      TPUCB_CUDA(cudaEventCreateWithFlags(&staging_free[i], cudaEventDisableTiming));
+      upload_done[i] = s.upload_done[i];
+      staging_free[i] = s.staging_free[i];
     }
-    TPUCB_CUDA(cudaMalloc(&d_err, sizeof(int)));
-    TPUCB_CUDA(cudaMemset(d_err, 0, sizeof(int)));
+    d_err = s.d_err;
   }
   ~Interpreter() {
     cudaSetDevice(device_);
-    cudaStreamSynchronize(stream);
+    cudaDeviceSynchronize(); // as cudaFree would: nobody's kernels still read a tensor of this module
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     kernels.clear();
     for (auto &kv : tensors)
-      if (kv.second->owns && kv.second->dev) cudaFree(kv.second->dev);
-    for (void *p : allocations) cudaFree(p);
-    if (staging) cudaFree(staging);
+      if (kv.second->owns) dfree(kv.second->dev);
+    for (void *p : allocations) dfree(p);
+    dfree(staging);
+    for (int i = 0; i < 2; ++i) dfree(async_staging[i]);
+    StreamSet s;
+    s.stream = stream;
+    s.copy_stream = copy_stream;
     for (int i = 0; i < 2; ++i) {
-      if (async_staging[i]) cudaFree(async_staging[i]);
-      cudaEventDestroy(upload_done[i]);
-      cudaEventDestroy(staging_free[i]);
+      s.upload_done[i] = upload_done[i];
+      s.staging_free[i] = staging_free[i];
     }
-    cudaFree(d_err);
-    cudaStreamDestroy(copy_stream);
-    cudaStreamDestroy(stream);
+    s.d_err = d_err;
+    pool->release(s);
   }
 
   void bind() {
@@ -128,21 +128,24 @@ public:
 
   // ---- device memory owned by the interpreter
   void *dalloc(size_t bytes) {
-    void *p = nullptr;
-    TPUCB_CUDA(cudaMalloc(&p, bytes ? bytes : 16));
+    void *p = pool->alloc(bytes, stream);
     allocations.push_back(p);
     return p;
   }
+  void dfree(void *p) {
+    if (p) cudaFreeAsync(p, stream);
+  }
   template <class T> T *upload(const std::vector<T> &v) {
     T *p = (T *)dalloc(v.size() * sizeof(T));
-    if (!v.empty()) TPUCB_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (!v.empty()) TPUCB_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream)); // pageable: staged before it returns
     return p;
   }
   float *ensure_staging(size_t bytes) {
     if (bytes > staging_bytes) {
-      TPUCB_CUDA(cudaStreamSynchronize(stream));
-      if (staging) cudaFree(staging);
-      TPUCB_CUDA(cudaMalloc(&staging, bytes));
+      dfree(staging);
+      staging = nullptr;
+      staging_bytes = 0;
+      staging = pool->alloc(bytes, stream);
       staging_bytes = bytes;
     }
     return (float *)staging;
@@ -178,8 +181,8 @@ public:
       t->wl = lr->second.wl;
       t->wphys = lr->second.wphys;
     }
-    TPUCB_CUDA(cudaMalloc(&t->dev, t->bytes()));
-    TPUCB_CUDA(cudaMemset(t->dev, 0, t->bytes()));
+    t->dev = pool->alloc(t->bytes(), stream);
+    TPUCB_CUDA(cudaMemsetAsync(t->dev, 0, t->bytes(), stream));
     return t;
   }
 
@@ -220,6 +223,7 @@ public:
   }
 
   int device_;
+  DevicePool *pool = nullptr;
   // MlirModuleInterpreter(int32_t batch) (MlirModuleInterpreter.h:35): the reference keeps `batch` copies ("slots") of
   // every activation and runs the kernels on one slot at a time. Here slot b is image group b of ONE device tensor
   // whose leading dimension is max_batch x the module's, so one launch covers every slot.
@@ -251,8 +255,8 @@ public:
     const size_t bytes = (size_t)pl.ws_tiles * 128 * 128 * sizeof(int32_t), cbytes = (size_t)pl.ws_tiles * sizeof(unsigned int);
     pl.p.ws = (int32_t *)dalloc(bytes);
     pl.p.ws_count = (unsigned int *)dalloc(cbytes);
-    TPUCB_CUDA(cudaMemset(pl.p.ws, 0, bytes));
-    TPUCB_CUDA(cudaMemset(pl.p.ws_count, 0, cbytes));
+    TPUCB_CUDA(cudaMemsetAsync(pl.p.ws, 0, bytes, stream));
+    TPUCB_CUDA(cudaMemsetAsync(pl.p.ws_count, 0, cbytes, stream));
     split_ws.push_back({pl.p.ws, bytes});
     split_ws.push_back({pl.p.ws_count, cbytes});
   }
@@ -277,6 +281,14 @@ public:
   cudaEvent_t upload_done[2], staging_free[2];
   bool staging_used[2] = {false, false};
   int async_next = 0;
+  void grow_async_staging(int k, size_t bytes) { // both streams are idle
+    dfree(async_staging[k]);
+    async_staging[k] = nullptr;
+    async_staging_bytes[k] = 0;
+    async_staging[k] = pool->alloc(bytes, stream);
+    TPUCB_CUDA(cudaStreamSynchronize(stream)); // the copy stream may use it from here on
+    async_staging_bytes[k] = bytes;
+  }
   void set_tensor_async(const std::string &name, const float *pinned, size_t numel);
   void set_tensor_async_i8(const std::string &name, const int8_t *pinned, size_t numel);
   void reenable_quant_of(const DevTensor *input);
@@ -1943,9 +1955,15 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
 inline void Interpreter::reset_module() {
   bind();
   invalidate_graph();
+  TPUCB_CUDA(cudaDeviceSynchronize());
   kernels.clear();
   for (auto &kv : tensors)
-    if (kv.second->owns && kv.second->dev) cudaFree(kv.second->dev);
+    if (kv.second->owns) dfree(kv.second->dev);
+  for (void *p : allocations) dfree(p);
+  allocations.clear();
+  split_ws.clear();
+  TPUCB_CUDA(cudaStreamSynchronize(stream));
+  pool->trim();
   tensors.clear();
   tensor_order.clear();
   input_details.clear();
@@ -2097,7 +2115,7 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
     } else if (op.type == "softmax") {
       k.reset(new SoftmaxOp(*this, op, opd(0), out));
     } else {
-      cudaFree(out->dev);
+      dfree(out->dev);
       throw Error(strfmt("op type '%s' (%s) is not implemented by the B200 backend", op.type.c_str(), op.name.c_str()));
     }
     k->name = op.name;
@@ -2121,7 +2139,7 @@ inline void Interpreter::finish_module() {
   output_details.clear();
   for (auto &k : kernels)
     if (!uses.count(k->name) && k->op_type != "input") output_details.push_back({k->name, k->result->numel() / (size_t)max_batch});
-  TPUCB_CUDA(cudaDeviceSynchronize());
+  TPUCB_CUDA(cudaStreamSynchronize(stream));
 }
 
 inline void Interpreter::load_module(const std::string &text) {
@@ -2235,9 +2253,7 @@ inline void Interpreter::set_tensor_async(const std::string &name, const float *
   if (bytes > async_staging_bytes[k]) {
     TPUCB_CUDA(cudaStreamSynchronize(stream));
     TPUCB_CUDA(cudaStreamSynchronize(copy_stream));
-    if (async_staging[k]) cudaFree(async_staging[k]);
-    TPUCB_CUDA(cudaMalloc(&async_staging[k], bytes));
-    async_staging_bytes[k] = bytes;
+    grow_async_staging(k, bytes);
     staging_used[k] = false;
   }
   // the previous conversion out of this staging buffer must have finished
@@ -2304,9 +2320,7 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
   if (numel > async_staging_bytes[k]) {
     TPUCB_CUDA(cudaStreamSynchronize(stream));
     TPUCB_CUDA(cudaStreamSynchronize(copy_stream));
-    if (async_staging[k]) cudaFree(async_staging[k]);
-    TPUCB_CUDA(cudaMalloc(&async_staging[k], numel));
-    async_staging_bytes[k] = numel;
+    grow_async_staging(k, numel);
     staging_used[k] = false;
   }
   if (staging_used[k]) TPUCB_CUDA(cudaStreamWaitEvent(copy_stream, staging_free[k], 0));
@@ -2405,8 +2419,8 @@ inline void Interpreter::sync_and_check() {
   int err = 0;
   TPUCB_CUDA(cudaMemcpy(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err != 0) {
-    TPUCB_CUDA(cudaMemset(d_err, 0, sizeof(int)));
-    for (auto &w : split_ws) TPUCB_CUDA(cudaMemset(w.first, 0, w.second)); // a failed launch may leave partial sums
+    TPUCB_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+    for (auto &w : split_ws) TPUCB_CUDA(cudaMemsetAsync(w.first, 0, w.second, stream)); // a failed launch may leave partial sums
     throw Error(strfmt("a convolution kernel gave up on a bounded wait (code %d: 1 = tile load never arrived, "
                        "2 = stage never freed, 3 = accumulator never completed or never handed back); the launch's "
                        "results are incomplete, the interpreter stays usable", err));

@@ -27,8 +27,9 @@ struct tpucb_interp {
   int stat_descs_cap = 0;
   explicit tpucb_interp(int device) : impl(device) {}
   ~tpucb_interp() {
-    if (tuner_sums) cudaFree(tuner_sums);
-    if (stat_descs) cudaFree(stat_descs);
+    cudaSetDevice(impl.device());
+    impl.dfree(tuner_sums);
+    impl.dfree(stat_descs);
   }
 };
 
@@ -481,10 +482,10 @@ int tpucb_tuner_distance(tpucb_interp *ref, const char *ref_name, tpucb_interp *
   TPUCB_CHECK(r->cp % 4 == 0 && t->cp % 4 == 0, "tpucb_tuner_distance: channel pitch is not a multiple of 4");
   T.bind();
   if (tgt->tuner_sums_cap < images) {
-    if (tgt->tuner_sums) TPUCB_CUDA(cudaFree(tgt->tuner_sums));
+    T.dfree(tgt->tuner_sums);
     tgt->tuner_sums = nullptr;
     tgt->tuner_sums_cap = 0;
-    TPUCB_CUDA(cudaMalloc(&tgt->tuner_sums, sizeof(double) * 2 * images));
+    tgt->tuner_sums = (double *)T.pool->alloc(sizeof(double) * 2 * images, T.stream);
     tgt->tuner_sums_cap = images;
   }
   TPUCB_CUDA(cudaStreamSynchronize(R.stream)); // the reference activations are complete
@@ -657,11 +658,10 @@ static const StatDesc *stat_descs_upload(tpucb_interp *it, const char *const *na
     d.pad_ = 0;
   }
   if (it->stat_descs_cap < count) {
-    TPUCB_CUDA(cudaStreamSynchronize(I.stream));
-    if (it->stat_descs) TPUCB_CUDA(cudaFree(it->stat_descs));
+    I.dfree(it->stat_descs);
     it->stat_descs = nullptr;
     it->stat_descs_cap = 0;
-    TPUCB_CUDA(cudaMalloc(&it->stat_descs, sizeof(StatDesc) * count));
+    it->stat_descs = (StatDesc *)I.pool->alloc(sizeof(StatDesc) * count, I.stream);
     it->stat_descs_cap = count;
   }
   TPUCB_CUDA(cudaMemcpyAsync(it->stat_descs, h.data(), sizeof(StatDesc) * count, cudaMemcpyHostToDevice, I.stream));
@@ -703,21 +703,16 @@ int tpucb_calib_kld(tpucb_interp *it, const int64_t *d_hist, const float *widths
   Interpreter &I = it->impl;
   I.bind();
   const int kl_num = bins / 128;
-  float *d_kl = nullptr;
-  TPUCB_CUDA(cudaMalloc(&d_kl, sizeof(float) * count * kl_num));
   size_t smem = (size_t)bins * (2 * sizeof(float) + sizeof(double));
   // always the limit of the largest bin count: the attribute is per function and device, shared with
   // tpucb_calib_kld_static and with other threads, so no call may lower it under another call's launch
-  cudaError_t e = cudaFuncSetAttribute(kld_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKldMaxSmem);
-  if (e != cudaSuccess) {
-    cudaFree(d_kl);
-    TPUCB_CUDA(e);
-  }
+  TPUCB_CUDA(cudaFuncSetAttribute(kld_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKldMaxSmem));
+  float *d_kl = (float *)I.pool->alloc(sizeof(float) * count * kl_num, I.stream);
   kld_kernel<<<count * kl_num, 256, smem, I.stream>>>((const long long *)d_hist, bins, d_kl);
   std::vector<float> kl((size_t)count * kl_num);
-  e = cudaMemcpyAsync(kl.data(), d_kl, kl.size() * sizeof(float), cudaMemcpyDeviceToHost, I.stream);
+  cudaError_t e = cudaMemcpyAsync(kl.data(), d_kl, kl.size() * sizeof(float), cudaMemcpyDeviceToHost, I.stream);
+  I.dfree(d_kl);
   if (e == cudaSuccess) e = cudaStreamSynchronize(I.stream);
-  cudaFree(d_kl);
   TPUCB_CUDA(e);
   // the_min_index + threshold (calibration_math.cpp:85-98, 321-322): first strict minimum.
   for (int t = 0; t < count; ++t) {
