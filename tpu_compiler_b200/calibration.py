@@ -59,6 +59,7 @@ class ActivationCalibrator:
         self.keep_activations_gb = keep_activations_gb   # None: 60% of the free device memory; 0: keep nothing
         self._kept = []          # per cached batch: (uint8 device buffer, images)
         self._kept_offsets = None
+        self._plan = None         # (bytes per batch, budget), see _keep_plan
         self._local_images = -1   # images this rank saw in pass 1
         self._pinned = None
         self._pinned_numel = 0
@@ -132,7 +133,15 @@ class ActivationCalibrator:
         return self._names_c
 
     def _keep_plan(self):
-        """(bytes one batch's fp32 activations take in the cache, byte budget of the cache)."""
+        """(bytes one batch's fp32 activations take in the cache, byte budget of the cache). Worked out once: the tensors do
+        not change, and asking the driver for the free memory takes its lock, which other processes of the machine hold
+        for up to 60 ms at a time (measured: single passes of 75 ms among passes of 18). If the memory has gone since,
+        the allocation fails and the batches from there on are recomputed."""
+        if self._plan is None:
+            self._plan = self._make_keep_plan()
+        return self._plan
+
+    def _make_keep_plan(self):
         if self.keep_activations_gb is not None and self.keep_activations_gb <= 0:
             return 0, 0
         offs, total = [], 0
