@@ -314,6 +314,15 @@ constexpr int kMaxStages = 8;
 constexpr int kMaxBN = 256;
 constexpr int kSmemHeader = 8192; // barriers + staged per-channel parameters
 
+// Records why a launch gave up, in the device word that later CTAs and kernels look at and in the host's own memory, whose
+// address stands 8 bytes behind the device word (ErrWord).
+__device__ __forceinline__ void report_error(int *err, int code) {
+  atomicExch(err, code);
+  int *host = *reinterpret_cast<int **>(err + 2);
+  *reinterpret_cast<volatile int *>(host) = code;
+  __threadfence_system();
+}
+
 enum ConvErr { kErrFullWait = 1, kErrEmptyWait = 2, kErrAccWait = 3 };
 
 // Per-channel requantisation constants, held in registers by the thread that owns the channel.
@@ -798,7 +807,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           const CUtensorMap *mapB = (TF32 && term == 1) ? &tmB2 : &tmB;
           if (it >= p.stages) {
             if (!ptx::mbar_wait_bounded(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
-              if (!*abort_flag) atomicExch(p.err, kErrEmptyWait);
+              if (!*abort_flag) report_error(p.err, kErrEmptyWait);
               *abort_flag = 1;
               ok = false;
               break;
@@ -880,7 +889,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const int ksteps = p.BK / 32;
       if (p.w_resident && (int)blockIdx.x < total_tiles) {
         if (!ptx::mbar_wait_bounded(bar_w, 0u, abort_flag, wait_rounds)) {
-          if (!*abort_flag) atomicExch(p.err, kErrFullWait);
+          if (!*abort_flag) report_error(p.err, kErrFullWait);
           *abort_flag = 1;
           ok = false;
         }
@@ -895,7 +904,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         if (t >= 2) {
           // the epilogue must have drained this accumulator buffer (its previous use)
           if (!ptx::mbar_wait_bounded(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
-            if (!*abort_flag) atomicExch(p.err, kErrAccWait);
+            if (!*abort_flag) report_error(p.err, kErrAccWait);
             *abort_flag = 1;
             ok = false;
             break;
@@ -906,7 +915,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         uint32_t wres_lo = desc_w_lo; // weight-resident mode: descriptor (low word) of K block `kit`
         for (int kit = k_begin; kit < k_end; ++kit, ++it) {
           if (!ptx::mbar_try_wait(m_full, mph) && !ptx::mbar_wait_bounded(m_full, mph, abort_flag, wait_rounds)) {
-            if (!*abort_flag) atomicExch(p.err, kErrFullWait);
+            if (!*abort_flag) report_error(p.err, kErrFullWait);
             *abort_flag = 1;
             ok = false;
             break;
@@ -986,7 +995,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       }
       ok = ptx::mbar_wait_bounded(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds);
       if (!ok && !*abort_flag) {
-        atomicExch(p.err, kErrAccWait);
+        report_error(p.err, kErrAccWait);
         *abort_flag = 1;
       }
       // the wait result may differ between lanes only on the error path; make it uniform

@@ -104,14 +104,14 @@ conv_stem_i8_kernel(const __grid_constant__ CUtensorMap tmB, const ConvStemParam
         // the copy is still owed: wait for it (bounded) before the CTA may release shared memory
         for (uint32_t it = 0; it < (1u << 20); ++it)
           if (ptx::mbar_try_wait(bar_b, 0u)) break;
-        if (!*abort_flag) atomicExch(p.err, kErrFullWait);
+        if (!*abort_flag) report_error(p.err, kErrFullWait);
         *abort_flag = 1;
       }
       int t = 0;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++t) {
         ok = ptx::mbar_wait_bounded(bar_a, (uint32_t)(t & 1), abort_flag);
         if (!ok) {
-          if (!*abort_flag) atomicExch(p.err, kErrFullWait);
+          if (!*abort_flag) report_error(p.err, kErrFullWait);
           *abort_flag = 1;
           break;
         }
@@ -195,7 +195,7 @@ conv_stem_i8_kernel(const __grid_constant__ CUtensorMap tmB, const ConvStemParam
       // ---- epilogue
       ok = ptx::mbar_wait_bounded(bar_acc, (uint32_t)(t & 1), abort_flag);
       if (!ok && !*abort_flag) {
-        atomicExch(p.err, kErrAccWait);
+        report_error(p.err, kErrAccWait);
         *abort_flag = 1;
       }
       ok = __all_sync(0xffffffffu, ok);

@@ -21,10 +21,29 @@ namespace tpucb {
 constexpr size_t kPoolKeepBytes = 256u << 20;
 constexpr size_t kPoolKeepStreams = 8;
 
+// The error word of an interpreter: kernels that give up write their code here and, through `host`, into pinned host
+// memory (report_error), so that the host learns of it from its own memory after an ordinary stream synchronisation: the
+// read-back of the device word cost every synchronous call a second driver round trip (14.5 us for a synchronisation with
+// it, 4 us without).
+struct ErrWord {
+  int code;
+  int pad_;
+  int *host;
+};
+
+constexpr size_t kUploadSlot = 1u << 20; // bytes of one of the pinned upload slots of a stream set
+constexpr int kUploadSlots = 4;
+constexpr size_t kDownloadBytes = 32u << 10; // its pinned download buffer (256 KB written that way: 11 us more than by a copy)
+
 struct StreamSet {
   cudaStream_t stream = nullptr, copy_stream = nullptr;
   cudaEvent_t upload_done[2] = {nullptr, nullptr}, staging_free[2] = {nullptr, nullptr};
-  int *d_err = nullptr; // the interpreter's device error word
+  ErrWord *d_err = nullptr; // the interpreter's device error word
+  int *h_err = nullptr;     // ... and its host part
+  // pinned, device-visible buffers of set_tensor / get_tensor, allocated at first use
+  float *download = nullptr;
+  uint8_t *upload = nullptr;
+  cudaEvent_t upload_read[kUploadSlots] = {}; // the kernels that read the slot are done
 };
 
 class DevicePool {
@@ -55,10 +74,14 @@ public:
         TPUCB_CUDA(cudaEventCreateWithFlags(&s.upload_done[i], cudaEventDisableTiming));
         TPUCB_CUDA(cudaEventCreateWithFlags(&s.staging_free[i], cudaEventDisableTiming));
       }
-      TPUCB_CUDA(cudaMallocFromPoolAsync((void **)&s.d_err, sizeof(int), mem_, s.stream));
+      TPUCB_CUDA(cudaMallocFromPoolAsync((void **)&s.d_err, sizeof(ErrWord), mem_, s.stream));
+      TPUCB_CUDA(cudaHostAlloc((void **)&s.h_err, 64, cudaHostAllocMapped));
+      const ErrWord w{0, 0, s.h_err};
+      TPUCB_CUDA(cudaMemcpyAsync(s.d_err, &w, sizeof(w), cudaMemcpyHostToDevice, s.stream));
     }
     ++live_;
-    TPUCB_CUDA(cudaMemsetAsync(s.d_err, 0, sizeof(int), s.stream));
+    *s.h_err = 0;
+    TPUCB_CUDA(cudaMemsetAsync(&s.d_err->code, 0, sizeof(int), s.stream));
     return s;
   }
   // ... and one less. Nothing may still run on its streams and all of its buffers are freed.
@@ -72,6 +95,11 @@ public:
       StreamSet &d = idle_.back();
       cudaFreeAsync(d.d_err, d.stream);
       cudaStreamSynchronize(d.stream);
+      cudaFreeHost(d.h_err);
+      if (d.download) cudaFreeHost(d.download);
+      if (d.upload) cudaFreeHost(d.upload);
+      for (cudaEvent_t e : d.upload_read)
+        if (e) cudaEventDestroy(e);
       for (int i = 0; i < 2; ++i) {
         cudaEventDestroy(d.upload_done[i]);
         cudaEventDestroy(d.staging_free[i]);

@@ -8,6 +8,7 @@
 #pragma once
 #include "conv_plan.cuh"
 #include "device_pool.h"
+#include "host_copy.h"
 #include "f32_kernels.cuh"
 #include "calib_kernels.cuh"
 #include "extra_kernels.cuh"
@@ -88,14 +89,9 @@ public:
     TPUCB_CUDA(cudaSetDevice(device));
     pool = &DevicePool::of(device);
     sm_count = pool->sm_count;
-    const StreamSet s = pool->acquire();
-    stream = s.stream;
-    copy_stream = s.copy_stream;
-    for (int i = 0; i < 2; ++i) {
-      upload_done[i] = s.upload_done[i];
-      staging_free[i] = s.staging_free[i];
-    }
-    d_err = s.d_err;
+    ss = pool->acquire();
+    stream = ss.stream;
+    copy_stream = ss.copy_stream;
   }
   ~Interpreter() {
     cudaSetDevice(device_);
@@ -107,15 +103,7 @@ public:
     for (void *p : allocations) dfree(p);
     dfree(staging);
     for (int i = 0; i < 2; ++i) dfree(async_staging[i]);
-    StreamSet s;
-    s.stream = stream;
-    s.copy_stream = copy_stream;
-    for (int i = 0; i < 2; ++i) {
-      s.upload_done[i] = upload_done[i];
-      s.staging_free[i] = staging_free[i];
-    }
-    s.d_err = d_err;
-    pool->release(s);
+    pool->release(ss);
   }
 
   void bind() {
@@ -232,7 +220,7 @@ public:
   std::map<std::string, int> uses;
   int sm_count = 148;
   cudaStream_t stream = nullptr;
-  int *d_err = nullptr;
+  StreamSet ss; // streams, events, error word, pinned buffers
   bool use_graph = true;
   // Programmatic dependent launch (option "pdl"): a kernel launched with the attribute may be scheduled while its
   // predecessor in the stream is still running; it sets up its barriers and tensor memory and then waits for that
@@ -278,7 +266,6 @@ public:
   cudaStream_t copy_stream = nullptr;
   void *async_staging[2] = {nullptr, nullptr};
   size_t async_staging_bytes[2] = {0, 0};
-  cudaEvent_t upload_done[2], staging_free[2];
   bool staging_used[2] = {false, false};
   int async_next = 0;
   void grow_async_staging(int k, size_t bytes) { // both streams are idle
@@ -289,6 +276,9 @@ public:
     TPUCB_CUDA(cudaStreamSynchronize(stream)); // the copy stream may use it from here on
     async_staging_bytes[k] = bytes;
   }
+  void upload_pageable(void *staging, const void *data, size_t bytes);
+  int upload_next = 0;    // upload slot of the next piece
+  int quants_disabled = 0; // quant ops that set_tensor_async_i8 has switched off
   void set_tensor_async(const std::string &name, const float *pinned, size_t numel);
   void set_tensor_async_i8(const std::string &name, const int8_t *pinned, size_t numel);
   void reenable_quant_of(const DevTensor *input);
@@ -462,7 +452,7 @@ public:
       p.out = (int8_t *)out->dev;
       p.ldc = out->cp * 2; // bytes
       p.c_off = 0;
-      p.err = I.d_err;
+      p.err = &I.ss.d_err->code;
       const int rows = g.n * g.oh * g.ow;
       const int k_bytes = in->cp * 2;
       const bool one_by_one_bf = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
@@ -548,7 +538,7 @@ public:
         p.out = (int8_t *)out->dev;
         p.ldc = out->cp * 4;
         p.c_off = 0;
-        p.err = I.d_err;
+        p.err = &I.ss.d_err->code;
         p.kh = p.kw = 1;
         p.a_mode = 0;
         const int kb = a.kp * 4;
@@ -594,7 +584,7 @@ public:
         p.out = (int8_t *)out->dev;
         p.ldc = out->cp * 4; // bytes
         p.c_off = 0;
-        p.err = I.d_err;
+        p.err = &I.ss.d_err->code;
         const int rows = g.n * g.oh * g.ow;
         const int k_bytes = in->cp * 4;
         const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
@@ -681,7 +671,7 @@ public:
       p.out = (int8_t *)out->dev;
       p.ldc = out->cp;
       p.c_off = 0;
-      p.err = I.d_err;
+      p.err = &I.ss.d_err->code;
       const int8_t *d_w = I.upload(pack_stem_weights(filt.data.data(), g.oc, g.ic, g.kh, g.kw, oc_pad));
       finish_stem_plan(sp, d_w, g.n * g.oh * g.ow, g.kh, oc_pad, I.sm_count);
       stem_plans_.push_back(sp);
@@ -720,7 +710,7 @@ public:
       p.out = (int8_t *)out->dev;
       p.ldc = out->cp;
       p.c_off = grp * ocg;
-      p.err = I.d_err;
+      p.err = &I.ss.d_err->code;
       const int rows = g.n * g.oh * g.ow;
       const float *wsrc = filt.data.data() + (size_t)grp * ocg * icg * g.kh * g.kw;
       int ocg_pad = groups == 1 ? oc_pad : ocg;
@@ -945,7 +935,7 @@ public:
       p.out = (int8_t *)out->dev;
       p.ldc = out->cp * 2;
       p.c_off = 0;
-      p.err = I.d_err;
+      p.err = &I.ss.d_err->code;
       p.OH = p.OW = 1; p.sh = p.sw = p.dh = p.dw = 1; p.kh = p.kw = 1;
       p.act = do_relu_ ? 1 : 0;
       p.a_mode = 0;
@@ -996,7 +986,7 @@ public:
     p.out = (int8_t *)out->dev;
     p.ldc = out->cp;
     p.c_off = 0;
-    p.err = I.d_err;
+    p.err = &I.ss.d_err->code;
     p.OH = p.OW = 1; p.sh = p.sw = p.dh = p.dw = 1; p.kh = p.kw = 1;
     // The reference applies ReLU to the float before the QDM requant; with a positive
     // multiplier the two orders give the same int8 result.
@@ -1957,6 +1947,7 @@ inline void Interpreter::reset_module() {
   invalidate_graph();
   TPUCB_CUDA(cudaDeviceSynchronize());
   kernels.clear();
+  quants_disabled = 0;
   for (auto &kv : tensors)
     if (kv.second->owns) dfree(kv.second->dev);
   for (void *p : allocations) dfree(p);
@@ -2223,7 +2214,7 @@ inline void Interpreter::set_tensor(const std::string &name, const float *data, 
   const SlotView v = slot_view(*t, slot, max_batch, "set_tensor");
   TPUCB_CHECK(numel == v.numel, "set_tensor %s: got %zu values, tensor has %zu", name.c_str(), numel, v.numel);
   float *stg = ensure_staging(numel * sizeof(float));
-  TPUCB_CUDA(cudaMemcpyAsync(stg, data, numel * sizeof(float), cudaMemcpyHostToDevice, stream));
+  upload_pageable(stg, data, numel * sizeof(float));
   const TensorGeom &g = v.g;
   const size_t pixels = (size_t)g.n * g.h * g.wphys;
   size_t total = pixels * t->cp;
@@ -2235,6 +2226,57 @@ inline void Interpreter::set_tensor(const std::string &name, const float *data, 
   else if (t->dtype == DT_BF16) launch_k(nchw_f32_to_dev_kernel<DT_BF16>, grid, 256, 0, stream, stg, v.dev, g);
   else launch_k(nchw_f32_to_dev_kernel<DT_F32>, grid, 256, 0, stream, stg, v.dev, g);
   TPUCB_CUDA(cudaGetLastError());
+}
+
+// Pageable host values -> device staging, on the compute stream; returns once the caller's array has been read. From 128 KB
+// on: blocks of 64 KB are copied into pinned slots (CopyHelpers: several host threads for 1 MB and more; at 600 KB waking
+// them costs what they save), and every piece of four blocks is sent as soon as it is complete, while the next ones are
+// being copied. The driver's own path for pageable memory copies on one thread: set_tensor of 2.1 MB and its arrival on the
+// device took 155-170 us and take 97-108 here, 29 MB 1640 us and 930. (Conversion kernels that read the pinned slot over the
+// link themselves were slower: 15-19 GB/s.)
+inline void Interpreter::upload_pageable(void *staging, const void *data, size_t bytes) {
+  if (bytes < (128u << 10)) {
+    TPUCB_CUDA(cudaMemcpyAsync(staging, data, bytes, cudaMemcpyHostToDevice, stream));
+    return;
+  }
+  if (!ss.upload) {
+    TPUCB_CUDA(cudaHostAlloc((void **)&ss.upload, kUploadSlot * kUploadSlots, cudaHostAllocDefault));
+    for (cudaEvent_t &e : ss.upload_read) TPUCB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  constexpr size_t kBlock = 64u << 10;
+  constexpr int kPiece = 4; // blocks
+  constexpr int kMaxPieces = (int)(kUploadSlot / (kBlock * kPiece));
+  const bool parallel = bytes >= (1u << 20);
+  for (size_t at = 0; at < bytes; at += kUploadSlot) {
+    const size_t len = std::min(kUploadSlot, bytes - at);
+    const int blocks = (int)((len + kBlock - 1) / kBlock), pieces = (blocks + kPiece - 1) / kPiece, slot = upload_next;
+    upload_next = (upload_next + 1) % kUploadSlots;
+    TPUCB_CUDA(cudaEventSynchronize(ss.upload_read[slot]));
+    uint8_t *pinned = ss.upload + (size_t)slot * kUploadSlot;
+    const uint8_t *src = (const uint8_t *)data + at;
+    std::atomic<int> done[kMaxPieces];
+    for (auto &d : done) d.store(0, std::memory_order_relaxed);
+    int sent = 0;
+    cudaError_t e = cudaSuccess; // an error must not leave run() while helpers still copy
+    CopyHelpers::run(
+        blocks, parallel,
+        [&](int i) {
+          stream_copy(pinned + i * kBlock, src + i * kBlock, std::min(kBlock, len - i * kBlock));
+          done[i / kPiece].fetch_add(1, std::memory_order_release);
+        },
+        [&] {
+          while (sent < pieces && done[sent].load(std::memory_order_acquire) == std::min(kPiece, blocks - sent * kPiece)) {
+            const size_t from = (size_t)sent * kPiece * kBlock;
+            const cudaError_t r = cudaMemcpyAsync((uint8_t *)staging + at + from, pinned + from, std::min(kPiece * kBlock, len - from),
+                                                  cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = r;
+            ++sent;
+          }
+          return sent == pieces;
+        });
+    TPUCB_CUDA(e);
+    TPUCB_CUDA(cudaEventRecord(ss.upload_read[slot], stream));
+  }
 }
 
 // Pipelined form of setTensor for serving loops: the host-to-device copy runs on a second stream
@@ -2257,10 +2299,10 @@ inline void Interpreter::set_tensor_async(const std::string &name, const float *
     staging_used[k] = false;
   }
   // the previous conversion out of this staging buffer must have finished
-  if (staging_used[k]) TPUCB_CUDA(cudaStreamWaitEvent(copy_stream, staging_free[k], 0));
+  if (staging_used[k]) TPUCB_CUDA(cudaStreamWaitEvent(copy_stream, ss.staging_free[k], 0));
   TPUCB_CUDA(cudaMemcpyAsync(async_staging[k], pinned, bytes, cudaMemcpyHostToDevice, copy_stream));
-  TPUCB_CUDA(cudaEventRecord(upload_done[k], copy_stream));
-  TPUCB_CUDA(cudaStreamWaitEvent(stream, upload_done[k], 0));
+  TPUCB_CUDA(cudaEventRecord(ss.upload_done[k], copy_stream));
+  TPUCB_CUDA(cudaStreamWaitEvent(stream, ss.upload_done[k], 0));
   TensorGeom g{t->n, t->c, t->h, t->w, t->cp, t->wl, t->wphys};
   size_t total = t->pixels() * t->cp;
   int grid = grid_for(total, 256, sm_count);
@@ -2272,16 +2314,18 @@ inline void Interpreter::set_tensor_async(const std::string &name, const float *
   else if (t->dtype == DT_BF16) launch_k(nchw_f32_to_dev_kernel<DT_BF16>, grid, 256, 0, stream, stg, t->dev, g);
   else launch_k(nchw_f32_to_dev_kernel<DT_F32>, grid, 256, 0, stream, stg, t->dev, g);
   TPUCB_CUDA(cudaGetLastError());
-  TPUCB_CUDA(cudaEventRecord(staging_free[k], stream));
+  TPUCB_CUDA(cudaEventRecord(ss.staging_free[k], stream));
   staging_used[k] = true;
 }
 
 // A quant op that was switched off by set_tensor_async_i8 runs again once its fp32 input is set the ordinary way.
 inline void Interpreter::reenable_quant_of(const DevTensor *input) {
+  if (quants_disabled == 0) return;
   for (auto &k : kernels) {
     auto *q = dynamic_cast<QuantOp *>(k.get());
     if (q && q->disabled && q->in().get() == input) {
       q->disabled = false;
+      --quants_disabled;
       invalidate_graph();
     }
   }
@@ -2312,6 +2356,7 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
     TPUCB_CHECK(ok, "set_tensor_async_i8 %s: only a module input or the quant op directly behind one can be supplied", name.c_str());
     if (!q->disabled) {
       q->disabled = true;
+      ++quants_disabled;
       invalidate_graph();
     }
   }
@@ -2323,10 +2368,10 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
     grow_async_staging(k, numel);
     staging_used[k] = false;
   }
-  if (staging_used[k]) TPUCB_CUDA(cudaStreamWaitEvent(copy_stream, staging_free[k], 0));
+  if (staging_used[k]) TPUCB_CUDA(cudaStreamWaitEvent(copy_stream, ss.staging_free[k], 0));
   TPUCB_CUDA(cudaMemcpyAsync(async_staging[k], pinned, numel, cudaMemcpyHostToDevice, copy_stream));
-  TPUCB_CUDA(cudaEventRecord(upload_done[k], copy_stream));
-  TPUCB_CUDA(cudaStreamWaitEvent(stream, upload_done[k], 0));
+  TPUCB_CUDA(cudaEventRecord(ss.upload_done[k], copy_stream));
+  TPUCB_CUDA(cudaStreamWaitEvent(stream, ss.upload_done[k], 0));
   TensorGeom g{t->n, t->c, t->h, t->w, t->cp, t->wl, t->wphys};
   const int8_t *stg = (const int8_t *)async_staging[k];
   if (t->cp == 4 && !t->padded_rows())
@@ -2334,7 +2379,7 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
              (size_t)t->h * t->w);
   else
     launch_k(nchw_i8_to_dev_kernel, grid_for(t->pixels() * t->cp, 256, sm_count), 256, 0, stream, stg, (int8_t *)t->dev, g);
-  TPUCB_CUDA(cudaEventRecord(staging_free[k], stream));
+  TPUCB_CUDA(cudaEventRecord(ss.staging_free[k], stream));
   staging_used[k] = true;
 }
 
@@ -2344,14 +2389,18 @@ inline void Interpreter::get_tensor(const std::string &name, float *out, size_t 
   TensorPtr t = tensor(name);
   const SlotView v = slot_view(*t, slot, max_batch, "get_tensor");
   TPUCB_CHECK(numel == v.numel, "get_tensor %s: buffer has %zu values, tensor has %zu", name.c_str(), numel, v.numel);
-  float *stg = ensure_staging(numel * sizeof(float));
+  // A small result is written straight into pinned host memory by the conversion kernel: no copy command behind it.
+  const bool direct = numel * sizeof(float) <= kDownloadBytes;
+  if (direct && !ss.download) TPUCB_CUDA(cudaHostAlloc((void **)&ss.download, kDownloadBytes, cudaHostAllocMapped));
+  float *stg = direct ? ss.download : ensure_staging(numel * sizeof(float));
   int grid = grid_for(numel, 256, sm_count);
   if (t->dtype == DT_I8) launch_k(dev_to_nchw_f32_kernel<DT_I8>, grid, 256, 0, stream, v.dev, stg, v.g);
   else if (t->dtype == DT_BF16) launch_k(dev_to_nchw_f32_kernel<DT_BF16>, grid, 256, 0, stream, v.dev, stg, v.g);
   else launch_k(dev_to_nchw_f32_kernel<DT_F32>, grid, 256, 0, stream, v.dev, stg, v.g);
   TPUCB_CUDA(cudaGetLastError());
-  TPUCB_CUDA(cudaMemcpyAsync(out, stg, numel * sizeof(float), cudaMemcpyDeviceToHost, stream));
+  if (!direct) TPUCB_CUDA(cudaMemcpyAsync(out, stg, numel * sizeof(float), cudaMemcpyDeviceToHost, stream));
   TPUCB_CUDA(cudaStreamSynchronize(stream));
+  if (direct) std::memcpy(out, stg, numel * sizeof(float));
 }
 
 // The op list captured as one CUDA graph, with the launch flag of the moment.
@@ -2416,10 +2465,10 @@ inline void Interpreter::fast_invoke_all_batch(const std::string &name, int batc
 inline void Interpreter::sync_and_check() {
   bind();
   TPUCB_CUDA(cudaStreamSynchronize(stream));
-  int err = 0;
-  TPUCB_CUDA(cudaMemcpy(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  const int err = *(volatile int *)ss.h_err;
   if (err != 0) {
-    TPUCB_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), stream));
+    *ss.h_err = 0;
+    TPUCB_CUDA(cudaMemsetAsync(&ss.d_err->code, 0, sizeof(int), stream));
     for (auto &w : split_ws) TPUCB_CUDA(cudaMemsetAsync(w.first, 0, w.second, stream)); // a failed launch may leave partial sums
     throw Error(strfmt("a convolution kernel gave up on a bounded wait (code %d: 1 = tile load never arrived, "
                        "2 = stage never freed, 3 = accumulator never completed or never handed back); the launch's "

@@ -63,6 +63,7 @@ class module:
             check(self._lib.tpucb_interp_create_batched(int(device), self.max_batch_size, C.byref(self._h)))
         self._weight_file = None
         self.op_info = []
+        self._shapes, self._detail = {}, {}
 
     def __del__(self):
         try:
@@ -119,11 +120,13 @@ class module:
 
     def load_text(self, text, weights):
         self.set_weights(weights)
+        self._shapes, self._detail = {}, {}
         check(self._lib.tpucb_interp_load_module(self._h, text.encode()))
         self._refresh_op_info()
 
     def _refresh_op_info(self):
         self.op_info = []
+        self._shapes, self._detail = {}, {}  # what the library has been asked about this module
         for line in _text(self._lib.tpucb_interp_get_op_info, self._h).splitlines():
             name, typ, dt, shape, ops, nbytes, bound = line.split("\t")
             self.op_info.append({"name": name, "type": typ, "dtype": dt,
@@ -160,10 +163,13 @@ class module:
         check(self._lib.tpucb_interp_wait_uploads(self._h))
 
     def get_tensor_shape(self, name):
-        shape = (C.c_int64 * 8)()
-        rank = C.c_int(0)
-        check(self._lib.tpucb_interp_get_tensor_shape(self._h, name.encode(), shape, C.byref(rank)))
-        return [int(shape[i]) for i in range(rank.value)]
+        known = self._shapes.get(name)
+        if known is None:
+            shape = (C.c_int64 * 8)()
+            rank = C.c_int(0)
+            check(self._lib.tpucb_interp_get_tensor_shape(self._h, name.encode(), shape, C.byref(rank)))
+            known = self._shapes[name] = [int(shape[i]) for i in range(rank.value)]
+        return list(known)
 
     def get_tensor(self, name, bidx=None):
         shape = self.get_tensor_shape(name)
@@ -192,12 +198,15 @@ class module:
         return {n: self.get_tensor(n, bidx) for n in self.get_all_tensor_names()}
 
     def _details(self, outputs, sizes=False):
-        out = []
-        for line in _text(self._lib.tpucb_interp_get_details, self._h, int(outputs)).splitlines():
-            if line:
-                n, sz = line.rsplit(":", 1)
-                out.append((n, int(sz)) if sizes else n)
-        return out
+        known = self._detail.get(outputs)
+        if known is None:
+            known = []
+            for line in _text(self._lib.tpucb_interp_get_details, self._h, int(outputs)).splitlines():
+                if line:
+                    n, sz = line.rsplit(":", 1)
+                    known.append((n, int(sz)))
+            self._detail[outputs] = known
+        return list(known) if sizes else [n for n, _ in known]
 
     def input_sizes(self):
         """input_details of the reference: (name, element count of one batch slot) in module order."""
