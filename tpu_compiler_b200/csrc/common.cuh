@@ -179,6 +179,59 @@ __device__ __forceinline__ uint32_t pack_sat_s8(int a, int b, uint32_t c) {
 __device__ __forceinline__ uint32_t pack4_sat(int q0, int q1, int q2, int q3) {
   return pack_sat_s8(q1, q0, pack_sat_s8(q3, q2, 0u));
 }
+// the same with unsigned saturation to [0, 255]
+__device__ __forceinline__ uint32_t pack_sat_u8(int a, int b, uint32_t c) {
+  uint32_t d;
+  asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// max(byte, 0) of four packed int8 values: the sign of every byte spread over it by one permute, then one logic operation
+__device__ __forceinline__ uint32_t relu_bytes(uint32_t w) {
+  uint32_t s;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(s) : "r"(w), "r"(0u), "r"(0xBA98u));
+  return w & ~s;
+}
+
+// ---- The requantisation on the floating-point pipes --------------------------------------------------------------------
+// Exact, with three (ReLU) or four full-rate instructions per value. The integer forms (requant_fast in conv_gemm_i8.cuh)
+// need a multiply-high at a quarter of that rate and shifts and multiply-adds at half of it, and their instruction pipes
+// bound every convolution with a short K. With s = acc + bias, the reference's
+//   hi = floor((s M + 2^30) / 2^31),  q = round half away from zero(hi / 2^r)
+// is computed as follows (m = M / 2^31; every quantity scaled by 2^-100, see below).
+//   f = the float with the bits of acc + sb: A + s, exact, because one unit of the bit pattern is 1 around A
+//   u = fma.rm(f, m, d), d = C + 1/2 - A m: rounds C + s m + 1/2 down to an integer, once: C + hi
+// ReLU (A = 2^23; negative s give some f below A and a result <= 0, which the caller clamps): C = 2^23 + 2^(r-1), and
+//   v = fma.rm(u, c, e), c = 2^-r, e = -2^23 c: floor((hi + 2^(r-1)) / 2^r)
+// else (A = 1.5 2^23, C = kFqC): h = u - C exactly, and
+//   v = fma.rn(h, c, 128), c = 2^-r (1 + 2^-23): the factor moves exact ties away from zero and nothing else across one
+// The products are scaled so that v's unit is 2^-149, the smallest subnormal: the bits of v ARE the integer (the sign bit
+// makes negative ones very negative integers, which saturate), and the packing instruction takes them as they are.
+// float_requant (host) checks per channel, from the sum of |weights|, that s and hi stay in range and that d is a float;
+// a layer that fails keeps the integer forms.
+struct FloatRequant {
+  uint32_t sb; // bias + bits of A
+  float m, d, c;
+};
+constexpr float kFqScale = 7.888609052210118e-31f; // 2^-100
+constexpr double kFqC = 8388608.0 + 2097152.0 - 8.0;
+
+#ifdef __CUDACC__
+// four values of one channel, packed
+template <bool RELU>
+__device__ __forceinline__ uint32_t float_requant4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const FloatRequant &q) {
+  const float e = q.c * -6.617444900424222e-24f; // -2^-77: the unit 2^-149 against c's 2^-49
+  auto one = [&](uint32_t a) {
+    float u, v;
+    asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(u) : "f"(__uint_as_float(a + q.sb)), "f"(q.m), "f"(q.d));
+    if (RELU) asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(u), "f"(q.c), "f"(e));
+    else asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(__fsub_rn(u, (float)kFqC * kFqScale)), "f"(q.c), "f"(__uint_as_float(128u)));
+    return __float_as_int(v);
+  };
+  if (RELU) return relu_bytes(pack_sat_s8(one(a1), one(a0), pack_sat_s8(one(a3), one(a2), 0u)));
+  return pack_sat_u8(one(a1), one(a0), pack_sat_u8(one(a3), one(a2), 0u)) ^ 0x80808080u;
+}
+#endif
+
 // sign-extended byte J of a word in one byte-permute: in prmt's default mode bit 3 of a selector
 // nibble replicates the sign of the selected byte (the __byte_perm intrinsic masks that bit off,
 // hence the inline PTX).

@@ -56,6 +56,7 @@ struct ConvGemmParams {
   const int32_t *bias;   // [n_valid]
   const int32_t *mult;   // [n_valid]
   const int32_t *rshift; // [n_valid]
+  const FloatRequant *fq; // [n_valid], or null: the floating-point form of the requantisation does not apply
   int8_t *out;
   int fastq;      // bit 0: the multiply-high form of the requantisation applies (requant_fast; set by the host);
                   // bit 1: every rshift of the layer is >= 1
@@ -438,10 +439,8 @@ __device__ __forceinline__ uint32_t add4_packed(uint32_t x, uint32_t y, uint32_t
   const int s2 = __dp4a((int)byte_pair<2>(x, y), (int)mm, rnd) >> r;
   const int s3 = __dp4a((int)byte_pair<3>(x, y), (int)mm, rnd) >> r;
   const uint32_t w = pack4_sat(s0, s1, s2, s3);
-  return relu ? __vmaxs4(w, 0u) : w;
+  return relu ? relu_bytes(w) : w;
 }
-// ReLU of four packed int8 values
-__device__ __forceinline__ uint32_t relu4(uint32_t w) { return __vmaxs4(w, 0u); }
 // INT8 leaky ReLU of a saturated convolution result (core/activation.cpp:126-153).
 __device__ __forceinline__ int leaky_of(int v, const ConvGemmParams &p) {
   if (v > 0) return p.leaky_mp != 0 ? mul_rshift_sat8(v, p.leaky_mp, p.leaky_rp) : v;
@@ -472,13 +471,26 @@ __device__ __forceinline__ uint32_t transpose4x4(uint32_t w, const TransposeSel 
 //   out4       output address of (pixel m0, this lane's 4-channel group)
 //   ch4_ok     the 4-channel group lies inside the valid channels
 //   ncols      pixel columns of the accumulator buffer (128; 256 for the two-SM tile)
-template <int ACT, bool FAST, bool R1 = false, bool FROM_WS = false>
+//   FORM       of the requantisation: 0 requant_one, 1 requant_fast, 2 requant_fast with every rshift >= 1, 3 float_requant4
+template <int ACT, int FORM, bool FROM_WS = false, class Consts = ChanConst>
 __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4,
                                                        bool ch4_ok, int m0, int half, int halves, int lane,
-                                                       const ChanConst &cc, const TransposeSel &ts, int ncols,
+                                                       const Consts &cc, const TransposeSel &ts, int ncols,
                                                        int32_t *ws_lane = nullptr) {
   constexpr int QACT = ACT == 3 ? 0 : ACT; // the fused add works on the plain (no activation) int8 result
-  auto rq = [&](uint32_t a) { return FAST ? requant_fast<QACT, R1>((int32_t)a, cc, p) : requant_one<QACT>((int32_t)a, cc, p); };
+  // four pixels of this lane's channel, packed
+  auto rq4 = [&](uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) -> uint32_t {
+    if constexpr (FORM == 3) {
+      return float_requant4<QACT == 1>(a0, a1, a2, a3, cc);
+    } else {
+      auto rq = [&](uint32_t a) {
+        if constexpr (FORM == 0) return requant_one<QACT>((int32_t)a, cc, p);
+        else return requant_fast<QACT, FORM == 2>((int32_t)a, cc, p);
+      };
+      const uint32_t w = pack4_sat(rq(a0), rq(a1), rq(a2), rq(a3));
+      return FORM != 0 && ACT == 1 ? relu_bytes(w) : w; // the multiply-high form leaves the ReLU clamp to the packed bytes
+    }
+  };
   const int pj = lane & 3;
   // (Software-pipelining these loads in 16-column pieces made the epilogue alone 14% faster and the whole
   // kernel 4% slower, so the two loads of a chunk are simply issued together.)
@@ -518,12 +530,8 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
     uint32_t w[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      w[k] = pack4_sat(rq(acc0[4 * k + 0]), rq(acc0[4 * k + 1]), rq(acc0[4 * k + 2]), rq(acc0[4 * k + 3]));
-      w[4 + k] = pack4_sat(rq(acc1[4 * k + 0]), rq(acc1[4 * k + 1]), rq(acc1[4 * k + 2]), rq(acc1[4 * k + 3]));
-      if (FAST && ACT == 1) { // the multiply-high form leaves the ReLU clamp to the packed bytes
-        w[k] = relu4(w[k]);
-        w[4 + k] = relu4(w[4 + k]);
-      }
+      w[k] = rq4(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3]);
+      w[4 + k] = rq4(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3]);
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) w[k] = transpose4x4(w[k], ts);
@@ -569,15 +577,6 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
         if (ch4_ok && m0 + colg + 4 * k + pj < p.M_total) *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
     }
   }
-}
-
-template <int ACT>
-__device__ __forceinline__ void epilogue_channels(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4,
-                                                  bool ch4_ok, int m0, int half, int halves, int lane,
-                                                  const ChanConst &cc, const TransposeSel &ts, int ncols = 128) {
-  if ((p.fastq & 3) == 3) epilogue_channels_impl<ACT, true, true>(p, lane_addr, out4, ch4_ok, m0, half, halves, lane, cc, ts, ncols);
-  else if (p.fastq & 1) epilogue_channels_impl<ACT, true, false>(p, lane_addr, out4, ch4_ok, m0, half, halves, lane, cc, ts, ncols);
-  else epilogue_channels_impl<ACT, false>(p, lane_addr, out4, ch4_ok, m0, half, halves, lane, cc, ts, ncols);
 }
 
 // Epilogue of a BF16 convolution (core/conv.cpp:90-98: fp32 result + fp32 bias, ReLU, BF16 rounding). The
@@ -658,6 +657,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
                                                const CUtensorMap &tmA2, const CUtensorMap &tmB2) {
   constexpr int KIND = TF32 ? 2 : (BF16 ? 1 : 0);
   constexpr int kTerms = TF32 ? 3 : 1;
+  constexpr bool FQ = ACTSEL >= 100; // one epilogue, the floating-point requantisation: ACTSEL - 100 is the activation
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -961,6 +961,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     const int half = (warp - 2) >> 2; // which alternate 32-pixel column groups it takes
     const TransposeSel ts = make_transpose_sel(lane);
     ChanConst cc = {};
+    FloatRequant fq = {};
     float bias_f = 0.0f;
     int staged_n0 = -1;
     int t = 0;
@@ -988,6 +989,10 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         if (BF16 || TF32) {
           const int ch = n0 + ch_base + lane;
           bias_f = ch < p.n_valid ? __int_as_float(p.bias[ch]) : 0.0f; // fp32 bias bits in the int32 array
+        } else if (FQ) {
+          const int ch = n0 + ch_base + lane;
+          const uint4 c = ch < p.n_valid ? __ldg(reinterpret_cast<const uint4 *>(p.fq) + ch) : make_uint4(0u, 0u, 0u, 0u);
+          fq = FloatRequant{c.x, __uint_as_float(c.y), __uint_as_float(c.z), __uint_as_float(c.w)};
         } else {
           cc = load_chan_const(p, n0 + ch_base + lane);
         }
@@ -1070,16 +1075,13 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + (size_t)m0 * p.ldc + (size_t)(p.c_off + (ch & ~1)) * 2;
           if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
           else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
-        } else if (ACTSEL == 1) { // kernels specialised for one epilogue (ACTSEL: 1 = ReLU, 10 = none with every rshift >= 1)
-          epilogue_channels_impl<1, FAST, false, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        } else if (ACTSEL == 10) {
-          epilogue_channels_impl<0, FAST, true, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        } else if (p.act == 1) epilogue_channels_impl<1, FAST, false, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else if (p.act == 2) epilogue_channels_impl<2, FAST, false, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else if (p.act == 3 && FAST && (p.fastq & 2)) epilogue_channels_impl<3, FAST, true>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128);
-        else if (p.act == 3) epilogue_channels_impl<3, FAST>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128);
-        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST, true, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else epilogue_channels_impl<0, FAST, false, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
+        } else if constexpr (FQ) {
+          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, fq, ts, 128);
+        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
+        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
+        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128);
+        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
+        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
       }
       if (SPLIT && ws_lane) continue; // split K: the accumulator buffer was handed back above
       // hand the accumulator buffer back to the MMA issuer
@@ -1104,13 +1106,13 @@ conv_gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     const ConvGemmParams p) {
   conv_gemm_body<false, true>(tmA, tmB, p, tmA, tmB);
 }
-// The two epilogues that carry most launches as kernels of their own (ReLU; no activation with every rshift >= 1):
-// the compiler allocates registers and schedules for that one epilogue instead of for all of them.
-template <int ACTSEL>
+// The floating-point requantisation (p.fq set), one kernel per activation (ConvGemmParams::act): the compiler allocates
+// registers and schedules for that one epilogue.
+template <int ACT>
 __global__ void __launch_bounds__(kConvThreads, 2)
-conv_gemm_i8_act_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                        const ConvGemmParams p) {
-  conv_gemm_body<false, true, false, false, ACTSEL>(tmA, tmB, p, tmA, tmB);
+conv_gemm_i8_fq_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                       const ConvGemmParams p) {
+  conv_gemm_body<false, true, false, false, 100 + ACT>(tmA, tmB, p, tmA, tmB);
 }
 // The split-K form of both (ConvGemmParams::split_k > 1): a kernel of its own, so that the ordinary ones carry none of
 // its code (with the switch at run time the epilogue-bound layers were 14% slower).

@@ -481,8 +481,10 @@ inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_cou
   } else if (pl.bf16) launch_k(conv_gemm_bf16_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1 && (pl.p.fastq & 1)) launch_k(conv_gemm_i8_split_kernel<true>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1) launch_k(conv_gemm_i8_split_kernel<false>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if ((pl.p.fastq & 1) && pl.p.act == 1) launch_k(conv_gemm_i8_act_kernel<1>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if ((pl.p.fastq & 3) == 3 && pl.p.act == 0) launch_k(conv_gemm_i8_act_kernel<10>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  else if (pl.p.fq && pl.p.act == 1) launch_k(conv_gemm_i8_fq_kernel<1>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  else if (pl.p.fq && pl.p.act == 0) launch_k(conv_gemm_i8_fq_kernel<0>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  else if (pl.p.fq && pl.p.act == 2) launch_k(conv_gemm_i8_fq_kernel<2>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  else if (pl.p.fq) launch_k(conv_gemm_i8_fq_kernel<3>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (!(pl.p.fastq & 1)) launch_k(conv_gemm_i8_wide_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else launch_k(conv_gemm_i8_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
 }
@@ -491,8 +493,10 @@ inline void conv_kernel_setup_once() {
   static bool done = [] {
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_act_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_act_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_split_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,

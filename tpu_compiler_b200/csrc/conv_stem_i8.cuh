@@ -207,10 +207,10 @@ conv_stem_i8_kernel(const __grid_constant__ CUtensorMap tmB, const ConvStemParam
         const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
         int8_t *out4 = p.out + (size_t)m0e * p.ldc + p.c_off + ch4;
         const bool ch4_ok = ch4 < p.n_valid;
-        if (RELU_ONLY || p.act == 1) epilogue_channels_impl<1, FAST>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
-        else if (p.act == 2) epilogue_channels_impl<2, FAST>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
-        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST, true>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
-        else epilogue_channels_impl<0, FAST>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
+        if (RELU_ONLY || p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
+        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
+        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
+        else epilogue_channels_impl<0, FAST ? 1 : 0>(ep, lane_addr, out4, ch4_ok, m0e, half, 2, lane, cc, ts, 128);
       }
     }
   }

@@ -318,6 +318,39 @@ inline int requant_fast_flags(const std::vector<float> &rshift, const std::vecto
   return f;
 }
 
+// Constants of the floating-point requantisation (FloatRequant) for the channels of a layer, padded to `pad_to`; empty when
+// a channel's sums may leave its range. filt: [oc][per_channel] integer-valued weights; |activation| <= 128.
+inline std::vector<FloatRequant> float_requant(const std::vector<float> &filt, const std::vector<float> &bias,
+                                               const std::vector<float> &mult, const std::vector<float> &rshift, bool relu,
+                                               int pad_to) {
+  const size_t oc = bias.size(), per = filt.size() / oc;
+  std::vector<FloatRequant> out(std::max<size_t>(oc, pad_to), FloatRequant{0u, 0.0f, 0.0f, 0.0f});
+  const double scale = kFqScale;
+  for (size_t o = 0; o < oc; ++o) {
+    double bound = std::fabs((double)bias[o]);
+    for (size_t i = 0; i < per; ++i) bound += 128.0 * std::fabs((double)filt[o * per + i]);
+    const double m = std::ldexp((double)mult[o], -31), r = rshift[o], rnd = r > 0 ? std::ldexp(1.0, (int)r - 1) : 0.0;
+    double d, c = std::ldexp(1.0, -49 - (int)r);
+    bool ok = r >= 0;
+    FloatRequant &q = out[o];
+    if (relu) {
+      ok = ok && r <= 22 && bound < 8388608.0 && bound * m + rnd + 1.0 <= 8388608.0;
+      q.sb = 0x4B000000u + (uint32_t)(int32_t)bias[o];
+      d = 8388608.0 + rnd + 0.5 - 8388608.0 * m;
+    } else {
+      ok = ok && r <= 31 && bound < 4194304.0 && bound * m < 2097152.0 - 16.0;
+      q.sb = 0x4B400000u + (uint32_t)(int32_t)bias[o];
+      d = kFqC + 0.5 - 12582912.0 * m;
+      c *= 1.0 + std::ldexp(1.0, -23);
+    }
+    q.m = (float)(m * scale);
+    q.d = (float)(d * scale);
+    q.c = (float)c;
+    if (!ok || (double)q.m != m * scale || (double)q.d != d * scale) return {};
+  }
+  return out;
+}
+
 // ---------------------------------------------------------------------------- Input
 // InputOpKernel (core/input.cpp:7-24): holds the tensor set_tensor writes; no device work.
 class InputOp : public OpKernel {
@@ -628,6 +661,9 @@ public:
     act_ = do_relu_ ? 1 : 0;
     const int fastq = requant_fast_flags(I.weight(op.in[5]).data, bias, (long long)(g.ic / g.g) * g.kh * g.kw);
 
+    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, I.weight(op.in[6]).data, I.weight(op.in[5]).data, do_relu_ != 0, oc_pad);
+    const FloatRequant *d_fq = fq.empty() ? nullptr : I.upload(fq);
+
     if (g.g == g.ic && g.g == g.oc && g.g > 1 && g.ins_h == 0 && g.ins_w == 0) {
       // depthwise
       dw_ = true;
@@ -707,6 +743,7 @@ public:
       p.act = act_;
       p.fastq = fastq;
       p.bias = d_bias_ + grp * ocg; p.mult = d_mult_ + grp * ocg; p.rshift = d_rsh_ + grp * ocg;
+      p.fq = d_fq ? d_fq + grp * ocg : nullptr;
       p.out = (int8_t *)out->dev;
       p.ldc = out->cp;
       p.c_off = grp * ocg;
@@ -992,6 +1029,8 @@ public:
     // multiplier the two orders give the same int8 result.
     p.act = do_relu_ ? 1 : 0;
     p.fastq = requant_fast_flags(rs, bias, k_);
+    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, mu, rs, do_relu_ != 0, n_pad);
+    if (!fq.empty()) p.fq = I.upload(fq);
     p.a_mode = 0;
     finish_plan(pl, m_, 1, kdev_, n_pad, I.sm_count);
     encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_, kdev_, p.BK, a_tile_rows(p));
