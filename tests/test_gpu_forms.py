@@ -1,0 +1,79 @@
+"""GPU parity of the forms that launch plans choose by size, type and value range, at the edges of their ranges."""
+import numpy as np
+import pytest
+
+from oracle import graph_runner
+from tpu_compiler_b200 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def run_model(text, weights, inputs, names):
+    from tpu_compiler_b200 import module
+    m = module(0)
+    m.load_text(text, weights)
+    for k, v in inputs.items():
+        m.set_tensor(k, v)
+    m.invoke()
+    ref = graph_runner.run(text, weights, inputs)
+    out = {n: (m.get_tensor(n), ref[n]) for n in names}
+    m.close()
+    return out
+
+
+def conv_text(dtype, n, ic, oc, hw, k, s, p, d, relu, int8=False, extra=""):
+    o = (hw + 2 * p - d * (k - 1) - 1) // s + 1
+    return ("conv_2d name=c in=x,f,b%s shape=%d,%d,%d,%d dtype=%s kh=%d kw=%d sh=%d sw=%d pt=%d pb=%d pl=%d pr=%d dh=%d dw=%d g=1 "
+            "do_relu=%d with_bias=1%s\n" % (",-,-,r,m" if int8 else "", n, oc, o, o, dtype, k, k, s, s, p, p, p, p, d, d, relu, extra))
+
+
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("mults", ["random", "power_of_two", "small"])
+def test_float_requantisation_edges(relu, mults):
+    """Every shift of the floating-point form's range, multipliers that make exact ties in the first rounding (powers of
+    two) or few significant bits, zero multipliers; sums close to both ends of the range."""
+    rng = np.random.default_rng(5 + relu)
+    ic, oc, hw = 32, 96, 12
+    f = rng.integers(-20, 21, (oc, ic, 1, 1)).astype(np.float32)
+    r = (np.arange(oc) % (23 if relu else 32)).astype(np.float32)
+    m = {"random": (rng.integers(2 ** 23, 2 ** 24, oc) * 128).astype(np.float32),
+         "power_of_two": np.float32(2.0) ** rng.integers(7, 31, oc).astype(np.float32),
+         "small": (rng.integers(0, 64, oc) * 2 ** 20).astype(np.float32)}[mults]
+    m[::17] = 0
+    b = rng.integers(-2 ** 18, 2 ** 18, oc).astype(np.float32)
+    b[:23] = rng.integers(-3, 4, 23)  # small sums around zero at every shift
+    text = "input name=x shape=2,%d,%d,%d dtype=INT8\n" % (ic, hw, hw) + conv_text("INT8", 2, ic, oc, hw, 1, 1, 0, 1, int(relu), True)
+    x = rng.integers(-128, 128, (2, ic, hw, hw)).astype(np.float32)
+    got, ref = run_model(text, {"f": f, "b": b, "r": r, "m": m}, {"x": x}, ["c"])["c"]
+    assert np.array_equal(got, ref)
+
+
+WINDOWS = [  # n, ic, oc, hw, k, stride, pad, dilation: pixel groups of 4, 2 and 1, tile remainders, 16-byte pixels
+    (2, 3, 32, 36, 3, 1, 1, 1), (1, 3, 24, 34, 3, 2, 1, 1), (3, 3, 64, 30, 7, 2, 3, 1), (1, 3, 64, 31, 5, 2, 2, 1),
+    (2, 4, 100, 18, 3, 1, 1, 2), (1, 1, 16, 9, 3, 1, 1, 1), (2, 2, 40, 26, 4, 2, 1, 1), (1, 3, 16, 17, 3, 4, 0, 1)]
+
+
+@pytest.mark.parametrize("case", WINDOWS + [(2, 12, 48, 20, 3, 1, 1, 1), (1, 7, 64, 24, 5, 2, 2, 1)])
+@pytest.mark.parametrize("shared", [False, True])  # True: another consumer of the input keeps it from the window layout
+def test_row_window_conv_i8(case, shared):
+    n, ic, oc, hw, k, s, p, d = case
+    model = graphs.single_conv_i8(n, ic, oc, hw, k, s, p, d, seed=3100 + ic + k)
+    text = model.text + ("relu name=other in=x shape=%d,%d,%d,%d dtype=INT8\n" % (n, ic, hw, hw) if shared else "")
+    for name, (got, ref) in run_model(text, model.weights, {"x": model.meta["x"]}, ["conv"] + ["other"] * shared + ["x"]).items():
+        assert np.array_equal(got, ref), name
+
+
+@pytest.mark.parametrize("dtype", ["BF16", "FP32"])
+@pytest.mark.parametrize("case", WINDOWS)
+def test_row_window_conv_float(dtype, case):
+    n, ic, oc, hw, k, s, p, d = case
+    rng = np.random.default_rng(41 + ic + k)
+    cut = graphs._bf16_np if dtype == "BF16" else (lambda v: np.asarray(v, np.float32))
+    w = {"f": cut(rng.normal(0, 0.2, (oc, ic, k, k))), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+    x = cut(rng.normal(0, 1, (n, ic, hw, hw)))
+    text = "input name=x shape=%d,%d,%d,%d dtype=%s\n" % (n, ic, hw, hw, dtype) + conv_text(dtype, n, ic, oc, hw, k, s, p, d, 1)
+    got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
+    if dtype == "BF16":
+        assert np.all(np.abs(got - ref) <= np.maximum(np.abs(ref) * 2.0 ** -7, 2.0 ** -8 * np.abs(ref).max() * 2.0 ** -6))
+    else:
+        assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()

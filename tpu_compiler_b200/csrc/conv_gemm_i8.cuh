@@ -46,8 +46,11 @@ struct ConvGemmParams {
   int stages;     // pipeline depth
   int dual;       // 1: at most 64 channels: two 128-pixel sub-tiles share the 128 TMEM lanes (see kernel)
   int w_resident; // 1: the CTA keeps all K blocks of its channel tile's weights in shared memory
-  int a_mode;     // 0: A is a 2-D [M][K] matrix, 1: im2col TMA, 2: row windows (stem)
-  int win_g;      // mode 2: output pixels per copy
+  int a_mode;     // 0: A is a 2-D [M][K] matrix, 1: im2col TMA
+  int ksteps;     // MMAs (32 bytes of K) per K block: BK / 32, fewer when the block's tail is padding
+  // Pixel groups (WindowPlan): > 1 means that a row of the implicit GEMM is `group` neighbouring output pixels, whose
+  // channels are 128 / group apart on the TMEM lanes; M_total, OW and ldc then count groups, ldc_px is one pixel's pitch.
+  int group, ldc_px;
   int act;        // 0 none, 1 ReLU, 2 leaky (non-QDM pos/neg rescale of the int8 result),
                   // 3 the eltwise add that consumes this convolution, with the residual tensor `res` (see add_*)
   int tmem_cols;  // 256: two accumulator buffers of 128 pixel columns
@@ -783,16 +786,6 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           w_base = q * p.sw - p.pl;
           h_base = pp * p.sh - p.pt;
         }
-        // mode 2: the (column, row, image) of the first pixel of each copy, computed once per tile
-        int bx_q[16], bx_h[16], bx_n[16];
-        const int n_boxes = p.a_mode == 2 ? 128 / p.win_g : 0;
-        for (int i = 0; i < n_boxes; ++i) {
-          const int m = m0 + i * p.win_g;
-          const int t = m / p.OW;
-          bx_q[i] = m - t * p.OW;
-          bx_n[i] = t / p.OH;
-          bx_h[i] = (t - bx_n[i] * p.OH) * p.sh - p.pt;
-        }
         // running (tap row, tap column, channel chunk) and ring (stage, phase) counters: this loop
         // is a single thread's instruction stream, so it carries no divisions
         int tap = 0, tr = 0, ts = 0, chunk = 0, term = 0;
@@ -823,11 +816,6 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
             // its issuing thread about 430 cycles whatever its size)
             ptx::tma_load_im2col_4d(a_dst, mapA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
                                     (uint16_t)(tr * p.dh));
-          } else if (p.a_mode == 2) {
-            // `tap` is the filter row; each copy brings win_g consecutive output pixels' windows.
-            for (int i = 0; i < n_boxes; ++i)
-              ptx::tma_load_4d(a_dst + (uint32_t)(i * p.win_g * p.BK), &tmA, fb, 0, bx_q[i],
-                               bx_h[i] + tap * p.dh, bx_n[i]);
           } else {
             ptx::tma_load_2d(a_dst, mapA, fb, c0, m0);
           }
@@ -886,7 +874,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const uint32_t stage_step = stage_bytes >> 4, a_step = a_bytes >> 4, w_step = b_bytes >> 4;
       const uint32_t sub_step = (128u * (uint32_t)p.BK) >> 4, dual_step = (64u * (uint32_t)p.BK) >> 4;
       uint32_t m_full = bar_full, m_empty = bar_empty, ring_lo = desc_ring_lo;
-      const int ksteps = p.BK / 32;
+      const int ksteps = p.ksteps;
       if (p.w_resident && (int)blockIdx.x < total_tiles) {
         if (!ptx::mbar_wait_bounded(bar_w, 0u, abort_flag, wait_rounds)) {
           if (!*abort_flag) report_error(p.err, kErrFullWait);
@@ -926,6 +914,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           const uint32_t acc_first = kit > k_begin ? 1u : 0u;
           if (!p.dual) {
             if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+            else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
             else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
             else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
           } else {
@@ -975,7 +964,8 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         tn = tile - tm * n_tiles;
       }
       // dual mode: lanes 0..63 are the channels of the first 128 pixels, lanes 64..127 of the second
-      const int ch_base = p.dual ? (quarter & 1) * 32 : quarter * 32;
+      // pixel groups: lane / (128 / group) is the pixel of the group
+      const int ch_base = p.dual ? (quarter & 1) * 32 : (p.group > 1 ? (quarter * 32) & (128 / p.group - 1) : quarter * 32);
       const int m0 = tm * m_tile + (p.dual ? 128 * (quarter >> 1) : 0);
       const int n0 = tn * p.BN;
       tm += walk_dm;
@@ -1061,18 +1051,19 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       }
       if (n0 + ch_base < p.n_valid && m0 < p.M_total) { // warp-uniform: this lane quarter holds real outputs
         const uint32_t lane_addr = tmem_base + (uint32_t)buf * acc_stride + ((uint32_t)(quarter * 32) << 16);
-        int8_t *out4 = p.out + (size_t)m0 * p.ldc + p.c_off + ch4;
+        const size_t out_m0 = (size_t)m0 * p.ldc + (p.group > 1 ? (quarter * 32 * p.group >> 7) * p.ldc_px : 0); // bytes
+        int8_t *out4 = p.out + out_m0 + p.c_off + ch4;
         const bool ch4_ok = ch4 < p.n_valid;
         if (TF32) {
           // byte addressing: 4 bytes per channel
           const int ch = n0 + ch_base + lane;
-          uint8_t *out_ch = reinterpret_cast<uint8_t *>(p.out) + (size_t)m0 * p.ldc + (size_t)(p.c_off + ch) * 4;
+          uint8_t *out_ch = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch) * 4;
           if (p.act == 1) epilogue_channels_f32<true>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
           else epilogue_channels_f32<false>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
         } else if (BF16) {
           // byte addressing: 2 bytes per channel, this lane's pair starts at its even channel
           const int ch = n0 + ch_base + lane;
-          uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + (size_t)m0 * p.ldc + (size_t)(p.c_off + (ch & ~1)) * 2;
+          uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + (ch & ~1)) * 2;
           if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
           else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
         } else if constexpr (FQ) {

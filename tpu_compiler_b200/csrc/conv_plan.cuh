@@ -4,10 +4,10 @@
 // output size taken from the result type, dilation, optional input zero-insertion.
 #pragma once
 #include "conv_gemm_i8.cuh"
-#include "conv_stem_i8.cuh"
 #include "host_common.h"
 #include "mem_kernels.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <cudaTypedefs.h>
@@ -89,10 +89,11 @@ struct ConvPlan {
   float *split_hi = nullptr, *split_lo = nullptr;
   size_t split_nvec = 0;
   bool use_patch = false;
-  int patch_elsize = 1; // bytes per element of the patch matrix: 1 INT8, 2 BF16, 4 fp32
   PatchArgs patch;
   int8_t *patch_buf = nullptr; // scratch: expanded patch matrix [M][kp]
   size_t patch_bytes = 0;
+  bool use_repack = false; // row windows: the input's rows are copied into the window layout first
+  RepackArgs repack;
   const int8_t *in = nullptr;
   double ops = 0, bytes = 0; // algorithmic work of one launch
 };
@@ -166,31 +167,6 @@ inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int ic
   return bytes;
 }
 
-// Weights of the patch-matrix form [oc_pad][kp], k = (r * kw + s) * icg + c, as 2-byte BF16 (part < 0) or as fp32
-// parts of a TF32 x 3 product (part 0: upper 19 bits, part 1: remainder).
-inline std::vector<int8_t> pack_patch_weights(const float *w, int oc, int icg, int kh, int kw, int oc_pad, int kp, int part,
-                                              int cstride = 0) {
-  if (cstride == 0) cstride = icg; // channel slots per tap (4 in patch_expand_tap_kernel's layout)
-  const size_t n = (size_t)oc_pad * kp;
-  std::vector<uint16_t> h(part < 0 ? n : 0, 0);
-  std::vector<float> f(part < 0 ? 0 : n, 0.0f);
-  for (int o = 0; o < oc; ++o)
-    for (int c = 0; c < icg; ++c)
-      for (int r = 0; r < kh; ++r)
-        for (int s = 0; s < kw; ++s) {
-          const float v = w[(((size_t)o * icg + c) * kh + r) * kw + s];
-          const size_t k = (size_t)o * kp + (size_t)(r * kw + s) * cstride + c;
-          if (part < 0) h[k] = (uint16_t)(f32_bits(v) >> 16);
-          else {
-            const float hi = bits_f32(f32_bits(v) & 0xffffe000u);
-            f[k] = part == 0 ? hi : v - hi;
-          }
-        }
-  std::vector<int8_t> bytes(part < 0 ? n * 2 : n * 4);
-  std::memcpy(bytes.data(), part < 0 ? (const void *)h.data() : (const void *)f.data(), bytes.size());
-  return bytes;
-}
-
 inline void encode_weight_map(CUtensorMap *tm, const int8_t *d_w, int oc_pad, int taps, int k_inner,
                               int BK, int BN) {
   cuuint64_t dims[3] = {(cuuint64_t)k_inner, (cuuint64_t)taps, (cuuint64_t)oc_pad};
@@ -218,6 +194,12 @@ inline void encode_matrix_map(CUtensorMap *tm, const int8_t *d_a, int rows, int 
   TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(matrix) failed: %d", (int)r);
 }
 
+// Drivers up to CUDA 13.1 encode im2col maps of tensors smaller than 128 KiB with a flag (bit 21 of the second 64-bit word)
+// that makes the load misbehave; the same correction is applied by NVIDIA's open-source CUTLASS when it builds these maps.
+inline void fix_small_im2col_map(CUtensorMap *tm, size_t tensor_bytes) {
+  if (tma_api().driver_version <= 13010 && tensor_bytes < 131072) reinterpret_cast<uint64_t *>(tm)[1] &= ~(1ull << 21);
+}
+
 inline void encode_im2col_map(CUtensorMap *tm, const int8_t *d_in, const ConvGeom &g, int cp,
                               int BK, int tile_rows) {
   cuuint64_t dims[4] = {(cuuint64_t)cp, (cuuint64_t)g.iw, (cuuint64_t)g.ih, (cuuint64_t)g.n};
@@ -241,125 +223,79 @@ inline void encode_im2col_map(CUtensorMap *tm, const int8_t *d_in, const ConvGeo
   TPUCB_CHECK(r == CUDA_SUCCESS,
               "cuTensorMapEncodeIm2col failed: %d (iw=%d ih=%d lower=%d,%d upper=%d,%d)", (int)r,
               g.iw, g.ih, lower[0], lower[1], upper[0], upper[1]);
-  // Drivers up to CUDA 13.1 encode im2col maps of tensors smaller than 128 KiB with a flag
-  // (bit 21 of the second 64-bit word) that makes the load misbehave; the same correction
-  // is applied by NVIDIA's open-source CUTLASS when it builds these maps.
-  size_t tensor_bytes = (size_t)cp * g.iw * g.ih * g.n;
-  if (tma_api().driver_version <= 13010 && tensor_bytes < 131072)
-    reinterpret_cast<uint64_t *>(tm)[1] &= ~(1ull << 21);
+  fix_small_im2col_map(tm, (size_t)cp * g.iw * g.ih * g.n);
 }
 
-// Few-channel ("stem") convolutions: with the input stored as zero-padded NHWC rows whose pixel
-// pitch is cp = 16 / stride_w bytes, the kw taps of one filter row of one output pixel are a
-// contiguous window that starts on a 16-byte boundary, and neighbouring output pixels' windows
-// start 16 bytes apart. A 4-D tiled tensor map with OVERLAPPING strides
-//   (window byte, output column q [16 B], input row [row pitch], image)
-// then delivers g consecutive output pixels' windows per copy; K has one step per filter row.
-struct StemLayout {
-  int cp = 0;     // channel pitch of the input tensor (bytes per pixel)
-  int wl = 0;     // zero pixels on the left of each row
-  int wphys = 0;  // physical row width in pixels
-  int bk = 0;     // window bytes, rounded up to a swizzle span (32/64/128)
-  int g = 0;      // output pixels per copy: gcd(OW, 128), at least 8
+// Few-channel convolutions (image stems) as row windows. The input is stored as zero-padded NHWC rows with a pixel pitch of
+// P = 4, 8 or 16 bytes, so that the taps of one filter row of one output pixel are one contiguous window. G neighbouring
+// output pixels form one row of the implicit GEMM: their windows overlap, so ONE window of (G - 1) strides more serves
+// all of them, against G copies of the filter shifted by one output stride each, which fill the 128 rows of the tensor
+// core's weight operand (64 output channels: G = 2, 32: G = 4) instead of zeros. G also makes the windows start on the 16-byte
+// boundaries that a tensor map needs. An im2col-mode tensor map whose "width" is the pixel group (stride G * sw * P, window
+// bytes as the "channels", overlapping) then brings the windows of a whole tile in one copy per filter row.
+struct WindowPlan {
+  int P = 0;      // bytes per input pixel
+  int G = 1;      // output pixels per GEMM row
+  int win = 0;    // window bytes that hold taps
+  int wphys = 0;  // pixels per stored row: pl zeros, the row, zeros
 };
-
-inline int gcd_int(int a, int b) { return b == 0 ? a : gcd_int(b, a % b); }
-
-inline bool stem_layout_for(const ConvGeom &g, StemLayout *out) {
-  if (g.g != 1 || g.ins_h || g.ins_w || g.dw != 1) return false;
-  if (!(g.sw == 1 || g.sw == 2 || g.sw == 4)) return false;
-  const int cp = 16 / g.sw;
-  if (g.ic > cp || g.ic >= 16) return false;
-  const int wl = round_up(g.pl, g.sw);
-  const int win_px = (wl - g.pl) + g.kw;
-  const int wb = win_px * cp;
-  if (wb > 128) return false;
-  const int bk = wb <= 32 ? 32 : (wb <= 64 ? 64 : 128);
-  const int gg = gcd_int(g.ow, 128);
-  if (gg < 8) return false;
-  int wphys = (g.ow - 1) * g.sw + bk / cp;
-  if (wphys < wl + g.iw) wphys = wl + g.iw;
-  wphys = round_up(wphys, g.sw);
-  if (((size_t)wphys * cp) % 16 != 0) return false;
-  out->cp = cp; out->wl = wl; out->wphys = wphys; out->bk = bk; out->g = gg;
-  return true;
+inline bool window_plan_for(const ConvGeom &g, int es, int oc_pad, WindowPlan *out) {
+  if (g.g != 1 || g.ins_h || g.ins_w || (g.kh == 1 && g.kw == 1) || g.ic * es > 16) return false;
+  if (g.sh > 8 || g.pt > 127 || g.pb > 127 || (g.kh - 1) * g.dh > 127) return false;
+  double best = 0;
+  bool found = false;
+  for (int G : {4, 2, 1})
+    for (int P : {4, 8, 16}) {
+      const int win = ((G - 1) * g.sw + (g.kw - 1) * g.dw + 1) * P;
+      if (P / es < g.ic || (G > 1 && (oc_pad > 128 / G || g.ow % G)) || G * g.sw * P % 16 || win > 128) continue;
+      const double cost = (double)((win + 31) / 32) / G; // tensor-core steps per output pixel and filter row
+      if (found && cost >= best) continue;
+      found = true;
+      best = cost;
+      const int bk = win <= 32 ? 32 : (win <= 64 ? 64 : 128);
+      int wphys = ((g.ow / G - 1) * G * g.sw * P + bk + P - 1) / P; // the last window, with its padding, stays inside the row
+      if (wphys < g.pl + g.iw) wphys = g.pl + g.iw;
+      while (wphys * P % 16) ++wphys;
+      out->P = P; out->G = G; out->win = win; out->wphys = wphys;
+    }
+  return found;
 }
 
-inline void encode_window_map(CUtensorMap *tm, const int8_t *d_in, const ConvGeom &g, int cp, int wphys,
-                              int BK, int gpix) {
-  const cuuint64_t row_pitch = (cuuint64_t)wphys * cp;
-  cuuint64_t dims[4] = {(cuuint64_t)BK, (cuuint64_t)g.ow, (cuuint64_t)g.ih, (cuuint64_t)g.n};
-  cuuint64_t strides[3] = {(cuuint64_t)g.sw * cp, row_pitch, row_pitch * g.ih};
-  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)gpix, 1, 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = tma_api().tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)d_in, dims, strides, box, es,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(BK),
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(row window) failed: %d", (int)r);
-}
-
-// Thread-gathered stem convolution (conv_stem_i8_kernel): at most 4 input channels stored as one
-// 32-bit word per pixel, kw <= 8, kh <= 8, no groups / insertion / horizontal dilation.
-inline bool stem4_applies(const ConvGeom &g) {
-  return g.g == 1 && !g.ins_h && !g.ins_w && g.dw == 1 && g.ic <= 4 && g.kw <= 8 && g.kh <= 8;
-}
-
-struct StemPlan {
-  CUtensorMap tmB;
-  ConvStemParams p;
-  dim3 grid;
-  size_t smem = 0;
-};
-
-inline void stem_kernel_setup_once() {
-  static bool done = [] {
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_i8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_i8_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_i8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    return true;
-  }();
-  (void)done;
-}
-
-// weights [kh][oc_pad][32]: byte s*4 + c of filter row r
-inline std::vector<int8_t> pack_stem_weights(const float *w, int oc, int ic, int kh, int kw, int oc_pad) {
-  std::vector<int8_t> out((size_t)kh * oc_pad * 32, 0);
-  for (int o = 0; o < oc; ++o)
-    for (int c = 0; c < ic; ++c)
-      for (int r = 0; r < kh; ++r)
-        for (int s = 0; s < kw; ++s)
-          out[((size_t)r * oc_pad + o) * 32 + s * 4 + c] = (int8_t)(int)w[(((size_t)o * ic + c) * kh + r) * kw + s];
+// Weights of the window form: rows [G][128 / G channels] (one row per channel for G = 1), per filter row BK bytes.
+// part: -2 int8, -1 BF16, 0 / 1 the TF32 parts
+inline std::vector<int8_t> pack_window_weights(const float *w, const ConvGeom &g, const WindowPlan &wp, int rows, int BK, int part) {
+  const int es = part == -2 ? 1 : (part == -1 ? 2 : 4), slot = 128 / wp.G;
+  std::vector<int8_t> out((size_t)rows * g.kh * BK, 0);
+  for (int j = 0; j < wp.G; ++j)
+    for (int o = 0; o < g.oc; ++o)
+      for (int c = 0; c < g.ic; ++c)
+        for (int r = 0; r < g.kh; ++r)
+          for (int s = 0; s < g.kw; ++s) {
+            const float v = w[(((size_t)o * g.ic + c) * g.kh + r) * g.kw + s];
+            int8_t *at = out.data() + ((size_t)(j * slot + o) * g.kh + r) * BK + (size_t)(j * g.sw + s * g.dw) * wp.P + c * es;
+            if (part == -2) *at = (int8_t)(int)v;
+            else if (part == -1) {
+              const uint16_t h = (uint16_t)(f32_bits(v) >> 16);
+              std::memcpy(at, &h, 2);
+            } else {
+              const float hi = bits_f32(f32_bits(v) & 0xffffe000u), f = part == 0 ? hi : v - hi;
+              std::memcpy(at, &f, 4);
+            }
+          }
   return out;
 }
 
-inline void finish_stem_plan(StemPlan &sp, const int8_t *d_w, int rows, int kh, int oc_pad, int sm_count) {
-  ConvStemParams &p = sp.p;
-  const int bn = 128; // channel tile = tensor-core M; rows past oc_pad are zero-filled by TMA
-  p.BN = bn;
-  p.n_valid = oc_pad;
-  p.tmem_cols = 128;
-  p.idesc = make_idesc_i8(128, bn);
-  p.M_total = rows;
-  p.kh = kh;
-  p.dual = (oc_pad <= 64 && rows > 128) ? 1 : 0;
-  const int m_tile = p.dual ? 256 : 128;
-  const int w_rows = p.dual ? 192 : bn;
-  sp.smem = kSmemHeader + 1024 + (size_t)kh * ((size_t)m_tile * 32 + (size_t)w_rows * 32);
-  const int m_tiles = (rows + m_tile - 1) / m_tile;
-  const int n_tiles = (oc_pad + bn - 1) / bn;
-  // persistent: two CTAs per SM, a multiple of the channel-tile count (a CTA's weights never change)
-  int grid = 2 * sm_count / n_tiles * n_tiles;
-  if (grid < n_tiles) grid = n_tiles;
-  if (grid > m_tiles * n_tiles) grid = m_tiles * n_tiles;
-  sp.grid = dim3((unsigned)grid, 1, 1);
-  cuuint64_t dims[3] = {32, (cuuint64_t)oc_pad, (cuuint64_t)kh};
-  cuuint64_t strides[2] = {32, (cuuint64_t)32 * oc_pad};
-  cuuint32_t box[3] = {32, (cuuint32_t)w_rows, (cuuint32_t)kh};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = tma_api().tiled(&sp.tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void *)d_w, dims, strides, box, es,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
-                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(stem weights) failed: %d", (int)r);
+inline void encode_window_map(CUtensorMap *tm, const void *d_in, const ConvGeom &g, const WindowPlan &wp, int BK, int tile_rows) {
+  const cuuint64_t row = (cuuint64_t)wp.wphys * wp.P;
+  cuuint64_t dims[4] = {(cuuint64_t)BK, (cuuint64_t)(g.ow / wp.G), (cuuint64_t)g.ih, (cuuint64_t)g.n};
+  cuuint64_t strides[3] = {(cuuint64_t)wp.G * g.sw * wp.P, row, row * g.ih};
+  int lower[2] = {0, -g.pt}, upper[2] = {0, (g.oh - 1) * g.sh + 1 - g.ih - g.pt};
+  cuuint32_t es[4] = {1, 1, (cuuint32_t)g.sh, 1};
+  CUresult r = tma_api().im2col(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)d_in, dims, strides, lower, upper, (cuuint32_t)BK,
+                                (cuuint32_t)tile_rows, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(BK),
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeIm2col(row windows) failed: %d", (int)r);
+  fix_small_im2col_map(tm, (size_t)row * g.ih * g.n);
 }
 
 // Build the launch plan for one GEMM-shaped problem.
@@ -371,15 +307,16 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   p.M_total = rows;
   p.BK = pick_bk(k_inner);
   p.c_chunks = (k_inner + p.BK - 1) / p.BK;
+  p.ksteps = p.c_chunks == 1 ? (k_inner + 31) / 32 : p.BK / 32;
   // Dual mode: layers with at most 64 output channels would leave half of the TMEM lanes (and half of
-  // the epilogue warps) idle; they run 256-pixel tiles instead (see the kernel). Not combined with the
-  // row-window activation mode.
+  // the epilogue warps) idle; they run 256-pixel tiles instead (see the kernel). Not combined with
+  // pixel groups, which fill them.
   {
     // ... unless the whole weight set is small enough to stay resident in plain mode, which feeds
     // fewer bytes per pixel (measured faster for the 1x1 layers with 64 outputs).
     const size_t w_plain = (size_t)taps * p.c_chunks * 128 * p.BK;
     const bool plain_resident = w_plain <= 48 * 1024 && 113 * 1024 - kSmemHeader - 1024 - w_plain >= 3 * (size_t)128 * p.BK;
-    p.dual = (oc_pad <= 64 && p.a_mode != 2 && rows > 128 && !plain_resident && !pl.tf32) ? 1 : 0;
+    p.dual = (oc_pad <= 64 && p.group <= 1 && rows > 128 && !plain_resident && !pl.tf32) ? 1 : 0;
   }
   const int m_tiles = (rows + (p.dual ? 255 : 127)) / (p.dual ? 256 : 128);
   // Transposed product: the channel tile is the tensor core's M (128 TMEM lanes, rows past the
@@ -401,8 +338,9 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   // sets would force one CTA per SM, which measured slower than re-fetching the weights from L2.
   const int ctas_per_sm = 2;
   const size_t budget = 113 * 1024;
-  p.w_resident = (!pl.tf32 && total_tiles >= 2LL * n_tiles && w_all <= 48 * 1024 &&
-                  budget - kSmemHeader - 1024 - w_all >= 3 * a_bytes) ? 1 : 0;
+  // (Pixel groups have small activation tiles: up to 60 KB of weights leave them four stages.)
+  p.w_resident = (!pl.tf32 && total_tiles >= 2LL * n_tiles && w_all <= (p.group > 1 ? 60 : 48) * 1024 &&
+                  budget - kSmemHeader - 1024 - w_all >= (p.group > 1 ? 4 : 3) * a_bytes) ? 1 : 0;
   const size_t stage_bytes = p.w_resident ? a_bytes : a_bytes + b_bytes;
   const size_t ring_budget = budget - kSmemHeader - 1024 - (p.w_resident ? w_all : 0);
   int stages = (int)(ring_budget / stage_bytes);
@@ -456,19 +394,14 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
 }
 
 inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_count) {
-  if (pl.use_patch) {
-    size_t total = (size_t)pl.p.M_total * pl.patch.kp;
-    if (pl.patch.cv == 4 && pl.patch_elsize == 4)
-      launch_k(patch_expand_tap_kernel<float>, grid_for(total / 4, 256, sm_count), 256, 0, stream, 
-          reinterpret_cast<const float *>(pl.in), reinterpret_cast<float *>(pl.patch_buf), pl.split_lo, pl.patch);
-    else if (pl.patch.cv == 4)
-      launch_k(patch_expand_tap_kernel<uint16_t>, grid_for(total / 4, 256, sm_count), 256, 0, stream, 
-          reinterpret_cast<const uint16_t *>(pl.in), reinterpret_cast<uint16_t *>(pl.patch_buf), nullptr, pl.patch);
-    else if (pl.patch_elsize == 2)
-      launch_k(patch_expand_kernel<uint16_t>, grid_for(total / 8, 256, sm_count), 256, 0, stream, 
-          reinterpret_cast<const uint16_t *>(pl.in), reinterpret_cast<uint16_t *>(pl.patch_buf), pl.patch);
-    else
-      launch_k(patch_expand_i8_kernel, grid_for(total, 256, sm_count), 256, 0, stream, pl.in, pl.patch_buf, pl.patch);
+  if (pl.use_patch)
+    launch_k(patch_expand_i8_kernel, grid_for((size_t)pl.p.M_total * pl.patch.kp, 256, sm_count), 256, 0, stream, pl.in, pl.patch_buf, pl.patch);
+  if (pl.use_repack) {
+    const RepackArgs &a = pl.repack;
+    const int grid = (int)std::min<size_t>(a.rows, (size_t)sm_count * 8);
+    if (a.es == 1) launch_k(window_repack_kernel<uint8_t>, grid, 256, 0, stream, a);
+    else if (a.es == 2) launch_k(window_repack_kernel<uint16_t>, grid, 256, 0, stream, a);
+    else launch_k(window_repack_kernel<uint32_t>, grid, 256, 0, stream, a);
   }
   const int threads = kConvThreads;
   PdlConvScope conv_class; // the tensor-core kernel and its helper passes may start while the predecessor finishes

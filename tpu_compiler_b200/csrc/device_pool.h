@@ -117,6 +117,8 @@ public:
     return p;
   }
 
+  cudaMemPool_t handle() const { return mem_; }
+
   // Gives the driver back what lies free above kPoolKeepBytes. Called where a module's buffers have been freed; in between
   // the pool holds on to what it has (its release threshold counts the memory in use too, so with any finite threshold
   // a process that holds a large module would unmap and map again at every synchronisation: 40 ms spikes).

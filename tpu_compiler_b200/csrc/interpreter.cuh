@@ -164,7 +164,7 @@ public:
     t->cp = round_up(t->c, lanes);
     t->wphys = t->w;
     auto lr = layout_requests.find(name);
-    if (lr != layout_requests.end() && dtype == DT_I8) {
+    if (lr != layout_requests.end() && dtype != DT_F32) {
       t->cp = lr->second.cp;
       t->wl = lr->second.wl;
       t->wphys = lr->second.wphys;
@@ -327,8 +327,22 @@ inline std::vector<FloatRequant> float_requant(const std::vector<float> &filt, c
   std::vector<FloatRequant> out(std::max<size_t>(oc, pad_to), FloatRequant{0u, 0.0f, 0.0f, 0.0f});
   const double scale = kFqScale;
   for (size_t o = 0; o < oc; ++o) {
-    double bound = std::fabs((double)bias[o]);
-    for (size_t i = 0; i < per; ++i) bound += 128.0 * std::fabs((double)filt[o * per + i]);
+    // sum of |w| in sixteen lanes: integers that stay exact in a float (2^24 / 128 weights and more per lane)
+    const float *w = filt.data() + o * per;
+    float lane[16] = {};
+    double sum = 0;
+    for (size_t i = 0; i < per; i += 16 << 16) {
+      const size_t end = std::min(per, i + (16u << 16));
+      size_t j = i;
+      for (; j + 16 <= end; j += 16)
+        for (int l = 0; l < 16; ++l) lane[l] += std::fabs(w[j + l]);
+      for (; j < end; ++j) lane[0] += std::fabs(w[j]);
+      for (float &l : lane) {
+        sum += l;
+        l = 0.0f;
+      }
+    }
+    const double bound = std::fabs((double)bias[o]) + 128.0 * sum;
     const double m = std::ldexp((double)mult[o], -31), r = rshift[o], rnd = r > 0 ? std::ldexp(1.0, (int)r - 1) : 0.0;
     double d, c = std::ldexp(1.0, -49 - (int)r);
     bool ok = r >= 0;
@@ -380,16 +394,14 @@ public:
   }
   void invoke(cudaStream_t s) override {
     TPUCB_CHECK(!in_->padded_rows(), "quant %s: padded-row input is not supported", name.c_str());
-    if (kind_ == 0 && in_->dtype == DT_F32 && in_->cp == 4 && (out_->cp == 4 || out_->cp == 8 || out_->cp == 16)) {
-      size_t total = out_->pixels();
-      launch_k(quant_input_pix_kernel, grid_for(total, 256, I_.sm_count), 256, 0, s, 
-          (const float4 *)in_->dev, out_->dev, out_->n, out_->h, out_->w, out_->c, out_->cp, out_->wl,
-          out_->wphys, scale_);
-      return;
-    }
-    if (kind_ == 5 && in_->dtype == DT_F32 && in_->cp == 4 && out_->cp == 16 && !out_->padded_rows()) {
-      launch_k(quant_f32c4_to_bf16c16_kernel, grid_for(out_->pixels(), 256, I_.sm_count), 256, 0, s, 
-          (const float4 *)in_->dev, (uint4 *)out_->dev, out_->pixels(), out_->c);
+    if ((kind_ == 0 || kind_ == 5) && in_->dtype == DT_F32 && in_->cp == 4 && (out_->cp == 4 || out_->cp == 8 || out_->cp == 16)) {
+      const int rows = out_->n * out_->h, grid = std::min(rows, I_.sm_count * 8);
+      if (kind_ == 0)
+        launch_k(quant_input_pix_kernel<false>, grid, 256, 0, s, (const float4 *)in_->dev, out_->dev, rows, out_->w, out_->c,
+                 out_->cp, out_->wl, out_->wphys, scale_);
+      else
+        launch_k(quant_input_pix_kernel<true>, grid, 256, 0, s, (const float4 *)in_->dev, out_->dev, rows, out_->w, out_->c,
+                 out_->cp, out_->wl, out_->wphys, scale_);
       return;
     }
     const bool same_layout = in_->cp == out_->cp && !out_->padded_rows() && out_->cp % 16 == 0;
@@ -452,7 +464,7 @@ public:
       // BF16 graphs (core/conv.cpp:90-98: fp32 convolution of BF16-valued operands, fp32 bias, ReLU, BF16 rounding):
       // the tensor-core pipeline with BF16 operands and fp32 accumulators; every K size and pitch is in bytes.
       TPUCB_CHECK(in->dtype == DT_BF16, "conv %s: a BF16 convolution needs a BF16 input", op.name.c_str());
-      if ((g.g > 1 || g.ins_h || g.ins_w) && !in->padded_rows()) {
+      if (g.g > 1 || g.ins_h || g.ins_w) {
         // grouped / depthwise layers and deconvolutions (input insertion): the direct kernel
         // (conv_bf16_grouped_kernel); weights as fp32 [oc][kh][kw][ic / g]
         std::vector<float> wt((size_t)g.oc * g.kh * g.kw * icg);
@@ -466,8 +478,9 @@ public:
         alg_bytes = 2.0 * ((double)in->numel() + out->numel()) + 4.0 * (filt.data.size() + g.oc);
         return;
       }
-      TPUCB_CHECK(g.g == 1 && !g.ins_h && !g.ins_w && !in->padded_rows() && g.pl <= 127 && g.pt <= 127 &&
-                      (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255,
+      WindowPlan wp;
+      const bool window = window_plan_for(g, 2, out->cp, &wp);
+      TPUCB_CHECK(window || (g.pl <= 127 && g.pt <= 127 && (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255),
                   "conv %s: BF16 convolution supports dense, ungrouped layers", op.name.c_str());
       conv_kernel_setup_once();
       std::vector<int32_t> bias_bits(out->cp, 0);
@@ -489,29 +502,8 @@ public:
       const int rows = g.n * g.oh * g.ow;
       const int k_bytes = in->cp * 2;
       const bool one_by_one_bf = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
-      if (g.ic < 8 && !one_by_one_bf) {
-        // few input channels (3-channel stems): expand the patches into a K-major matrix first
-        pl.use_patch = true;
-        pl.patch_elsize = 2;
-        PatchArgs &a = pl.patch;
-        a.n = g.n; a.c = g.ic; a.cp = in->cp; a.ih = g.ih; a.iw = g.iw; a.oh = g.oh; a.ow = g.ow;
-        a.kh = g.kh; a.kw = g.kw; a.sh = g.sh; a.sw = g.sw; a.pt = g.pt; a.pl = g.pl; a.dh = g.dh; a.dw = g.dw;
-        a.ins_h = 0; a.ins_w = 0; a.c_first = 0; a.c_count = g.ic; a.wl = in->wl; a.wphys = in->wphys;
-        a.cv = g.ic <= 4 ? 4 : 0; // four channel slots per tap: one 8-byte copy per tap
-        a.kp = a.cv ? round_up(g.kh * g.kw * 4, 8) : round_up(g.kh * g.kw * g.ic, 16);
-        pl.patch_bytes = (size_t)rows * a.kp * 2;
-        pl.patch_buf = (int8_t *)I.dalloc(pl.patch_bytes);
-        const int8_t *d_wp = I.upload(pack_patch_weights(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, a.kp, -1, a.cv));
-        p.kh = p.kw = 1;
-        p.a_mode = 0;
-        finish_plan(pl, rows, 1, a.kp * 2, out->cp, I.sm_count);
-        encode_matrix_map(&pl.tmA, pl.patch_buf, rows, a.kp * 2, a.kp * 2, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_wp, out->cp, 1, a.kp * 2, p.BK, p.dual ? 192 : p.BN);
-        p.idesc = make_idesc_bf16(128, p.BN);
-        pl.ops = alg_ops;
-        I.attach_split_ws(pl);
-        plans_.push_back(pl);
-        alg_bytes = 2.0 * ((double)in->numel() + out->numel() + filt.data.size()) + 4.0 * g.oc;
+      if (window) { // few input channels (3-channel stems)
+        setup_window(I, pl, wp, filt, -1);
         return;
       }
       const int8_t *d_w = I.upload(pack_conv_weights_bf16(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, in->cp));
@@ -537,10 +529,8 @@ public:
     }
     if (out->dtype == DT_F32) {
       TPUCB_CHECK(in->dtype == DT_F32, "conv %s: an fp32 convolution needs an fp32 input", op.name.c_str());
-      if (I.fp32_tensor_cores && g.g == 1 && !g.ins_h && !g.ins_w && g.ic <= 4 && in->cp == 4 && !(g.kh == 1 && g.kw == 1)) {
-        // Image stem (at most 4 channels, NHWC4 input): the patches are expanded into a K-major matrix with four channel
-        // slots per tap (one 16-byte copy per tap; the expansion also writes the remainder part), which is then the
-        // activation operand of the TF32 x 3 product: 49 taps become 7 K blocks per term.
+      WindowPlan wp;
+      if (I.fp32_tensor_cores && window_plan_for(g, 4, out->cp, &wp)) { // image stems
         conv_kernel_setup_once();
         std::vector<int32_t> bias_bits(out->cp, 0);
         for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
@@ -549,47 +539,13 @@ public:
         ConvPlan pl;
         std::memset(&pl.p, 0, sizeof(pl.p));
         pl.tf32 = true;
-        pl.use_patch = true;
-        pl.patch_elsize = 4;
-        pl.in = (const int8_t *)in->dev;
-        const int rows = g.n * g.oh * g.ow;
-        PatchArgs &a = pl.patch;
-        a.n = g.n; a.c = g.ic; a.cp = in->cp; a.ih = g.ih; a.iw = g.iw; a.oh = g.oh; a.ow = g.ow;
-        a.kh = g.kh; a.kw = g.kw; a.sh = g.sh; a.sw = g.sw; a.pt = g.pt; a.pl = g.pl; a.dh = g.dh; a.dw = g.dw;
-        a.ins_h = 0; a.ins_w = 0; a.c_first = 0; a.c_count = g.ic; a.wl = in->wl; a.wphys = in->wphys;
-        a.cv = 4;
-        a.kp = g.kh * g.kw * 4;
-        pl.patch_bytes = (size_t)rows * a.kp * 4;
-        pl.patch_buf = (int8_t *)I.dalloc(pl.patch_bytes);
-        pl.split_src = nullptr; // the expansion writes the remainder itself
-        pl.split_hi = nullptr;
-        pl.split_lo = (float *)I.dalloc(pl.patch_bytes);
-        ConvGemmParams &p = pl.p;
-        p.OH = g.oh; p.OW = g.ow; p.sh = p.sw = p.dh = p.dw = 1;
-        p.act = act_;
-        p.bias = d_bias_; p.mult = d_bias_; p.rshift = d_bias_;
-        p.out = (int8_t *)out->dev;
-        p.ldc = out->cp * 4;
-        p.c_off = 0;
-        p.err = &I.ss.d_err->code;
-        p.kh = p.kw = 1;
-        p.a_mode = 0;
-        const int kb = a.kp * 4;
-        const int8_t *d_ph = I.upload(pack_patch_weights(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, a.kp, 0, 4));
-        const int8_t *d_pl = I.upload(pack_patch_weights(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, a.kp, 1, 4));
-        finish_plan(pl, rows, 1, kb, out->cp, I.sm_count);
-        encode_matrix_map(&pl.tmA, pl.patch_buf, rows, kb, kb, p.BK, a_tile_rows(p));
-        encode_matrix_map(&pl.tmA2, (const int8_t *)pl.split_lo, rows, kb, kb, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_ph, out->cp, 1, kb, p.BK, p.BN);
-        encode_weight_map(&pl.tmB2, d_pl, out->cp, 1, kb, p.BK, p.BN);
-        p.idesc = make_idesc_tf32(128, p.BN);
-        pl.ops = alg_ops;
-        I.attach_split_ws(pl);
-        plans_.push_back(pl);
-        alg_bytes = 4.0 * ((double)in->numel() + out->numel() + filt.data.size() + g.oc);
+        pl.p.act = act_;
+        pl.p.bias = d_bias_; pl.p.mult = d_bias_; pl.p.rshift = d_bias_;
+        pl.p.err = &I.ss.d_err->code;
+        setup_window(I, pl, wp, filt, 0);
         return;
       }
-      if (I.fp32_tensor_cores && g.g == 1 && !g.ins_h && !g.ins_w && !in->padded_rows() && in->cp % 8 == 0 &&
+      if (I.fp32_tensor_cores && g.g == 1 && !g.ins_h && !g.ins_w && in->cp % 8 == 0 &&
           g.pl <= 127 && g.pt <= 127 && (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255) {
         // fp32 convolution on the tensor cores as three TF32 products with fp32 accumulation (x w = xh wh + xl wh +
         // xh wl, 2^-22 relative: inside the 1e-4 of the fp32 path, where a single TF32 product would not be). The
@@ -693,45 +649,26 @@ public:
       return;
     }
 
-    if (in->cp == 4 && !in->padded_rows() && stem4_applies(g)) {
-      stem_kernel_setup_once();
-      StemPlan sp;
-      std::memset(&sp.p, 0, sizeof(sp.p));
-      ConvStemParams &p = sp.p;
-      p.OH = g.oh; p.OW = g.ow; p.H = g.ih; p.W = g.iw;
-      p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.kw = g.kw;
-      p.act = act_;
-      p.fastq = fastq;
-      p.in = (const uint32_t *)in->dev;
-      p.bias = d_bias_; p.mult = d_mult_; p.rshift = d_rsh_;
-      p.out = (int8_t *)out->dev;
-      p.ldc = out->cp;
-      p.c_off = 0;
-      p.err = &I.ss.d_err->code;
-      const int8_t *d_w = I.upload(pack_stem_weights(filt.data.data(), g.oc, g.ic, g.kh, g.kw, oc_pad));
-      finish_stem_plan(sp, d_w, g.n * g.oh * g.ow, g.kh, oc_pad, I.sm_count);
-      stem_plans_.push_back(sp);
-      return;
+    {
+      WindowPlan wp;
+      if (window_plan_for(g, 1, oc_pad, &wp)) { // few input channels (3-channel stems)
+        conv_kernel_setup_once();
+        ConvPlan pl;
+        std::memset(&pl.p, 0, sizeof(pl.p));
+        pl.p.act = act_;
+        pl.p.fastq = fastq;
+        pl.p.bias = d_bias_; pl.p.mult = d_mult_; pl.p.rshift = d_rsh_;
+        pl.p.fq = d_fq;
+        pl.p.err = &I.ss.d_err->code;
+        setup_window(I, pl, wp, filt, -2);
+        return;
+      }
     }
-
     conv_kernel_setup_once();
     const bool one_by_one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 &&
                             g.oh == g.ih && g.ow == g.iw;
     const bool small_c = g.ic < 16;
-    StemLayout stem;
-    bool stem_ok = in->padded_rows() && stem_layout_for(g, &stem) && stem.cp == in->cp &&
-                   stem.wl == in->wl && stem.wphys == in->wphys;
-    if (stem_ok) {
-      // The window tensor map has overlapping strides; if the driver refuses to encode it, the
-      // patch-expansion path (which understands padded rows) takes over.
-      try {
-        CUtensorMap probe;
-        encode_window_map(&probe, (const int8_t *)in->dev, g, in->cp, in->wphys, stem.bk, stem.g);
-      } catch (const Error &) {
-        stem_ok = false;
-      }
-    }
-    const bool need_patch = !stem_ok && (g.g > 1 || g.ins_h || g.ins_w || (small_c && !one_by_one) || in->padded_rows() || in->cp % 16 != 0 ||
+    const bool need_patch = (g.g > 1 || g.ins_h || g.ins_w || (small_c && !one_by_one) || in->padded_rows() || in->cp % 16 != 0 ||
                             g.pl > 127 || g.pt > 127 || (g.kw - 1) * g.dw > 255 || (g.kh - 1) * g.dh > 255);
     const int groups = g.g;
     for (int grp = 0; grp < groups; ++grp) {
@@ -753,27 +690,7 @@ public:
       int ocg_pad = groups == 1 ? oc_pad : ocg;
       TPUCB_CHECK(groups == 1 || ocg % 16 == 0, "conv %s: grouped convolution needs oc/g to be a multiple of 16",
                   op.name.c_str());
-      if (stem_ok) {
-        // Row-window path: one K step per filter row; the window of (left slack + kw) pixels x
-        // cp channels is contiguous in the zero-padded NHWC rows.
-        const int BKs = stem.bk;
-        std::vector<int8_t> w((size_t)ocg_pad * g.kh * BKs, 0);
-        for (int o = 0; o < ocg; ++o)
-          for (int c = 0; c < icg; ++c)
-            for (int r = 0; r < g.kh; ++r)
-              for (int ss = 0; ss < g.kw; ++ss)
-                w[((size_t)o * g.kh + r) * BKs + (size_t)(ss + stem.wl - g.pl) * in->cp + c] =
-                    (int8_t)(int)wsrc[(((size_t)o * icg + c) * g.kh + r) * g.kw + ss];
-        const int8_t *d_w = I.upload(w);
-        p.kh = g.kh;
-        p.kw = 1;
-        p.a_mode = 2;
-        p.win_g = stem.g;
-        finish_plan(pl, rows, g.kh, BKs, ocg_pad, I.sm_count);
-        TPUCB_CHECK(p.BK == BKs && p.c_chunks == 1, "conv %s: stem tile shape mismatch", op.name.c_str());
-        encode_window_map(&pl.tmA, (const int8_t *)in->dev, g, in->cp, in->wphys, BKs, stem.g);
-        encode_weight_map(&pl.tmB, d_w, ocg_pad, g.kh, BKs, p.BK, p.dual ? 192 : p.BN);
-      } else if (need_patch) {
+      if (need_patch) {
         pl.use_patch = true;
         PatchArgs &a = pl.patch;
         a.n = g.n; a.c = g.ic; a.cp = in->cp; a.ih = g.ih; a.iw = g.iw; a.oh = g.oh; a.ow = g.ow;
@@ -816,10 +733,58 @@ public:
       plans_.push_back(pl);
     }
   }
+  // The row-window form (WindowPlan) of the layer. The input tensor has the window layout when it was asked for at load
+  // and granted; else (and always for fp32, whose remainder operand has to be made anyway) a copy of its rows is made
+  // before the launch. part: as in pack_window_weights (0: TF32, both parts)
+  void setup_window(Interpreter &I, ConvPlan &pl, const WindowPlan &wp, const HostWeight &filt, int part) {
+    const ConvGeom &g = g_;
+    const int es = part == -2 ? 1 : (part == -1 ? 2 : 4);
+    ConvGemmParams &p = pl.p;
+    const void *rows = in_->dev, *rows_lo = nullptr;
+    if (part == 0 || in_->cp * es != wp.P || in_->wl != g.pl || in_->wphys != wp.wphys) {
+      const size_t bytes = (size_t)g.n * g.ih * wp.wphys * wp.P;
+      pl.use_repack = true;
+      RepackArgs &a = pl.repack;
+      a.in = in_->dev;
+      a.out = I.dalloc(bytes);
+      a.lo = part == 0 ? I.dalloc(bytes) : nullptr;
+      a.rows = (size_t)g.n * g.ih;
+      a.w = g.iw; a.c = g.ic; a.cps = in_->cp; a.in_wl = in_->wl; a.in_wphys = in_->wphys;
+      a.cpd = wp.P / es; a.wl = g.pl; a.wphys = wp.wphys; a.es = es;
+      rows = a.out;
+      rows_lo = a.lo;
+    }
+    p.OH = g.oh; p.OW = g.ow / wp.G; p.sh = g.sh; p.sw = 1; p.pt = g.pt; p.pl = 0; p.dh = g.dh; p.dw = 0;
+    p.kh = g.kh; p.kw = 1;
+    p.a_mode = 1;
+    p.out = (int8_t *)out_->dev;
+    p.c_off = 0;
+    p.group = wp.G;
+    p.ldc_px = out_->cp * es;
+    p.ldc = p.ldc_px * wp.G;
+    finish_plan(pl, g.n * g.oh * p.OW, g.kh, wp.win, out_->cp, I.sm_count);
+    const int w_rows = wp.G > 1 ? 128 : out_->cp;
+    auto weights = [&](CUtensorMap *tm, int pt) {
+      encode_weight_map(tm, I.upload(pack_window_weights(filt.data.data(), g, wp, w_rows, p.BK, pt)), w_rows, g.kh, p.BK, p.BK,
+                        p.dual ? 192 : p.BN);
+    };
+    encode_window_map(&pl.tmA, rows, g, wp, p.BK, a_tile_rows(p));
+    weights(&pl.tmB, part);
+    if (part == 0) {
+      encode_window_map(&pl.tmA2, rows_lo, g, wp, p.BK, a_tile_rows(p));
+      weights(&pl.tmB2, 1);
+    }
+    if (part == 0) p.idesc = make_idesc_tf32(128, p.BN);
+    else if (part == -1) p.idesc = make_idesc_bf16(128, p.BN);
+    pl.ops = alg_ops;
+    I.attach_split_ws(pl);
+    plans_.push_back(pl);
+    alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.data.size()) + (part == -2 ? 12.0 : 4.0) * g.oc;
+  }
   // Fused leaky ReLU (tensor-core plans only): the epilogue writes the plain result to this op's tensor
   // and the activation result to `act_out`.
   bool can_fuse_leaky() const {
-    return !(f32_ || dw_ || bf16g_ || !stem_plans_.empty() || act_ != 0 || plans_.empty()) && in_->dtype == DT_I8;
+    return !(f32_ || dw_ || bf16g_ || act_ != 0 || plans_.empty()) && in_->dtype == DT_I8;
   }
   void set_leaky(int mp, int rp, int mn, int rn, int8_t *act_out) {
     for (auto &pl : plans_) {
@@ -832,7 +797,7 @@ public:
   // Fused eltwise add (tensor-core INT8 plans without an activation of their own): the epilogue also forms
   // sat8(relu?((conv * ms + residual * mr + 2^(r-1)) >> r)) into `sum_out`; this op's own tensor is still written.
   bool can_fuse_add() const {
-    return can_fuse_leaky() && plans_.size() == 1 && in_->dtype == DT_I8 && plans_[0].p.split_k <= 1;
+    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1;
   }
   void set_residual_add(const int8_t *residual, int8_t *sum_out, int ms, int mr, int rshift, int relu) {
     for (auto &pl : plans_) {
@@ -846,8 +811,8 @@ public:
   }
   const TensorPtr &out() const { return out_; }
   const TensorPtr &in() const { return in_; }
-  // TF32 x 3 plans (not the patch-matrix stem, whose remainder belongs to the patch matrix)
-  bool is_tf32() const { return !plans_.empty() && plans_[0].tf32 && !plans_[0].use_patch; }
+  // TF32 x 3 plans (not the row-window stem, whose remainder belongs to its own copy of the rows)
+  bool is_tf32() const { return !plans_.empty() && plans_[0].tf32 && !plans_[0].use_repack; }
   bool can_write_remainder() const { return !plans_.empty() && plans_[0].tf32; }
   void set_remainder_out(void *lo) {
     for (auto &pl : plans_) pl.p.out2 = (int8_t *)lo;
@@ -891,25 +856,17 @@ public:
       launch_k(dwconv_i8_kernel, grid_for(total, 128, I_.sm_count), 128, 0, s, (const int8_t *)in_->dev,
                                                                           (int8_t *)out_->dev, dwargs_);
     } else {
-      for (auto &sp : stem_plans_) {
-        PdlConvScope conv_class;
-        if ((sp.p.fastq & 1) && sp.p.act == 1) // the ReLU epilogue alone: most stems
-          launch_k(conv_stem_i8_kernel<true, true>, sp.grid, kStemThreads, sp.smem, s, sp.tmB, sp.p);
-        else if (sp.p.fastq & 1) launch_k(conv_stem_i8_kernel<true>, sp.grid, kStemThreads, sp.smem, s, sp.tmB, sp.p);
-        else launch_k(conv_stem_i8_kernel<false>, sp.grid, kStemThreads, sp.smem, s, sp.tmB, sp.p);
-      }
       for (auto &pl : plans_) launch_conv_plan(pl, s, I_.sm_count);
     }
   }
   int kernel_launches() const override {
     if (f32_ || dw_ || bf16g_) return 1;
-    int k = (int)stem_plans_.size();
-    for (auto &pl : plans_) k += 1 + (pl.use_patch ? 1 : 0) + ((pl.tf32 && pl.split_src) ? 1 : 0);
+    int k = 0;
+    for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack ? 1 : 0) + ((pl.tf32 && pl.split_src) ? 1 : 0);
     return k;
   }
   bool is_tensor_core() const { return !f32_ && !dw_ && !bf16g_; }
   std::vector<ConvPlan> plans_;
-  std::vector<StemPlan> stem_plans_;
 
 private:
   Interpreter &I_;
@@ -2184,8 +2141,8 @@ inline void Interpreter::load_module(const std::string &text) {
       parsed.push_back(parse_line(line.substr(b)));
     }
   }
-  // Pre-pass: a few-channel convolution whose input is produced by an input or quant op and has
-  // no other consumer asks for that tensor to be stored with zero-padded rows (stem path).
+  // Pre-pass: a few-channel convolution whose input is produced by an input or quant op and has no
+  // other consumer asks for that tensor to be stored in its window layout (WindowPlan).
   layout_requests.clear();
   {
     std::map<std::string, const ParsedOp *> by_name;
@@ -2195,11 +2152,11 @@ inline void Interpreter::load_module(const std::string &text) {
       for (auto &nm : op.in) n_uses[nm]++;
     }
     for (auto &op : parsed) {
-      if (op.type != "conv_2d" || op.dtype != "INT8" || op.in.empty()) continue;
+      if (op.type != "conv_2d" || (op.dtype != "INT8" && op.dtype != "BF16") || op.in.empty()) continue;
       auto it = by_name.find(op.in[0]);
       if (it == by_name.end() || n_uses[op.in[0]] != 1) continue;
       const ParsedOp &src = *it->second;
-      if (!(src.type == "input" || src.type == "quant") || src.dtype != "INT8" || src.shape.size() != 4 ||
+      if (!(src.type == "input" || src.type == "quant") || src.dtype != op.dtype || src.shape.size() != 4 ||
           op.shape.size() != 4)
         continue;
       ConvGeom g;
@@ -2209,17 +2166,26 @@ inline void Interpreter::load_module(const std::string &text) {
       g.sw = op.geti("sw", 1); g.pt = op.geti("pt", 0); g.pb = op.geti("pb", 0); g.pl = op.geti("pl", 0);
       g.pr = op.geti("pr", 0); g.dh = op.geti("dh", 1); g.dw = op.geti("dw", 1);
       g.ins_h = op.geti("ins_h", 0); g.ins_w = op.geti("ins_w", 0);
-      StemLayout st;
-      if (stem4_applies(g)) {
+      WindowPlan wp;
+      const int es = op.dtype == "INT8" ? 1 : 2;
+      if (window_plan_for(g, es, round_up(g.oc, 16), &wp)) {
         RowLayout rl;
-        rl.cp = 4; rl.wl = 0; rl.wphys = g.iw;
-        layout_requests[src.name] = rl;
-      } else if (stem_layout_for(g, &st)) {
-        RowLayout rl;
-        rl.cp = st.cp; rl.wl = st.wl; rl.wphys = st.wphys;
+        rl.cp = wp.P / es; rl.wl = g.pl; rl.wphys = wp.wphys;
         layout_requests[src.name] = rl;
       }
     }
+  }
+  // The pool grows once, by about what the tensors of a large module need, instead of tensor by tensor.
+  size_t need = 0;
+  for (const ParsedOp &op : parsed) {
+    size_t v = (size_t)max_batch * (op.dtype == "INT8" ? 1 : (op.dtype == "BF16" ? 2 : 4));
+    for (int64_t d : op.shape) v *= (size_t)std::max<int64_t>(d, 1);
+    if (op.type != "reshape") need += v;
+  }
+  if (need >= (64u << 20)) {
+    void *p = nullptr; // (a request that is too large by its rounding is no error: the tensors will tell)
+    if (cudaMallocFromPoolAsync(&p, need, pool->handle(), stream) == cudaSuccess) dfree(p);
+    else cudaGetLastError();
   }
   for (const ParsedOp &op : parsed) add_op(op);
   finish_module();
@@ -2413,9 +2379,9 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
   TPUCB_CUDA(cudaStreamWaitEvent(stream, ss.upload_done[k], 0));
   TensorGeom g{t->n, t->c, t->h, t->w, t->cp, t->wl, t->wphys};
   const int8_t *stg = (const int8_t *)async_staging[k];
-  if (t->cp == 4 && !t->padded_rows())
-    launch_k(nchw_i8_to_nhwc4_kernel, grid_for(t->pixels(), 256, sm_count), 256, 0, stream, stg, (uint32_t *)t->dev, t->n, t->c,
-             (size_t)t->h * t->w);
+  if (t->c <= 4 && (t->cp == 4 || t->cp == 8 || t->cp == 16))
+    launch_k(nchw_i8_to_pix_kernel, std::min(t->n * t->h, sm_count * 8), 256, 0, stream, (const uint8_t *)stg, t->dev, t->n, t->c,
+             t->h, t->w, t->cp, t->wl, t->wphys);
   else
     launch_k(nchw_i8_to_dev_kernel, grid_for(t->pixels() * t->cp, 256, sm_count), 256, 0, stream, stg, (int8_t *)t->dev, g);
   TPUCB_CUDA(cudaEventRecord(ss.staging_free[k], stream));

@@ -66,7 +66,7 @@ __global__ void nchw_f32_to_nhwc4_kernel(const float *__restrict__ src, float4 *
 }
 
 // upload of already quantised int8 values (NCHW order) into an INT8 tensor: the generic form (any channel pitch,
-// padded rows) and the image form (at most 4 channels, one 32-bit word per pixel).
+// padded rows) and the image form (at most 4 channels in a pitch of 4, 8 or 16; one block per row).
 __global__ void nchw_i8_to_dev_kernel(const int8_t *__restrict__ src, int8_t *__restrict__ dst, TensorGeom g) {
   pdl_prologue();
   const size_t total = (size_t)g.n * g.h * g.wphys * g.cp;
@@ -80,17 +80,27 @@ __global__ void nchw_i8_to_dev_kernel(const int8_t *__restrict__ src, int8_t *__
     dst[i] = (c < g.c && x >= 0 && x < g.w) ? src[(((size_t)b * g.c + c) * g.h + y) * g.w + x] : (int8_t)0;
   }
 }
-__global__ void nchw_i8_to_nhwc4_kernel(const int8_t *__restrict__ src, uint32_t *__restrict__ dst, int n, int c, size_t hw) {
+__global__ void nchw_i8_to_pix_kernel(const uint8_t *__restrict__ src, void *__restrict__ dst, int n, int c, int h, int w, int cp,
+                                      int wl, int wphys) {
   pdl_prologue();
-  const size_t total = (size_t)n * hw;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t b = i / hw, p = i - b * hw;
-    const uint8_t *s = reinterpret_cast<const uint8_t *>(src) + b * c * hw + p;
-    uint32_t v = s[0];
-    if (c > 1) v |= (uint32_t)s[hw] << 8;
-    if (c > 2) v |= (uint32_t)s[2 * hw] << 16;
-    if (c > 3) v |= (uint32_t)s[3 * hw] << 24;
-    dst[i] = v;
+  for (int row = blockIdx.x; row < n * h; row += gridDim.x) {
+    const int b = row / h, y = row - b * h;
+    const uint8_t *s = src + ((size_t)b * c * h + y) * w;
+    const size_t plane = (size_t)h * w;
+    for (int i = threadIdx.x; i < wphys; i += blockDim.x) {
+      const int x = i - wl;
+      uint32_t v = 0;
+      if (x >= 0 && x < w) {
+        v = s[x];
+        if (c > 1) v |= (uint32_t)s[plane + x] << 8;
+        if (c > 2) v |= (uint32_t)s[2 * plane + x] << 16;
+        if (c > 3) v |= (uint32_t)s[3 * plane + x] << 24;
+      }
+      const size_t at = (size_t)row * wphys + i;
+      if (cp == 4) reinterpret_cast<uint32_t *>(dst)[at] = v;
+      else if (cp == 8) reinterpret_cast<uint2 *>(dst)[at] = make_uint2(v, 0u);
+      else reinterpret_cast<uint4 *>(dst)[at] = make_uint4(v, 0u, 0u, 0u);
+    }
   }
 }
 
@@ -134,19 +144,6 @@ __device__ __forceinline__ void store_from_f32(void *p, int dt, size_t i, float 
   if (dt == DT_I8) reinterpret_cast<int8_t *>(p)[i] = (int8_t)(int)v;
   else if (dt == DT_BF16) reinterpret_cast<uint16_t *>(p)[i] = (uint16_t)(f32_bits(v) >> 16);
   else reinterpret_cast<float *>(p)[i] = v;
-}
-
-// fp32 NHWC4 input image -> BF16 tensor with a 16-channel pitch (quant NONE -> BF16: the upper half of each fp32
-// word, no rounding, QuantOpKernel's cast): one pixel per thread, one 16-byte read, two 16-byte writes.
-__global__ void quant_f32c4_to_bf16c16_kernel(const float4 *__restrict__ in, uint4 *__restrict__ out, size_t pixels, int c) {
-  pdl_prologue();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < pixels; i += (size_t)gridDim.x * blockDim.x) {
-    const float4 v = __ldg(in + i);
-    const uint32_t h0 = __float_as_uint(v.x) >> 16, h1 = c > 1 ? __float_as_uint(v.y) >> 16 : 0u;
-    const uint32_t h2 = c > 2 ? __float_as_uint(v.z) >> 16 : 0u, h3 = c > 3 ? __float_as_uint(v.w) >> 16 : 0u;
-    out[2 * i] = make_uint4(h0 | (h1 << 16), h2 | (h3 << 16), 0u, 0u);
-    out[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
-  }
 }
 
 __global__ void quant_kernel(const void *__restrict__ src, void *__restrict__ dst, size_t rows, int w,
@@ -230,32 +227,49 @@ __global__ void quant_bf16_to_i8_vec_kernel(const uint4 *__restrict__ src, uint4
   }
 }
 
-// fp32 -> int8 at the graph input (kind 0) from an NHWC4 fp32 tensor (c <= 4) into an int8
-// tensor with channel pitch 4, 8 or 16 and optionally zero-padded rows: one thread per physical
-// destination pixel, one 16-byte load and one 8/16-byte store.
-__global__ void quant_input_pix_kernel(const float4 *__restrict__ src, void *__restrict__ dst, int n,
-                                       int h, int w, int c, int cpd, int wl, int wphys, float scale) {
+// The quantisation of an NHWC4 fp32 input image (c <= 4) into an INT8 or BF16 tensor with a pitch of 4, 8 or 16 channels and
+// optionally zero-padded rows: kind 0 (int8, round half away from zero) or 5 (BF16, the upper half of the word). One thread
+// per stored pixel, blocks over rows (no divisions), two rows in flight: one 16-byte read, one write of the pixel.
+template <bool BF16>
+__global__ void __launch_bounds__(256) quant_input_pix_kernel(const float4 *__restrict__ src, void *__restrict__ dst, int rows, int w,
+                                                              int c, int cpd, int wl, int wphys, float scale) {
   pdl_prologue();
-  const size_t total = (size_t)n * h * wphys;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-       i += (size_t)gridDim.x * blockDim.x) {
-    int x = (int)(i % wphys) - wl;
-    size_t row = i / wphys;
-    uint32_t lo = 0;
-    if (x >= 0 && x < w) {
-      float4 v = src[row * w + x];
-      float f[4] = {v.x, v.y, v.z, v.w};
+  auto put = [&](int row, int i, const float4 &v, bool real) {
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    uint32_t lo = 0, hi = 0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (k < c) {
-          float r = fminf(fmaxf(roundf(__fmul_rn(f[k], scale)), -128.0f), 127.0f);
-          lo |= ((uint32_t)((int)r & 0xff)) << (8 * k);
-        }
+    for (int k = 0; k < 4; ++k) {
+      if (!real || k >= c) continue;
+      if (BF16) {
+        const uint32_t h = __float_as_uint(f[k]) >> 16;
+        if (k < 2) lo |= h << (16 * k);
+        else hi |= h << (16 * k - 32);
+      } else {
+        const float r = fminf(fmaxf(roundf(__fmul_rn(f[k], scale)), -128.0f), 127.0f);
+        lo |= ((uint32_t)((int)r & 0xff)) << (8 * k);
       }
     }
-    if (cpd == 4) reinterpret_cast<uint32_t *>(dst)[i] = lo;
-    else if (cpd == 8) reinterpret_cast<uint2 *>(dst)[i] = make_uint2(lo, 0u);
-    else reinterpret_cast<uint4 *>(dst)[i] = make_uint4(lo, 0u, 0u, 0u);
+    const size_t at = (size_t)row * wphys + i;
+    const int bytes = cpd * (BF16 ? 2 : 1);
+    if (bytes == 4) reinterpret_cast<uint32_t *>(dst)[at] = lo;
+    else if (bytes == 8) reinterpret_cast<uint2 *>(dst)[at] = make_uint2(lo, hi);
+    else {
+      uint4 *o = reinterpret_cast<uint4 *>(dst) + at * (bytes / 16);
+      o[0] = make_uint4(lo, hi, 0u, 0u);
+      if (bytes == 32) o[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  for (int row = blockIdx.x; row < rows; row += 2 * gridDim.x) {
+    const int row2 = row + gridDim.x;
+    for (int i = threadIdx.x; i < wphys; i += blockDim.x) {
+      const int x = i - wl;
+      const bool real = x >= 0 && x < w;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+      if (real) a = __ldg(src + (size_t)row * w + x);
+      if (real && row2 < rows) b = __ldg(src + (size_t)row2 * w + x);
+      put(row, i, a, real);
+      if (row2 < rows) put(row2, i, b, real);
+    }
   }
 }
 
@@ -757,7 +771,6 @@ struct PatchArgs {
   int c_first, c_count; // channel slice (grouped convolution)
   int kp;
   int wl, wphys;        // physical row layout of the input
-  int cv = 0;           // 4: patch_expand_tap_kernel's layout, four channel slots per filter tap (k = tap * 4 + c)
 };
 __global__ void patch_expand_i8_kernel(const int8_t *__restrict__ in, int8_t *__restrict__ out,
                                        PatchArgs a) {
@@ -788,79 +801,33 @@ __global__ void patch_expand_i8_kernel(const int8_t *__restrict__ in, int8_t *__
   }
 }
 
-// The same expansion for 2-byte (BF16) and 4-byte (fp32) elements, one thread per 16-byte vector of the patch
-// matrix: few-channel BF16 / fp32 convolutions (3-channel stems) would otherwise run one 32-byte K step per filter
-// tap; the expanded matrix [M][kp] is a plain K-major operand with a handful of 128-byte K blocks.
+// Rows of a few-channel tensor copied into the window layout (WindowPlan): one block per row, one thread per pixel of the
+// stored row. Runs when the tensor itself could not be given that layout (several consumers, an fp32 input). With `lo` (fp32)
+// the remainder operand of the TF32 x 3 product, x - (upper 19 bits of x), is written beside it.
+struct RepackArgs {
+  const void *in;
+  void *out, *lo;
+  size_t rows; // n * h
+  int w, c, cps, in_wl, in_wphys;
+  int cpd, wl, wphys;
+  int es;
+};
 template <typename T>
-__global__ void patch_expand_kernel(const T *__restrict__ in, T *__restrict__ out, PatchArgs a) {
+__global__ void window_repack_kernel(RepackArgs a) {
   pdl_prologue();
-  constexpr int V = 16 / (int)sizeof(T);
-  const size_t total = (size_t)a.n * a.oh * a.ow * (a.kp / V);
-  const int kreal = a.kh * a.kw * a.c_count;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int kv = (int)(i % (a.kp / V));
-    const size_t pix = i / (a.kp / V);
-    const int x = (int)(pix % a.ow);
-    const size_t t = pix / a.ow;
-    const int y = (int)(t % a.oh);
-    const int b = (int)(t / a.oh);
-    T v[V];
-#pragma unroll
-    for (int j = 0; j < V; ++j) {
-      const int k = kv * V + j;
-      v[j] = (T)0;
-      if (k < kreal) {
-        const int c = k % a.c_count, tap = k / a.c_count;
-        const int s = tap % a.kw, r = tap / a.kw;
-        const int yy = y * a.sh - a.pt + r * a.dh, xx = x * a.sw - a.pl + s * a.dw;
-        if (yy >= 0 && yy < a.ih && xx >= 0 && xx < a.iw)
-          v[j] = in[(((size_t)b * a.ih + yy) * a.wphys + a.wl + xx) * a.cp + a.c_first + c];
-      }
-    }
-    reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(v);
-  }
-}
-
-// At most 4 input channels (image stems): every filter tap keeps four channel slots in the patch matrix,
-// k = tap * 4 + c, so a thread copies one tap of one output pixel as ONE vector (16 bytes of fp32, 8 bytes of BF16)
-// without any per-element index arithmetic. With `lo` (fp32) the remainder part of the TF32 x 3 product,
-// x - (upper 19 bits of x), is written beside it, which saves the separate split pass over the matrix.
-template <typename T>
-__global__ void patch_expand_tap_kernel(const T *__restrict__ in, T *__restrict__ out, T *__restrict__ lo, PatchArgs a) {
-  pdl_prologue();
-  const int taps = a.kh * a.kw;
-  const int slots = a.kp / 4; // vectors per row, the last ones are padding
-  const size_t total = (size_t)a.n * a.oh * a.ow * slots;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int tap = (int)(i % slots);
-    const size_t pix = i / slots;
-    const int x = (int)(pix % a.ow);
-    const size_t t = pix / a.ow;
-    const int y = (int)(t % a.oh);
-    const int b = (int)(t / a.oh);
-    T v[4] = {(T)0, (T)0, (T)0, (T)0};
-    if (tap < taps) {
-      const int s = tap % a.kw, r = tap / a.kw;
-      const int yy = y * a.sh - a.pt + r * a.dh, xx = x * a.sw - a.pl + s * a.dw;
-      if (yy >= 0 && yy < a.ih && xx >= 0 && xx < a.iw) {
-        const T *src = in + (((size_t)b * a.ih + yy) * a.wphys + a.wl + xx) * a.cp;
-        if (sizeof(T) == 4) *reinterpret_cast<uint4 *>(v) = __ldg(reinterpret_cast<const uint4 *>(src));
-        else *reinterpret_cast<uint2 *>(v) = __ldg(reinterpret_cast<const uint2 *>(src));
-      }
-    }
-    if (sizeof(T) == 4) {
-      reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(v);
-      if (lo) {
-        float l[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float f = reinterpret_cast<const float *>(v)[j];
-          l[j] = __fsub_rn(f, __uint_as_float(__float_as_uint(f) & 0xffffe000u));
+  for (size_t row = blockIdx.x; row < a.rows; row += gridDim.x) {
+    const T *src = reinterpret_cast<const T *>(a.in) + (row * a.in_wphys + a.in_wl) * a.cps;
+    for (int i = threadIdx.x; i < a.wphys; i += blockDim.x) {
+      const int x = i - a.wl;
+      const size_t at = (row * a.wphys + i) * a.cpd;
+      for (int k = 0; k < a.cpd; ++k) {
+        const T v = (x >= 0 && x < a.w && k < a.c) ? src[(size_t)x * a.cps + k] : (T)0;
+        reinterpret_cast<T *>(a.out)[at + k] = v;
+        if (sizeof(T) == 4 && a.lo) {
+          const float f = __uint_as_float((uint32_t)v);
+          reinterpret_cast<float *>(a.lo)[at + k] = __fsub_rn(f, __uint_as_float((uint32_t)v & 0xffffe000u));
         }
-        reinterpret_cast<uint4 *>(lo)[i] = *reinterpret_cast<const uint4 *>(l);
       }
-    } else {
-      reinterpret_cast<uint2 *>(out)[i] = *reinterpret_cast<const uint2 *>(v);
     }
   }
 }
