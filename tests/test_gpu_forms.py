@@ -77,3 +77,32 @@ def test_row_window_conv_float(dtype, case):
         assert np.all(np.abs(got - ref) <= np.maximum(np.abs(ref) * 2.0 ** -7, 2.0 ** -8 * np.abs(ref).max() * 2.0 ** -6))
     else:
         assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dtype", ["INT8", "BF16", "FP32"])
+@pytest.mark.parametrize("case", [
+    # n, ic, oc, hw, k, stride, pad, dilation
+    (3, 64, 64, 14, 3, 1, 1, 1),    # pixel pairs, steps of K skipped at both ends
+    (2, 32, 32, 10, 5, 1, 2, 1), (1, 48, 24, 12, 3, 1, 0, 1), (2, 64, 48, 12, 3, 1, 2, 2),  # pairs: other filters, pads
+    (2, 16, 16, 20, 1, 1, 0, 1), (3, 96, 40, 6, 1, 1, 0, 1),  # pairs twice; pairs of a 1x1 with a long K
+    (5, 128, 96, 7, 3, 1, 1, 1),    # several images per tile
+    (2, 40, 136, 13, 3, 1, 2, 2), (1, 64, 130, 31, 3, 1, 1, 1), (1, 72, 80, 57, 5, 1, 1, 1),  # odd extents, ragged tiles
+    (1, 512, 64, 9, 3, 1, 1, 1), (1, 256, 200, 5, 1, 1, 0, 1),  # few tiles and a long K
+    (2, 64, 96, 11, 3, 2, 1, 1)])   # a stride
+def test_conv_forms(dtype, case):
+    n, ic, oc, hw, k, s, p, d = case
+    if dtype == "INT8":
+        model = graphs.single_conv_i8(n, ic, oc, hw, k, s, p, d, seed=5200 + ic + k)
+        got, ref = run_model(model.text, model.weights, {"x": model.meta["x"]}, ["conv"])["conv"]
+        assert np.array_equal(got, ref)
+        return
+    rng = np.random.default_rng(43 + ic + k)
+    cut = graphs._bf16_np if dtype == "BF16" else (lambda v: np.asarray(v, np.float32))
+    w = {"f": cut(rng.normal(0, (2.0 / (ic * k * k)) ** 0.5, (oc, ic, k, k))), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+    x = cut(rng.normal(0, 1, (n, ic, hw, hw)))
+    text = "input name=x shape=%d,%d,%d,%d dtype=%s\n" % (n, ic, hw, hw, dtype) + conv_text(dtype, n, ic, oc, hw, k, s, p, d, 1)
+    got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
+    if dtype == "BF16":
+        assert np.all(np.abs(got - ref) <= np.maximum(np.abs(ref) * 2.0 ** -7, 2.0 ** -14 * np.abs(ref).max()))
+    else:
+        assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()

@@ -252,7 +252,6 @@ public:
   bool fuse_residual_add = false; // set before load_module: eltwise adds run in the producing convolution's epilogue
   bool fp32_tensor_cores = true; // set before load_module: fp32 convolutions as three TF32 products
   void fuse_activation_chains(const std::map<std::string, int> &uses);
-  void link_tf32_remainders();
   cudaGraphExec_t graph_exec = nullptr;
   std::map<std::string, HostWeight> weights;
   std::map<std::string, TensorPtr> tensors;
@@ -482,121 +481,18 @@ public:
       const bool window = window_plan_for(g, 2, out->cp, &wp);
       TPUCB_CHECK(window || (g.pl <= 127 && g.pt <= 127 && (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255),
                   "conv %s: BF16 convolution supports dense, ungrouped layers", op.name.c_str());
-      conv_kernel_setup_once();
-      std::vector<int32_t> bias_bits(out->cp, 0);
-      for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
-      d_bias_ = I.upload(bias_bits);
-      act_ = do_relu_ ? 1 : 0;
-      ConvPlan pl;
-      std::memset(&pl.p, 0, sizeof(pl.p));
-      pl.bf16 = true;
-      pl.in = (const int8_t *)in->dev;
-      ConvGemmParams &p = pl.p;
-      p.OH = g.oh; p.OW = g.ow; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
-      p.act = act_;
-      p.bias = d_bias_; p.mult = d_bias_; p.rshift = d_bias_;
-      p.out = (int8_t *)out->dev;
-      p.ldc = out->cp * 2; // bytes
-      p.c_off = 0;
-      p.err = &I.ss.d_err->code;
-      const int rows = g.n * g.oh * g.ow;
-      const int k_bytes = in->cp * 2;
-      const bool one_by_one_bf = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
-      if (window) { // few input channels (3-channel stems)
-        setup_window(I, pl, wp, filt, -1);
-        return;
-      }
-      const int8_t *d_w = I.upload(pack_conv_weights_bf16(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, in->cp));
-      if (one_by_one_bf) {
-        p.kh = p.kw = 1;
-        p.a_mode = 0;
-        finish_plan(pl, rows, 1, k_bytes, out->cp, I.sm_count);
-        encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_w, out->cp, 1, k_bytes, p.BK, p.dual ? 192 : p.BN);
-      } else {
-        p.kh = g.kh; p.kw = g.kw;
-        p.a_mode = 1;
-        finish_plan(pl, rows, g.kh * g.kw, k_bytes, out->cp, I.sm_count);
-        encode_im2col_map(&pl.tmA, (const int8_t *)in->dev, g, k_bytes, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_w, out->cp, g.kh * g.kw, k_bytes, p.BK, p.dual ? 192 : p.BN);
-      }
-      p.idesc = make_idesc_bf16(128, p.BN);
-      pl.ops = alg_ops;
-      I.attach_split_ws(pl);
-      plans_.push_back(pl);
-      alg_bytes = 2.0 * ((double)in->numel() + out->numel() + filt.data.size()) + 4.0 * g.oc;
+      setup_tensor_core(I, 1, filt.data, bias, {}, {}, window ? &wp : nullptr);
       return;
     }
     if (out->dtype == DT_F32) {
       TPUCB_CHECK(in->dtype == DT_F32, "conv %s: an fp32 convolution needs an fp32 input", op.name.c_str());
       WindowPlan wp;
-      if (I.fp32_tensor_cores && window_plan_for(g, 4, out->cp, &wp)) { // image stems
-        conv_kernel_setup_once();
-        std::vector<int32_t> bias_bits(out->cp, 0);
-        for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
-        d_bias_ = I.upload(bias_bits);
-        act_ = do_relu_ ? 1 : 0;
-        ConvPlan pl;
-        std::memset(&pl.p, 0, sizeof(pl.p));
-        pl.tf32 = true;
-        pl.p.act = act_;
-        pl.p.bias = d_bias_; pl.p.mult = d_bias_; pl.p.rshift = d_bias_;
-        pl.p.err = &I.ss.d_err->code;
-        setup_window(I, pl, wp, filt, 0);
-        return;
-      }
-      if (I.fp32_tensor_cores && g.g == 1 && !g.ins_h && !g.ins_w && in->cp % 8 == 0 &&
-          g.pl <= 127 && g.pt <= 127 && (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255) {
-        // fp32 convolution on the tensor cores as three TF32 products with fp32 accumulation (x w = xh wh + xl wh +
-        // xh wl, 2^-22 relative: inside the 1e-4 of the fp32 path, where a single TF32 product would not be). The
-        // activations are split into their two parts by a vector kernel right before the launch; the weights once, here.
-        conv_kernel_setup_once();
-        std::vector<int32_t> bias_bits(out->cp, 0);
-        for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
-        d_bias_ = I.upload(bias_bits);
-        act_ = do_relu_ ? 1 : 0;
-        ConvPlan pl;
-        std::memset(&pl.p, 0, sizeof(pl.p));
-        pl.tf32 = true;
-        pl.in = (const int8_t *)in->dev;
-        pl.split_src = (const float *)in->dev;
-        // The tensor core ignores the low 13 mantissa bits of an fp32 operand (measured: results are bit-identical with
-        // the upper part materialised or not), so the tensor itself serves as xh and only xl is written.
-        pl.split_hi = nullptr;
-        if (!in->lo_dev) in->lo_dev = I.dalloc(in->bytes()); // shared by every convolution that reads this tensor
-        pl.split_lo = (float *)in->lo_dev;
-        pl.split_nvec = in->bytes() / 16;
-        ConvGemmParams &p = pl.p;
-        p.OH = g.oh; p.OW = g.ow; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
-        p.act = act_;
-        p.bias = d_bias_; p.mult = d_bias_; p.rshift = d_bias_;
-        p.out = (int8_t *)out->dev;
-        p.ldc = out->cp * 4; // bytes
-        p.c_off = 0;
-        p.err = &I.ss.d_err->code;
-        const int rows = g.n * g.oh * g.ow;
-        const int k_bytes = in->cp * 4;
-        const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
-        const int8_t *d_wh = I.upload(pack_conv_weights_tf32(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, in->cp, 0));
-        const int8_t *d_wl = I.upload(pack_conv_weights_tf32(filt.data.data(), g.oc, g.ic, g.kh, g.kw, out->cp, in->cp, 1));
-        const int taps = one ? 1 : g.kh * g.kw;
-        p.kh = one ? 1 : g.kh; p.kw = one ? 1 : g.kw;
-        p.a_mode = one ? 0 : 1;
-        finish_plan(pl, rows, taps, k_bytes, out->cp, I.sm_count);
-        if (one) {
-          encode_matrix_map(&pl.tmA, pl.split_hi ? (const int8_t *)pl.split_hi : (const int8_t *)in->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-          encode_matrix_map(&pl.tmA2, (const int8_t *)pl.split_lo, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-        } else {
-          encode_im2col_map(&pl.tmA, pl.split_hi ? (const int8_t *)pl.split_hi : (const int8_t *)in->dev, g, k_bytes, p.BK, a_tile_rows(p));
-          encode_im2col_map(&pl.tmA2, (const int8_t *)pl.split_lo, g, k_bytes, p.BK, a_tile_rows(p));
-        }
-        encode_weight_map(&pl.tmB, d_wh, out->cp, taps, k_bytes, p.BK, p.BN);
-        encode_weight_map(&pl.tmB2, d_wl, out->cp, taps, k_bytes, p.BK, p.BN);
-        p.idesc = make_idesc_tf32(128, p.BN);
-        pl.ops = alg_ops;
-        I.attach_split_ws(pl);
-        plans_.push_back(pl);
-        alg_bytes = 4.0 * ((double)in->numel() + out->numel() + filt.data.size() + g.oc);
+      const bool window = window_plan_for(g, 4, out->cp, &wp); // image stems
+      // fp32 convolution on the tensor cores as three TF32 products with fp32 accumulation (x w = xh wh + xl wh + xh wl,
+      // 2^-22 relative: inside the 1e-4 of the fp32 path, where a single TF32 product would not be)
+      if (I.fp32_tensor_cores && (window || (g.g == 1 && !g.ins_h && !g.ins_w && in->cp % 8 == 0 && g.pl <= 127 && g.pt <= 127 &&
+                                             (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255))) {
+        setup_tensor_core(I, 2, filt.data, bias, {}, {}, window ? &wp : nullptr);
         return;
       }
       f32_ = true;
@@ -610,14 +506,24 @@ public:
                 "conv %s: INT8 convolution needs rshift and multiplier operands (RSHIFT_AND_M_I32)", op.name.c_str());
     const int oc_pad = out->cp;
     check_q31_multipliers(I.weight(op.in[6]).data, op.name);
-    d_bias_ = I.upload(to_i32(bias, oc_pad));
-    d_mult_ = I.upload(to_i32(I.weight(op.in[6]).data, oc_pad, true));
-    d_rsh_ = I.upload(to_i32(I.weight(op.in[5]).data, oc_pad, true));
+    const auto &mult = I.weight(op.in[6]).data, &rshift = I.weight(op.in[5]).data;
     alg_bytes = (double)in->numel() + out->numel() + filt.data.size() + 12.0 * g.oc;
     act_ = do_relu_ ? 1 : 0;
-    const int fastq = requant_fast_flags(I.weight(op.in[5]).data, bias, (long long)(g.ic / g.g) * g.kh * g.kw);
-
-    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, I.weight(op.in[6]).data, I.weight(op.in[5]).data, do_relu_ != 0, oc_pad);
+    const int fastq = requant_fast_flags(rshift, bias, (long long)(g.ic / g.g) * g.kh * g.kw);
+    WindowPlan wp;
+    const bool window = window_plan_for(g, 1, oc_pad, &wp); // few input channels (3-channel stems)
+    const bool one_by_one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 &&
+                            g.oh == g.ih && g.ow == g.iw;
+    const bool need_patch = g.g > 1 || g.ins_h || g.ins_w || (g.ic < 16 && !one_by_one) || in->padded_rows() || in->cp % 16 != 0 ||
+                            g.pl > 127 || g.pt > 127 || (g.kw - 1) * g.dw > 255 || (g.kh - 1) * g.dh > 255;
+    if (window || !need_patch) {
+      setup_tensor_core(I, 0, filt.data, bias, mult, rshift, window ? &wp : nullptr);
+      return;
+    }
+    d_bias_ = I.upload(to_i32(bias, oc_pad));
+    d_mult_ = I.upload(to_i32(mult, oc_pad, true));
+    d_rsh_ = I.upload(to_i32(rshift, oc_pad, true));
+    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, mult, rshift, do_relu_ != 0, oc_pad);
     const FloatRequant *d_fq = fq.empty() ? nullptr : I.upload(fq);
 
     if (g.g == g.ic && g.g == g.oc && g.g > 1 && g.ins_h == 0 && g.ins_w == 0) {
@@ -649,27 +555,7 @@ public:
       return;
     }
 
-    {
-      WindowPlan wp;
-      if (window_plan_for(g, 1, oc_pad, &wp)) { // few input channels (3-channel stems)
-        conv_kernel_setup_once();
-        ConvPlan pl;
-        std::memset(&pl.p, 0, sizeof(pl.p));
-        pl.p.act = act_;
-        pl.p.fastq = fastq;
-        pl.p.bias = d_bias_; pl.p.mult = d_mult_; pl.p.rshift = d_rsh_;
-        pl.p.fq = d_fq;
-        pl.p.err = &I.ss.d_err->code;
-        setup_window(I, pl, wp, filt, -2);
-        return;
-      }
-    }
-    conv_kernel_setup_once();
-    const bool one_by_one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 &&
-                            g.oh == g.ih && g.ow == g.iw;
-    const bool small_c = g.ic < 16;
-    const bool need_patch = (g.g > 1 || g.ins_h || g.ins_w || (small_c && !one_by_one) || in->padded_rows() || in->cp % 16 != 0 ||
-                            g.pl > 127 || g.pt > 127 || (g.kw - 1) * g.dw > 255 || (g.kh - 1) * g.dh > 255);
+    conv_kernel_setup_once(); // grouped layers, input insertion: one launch per group over an expanded patch matrix
     const int groups = g.g;
     for (int grp = 0; grp < groups; ++grp) {
       ConvPlan pl;
@@ -690,7 +576,7 @@ public:
       int ocg_pad = groups == 1 ? oc_pad : ocg;
       TPUCB_CHECK(groups == 1 || ocg % 16 == 0, "conv %s: grouped convolution needs oc/g to be a multiple of 16",
                   op.name.c_str());
-      if (need_patch) {
+      {
         pl.use_patch = true;
         PatchArgs &a = pl.patch;
         a.n = g.n; a.c = g.ic; a.cp = in->cp; a.ih = g.ih; a.iw = g.iw; a.oh = g.oh; a.ow = g.ow;
@@ -708,22 +594,6 @@ public:
         finish_plan(pl, rows, 1, a.kp, ocg_pad, I.sm_count);
         encode_matrix_map(&pl.tmA, pl.patch_buf, rows, a.kp, a.kp, p.BK, a_tile_rows(p));
         encode_weight_map(&pl.tmB, d_w, ocg_pad, 1, a.kp, p.BK, p.dual ? 192 : p.BN);
-      } else if (one_by_one) {
-        auto w = pack_conv_weights(wsrc, ocg, icg, 1, 1, ocg_pad, in->cp, false, 0);
-        const int8_t *d_w = I.upload(w);
-        p.kh = p.kw = 1;
-        p.a_mode = 0;
-        finish_plan(pl, rows, 1, in->cp, ocg_pad, I.sm_count);
-        encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, rows, in->cp, in->cp, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_w, ocg_pad, 1, in->cp, p.BK, p.dual ? 192 : p.BN);
-      } else {
-        auto w = pack_conv_weights(wsrc, ocg, icg, g.kh, g.kw, ocg_pad, in->cp, false, 0);
-        const int8_t *d_w = I.upload(w);
-        p.kh = g.kh; p.kw = g.kw;
-        p.a_mode = 1;
-        finish_plan(pl, rows, g.kh * g.kw, in->cp, ocg_pad, I.sm_count);
-        encode_im2col_map(&pl.tmA, (const int8_t *)in->dev, g, in->cp, p.BK, a_tile_rows(p));
-        encode_weight_map(&pl.tmB, d_w, ocg_pad, g.kh * g.kw, in->cp, p.BK, p.dual ? 192 : p.BN);
       }
       if (I.selftest_lost_arrival > 0) {
         pl.p.wait_rounds = I.selftest_lost_arrival;
@@ -733,53 +603,146 @@ public:
       plans_.push_back(pl);
     }
   }
-  // The row-window form (WindowPlan) of the layer. The input tensor has the window layout when it was asked for at load
-  // and granted; else (and always for fp32, whose remainder operand has to be made anyway) a copy of its rows is made
-  // before the launch. part: as in pack_window_weights (0: TF32, both parts)
-  void setup_window(Interpreter &I, ConvPlan &pl, const WindowPlan &wp, const HostWeight &filt, int part) {
-    const ConvGeom &g = g_;
-    const int es = part == -2 ? 1 : (part == -1 ? 2 : 4);
+  // Ungrouped layers on the tensor cores. kind: 0 INT8, 1 BF16, 2 fp32 as three TF32 products. Three forms: row windows
+  // (wp), tap blocks (fp32 only), K blocks of a matrix or im2col map. fp32 runs on conv_tf32x3.cuh, the others on
+  // conv_gemm_i8.cuh.
+  void setup_tensor_core(Interpreter &I, int kind, const std::vector<float> &filt, const std::vector<float> &bias,
+                         const std::vector<float> &mult, const std::vector<float> &rshift, const WindowPlan *wp) {
+    conv_kernel_setup_once();
+    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4);
+    act_ = do_relu_ ? 1 : 0;
+    alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.size()) + (kind == 0 ? 12.0 : 4.0) * g_.oc;
+    DenseLayer d;
+    d.g = g_; d.in_cp = in_->cp; d.out_cp = out_->cp;
+    d.w = filt; d.bias = bias; d.mult = mult; d.rshift = rshift;
+    // (1x1 layers of 16 or 32 channels twice)
+    while (!wp && pair_applies(d.g, d.in_cp, d.out_cp, es) && (g_.kw == 1 || !d.paired)) pair_layer(d);
+    const ConvGeom &g = d.g;
+    ConvPlan pl;
+    std::memset(&pl.p, 0, sizeof(pl.p));
+    pl.bf16 = kind == 1;
+    pl.tf32 = kind == 2;
+    pl.in = (const int8_t *)in_->dev;
+    pl.ops = alg_ops;
     ConvGemmParams &p = pl.p;
-    const void *rows = in_->dev, *rows_lo = nullptr;
-    if (part == 0 || in_->cp * es != wp.P || in_->wl != g.pl || in_->wphys != wp.wphys) {
-      const size_t bytes = (size_t)g.n * g.ih * wp.wphys * wp.P;
+    p.act = act_;
+    p.err = &I.ss.d_err->code;
+    p.out = (int8_t *)out_->dev;
+    p.ldc = d.out_cp * es;
+    if (kind == 0) {
+      p.fastq = requant_fast_flags(rshift, bias, (long long)g_.ic * g_.kh * g_.kw);
+      p.bias = I.upload(to_i32(d.bias, d.out_cp));
+      p.mult = I.upload(to_i32(d.mult, d.out_cp, true));
+      p.rshift = I.upload(to_i32(d.rshift, d.out_cp, true));
+      const std::vector<FloatRequant> fq = float_requant(d.w, d.bias, d.mult, d.rshift, do_relu_ != 0, d.out_cp);
+      if (!fq.empty()) p.fq = I.upload(fq);
+      if (I.selftest_lost_arrival > 0) {
+        p.wait_rounds = I.selftest_lost_arrival;
+        p.lose_arrival = 1;
+      }
+    } else {
+      std::vector<int32_t> bias_bits(d.out_cp, 0);
+      for (size_t o = 0; o < d.bias.size(); ++o) bias_bits[o] = (int32_t)f32_bits(d.bias[o]);
+      p.bias = p.mult = p.rshift = I.upload(bias_bits);
+    }
+    p.OH = g.oh; p.OW = g.ow; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
+    p.kh = g.kh; p.kw = g.kw;
+    if (wp) setup_window(I, pl, *wp, filt, kind);
+    else setup_blocks(I, pl, d, kind);
+    if (kind == 2 && pl.q.parts > 1) { // partial sums to a workspace, bias and activation in the reducing pass
+      pl.reduce_out = (float *)p.out;
+      pl.reduce_bias = (const float *)p.bias;
+      pl.reduce_bytes = out_->bytes();
+      pl.reduce_act = p.act;
+      pl.q.part_bytes = out_->bytes();
+      p.out = (int8_t *)I.dalloc(out_->bytes() * pl.q.parts);
+      p.act = 0;
+      p.bias = I.upload(std::vector<int32_t>(d.out_cp, 0));
+    }
+    I.attach_split_ws(pl);
+    plans_.push_back(pl);
+  }
+  // The row-window form (WindowPlan). The input tensor has the window layout when it was asked for at load and granted;
+  // else a copy of its rows is made before the launch.
+  void setup_window(Interpreter &I, ConvPlan &pl, const WindowPlan &wp, const std::vector<float> &filt, int kind) {
+    const ConvGeom &g = g_;
+    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4);
+    ConvGemmParams &p = pl.p;
+    const void *rows = in_->dev;
+    if (in_->cp * es != wp.P || in_->wl != g.pl || in_->wphys != wp.wphys) {
       pl.use_repack = true;
       RepackArgs &a = pl.repack;
       a.in = in_->dev;
-      a.out = I.dalloc(bytes);
-      a.lo = part == 0 ? I.dalloc(bytes) : nullptr;
+      a.out = I.dalloc((size_t)g.n * g.ih * wp.wphys * wp.P);
       a.rows = (size_t)g.n * g.ih;
       a.w = g.iw; a.c = g.ic; a.cps = in_->cp; a.in_wl = in_->wl; a.in_wphys = in_->wphys;
       a.cpd = wp.P / es; a.wl = g.pl; a.wphys = wp.wphys; a.es = es;
       rows = a.out;
-      rows_lo = a.lo;
     }
-    p.OH = g.oh; p.OW = g.ow / wp.G; p.sh = g.sh; p.sw = 1; p.pt = g.pt; p.pl = 0; p.dh = g.dh; p.dw = 0;
-    p.kh = g.kh; p.kw = 1;
+    p.OW = g.ow / wp.G; p.sw = 1; p.pl = 0; p.dw = 0;
+    p.kw = 1;
     p.a_mode = 1;
-    p.out = (int8_t *)out_->dev;
-    p.c_off = 0;
     p.group = wp.G;
-    p.ldc_px = out_->cp * es;
-    p.ldc = p.ldc_px * wp.G;
+    p.ldc_px = p.ldc;
+    p.ldc *= wp.G;
     finish_plan(pl, g.n * g.oh * p.OW, g.kh, wp.win, out_->cp, I.sm_count);
-    const int w_rows = wp.G > 1 ? 128 : out_->cp;
-    auto weights = [&](CUtensorMap *tm, int pt) {
-      encode_weight_map(tm, I.upload(pack_window_weights(filt.data.data(), g, wp, w_rows, p.BK, pt)), w_rows, g.kh, p.BK, p.BK,
-                        p.dual ? 192 : p.BN);
-    };
-    encode_window_map(&pl.tmA, rows, g, wp, p.BK, a_tile_rows(p));
-    weights(&pl.tmB, part);
-    if (part == 0) {
-      encode_window_map(&pl.tmA2, rows_lo, g, wp, p.BK, a_tile_rows(p));
-      weights(&pl.tmB2, 1);
+    const int w_rows = wp.G > 1 ? 128 : out_->cp, n_tiles = (out_->cp + 127) / 128;
+    if (kind == 2) {
+      finish_tf32_plan(pl, plain_tap_tiles(p, 1, p.M_total), n_tiles, I.sm_count);
+    } else if (kind == 1) {
+      p.idesc = make_idesc_bf16(128, p.BN);
     }
-    if (part == 0) p.idesc = make_idesc_tf32(128, p.BN);
-    else if (part == -1) p.idesc = make_idesc_bf16(128, p.BN);
-    pl.ops = alg_ops;
-    I.attach_split_ws(pl);
-    plans_.push_back(pl);
-    alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.data.size()) + (part == -2 ? 12.0 : 4.0) * g.oc;
+    auto weights = [&](CUtensorMap *tm, int part) {
+      encode_weight_map(tm, I.upload(pack_window_weights(filt.data(), g, wp, w_rows, p.BK, part)), w_rows, g.kh, p.BK, p.BK,
+                        p.dual ? 192 : 128);
+    };
+    weights(&pl.tmB, kind == 0 ? -2 : (kind == 1 ? -1 : 0));
+    if (kind == 2) weights(&pl.tmB2, 1);
+    encode_window_map(&pl.tmA, rows, g, wp, p.BK, a_tile_rows(p));
+  }
+  void setup_blocks(Interpreter &I, ConvPlan &pl, const DenseLayer &d, int kind) {
+    const ConvGeom &g = d.g;
+    ConvGemmParams &p = pl.p;
+    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4), k_bytes = d.in_cp * es, rows = g.n * g.oh * g.ow;
+    const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.oh == g.ih && g.ow == g.iw;
+    const int taps = g.kh * g.kw, n_tiles = (d.out_cp + 127) / 128;
+    p.a_mode = one ? 0 : 1;
+    finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count);
+    if (kind == 2) {
+      const int all = (k_bytes + 31) / 32;
+      TapParams q = plain_tap_tiles(p, one ? 0 : 1, rows), t;
+      double t_clocks = 0;
+      int skip = 0, keep = 1 << 20; // steps of K that tap blocks skip
+      if (d.paired && k_bytes % 64 == 0) {
+        if (g_.pl % 2) skip = all / 2;
+        if ((1 + (g_.kw - 1) * g_.dw - g_.pl) % 2 == 0) keep = all / 2;
+      }
+      const double steps = (double)g.kh * (g.kw * all - skip - std::max(all - keep, 0));
+      if (taps > 1 && choose_tap_tile(g, k_bytes, n_tiles, steps, I.sm_count, &t, &t_clocks) &&
+          t_clocks < tf32_clocks(q, 1, p.BK, (double)taps * all, n_tiles, I.sm_count)) {
+        q = t;
+        q.skip_first = skip;
+        q.keep_last = keep;
+      }
+      finish_tf32_plan(pl, q, n_tiles, I.sm_count);
+      if (q.mode == 2) encode_block_map(&pl.tmA, in_->dev, g, k_bytes, p.BK, q);
+    } else if (kind == 1) {
+      p.idesc = make_idesc_bf16(128, p.BN);
+    }
+    if (pl.q.mode != 2) {
+      if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
+      else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, a_tile_rows(p));
+    }
+    auto weights = [&](CUtensorMap *tm, const std::vector<int8_t> &w) {
+      encode_weight_map(tm, I.upload(w), d.out_cp, taps, k_bytes, p.BK, p.dual ? 192 : 128);
+    };
+    const float *w = d.w.data();
+    if (kind == 0) weights(&pl.tmB, pack_conv_weights(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, false, 0));
+    else if (kind == 1) weights(&pl.tmB, pack_conv_weights_bf16(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp));
+    else {
+      weights(&pl.tmB, pack_conv_weights_tf32(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, 0));
+      weights(&pl.tmB2, pack_conv_weights_tf32(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, 1));
+    }
   }
   // Fused leaky ReLU (tensor-core plans only): the epilogue writes the plain result to this op's tensor
   // and the activation result to `act_out`.
@@ -811,15 +774,6 @@ public:
   }
   const TensorPtr &out() const { return out_; }
   const TensorPtr &in() const { return in_; }
-  // TF32 x 3 plans (not the row-window stem, whose remainder belongs to its own copy of the rows)
-  bool is_tf32() const { return !plans_.empty() && plans_[0].tf32 && !plans_[0].use_repack; }
-  bool can_write_remainder() const { return !plans_.empty() && plans_[0].tf32; }
-  void set_remainder_out(void *lo) {
-    for (auto &pl : plans_) pl.p.out2 = (int8_t *)lo;
-  }
-  void skip_split() {
-    for (auto &pl : plans_) pl.split_src = nullptr;
-  }
   void invoke(cudaStream_t s) override {
     if (bf16g_) {
       ConvBf16GroupArgs a{g_.n, g_.ic, in_->cp, g_.ih, g_.iw, g_.oc, out_->cp, g_.oh, g_.ow, g_.kh, g_.kw, g_.sh, g_.sw,
@@ -862,7 +816,7 @@ public:
   int kernel_launches() const override {
     if (f32_ || dw_ || bf16g_) return 1;
     int k = 0;
-    for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack ? 1 : 0) + ((pl.tf32 && pl.split_src) ? 1 : 0);
+    for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack ? 1 : 0) + (pl.q.parts > 1 ? 1 : 0);
     return k;
   }
   bool is_tensor_core() const { return !f32_ && !dw_ && !bf16g_; }
@@ -1140,7 +1094,6 @@ public:
     } else {
       TPUCB_CHECK(out->dtype == DT_F32 && !is_mul, "eltwise %s: fp32 supports add only", op.name.c_str());
       f_.nin = nin;
-      f_.lo = nullptr;
       f_.do_relu = do_relu_;
       for (int i = 0; i < nin; ++i) {
         f_.in[i] = (const float *)ins[i]->dev;
@@ -1154,9 +1107,6 @@ public:
   const std::vector<TensorPtr> &inputs() const { return ins_; }
   const TensorPtr &out() const { return out_; }
   const EltwiseArgs &i8_args() const { return a_; }
-  // fp32 add whose result feeds a TF32 x 3 convolution: also write that convolution's remainder operand
-  bool can_write_remainder() const { return out_->dtype == DT_F32 && !is_mul_; }
-  void set_remainder_out(float *lo) { f_.lo = lo; }
   static void parse_coeff(const ParsedOp &op, float *coeff, int nin) {
     std::string co = op.gets("coeff", "");
     if (co.empty()) return;
@@ -1814,38 +1764,6 @@ inline ParsedOp parse_line(const std::string &line) {
 
 // Replaces every quant(INT8->BF16) -> slope-table activation -> quant(BF16->INT8) chain whose
 // intermediates feed nothing else by one ActChainOp at the first op's position.
-// Who writes the remainder operand (x minus the upper 19 bits of x) of the fp32 tensors that TF32 x 3 convolutions read:
-// the kernel that produces the tensor when it can (an fp32 eltwise add or another TF32 x 3 convolution: 4 more bytes
-// written per value, no separate pass), else the split pass of the FIRST convolution that reads it; later readers of
-// the same tensor reuse the buffer. Ops run in program order, so the first reader always runs before the others.
-inline void Interpreter::link_tf32_remainders() {
-  for (auto &k : kernels) {
-    auto *cv = dynamic_cast<Conv2DOp *>(k.get());
-    if (!cv || !cv->is_tf32()) continue;
-    DevTensor *t = cv->in().get();
-    if (t->lo_by != 0) { // already filled by the producer or by an earlier reader
-      cv->skip_split();
-      continue;
-    }
-    OpKernel *prod = nullptr;
-    for (auto &q : kernels)
-      if (q->result.get() == t) prod = q.get();
-    if (auto *pe = dynamic_cast<EltwiseOp *>(prod)) {
-      if (pe->can_write_remainder()) {
-        pe->set_remainder_out((float *)t->lo_dev);
-        t->lo_by = 1;
-      }
-    } else if (auto *pc = dynamic_cast<Conv2DOp *>(prod)) {
-      if (pc->can_write_remainder()) {
-        pc->set_remainder_out(t->lo_dev);
-        t->lo_by = 1;
-      }
-    }
-    if (t->lo_by == 1) cv->skip_split();
-    else t->lo_by = 2; // this convolution's split pass fills it
-  }
-}
-
 inline void Interpreter::fuse_activation_chains(const std::map<std::string, int> &uses) {
   auto single_use = [&](const std::string &nm) {
     auto it = uses.find(nm);
@@ -2122,7 +2040,6 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
 
 inline void Interpreter::finish_module() {
   if (fuse_activations) fuse_activation_chains(uses);
-  link_tf32_remainders();
   output_details.clear();
   for (auto &k : kernels)
     if (!uses.count(k->name) && k->op_type != "input") output_details.push_back({k->name, k->result->numel() / (size_t)max_batch});

@@ -368,7 +368,6 @@ struct EltwiseF32Args {
   float coeff[4];
   int nin;
   int do_relu;
-  float *lo; // when set: also write x - (upper 19 bits of x), the remainder operand of a TF32 x 3 convolution that reads x
 };
 // One 16-byte vector per thread and step (fp32 tensors are a whole number of them: the channel pitch is a
 // multiple of 4); operand by operand, product and sum rounded separately, as the reference's loop.
@@ -393,14 +392,6 @@ __global__ void eltwise_add_f32_kernel(EltwiseF32Args a, float *__restrict__ out
       acc.w = acc.w < 0 ? 0.0f : acc.w;
     }
     reinterpret_cast<float4 *>(out)[i] = acc;
-    if (a.lo) {
-      float4 l;
-      l.x = __fsub_rn(acc.x, __uint_as_float(__float_as_uint(acc.x) & 0xffffe000u));
-      l.y = __fsub_rn(acc.y, __uint_as_float(__float_as_uint(acc.y) & 0xffffe000u));
-      l.z = __fsub_rn(acc.z, __uint_as_float(__float_as_uint(acc.z) & 0xffffe000u));
-      l.w = __fsub_rn(acc.w, __uint_as_float(__float_as_uint(acc.w) & 0xffffe000u));
-      reinterpret_cast<float4 *>(a.lo)[i] = l;
-    }
   }
 }
 
@@ -802,11 +793,10 @@ __global__ void patch_expand_i8_kernel(const int8_t *__restrict__ in, int8_t *__
 }
 
 // Rows of a few-channel tensor copied into the window layout (WindowPlan): one block per row, one thread per pixel of the
-// stored row. Runs when the tensor itself could not be given that layout (several consumers, an fp32 input). With `lo` (fp32)
-// the remainder operand of the TF32 x 3 product, x - (upper 19 bits of x), is written beside it.
+// stored row. Runs when the tensor itself could not be given that layout (several consumers, an fp32 input).
 struct RepackArgs {
   const void *in;
-  void *out, *lo;
+  void *out;
   size_t rows; // n * h
   int w, c, cps, in_wl, in_wphys;
   int cpd, wl, wphys;
@@ -823,10 +813,6 @@ __global__ void window_repack_kernel(RepackArgs a) {
       for (int k = 0; k < a.cpd; ++k) {
         const T v = (x >= 0 && x < a.w && k < a.c) ? src[(size_t)x * a.cps + k] : (T)0;
         reinterpret_cast<T *>(a.out)[at + k] = v;
-        if (sizeof(T) == 4 && a.lo) {
-          const float f = __uint_as_float((uint32_t)v);
-          reinterpret_cast<float *>(a.lo)[at + k] = __fsub_rn(f, __uint_as_float((uint32_t)v & 0xffffe000u));
-        }
       }
     }
   }
