@@ -223,11 +223,11 @@ public:
   StreamSet ss; // streams, events, error word, pinned buffers
   bool use_graph = true;
   // Programmatic dependent launch (option "pdl"): a kernel launched with the attribute may be scheduled while its
-  // predecessor in the stream is still running; it sets up its barriers and tensor memory and then waits for that
-  // kernel's results (pdl_wait). 1 (default): the tensor-core convolution kernels carry the attribute; 0: none; 2: every
-  // kernel. Measured per class (ms per graph launch, off / all / convolutions only): INT8 ResNet-50 batch 1 0.379 / 0.348 /
+  // predecessor in the stream is still running; it sets up its barriers, tensor memory or table and then waits for that
+  // kernel's results (pdl_wait). 1 (default): the tensor-core convolution kernels and the activation chains carry the
+  // attribute; 0: none; 2: every kernel. Measured per class (ms per graph launch, off / all / convolutions only): INT8 ResNet-50 batch 1 0.379 / 0.348 /
   // 0.334, batch 32 0.697 / 0.668 / 0.657, batch 256 3.074 / 3.193 / 3.063; YOLOv4-style batch 8 2.361 / 2.412 / 2.265;
-  // MobileNet-v2 batch 32 0.526 / 0.504 / 0.485. On the memory-bound kernels alone the attribute costs 1-5%: their blocks
+  // MobileNet-v2 batch 32 0.526 / 0.504 / 0.485. On the other memory-bound kernels alone the attribute costs 1-5%: their blocks
   // then take their SMs in the order the predecessor's CTAs leave instead of evenly.
   int use_pdl = 1;
   cudaGraphExec_t capture_graph();
@@ -1352,22 +1352,24 @@ private:
 class ActChainOp : public OpKernel {
 public:
   ActChainOp(Interpreter &I, const QuantOp &q0, const LutOp &lut, const QuantOp &q1)
-      : I_(I), in_(q0.in()), deq_(q0.out()), act_(lut.out()), out_(q1.out()), s_in_(q0.scale()),
-        s_lut_(lut.scale()), s_out_(q1.scale()), base_(lut.base_table()), slope_(lut.slope_table()) {
+      : I_(I), in_(q0.in()), deq_(q0.out()), act_(lut.out()), out_(q1.out()) {
     alg_bytes = 6.0 * out_->numel();
+    table_ = (uint2 *)I.dalloc(256 * sizeof(uint2));
+    act_table_kernel<<<1, 256, 0, I.stream>>>(table_, q0.scale(), lut.scale(), lut.base_table(), lut.slope_table(), q1.scale());
+    TPUCB_CUDA(cudaGetLastError());
   }
   void invoke(cudaStream_t s) override {
-    size_t nvec = out_->pixels() * out_->cp / 16;
-    launch_k(act_chain_i8_kernel, grid_for(nvec, 256, I_.sm_count), 256, 0, s, 
-        (const uint4 *)in_->dev, (uint4 *)deq_->dev, (uint4 *)act_->dev, (uint4 *)out_->dev, nvec, s_in_, s_lut_,
-        base_, slope_, s_out_);
+    const size_t nvec = out_->pixels() * out_->cp / 8;
+    const int grid = (int)std::min<size_t>((nvec + 255) / 256, (size_t)I_.sm_count * 8);
+    PdlConvScope pdl; // stands behind a convolution: its table is in place when the convolution ends
+    launch_k(act_chain_i8_kernel, grid, 256, 0, s, (const uint2 *)in_->dev, (uint4 *)deq_->dev, (uint4 *)act_->dev,
+             (uint2 *)out_->dev, nvec, table_);
   }
 
 private:
   Interpreter &I_;
   TensorPtr in_, deq_, act_, out_;
-  float s_in_, s_lut_, s_out_;
-  const float *base_, *slope_;
+  uint2 *table_ = nullptr;
 };
 
 class FusedAwayOp : public OpKernel {
