@@ -140,8 +140,9 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          "pdl" (0 off, 1 = default, 2 every kernel): programmatic dependent launch. A kernel launched with the
  *          attribute may be scheduled while its predecessor in the stream is still running: its launch and set-up
  *          (barriers, tensor memory) overlap that kernel's tail, and it waits for that kernel's results before its first
- *          global access. 1 gives the attribute to the tensor-core convolution kernels only, which measured faster than
- *          none and than all on every graph and batch tried (on the memory-bound kernels alone it costs 1-5%).
+ *          global access. 1 gives the attribute to the tensor-core convolution kernels, the activation chains and
+ *          launches too small to fill the chip, which measured faster than none and than all (on large memory-bound
+ *          kernels it costs 1-5%).
  *          "split_k" (0/1, default 1; read by the next load_module): INT8 convolutions and inner products with few
  *          tiles and 24 K blocks or more share each tile among several CTAs (exact: int32 partial sums).
  *          "fuse_activations" (0/1, default 1; read by the next load_module): run each

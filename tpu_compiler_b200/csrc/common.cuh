@@ -95,10 +95,12 @@ TPUCB_HD float bf16_round(float f, bool rounding = true) {
 // before its own first global access (pdl_wait). Both are no-ops in a kernel launched the ordinary way.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// first statement of every kernel that has no set-up worth overlapping
+// First statement of every kernel that has no set-up worth overlapping. It waits before it lets its successor in: with
+// nothing to overlap, blocks of the successor that stand about early only take room from this kernel's own (MobileNet-v2
+// batch 7: 231 us, the other way round 261).
 __device__ __forceinline__ void pdl_prologue() {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
 }
 
 // Two F32ToBF16 roundings in one conversion instruction: {bf16(hi), bf16(lo)} packed in a word.

@@ -110,7 +110,11 @@ inline void launch_k(void (*kernel)(KArgs...), G grid, B block, size_t smem, cud
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const bool pdl = launch_pdl_flag();
+  // Mode 1 marks small launches of the other kernels too: one that has no more than a block's worth of threads per SM
+  // cannot be placed badly by the order in which its predecessor's blocks leave, and its scheduling is most of what it
+  // costs (MobileNet-v2 batch 1 227 -> 218 us, 12 307 -> 296; YOLOv4-style batch 1 1181 -> 1160; twice the threads: a loss).
+  const bool pdl = launch_pdl_flag() || (pdl_mode() == 1 && (size_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z *
+                                             cfg.blockDim.x * cfg.blockDim.y * cfg.blockDim.z <= 148 * 256);
   // The arguments are converted to the kernel's own parameter types and passed by address; without the attribute the
   // launch goes through the classic entry point.
   auto go = [&](KArgs... a) {

@@ -225,7 +225,7 @@ public:
   // Programmatic dependent launch (option "pdl"): a kernel launched with the attribute may be scheduled while its
   // predecessor in the stream is still running; it sets up its barriers, tensor memory or table and then waits for that
   // kernel's results (pdl_wait). 1 (default): the tensor-core convolution kernels and the activation chains carry the
-  // attribute; 0: none; 2: every kernel. Measured per class (ms per graph launch, off / all / convolutions only): INT8 ResNet-50 batch 1 0.379 / 0.348 /
+  // attribute, and every launch too small to fill the chip (launch_k); 0: none; 2: every kernel. Measured per class (ms per graph launch, off / all / convolutions only): INT8 ResNet-50 batch 1 0.379 / 0.348 /
   // 0.334, batch 32 0.697 / 0.668 / 0.657, batch 256 3.074 / 3.193 / 3.063; YOLOv4-style batch 8 2.361 / 2.412 / 2.265;
   // MobileNet-v2 batch 32 0.526 / 0.504 / 0.485. On the other memory-bound kernels alone the attribute costs 1-5%: their blocks
   // then take their SMs in the order the predecessor's CTAs leave instead of evenly.
