@@ -106,3 +106,29 @@ def test_conv_forms(dtype, case):
         assert np.all(np.abs(got - ref) <= np.maximum(np.abs(ref) * 2.0 ** -7, 2.0 ** -14 * np.abs(ref).max()))
     else:
         assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("graph", [1, 0])
+def test_large_result_read_before_the_end(graph):
+    """A large result that ends before the module does is fetched beside the ops behind it: launch after launch, each with
+    inputs of its own, in any order of fetching, and behind something else than a launch."""
+    from tpu_compiler_b200 import module
+    rng = np.random.default_rng(9)
+    text = ("input name=x shape=4,64,64,64 dtype=INT8\n"
+            "relu name=early in=x shape=4,64,64,64 dtype=INT8\n"  # 4 MB as fp32, nothing reads it
+            "pool_max_2d name=p in=x shape=4,64,64,64 dtype=INT8 kh=3 kw=3 sh=1 sw=1 pt=1 pb=1 pl=1 pr=1\n"
+            "pool_max_2d name=q in=p shape=4,64,32,32 dtype=INT8 kh=2 kw=2 sh=2 sw=2 pt=0 pb=0 pl=0 pr=0\n"
+            "relu name=late in=q shape=4,64,32,32 dtype=INT8\n")
+    m = module(0)
+    m.load_text(text, {})
+    m.set_option("cuda_graph", graph)
+    for i in range(8):
+        x = rng.integers(-128, 128, (4, 64, 64, 64)).astype(np.float32)
+        m.set_tensor("x", x)
+        m.launch()
+        if i == 5:
+            m.set_tensor("x", -x - 1)  # the launch in flight keeps its input
+        ref = graph_runner.run(text, {}, {"x": x})
+        for name in (["early", "late", "early"], ["late", "early", "p"])[i % 2]:
+            assert np.array_equal(m.get_tensor(name), ref[name]), (i, name)
+    m.close()

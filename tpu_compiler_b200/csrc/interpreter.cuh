@@ -96,7 +96,7 @@ public:
   ~Interpreter() {
     cudaSetDevice(device_);
     cudaDeviceSynchronize(); // as cudaFree would: nobody's kernels still read a tensor of this module
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    invalidate_graph();
     kernels.clear();
     for (auto &kv : tensors)
       if (kv.second->owns) dfree(kv.second->dev);
@@ -107,6 +107,7 @@ public:
   }
 
   void bind() {
+    early_valid = false; // whatever comes now may write a tensor
     TPUCB_CUDA(cudaSetDevice(device_));
     pdl_mode() = use_pdl;
     launch_pdl_flag() = use_pdl >= 2;
@@ -130,6 +131,7 @@ public:
   }
   float *ensure_staging(size_t bytes) {
     if (bytes > staging_bytes) {
+      early_valid = false; // ordered behind the launch in flight
       dfree(staging);
       staging = nullptr;
       staging_bytes = 0;
@@ -204,10 +206,11 @@ public:
   void launch_to(const std::string &name);
   void sync_and_check();
   void invalidate_graph() {
-    if (graph_exec) {
-      cudaGraphExecDestroy(graph_exec);
-      graph_exec = nullptr;
+    for (GraphPart &p : graph) {
+      if (p.exec) cudaGraphExecDestroy(p.exec);
+      if (p.done) cudaEventDestroy(p.done);
     }
+    graph.clear();
   }
 
   int device_;
@@ -230,7 +233,7 @@ public:
   // MobileNet-v2 batch 32 0.526 / 0.504 / 0.485. On the other memory-bound kernels alone the attribute costs 1-5%: their blocks
   // then take their SMs in the order the predecessor's CTAs leave instead of evenly.
   int use_pdl = 1;
-  cudaGraphExec_t capture_graph();
+  void capture_graph();
   // Self-test (option "selftest_lost_arrival", read by the next load_module): > 0 makes every INT8 tensor-core
   // convolution built from then on lose its accumulator hand-back and wait only that many rounds of 1024 polls
   // (ConvGemmParams::wait_rounds / lose_arrival), so that a launch ends with a bounded-wait error status.
@@ -252,7 +255,16 @@ public:
   bool fuse_residual_add = false; // set before load_module: eltwise adds run in the producing convolution's epilogue
   bool fp32_tensor_cores = true; // set before load_module: fp32 convolutions as three TF32 products
   void fuse_activation_chains(const std::map<std::string, int> &uses);
-  cudaGraphExec_t graph_exec = nullptr;
+  // The op list as CUDA graphs that follow one another: a part ends behind each large result that nothing in the module
+  // reads, so that its download need not wait for the ops behind it (get_tensor).
+  struct GraphPart {
+    cudaGraphExec_t exec = nullptr;
+    const DevTensor *out = nullptr; // ... and the event behind it, unless it is the last part
+    cudaEvent_t done = nullptr;
+  };
+  std::vector<GraphPart> graph;
+  static constexpr size_t kEarlyBytes = 1u << 20; // 20 us of the link, against a few us for one graph more
+  bool early_valid = false; // nothing but downloads since the graph launch in flight
   std::map<std::string, HostWeight> weights;
   std::map<std::string, TensorPtr> tensors;
   std::vector<std::string> tensor_order;
@@ -2307,8 +2319,11 @@ inline void Interpreter::set_tensor_async_i8(const std::string &name, const int8
   staging_used[k] = true;
 }
 
-// getTensor (MlirModuleInterpreter.cpp:419-427): deep copy out as fp32 NCHW.
+// getTensor (MlirModuleInterpreter.cpp:419-427): deep copy out as fp32 NCHW. A large result that ends a part of the graph
+// is converted and copied on the copy stream as soon as that part is done, beside the ops behind it: of a detector's three
+// heads the first is three quarters of the bytes (22 MB at a batch of eight, 400 us of the link).
 inline void Interpreter::get_tensor(const std::string &name, float *out, size_t numel, int slot) {
+  const bool launched = early_valid;
   bind();
   TensorPtr t = tensor(name);
   const SlotView v = slot_view(*t, slot, max_batch, "get_tensor");
@@ -2316,42 +2331,70 @@ inline void Interpreter::get_tensor(const std::string &name, float *out, size_t 
   // A small result is written straight into pinned host memory by the conversion kernel: no copy command behind it.
   const bool direct = numel * sizeof(float) <= kDownloadBytes;
   if (direct && !ss.download) TPUCB_CUDA(cudaHostAlloc((void **)&ss.download, kDownloadBytes, cudaHostAllocMapped));
+  early_valid = launched;
   float *stg = direct ? ss.download : ensure_staging(numel * sizeof(float));
-  int grid = grid_for(numel, 256, sm_count);
-  if (t->dtype == DT_I8) launch_k(dev_to_nchw_f32_kernel<DT_I8>, grid, 256, 0, stream, v.dev, stg, v.g);
-  else if (t->dtype == DT_BF16) launch_k(dev_to_nchw_f32_kernel<DT_BF16>, grid, 256, 0, stream, v.dev, stg, v.g);
-  else launch_k(dev_to_nchw_f32_kernel<DT_F32>, grid, 256, 0, stream, v.dev, stg, v.g);
+  cudaStream_t on = stream;
+  if (early_valid)
+    for (const GraphPart &p : graph)
+      if (p.done && p.out == t.get()) {
+        on = copy_stream;
+        TPUCB_CUDA(cudaStreamWaitEvent(on, p.done, 0));
+      }
+  const dim3 grid((unsigned)((v.g.n * (size_t)v.g.h * v.g.w + 63) / 64), (unsigned)((v.g.c + 63) / 64));
+  if (t->dtype == DT_I8) launch_k(dev_to_nchw_f32_kernel<DT_I8>, grid, 256, 0, on, v.dev, stg, v.g);
+  else if (t->dtype == DT_BF16) launch_k(dev_to_nchw_f32_kernel<DT_BF16>, grid, 256, 0, on, v.dev, stg, v.g);
+  else launch_k(dev_to_nchw_f32_kernel<DT_F32>, grid, 256, 0, on, v.dev, stg, v.g);
   TPUCB_CUDA(cudaGetLastError());
-  if (!direct) TPUCB_CUDA(cudaMemcpyAsync(out, stg, numel * sizeof(float), cudaMemcpyDeviceToHost, stream));
-  TPUCB_CUDA(cudaStreamSynchronize(stream));
+  if (!direct) TPUCB_CUDA(cudaMemcpyAsync(out, stg, numel * sizeof(float), cudaMemcpyDeviceToHost, on));
+  TPUCB_CUDA(cudaStreamSynchronize(on));
   if (direct) std::memcpy(out, stg, numel * sizeof(float));
 }
 
-// The op list captured as one CUDA graph, with the launch flag of the moment.
-inline cudaGraphExec_t Interpreter::capture_graph() {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  TPUCB_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+// The op list captured as CUDA graphs, with the launch flag of the moment.
+inline void Interpreter::capture_graph() {
+  size_t at = 0;
   try {
-    for (auto &k : kernels) k->run(stream);
+    while (at < kernels.size()) {
+      graph.emplace_back();
+      GraphPart &part = graph.back();
+      cudaGraph_t g = nullptr;
+      TPUCB_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+      try {
+        while (at < kernels.size()) {
+          OpKernel &k = *kernels[at++];
+          k.run(stream);
+          if (at < kernels.size() && k.result && !uses.count(k.name) && k.result->numel() * sizeof(float) >= kEarlyBytes) {
+            part.out = k.result.get();
+            break;
+          }
+        }
+      } catch (...) {
+        cudaStreamEndCapture(stream, &g);
+        if (g) cudaGraphDestroy(g);
+        throw;
+      }
+      TPUCB_CUDA(cudaStreamEndCapture(stream, &g));
+      const cudaError_t e = cudaGraphInstantiate(&part.exec, g, 0);
+      cudaGraphDestroy(g);
+      TPUCB_CUDA(e);
+      if (part.out) TPUCB_CUDA(cudaEventCreateWithFlags(&part.done, cudaEventDisableTiming));
+    }
   } catch (...) {
-    cudaStreamEndCapture(stream, &graph);
-    if (graph) cudaGraphDestroy(graph);
+    invalidate_graph();
     throw;
   }
-  TPUCB_CUDA(cudaStreamEndCapture(stream, &graph));
-  cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  TPUCB_CUDA(e);
-  return exec;
 }
 
-// invoke (MlirModuleInterpreter.cpp:371-381): the op loop; replayed as one CUDA graph.
+// invoke (MlirModuleInterpreter.cpp:371-381): the op loop; replayed as CUDA graphs.
 inline void Interpreter::launch_all() {
   bind();
   if (use_graph) {
-    if (!graph_exec) graph_exec = capture_graph();
-    TPUCB_CUDA(cudaGraphLaunch(graph_exec, stream));
+    if (graph.empty()) capture_graph();
+    for (const GraphPart &p : graph) {
+      TPUCB_CUDA(cudaGraphLaunch(p.exec, stream));
+      if (p.done) TPUCB_CUDA(cudaEventRecord(p.done, stream));
+    }
+    early_valid = true;
   } else {
     for (auto &k : kernels) k->run(stream);
     TPUCB_CUDA(cudaGetLastError());

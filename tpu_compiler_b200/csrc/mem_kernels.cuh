@@ -104,28 +104,37 @@ __global__ void nchw_i8_to_pix_kernel(const uint8_t *__restrict__ src, void *__r
   }
 }
 
-// download: device NHWC -> fp32 NCHW. One thread per NCHW element; reads of a warp
-// stride by cp but stay inside L2-resident rows for the sizes that are fetched.
+__device__ __forceinline__ float load_as_f32(const void *p, int dt, size_t i) {
+  if (dt == DT_I8) return (float)reinterpret_cast<const int8_t *>(p)[i];
+  if (dt == DT_BF16) return bits_f32((uint32_t)reinterpret_cast<const uint16_t *>(p)[i] << 16);
+  return reinterpret_cast<const float *>(p)[i];
+}
+
+// download: device NHWC -> fp32 NCHW, a tile of 64 pixels by 64 channels per block (256 threads) through shared memory:
+// reads run along the channels, writes along the pixels of one channel.
 template <int DT>
-__global__ void dev_to_nchw_f32_kernel(const void *__restrict__ src, float *__restrict__ dst,
-                                       TensorGeom g) {
+__global__ void __launch_bounds__(256) dev_to_nchw_f32_kernel(const void *__restrict__ src, float *__restrict__ dst, TensorGeom g) {
   pdl_prologue();
-  const size_t total = (size_t)g.n * g.c * g.h * g.w;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-       i += (size_t)gridDim.x * blockDim.x) {
-    int x = (int)(i % g.w);
-    size_t t = i / g.w;
-    int y = (int)(t % g.h);
-    t /= g.h;
-    int c = (int)(t % g.c);
-    int b = (int)(t / g.c);
-    size_t s = (((size_t)b * g.h + y) * g.wphys + g.wl + x) * g.cp + c;
-    float v;
-    if (DT == DT_I8) v = (float)reinterpret_cast<const int8_t *>(src)[s];
-    else if (DT == DT_BF16) v = bits_f32((uint32_t)reinterpret_cast<const uint16_t *>(src)[s] << 16);
-    else v = reinterpret_cast<const float *>(src)[s];
-    dst[i] = v;
+  __shared__ float s_v[64][65];
+  const size_t hw = (size_t)g.h * g.w, pixels = g.n * hw, p0 = blockIdx.x * (size_t)64;
+  const int c0 = blockIdx.y * 64, lane = threadIdx.x & 63;
+  if (c0 + lane < g.c) {
+#pragma unroll 4
+    for (int j = threadIdx.x >> 6; j < 64; j += 4) {
+      const size_t pix = p0 + j;
+      if (pix >= pixels) break;
+      const size_t row = pix / g.w;
+      const size_t i = (row * g.wphys + g.wl + (pix - row * g.w)) * g.cp + c0 + lane;
+      s_v[lane][j] = load_as_f32(src, DT, i);
+    }
   }
+  __syncthreads();
+  const size_t pix = p0 + lane;
+  if (pix >= pixels) return;
+  const size_t b = pix / hw;
+  float *to = dst + b * g.c * hw + (pix - b * hw);
+#pragma unroll 4
+  for (int j = threadIdx.x >> 6; j < 64 && c0 + j < g.c; j += 4) to[(size_t)(c0 + j) * hw] = s_v[j][lane];
 }
 
 // ------------------------------------------------------------------------- quant
@@ -135,11 +144,6 @@ __global__ void dev_to_nchw_f32_kernel(const void *__restrict__ src, float *__re
 //       4 bf16->int8                                                  quant.cpp:87-94
 //       5 fp32->bf16 (truncate)                                       quant.cpp:41-52
 // Source and destination may have different channel pitches (cps / cpd).
-__device__ __forceinline__ float load_as_f32(const void *p, int dt, size_t i) {
-  if (dt == DT_I8) return (float)reinterpret_cast<const int8_t *>(p)[i];
-  if (dt == DT_BF16) return bits_f32((uint32_t)reinterpret_cast<const uint16_t *>(p)[i] << 16);
-  return reinterpret_cast<const float *>(p)[i];
-}
 __device__ __forceinline__ void store_from_f32(void *p, int dt, size_t i, float v) {
   if (dt == DT_I8) reinterpret_cast<int8_t *>(p)[i] = (int8_t)(int)v;
   else if (dt == DT_BF16) reinterpret_cast<uint16_t *>(p)[i] = (uint16_t)(f32_bits(v) >> 16);
