@@ -909,6 +909,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
               const uint32_t b_lo = ring_lo + (uint32_t)sub * sub_step;
               const uint32_t first = (kit > k_begin || sub > 0) ? 1u : 0u;
               if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+              else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
               else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
               else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
             }

@@ -355,24 +355,23 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
     grid = grid / n_tiles * n_tiles; // a CTA's channel tile must not change
     if (grid < n_tiles) grid = n_tiles;
   }
-  // Split K: a launch with fewer tiles than CTA slots and a long K gives each tile to several CTAs (ConvGemmParams::
-  // split_k): at least six K blocks per CTA, at most sixteen CTAs per tile, no more CTAs than slots. The exchange
-  // through global memory costs about 3 us of latency (reductions, fence, count, read back) and a K block 0.4 us, so
-  // only layers of 24 K blocks or more are split (3x3 with 512 channels: 36 blocks, 16.4 -> 10.3 us at batch 1; with 16
-  // or 18 blocks the two forms measured equal, below that the split is slower). The weights are then not kept resident
-  // (a CTA needs only its own K range once).
+  // Split K: a launch with fewer tiles than SMs and a long K gives each tile to several CTAs (ConvGemmParams::split_k): at
+  // least six K blocks per CTA, at most sixteen CTAs per tile, no more CTAs than SMs. A K block takes 0.33 us of a CTA that
+  // has its SM to itself; the exchange through global memory (reductions, fence, count, read back) costs 4 us and 0.035 us
+  // for each of up to a hundred CTAs. Split where that pays by half a microsecond (3x3, 512 channels, 7x7, batch 1: 15.6 ->
+  // 9.2 us; batch 19: 16.4 -> 15.2). Two CTAs per SM were a loss wherever other work fills the gaps (5x5, 64 -> 128
+  // channels, 7 x 45 x 45, 222 CTAs: 16.1 us against 12.7 unsplit, three streams at once 9.8 against 5.3). The weights are
+  // then not kept resident (a CTA needs only its own K range once).
   p.split_k = 1;
   p.k_per = k_iters;
-  if (conv_split_k_enabled() && !pl.bf16 && !p.dual && k_iters >= 24 && total_tiles * 2 <= ctas_per_sm * sm_count) {
-    int want = (int)((ctas_per_sm * sm_count) / total_tiles);
-    if (want > 16) want = 16;
-    if (want > k_iters / 6) want = k_iters / 6;
+  if (conv_split_k_enabled() && !pl.bf16 && !p.dual) {
+    const int want = (int)std::min<long long>(std::min(16, k_iters / 6), sm_count / total_tiles);
     if (want >= 2) {
-      p.k_per = (k_iters + want - 1) / want;
-      p.split_k = (k_iters + p.k_per - 1) / p.k_per;
-      if (p.split_k < 2) {
-        p.split_k = 1;
-        p.k_per = k_iters;
+      const int per = (k_iters + want - 1) / want, parts = (k_iters + per - 1) / per;
+      const double exchange = 4.0 + 0.035 * std::min<double>((double)total_tiles * parts, 100.0);
+      if (0.33 * (k_iters - per) > exchange + 0.5) {
+        p.k_per = per;
+        p.split_k = parts;
       }
     }
   }
