@@ -106,7 +106,7 @@ def test_conv_forms(dtype, case):
     if dtype == "BF16":
         assert np.all(np.abs(got - ref) <= np.maximum(np.abs(ref) * 2.0 ** -7, 2.0 ** -14 * np.abs(ref).max()))
     else:
-        assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+        assert np.abs(got - ref).max() <= 3e-5 * np.abs(ref).max()
 
 
 @pytest.mark.parametrize("graph", [1, 0])

@@ -90,6 +90,16 @@ TPUCB_HD float bf16_round(float f, bool rounding = true) {
 }
 
 #ifdef __CUDACC__
+// the part of x that a kind::tf32 product does not read: x - (upper 19 bits of x), exact
+__device__ __forceinline__ float4 tf32_remainder(const float4 &x) {
+  float4 l;
+  l.x = __fsub_rn(x.x, __uint_as_float(__float_as_uint(x.x) & 0xffffe000u));
+  l.y = __fsub_rn(x.y, __uint_as_float(__float_as_uint(x.y) & 0xffffe000u));
+  l.z = __fsub_rn(x.z, __uint_as_float(__float_as_uint(x.z) & 0xffffe000u));
+  l.w = __fsub_rn(x.w, __uint_as_float(__float_as_uint(x.w) & 0xffffe000u));
+  return l;
+}
+
 // Programmatic dependent launch (kernels launched through launch_k with the stream-serialisation attribute): a kernel
 // lets its successor in the stream be scheduled early (pdl_trigger) and waits for its predecessor's memory operations
 // before its own first global access (pdl_wait). Both are no-ops in a kernel launched the ordinary way.

@@ -617,31 +617,29 @@ __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, 
   }
 }
 
-// Where the columns of a tap block's accumulator go: column c to pixel pix[c] (shared memory) counted from the tile's first,
-// where that lies below `lim`.
-struct TableMap {
-  const int *pix;
-  int lim;
-};
-
-// Epilogue of an fp32 convolution computed as three TF32 products (calibration forward; core/conv.cpp:80-89): the sum of the
-// two fp32 accumulators (large terms, small terms `small_at` columns further) + fp32 bias, ReLU, stored as fp32. A lane owns a
-// channel: for every pixel the warp writes 32 consecutive channels (128 contiguous bytes). `out_ch` addresses (the tile's
-// first pixel, this lane's channel).
+// Epilogue of an fp32 convolution computed as three TF32 products (calibration forward; core/conv.cpp:80-89): fp32
+// accumulator + fp32 bias, ReLU, stored as fp32. A lane owns a channel: for every pixel the warp writes 32 consecutive
+// channels (128 contiguous bytes). `out_ch` addresses (pixel m0, this lane's channel); `pitch` is the row pitch in bytes.
 template <bool RELU>
 __device__ __forceinline__ void epilogue_channels_f32(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out_ch, bool ch_ok,
-                                                      int half, int halves, float bias, int ncols, uint32_t small_at, const TableMap &map) {
-  for (int colg = half * 16; colg < ncols; colg += 16 * halves) {
-    uint32_t big[16], small[16];
-    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, big);
-    ptx::tcgen05_ld_x16(lane_addr + small_at + (uint32_t)colg, small);
+                                                      int m0, int half, int halves, float bias, int ncols = 128) {
+  const size_t pitch = (size_t)p.ldc;
+  uint8_t *lo_ch = p.out2 ? reinterpret_cast<uint8_t *>(p.out2) + (out_ch - reinterpret_cast<uint8_t *>(p.out)) : nullptr;
+  for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
+    if (m0 + colg >= p.M_total) break;
+    uint32_t acc0[16], acc1[16];
+    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
+    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
     ptx::tcgen05_wait_ld();
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      float v = __fadd_rn(__fadd_rn(bits_f32(big[j]), bits_f32(small[j])), bias);
+    for (int j = 0; j < 32; ++j) {
+      float v = __fadd_rn(bits_f32(j < 16 ? acc0[j & 15] : acc1[j & 15]), bias);
       if (RELU) v = v > 0.0f ? v : 0.0f;
-      const int px = map.pix[colg + j];
-      if (ch_ok && px < map.lim) *reinterpret_cast<float *>(out_ch + (size_t)(unsigned)px * (unsigned)p.ldc) = v;
+      if (ch_ok && m0 + colg + j < p.M_total) {
+        *reinterpret_cast<float *>(out_ch + (size_t)(colg + j) * pitch) = v;
+        // the remainder operand of a TF32 x 3 convolution that reads this result, when one does
+        if (lo_ch) *reinterpret_cast<float *>(lo_ch + (size_t)(colg + j) * pitch) = __fsub_rn(v, __uint_as_float(__float_as_uint(v) & 0xffffe000u));
+      }
     }
   }
 }
@@ -650,9 +648,18 @@ __device__ __forceinline__ void epilogue_channels_f32(const ConvGemmParams &p, u
 // vary fastest so that CTAs working at the same time share activation tiles through L2). The
 // producer runs ahead through the shared-memory ring across tile boundaries and the accumulator is
 // double-buffered in TMEM, so the loads and MMAs of tile i+1 overlap the epilogue of tile i.
-template <bool BF16, bool FAST = true, bool SPLIT = false, int ACTSEL = -1>
-__device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUtensorMap &tmB, const ConvGemmParams &p) {
-  constexpr int KIND = BF16 ? 1 : 0;
+// TF32: an fp32 convolution as three kind::tf32 products accumulated in one pass over K: with x = xh + xl and
+// w = wh + wl (h: the upper 19 bits of the fp32 word, l: the exact remainder), x w = xh wh + xl wh + xh wl up to
+// 2^-22 relative. The K loop runs three times over the taps: term 0 reads (tmA2, tmB) = (xl, wh), term 1
+// (tmA, tmB2) = (xh, wl), term 2 (tmA, tmB) = (xh, wh); the accumulator never leaves TMEM in between. The two small
+// terms come first: the tensor core truncates every partial sum at the accumulator's own precision, so each MMA
+// step costs up to an ulp of what has been accumulated so far, and only the steps of the last term see the
+// full magnitude (measured: the error against a double-accumulated convolution drops by the expected factor 3).
+template <bool BF16, bool FAST = true, bool TF32 = false, bool SPLIT = false, int ACTSEL = -1>
+__device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUtensorMap &tmB, const ConvGemmParams &p,
+                                               const CUtensorMap &tmA2, const CUtensorMap &tmB2) {
+  constexpr int KIND = TF32 ? 2 : (BF16 ? 1 : 0);
+  constexpr int kTerms = TF32 ? 3 : 1;
   constexpr bool FQ = ACTSEL >= 100; // one epilogue, the floating-point requantisation: ACTSEL - 100 is the activation
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -754,7 +761,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       bool ok = true;
       int tm = walk_m0, tn = walk_n0; // (resident weights: their copies were started before the wait above)
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-        int k_begin = 0, k_end = k_iters;
+        int k_begin = 0, k_end = kTerms * k_iters;
         if (split_k > 1) { // few items per CTA: the divisions do not matter here
           const int tile = item / split_k;
           tm = tile / n_tiles;
@@ -781,7 +788,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         }
         // running (tap row, tap column, channel chunk) and ring (stage, phase) counters: this loop
         // is a single thread's instruction stream, so it carries no divisions
-        int tap = 0, tr = 0, ts = 0, chunk = 0;
+        int tap = 0, tr = 0, ts = 0, chunk = 0, term = 0;
         if (k_begin > 0) {
           tap = k_begin / p.c_chunks;
           chunk = k_begin - tap * p.c_chunks;
@@ -789,6 +796,8 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           ts = tap - tr * p.kw;
         }
         for (int kit = k_begin; kit < k_end; ++kit, ++it) {
+          const CUtensorMap *mapA = (TF32 && term == 0) ? &tmA2 : &tmA;
+          const CUtensorMap *mapB = (TF32 && term == 1) ? &tmB2 : &tmB;
           if (it >= p.stages) {
             if (!ptx::mbar_wait_bounded(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
               if (!*abort_flag) report_error(p.err, kErrEmptyWait);
@@ -805,18 +814,24 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           if (p.a_mode == 1) {
             // one copy per tile, also in dual mode (the map's pixel count per copy is the tile's: every copy costs
             // its issuing thread about 430 cycles whatever its size)
-            ptx::tma_load_im2col_4d(a_dst, &tmA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
+            ptx::tma_load_im2col_4d(a_dst, mapA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
                                     (uint16_t)(tr * p.dh));
           } else {
-            ptx::tma_load_2d(a_dst, &tmA, fb, c0, m0);
+            ptx::tma_load_2d(a_dst, mapA, fb, c0, m0);
           }
-          if (!p.w_resident) ptx::tma_load_3d(b_dst, &tmB, fb, c0, tap, n0);
+          if (!p.w_resident) ptx::tma_load_3d(b_dst, mapB, fb, c0, tap, n0);
           if (++chunk == p.c_chunks) {
             chunk = 0;
             ++tap;
             if (++ts == p.kw) {
               ts = 0;
               ++tr;
+            }
+            if (TF32 && tap == taps) { // next term: the same taps over the other operand pair
+              tap = 0;
+              tr = 0;
+              ts = 0;
+              ++term;
             }
           }
           if (++ps == p.stages) {
@@ -868,7 +883,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         }
       }
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++t) {
-        int k_begin = 0, k_end = k_iters;
+        int k_begin = 0, k_end = kTerms * k_iters;
         if (split_k > 1) {
           k_begin = (item % split_k) * p.k_per;
           k_end = min(k_iters, k_begin + p.k_per);
@@ -962,7 +977,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       }
       const int buf = t & 1;
       if (n0 != staged_n0) {
-        if (BF16) {
+        if (BF16 || TF32) {
           const int ch = n0 + ch_base + lane;
           bias_f = ch < p.n_valid ? __int_as_float(p.bias[ch]) : 0.0f; // fp32 bias bits in the int32 array
         } else if (FQ) {
@@ -1040,7 +1055,13 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         const size_t out_m0 = (size_t)m0 * p.ldc + (p.group > 1 ? (quarter * 32 * p.group >> 7) * p.ldc_px : 0); // bytes
         int8_t *out4 = p.out + out_m0 + p.c_off + ch4;
         const bool ch4_ok = ch4 < p.n_valid;
-        if (BF16) {
+        if (TF32) {
+          // byte addressing: 4 bytes per channel
+          const int ch = n0 + ch_base + lane;
+          uint8_t *out_ch = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch) * 4;
+          if (p.act == 1) epilogue_channels_f32<true>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
+          else epilogue_channels_f32<false>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
+        } else if (BF16) {
           // byte addressing: 2 bytes per channel, this lane's pair starts at its even channel
           const int ch = n0 + ch_base + lane;
           uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + (ch & ~1)) * 2;
@@ -1075,7 +1096,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
 __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const ConvGemmParams p) {
-  conv_gemm_body<false, true>(tmA, tmB, p);
+  conv_gemm_body<false, true>(tmA, tmB, p, tmA, tmB);
 }
 // The floating-point requantisation (p.fq set), one kernel per activation (ConvGemmParams::act): the compiler allocates
 // registers and schedules for that one epilogue.
@@ -1083,7 +1104,7 @@ template <int ACT>
 __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_i8_fq_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const ConvGemmParams p) {
-  conv_gemm_body<false, true, false, 100 + ACT>(tmA, tmB, p);
+  conv_gemm_body<false, true, false, false, 100 + ACT>(tmA, tmB, p, tmA, tmB);
 }
 // The split-K form of both (ConvGemmParams::split_k > 1): a kernel of its own, so that the ordinary ones carry none of
 // its code (with the switch at run time the epilogue-bound layers were 14% slower).
@@ -1091,13 +1112,13 @@ template <bool FAST>
 __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_i8_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           const ConvGemmParams p) {
-  conv_gemm_body<false, FAST, true>(tmA, tmB, p);
+  conv_gemm_body<false, FAST, false, true>(tmA, tmB, p, tmA, tmB);
 }
 // the same with the 64-bit multiply-add requantisation (requant_one), for layers outside requant_fast's domain
 __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_i8_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const ConvGemmParams p) {
-  conv_gemm_body<false, false>(tmA, tmB, p);
+  conv_gemm_body<false, false>(tmA, tmB, p, tmA, tmB);
 }
 // The same pipeline for BF16 graphs: BF16 operands (tcgen05 kind::f16), fp32 accumulators, BF16 results.
 // All sizes in ConvGemmParams that count K or row pitches are in BYTES, so only the MMA kind and the
@@ -1105,7 +1126,22 @@ conv_gemm_i8_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const ConvGemmParams p) {
-  conv_gemm_body<true, false>(tmA, tmB, p);
+  conv_gemm_body<true, false>(tmA, tmB, p, tmA, tmB);
+}
+
+// fp32 convolution on the tensor cores as three TF32 products (see conv_gemm_body): tmA / tmA2 are the upper and
+// the remainder part of the activations, tmB / tmB2 of the weights.
+__global__ void __launch_bounds__(kConvThreads, 2)
+conv_gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                        const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB2,
+                        const ConvGemmParams p) {
+  conv_gemm_body<false, false, true>(tmA, tmB, p, tmA2, tmB2);
+}
+
+// x -> remainder x - (upper 19 bits of x), exact; the upper part is what a kind::tf32 product reads of x itself.
+__global__ void tf32_split_kernel(const float4 *__restrict__ x, float4 *__restrict__ lo, size_t nvec) {
+  pdl_prologue();
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nvec; i += (size_t)gridDim.x * blockDim.x) lo[i] = tf32_remainder(x[i]);
 }
 
 } // namespace tpucb

@@ -3,7 +3,7 @@
 // (lib/Dialect/TPU/IR/TPUOperationSupport.cpp:366-428): four independent pads, the
 // output size taken from the result type, dilation, optional input zero-insertion.
 #pragma once
-#include "conv_tf32x3.cuh"
+#include "conv_gemm_i8.cuh"
 #include "host_common.h"
 #include "mem_kernels.cuh"
 
@@ -83,14 +83,11 @@ struct ConvPlan {
   size_t smem = 0;
   int ws_tiles = 0;  // split K: tiles of the partial-sum workspace (p.ws, p.ws_count), allocated by the op that owns the plan
   bool bf16 = false; // runs conv_gemm_bf16_kernel (K sizes and pitches in bytes, 2 per element)
-  bool tf32 = false; // runs conv_tf32x3_kernel (fp32 operands, 4 bytes per element): TapParams
-  TapParams q = {};
-  CUtensorMap tmB2;  // tf32: remainder part of the weights
-  // tf32 with parts (TapParams::parts): the result, its bias and activation for the reducing pass
-  float *reduce_out = nullptr;
-  const float *reduce_bias = nullptr;
-  size_t reduce_bytes = 0;
-  int reduce_act = 0;
+  bool tf32 = false; // runs conv_gemm_tf32x3_kernel (fp32 operands, 4 bytes per element; three K passes)
+  CUtensorMap tmA2, tmB2;           // tf32: remainder parts of the activations and of the weights
+  const float *split_src = nullptr; // tf32: the fp32 input, whose remainder is written to split_lo before the launch
+  float *split_lo = nullptr;
+  size_t split_nvec = 0;
   bool use_patch = false;
   PatchArgs patch;
   int8_t *patch_buf = nullptr; // scratch: expanded patch matrix [M][kp]
@@ -165,6 +162,21 @@ inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int ic
           const float hi = bits_f32(f32_bits(v) & 0xffffe000u);
           out[((size_t)o * taps + (r * kw + s)) * cin_pad + c] = part == 0 ? hi : v - hi;
         }
+  std::vector<int8_t> bytes(out.size() * 4);
+  std::memcpy(bytes.data(), out.data(), bytes.size());
+  return bytes;
+}
+
+// the same for the patch matrix of an fp32 image stem: four channel slots per tap, k = tap * 4 + c
+inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeom &g, int oc_pad, int part) {
+  const int kp = g.kh * g.kw * 4;
+  std::vector<float> out((size_t)oc_pad * kp, 0.0f);
+  for (int o = 0; o < g.oc; ++o)
+    for (int c = 0; c < g.ic; ++c)
+      for (int t = 0; t < g.kh * g.kw; ++t) {
+        const float v = w[((size_t)o * g.ic + c) * g.kh * g.kw + t], hi = bits_f32(f32_bits(v) & 0xffffe000u);
+        out[(size_t)o * kp + t * 4 + c] = part == 0 ? hi : v - hi;
+      }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
   return bytes;
@@ -265,9 +277,8 @@ inline bool window_plan_for(const ConvGeom &g, int es, int oc_pad, WindowPlan *o
 }
 
 // Weights of the window form: rows [G][128 / G channels] (one row per channel for G = 1), per filter row BK bytes.
-// part: -2 int8, -1 BF16, 0 / 1 the TF32 parts
-inline std::vector<int8_t> pack_window_weights(const float *w, const ConvGeom &g, const WindowPlan &wp, int rows, int BK, int part) {
-  const int es = part == -2 ? 1 : (part == -1 ? 2 : 4), slot = 128 / wp.G;
+inline std::vector<int8_t> pack_window_weights(const float *w, const ConvGeom &g, const WindowPlan &wp, int rows, int BK, bool bf16) {
+  const int es = bf16 ? 2 : 1, slot = 128 / wp.G;
   std::vector<int8_t> out((size_t)rows * g.kh * BK, 0);
   for (int j = 0; j < wp.G; ++j)
     for (int o = 0; o < g.oc; ++o)
@@ -276,13 +287,11 @@ inline std::vector<int8_t> pack_window_weights(const float *w, const ConvGeom &g
           for (int s = 0; s < g.kw; ++s) {
             const float v = w[(((size_t)o * g.ic + c) * g.kh + r) * g.kw + s];
             int8_t *at = out.data() + ((size_t)(j * slot + o) * g.kh + r) * BK + (size_t)(j * g.sw + s * g.dw) * wp.P + c * es;
-            if (part == -2) *at = (int8_t)(int)v;
-            else if (part == -1) {
+            if (bf16) {
               const uint16_t h = (uint16_t)(f32_bits(v) >> 16);
               std::memcpy(at, &h, 2);
             } else {
-              const float hi = bits_f32(f32_bits(v) & 0xffffe000u), f = part == 0 ? hi : v - hi;
-              std::memcpy(at, &f, 4);
+              *at = (int8_t)(int)v;
             }
           }
   return out;
@@ -319,7 +328,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
     // fewer bytes per pixel (measured faster for the 1x1 layers with 64 outputs).
     const size_t w_plain = (size_t)taps * p.c_chunks * 128 * p.BK;
     const bool plain_resident = w_plain <= 48 * 1024 && 113 * 1024 - kSmemHeader - 1024 - w_plain >= 3 * (size_t)128 * p.BK;
-    p.dual = (oc_pad <= 64 && p.group <= 1 && rows > 128 && !plain_resident) ? 1 : 0;
+    p.dual = (oc_pad <= 64 && p.group <= 1 && rows > 128 && !plain_resident && !pl.tf32) ? 1 : 0;
   }
   const int m_tiles = (rows + (p.dual ? 255 : 127)) / (p.dual ? 256 : 128);
   // Transposed product: the channel tile is the tensor core's M (128 TMEM lanes, rows past the
@@ -342,7 +351,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   const int ctas_per_sm = 2;
   const size_t budget = 113 * 1024;
   // (Pixel groups have small activation tiles: up to 60 KB of weights leave them four stages.)
-  p.w_resident = (total_tiles >= 2LL * n_tiles && w_all <= (p.group > 1 ? 60 : 48) * 1024 &&
+  p.w_resident = (!pl.tf32 && total_tiles >= 2LL * n_tiles && w_all <= (p.group > 1 ? 60 : 48) * 1024 &&
                   budget - kSmemHeader - 1024 - w_all >= (p.group > 1 ? 4 : 3) * a_bytes) ? 1 : 0;
   const size_t stage_bytes = p.w_resident ? a_bytes : a_bytes + b_bytes;
   const size_t ring_budget = budget - kSmemHeader - 1024 - (p.w_resident ? w_all : 0);
@@ -364,7 +373,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   // then not kept resident (a CTA needs only its own K range once).
   p.split_k = 1;
   p.k_per = k_iters;
-  if (conv_split_k_enabled() && !pl.bf16 && !p.dual) {
+  if (conv_split_k_enabled() && !pl.tf32 && !pl.bf16 && !p.dual) {
     const int want = (int)std::min<long long>(std::min(16, k_iters / 6), sm_count / total_tiles);
     if (want >= 2) {
       const int per = (k_iters + want - 1) / want, parts = (k_iters + per - 1) / per;
@@ -387,7 +396,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   }
   const size_t stage_bytes_final = p.w_resident ? a_bytes : a_bytes + b_bytes;
   const long long iters_per_cta = p.split_k > 1 ? p.k_per
-                                                : ((total_tiles + grid - 1) / grid) * k_iters;
+                                                : ((total_tiles + grid - 1) / grid) * k_iters * (pl.tf32 ? 3 : 1);
   if (stages > iters_per_cta) stages = (int)iters_per_cta;
   if (stages < 1) stages = 1;
   p.stages = stages;
@@ -400,7 +409,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
 // pixels of cp channels are one pixel of 2 cp channels, on both sides, so the layer is also a convolution of half the width
 // from 2 cp to 2 cp channels, whose filter holds the original one twice, the second time a pixel (half a channel block)
 // further. The rows fill up, tile rows are twice as long, and of a 3x3 filter's nine taps of twice the channels a third meets
-// only zero weights: those steps of K are skipped in tap blocks (TapParams::skip_first, keep_last).
+// only zero weights.
 struct DenseLayer {
   ConvGeom g; // g.ic = in_cp and g.oc = out_cp once paired
   int in_cp, out_cp;
@@ -446,127 +455,25 @@ inline void pair_layer(DenseLayer &d) {
   d.paired = true;
 }
 
-// ---- TF32 x 3 plans ----------------------------------------------------------------------------------------------------
-// Cost model of one SM, in clocks (see conv_tf32x3.cuh): `steps` products of 128 x N x 32 bytes, three for each 32 bytes of
-// K, against 128 bytes per clock of shared memory for their operands, the copied tiles and the split of the blocks (`bytes`);
-// the epilogue overlaps with two accumulators (N <= 128) only.
-inline double tf32_tile_clocks(double steps, int N, double bytes) {
-  const double work = std::max(steps * 68.0 * std::max(N, 64) / 128.0, steps * (128 + N) / 4.0 + bytes / 128.0), epi = 12.0 * N;
-  return (N > 128 ? work + epi : std::max(work, epi)) + 500.0;
-}
-constexpr int kTf32Smem = 222 * 1024 - kSmemHeader - 1024;
-// How many CTAs share a tile: a weight tile is 0.4 us of a CTA's time and the reducing pass 2.5 us, so at least a dozen
-// weight tiles in all.
-inline int tf32_parts(const TapParams &q, int weight_tiles, int n_tiles, int sm_count) {
-  if (q.m_tiles * n_tiles * 2 > sm_count || weight_tiles < 12) return 1;
-  return std::max(1, std::min(std::min(q.blocks, 8), sm_count / (q.m_tiles * n_tiles)));
-}
-inline double tf32_clocks(const TapParams &q, int taps_per_block, int BK, double steps, int n_tiles, int sm_count) {
-  const int weight_tiles = q.blocks * taps_per_block;
-  const double bytes = (double)q.blocks * (q.act_bytes * 3.0 + (double)taps_per_block * 256 * BK);
-  const int parts = tf32_parts(q, weight_tiles, n_tiles, sm_count);
-  return std::ceil((double)q.m_tiles * n_tiles / sm_count) * tf32_tile_clocks(3 * steps, q.N, bytes) / parts + (parts > 1 ? 4000.0 : 0.0);
-}
-// Chooses the tile of a stride-1 layer for tap blocks: image rows x columns (x whole images), so that the columns of a
-// product are many and well used. steps: 32-byte steps of K that a tile needs. False: no tile fits.
-inline bool choose_tap_tile(const ConvGeom &g, int k_bytes, int n_tiles, double steps, int sm_count, TapParams *q, double *clocks) {
-  if (g.sh != 1 || g.sw != 1 || g.pr < 0 || g.pb < 0 || g.oh != g.ih + g.pt + g.pb - (g.kh - 1) * g.dh ||
-      g.ow != g.iw + g.pl + g.pr - (g.kw - 1) * g.dw)
-    return false;
-  const int bk = pick_bk(k_bytes), chunks = (k_bytes + bk - 1) / bk, taps = g.kh * g.kw;
-  bool found = false;
-  for (int cw = std::min(g.ow, 256); cw >= 1; --cw) {
-    if (g.ow % cw) continue;
-    const int pc = cw == g.ow ? g.iw + std::max(g.pl, g.pr) : cw + (g.kw - 1) * g.dw;
-    for (int r = 1; r <= g.oh; ++r) {
-      const int rl = r + (g.kh - 1) * g.dh;
-      if ((r - 1) * pc + cw > 256 || pc > 256 || rl > 256) break;
-      for (int im = 1; im <= (cw == g.ow && r == g.oh ? g.n : 1); ++im) {
-        const int used = (im - 1) * rl * pc + (r - 1) * pc + cw;
-        if (used > 256 || im > 256) break;
-        TapParams t = {};
-        t.mode = 2;
-        t.blocks = chunks;
-        t.nb = 2;
-        t.N = round_up(used, 16);
-        t.n_used = used;
-        t.act_bytes = im * rl * pc * bk;
-        const int last = t.N - 1 + (g.kh - 1) * g.dh * pc + (g.kw - 1) * g.dw; // last pixel a product may read
-        t.act_stride = round_up(std::max((last + 1) * bk, t.act_bytes), 1024);
-        if (4 * t.act_stride + 2 * 256 * bk > kTf32Smem) continue;
-        t.R = r; t.I = im; t.Cw = cw; t.Pc = pc; t.Rl = rl; t.images = g.n;
-        t.tiles_x = g.ow / cw;
-        t.tiles_y = (g.oh + r - 1) / r;
-        t.m_tiles = (g.n + im - 1) / im * t.tiles_x * t.tiles_y;
-        const double c = tf32_clocks(t, taps, bk, steps, n_tiles, sm_count) + t.m_tiles * 1e-3;
-        if (found && c >= *clocks) continue;
-        found = true;
-        *clocks = c;
-        *q = t;
-      }
-    }
-  }
-  return found;
-}
-// A matrix (mode 0) or an im2col / row-window map (mode 1), `rows` rows in tiles of 128
-inline TapParams plain_tap_tiles(const ConvGemmParams &p, int mode, int rows) {
-  TapParams q = {};
-  q.mode = mode;
-  q.blocks = p.c_chunks * (mode == 1 ? p.kh * p.kw : 1);
-  q.nb = 3;
-  q.act_bytes = q.act_stride = 128 * p.BK;
-  q.N = q.n_used = 128;
-  q.m_tiles = (rows + 127) / 128;
-  return q;
-}
-// Launch shape of a plan whose TapParams are chosen
-inline void finish_tf32_plan(ConvPlan &pl, const TapParams &chosen, int n_tiles, int sm_count) {
-  ConvGemmParams &p = pl.p;
-  TapParams &q = pl.q;
-  q = chosen;
-  p.dual = 0; p.w_resident = 0; p.split_k = 1;
-  pl.ws_tiles = 0;
-  const int w_bytes = 256 * p.BK, acts = 2 * q.nb * q.act_stride;
-  const int weight_tiles = q.blocks * (q.mode == 2 ? p.kh * p.kw : 1);
-  q.parts = tf32_parts(q, weight_tiles, n_tiles, sm_count);
-  q.acc_bufs = q.N > 128 ? 1 : 2;
-  p.stages = std::min(std::min((kTf32Smem - acts) / w_bytes, kMaxStages), weight_tiles);
-  p.BN = 128;
-  p.tmem_cols = 512;
-  p.idesc = make_idesc_tf32(128, q.N);
-  pl.smem = kSmemHeader + 1024 + acts + (size_t)p.stages * w_bytes;
-  pl.grid = dim3((unsigned)std::min(q.m_tiles * n_tiles * q.parts, sm_count), 1, 1);
-}
-inline void encode_block_map(CUtensorMap *tm, const void *d_in, const ConvGeom &g, int cp_bytes, int BK, const TapParams &q) {
-  cuuint64_t dims[4] = {(cuuint64_t)cp_bytes, (cuuint64_t)g.iw, (cuuint64_t)g.ih, (cuuint64_t)g.n};
-  cuuint64_t strides[3] = {(cuuint64_t)cp_bytes, (cuuint64_t)cp_bytes * g.iw, (cuuint64_t)cp_bytes * g.iw * g.ih};
-  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)q.Pc, (cuuint32_t)q.Rl, (cuuint32_t)q.I};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = tma_api().tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void *)d_in, dims, strides, box, es,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(BK), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(tap blocks) failed: %d", (int)r);
-}
-
 inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_count) {
-  if (pl.use_patch)
+  if (pl.use_patch && pl.tf32)
+    launch_k(patch_expand_f32_kernel, grid_for((size_t)pl.p.M_total * pl.patch.kp / 4, 256, sm_count), 256, 0, stream,
+             reinterpret_cast<const float4 *>(pl.in), reinterpret_cast<float4 *>(pl.patch_buf), reinterpret_cast<float4 *>(pl.split_lo), pl.patch);
+  else if (pl.use_patch)
     launch_k(patch_expand_i8_kernel, grid_for((size_t)pl.p.M_total * pl.patch.kp, 256, sm_count), 256, 0, stream, pl.in, pl.patch_buf, pl.patch);
   if (pl.use_repack) {
     const RepackArgs &a = pl.repack;
     const int grid = (int)std::min<size_t>(a.rows, (size_t)sm_count * 8);
     if (a.es == 1) launch_k(window_repack_kernel<uint8_t>, grid, 256, 0, stream, a);
-    else if (a.es == 2) launch_k(window_repack_kernel<uint16_t>, grid, 256, 0, stream, a);
-    else launch_k(window_repack_kernel<uint32_t>, grid, 256, 0, stream, a);
+    else launch_k(window_repack_kernel<uint16_t>, grid, 256, 0, stream, a);
   }
   const int threads = kConvThreads;
   PdlConvScope conv_class; // the tensor-core kernel and its helper passes may start while the predecessor finishes
   if (pl.tf32) {
-    launch_k(conv_tf32x3_kernel, pl.grid, threads + 32 * kTransformWarps, pl.smem, stream, pl.tmA, pl.tmB, pl.tmB2, pl.p, pl.q);
-    if (pl.q.parts > 1) {
-      const size_t nvec = pl.reduce_bytes / 16;
-      launch_k(tf32_reduce_kernel, grid_for(nvec, 128, sm_count), 128, 0, stream, (const float4 *)pl.p.out, (float4 *)pl.reduce_out,
-               (const float4 *)pl.reduce_bias, nvec, pl.p.n_valid / 4, pl.q.parts, pl.reduce_act);
-    }
+    if (pl.split_src)
+      launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
+               reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
+    launch_k(conv_gemm_tf32x3_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.p);
   } else if (pl.bf16) launch_k(conv_gemm_bf16_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1 && (pl.p.fastq & 1)) launch_k(conv_gemm_i8_split_kernel<true>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1) launch_k(conv_gemm_i8_split_kernel<false>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
@@ -594,7 +501,7 @@ inline void conv_kernel_setup_once() {
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     return true;
   }();
   (void)done;

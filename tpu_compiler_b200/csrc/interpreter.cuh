@@ -254,6 +254,7 @@ public:
   bool fuse_activations = true; // set before load_module
   bool fuse_residual_add = false; // set before load_module: eltwise adds run in the producing convolution's epilogue
   bool fp32_tensor_cores = true; // set before load_module: fp32 convolutions as three TF32 products
+  void link_tf32_remainders();
   void fuse_activation_chains(const std::map<std::string, int> &uses);
   // The op list as CUDA graphs that follow one another: a part ends behind each large result that nothing in the module
   // reads, so that its download need not wait for the ops behind it (get_tensor).
@@ -498,13 +499,12 @@ public:
     }
     if (out->dtype == DT_F32) {
       TPUCB_CHECK(in->dtype == DT_F32, "conv %s: an fp32 convolution needs an fp32 input", op.name.c_str());
-      WindowPlan wp;
-      const bool window = window_plan_for(g, 4, out->cp, &wp); // image stems
       // fp32 convolution on the tensor cores as three TF32 products with fp32 accumulation (x w = xh wh + xl wh + xh wl,
       // 2^-22 relative: inside the 1e-4 of the fp32 path, where a single TF32 product would not be)
-      if (I.fp32_tensor_cores && (window || (g.g == 1 && !g.ins_h && !g.ins_w && in->cp % 8 == 0 && g.pl <= 127 && g.pt <= 127 &&
-                                             (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255))) {
-        setup_tensor_core(I, 2, filt.data, bias, {}, {}, window ? &wp : nullptr);
+      const bool stem = g.ic <= 4 && in->cp == 4 && !(g.kh == 1 && g.kw == 1);
+      if (I.fp32_tensor_cores && g.g == 1 && !g.ins_h && !g.ins_w &&
+          (stem || (in->cp % 8 == 0 && g.pl <= 127 && g.pt <= 127 && (g.kw - 1) * g.dw <= 255 && (g.kh - 1) * g.dh <= 255))) {
+        setup_tf32(I, filt.data, bias, stem);
         return;
       }
       f32_ = true;
@@ -615,13 +615,76 @@ public:
       plans_.push_back(pl);
     }
   }
-  // Ungrouped layers on the tensor cores. kind: 0 INT8, 1 BF16, 2 fp32 as three TF32 products. Three forms: row windows
-  // (wp), tap blocks (fp32 only), K blocks of a matrix or im2col map. fp32 runs on conv_tf32x3.cuh, the others on
-  // conv_gemm_i8.cuh.
+  // fp32 as three TF32 products. Image stems read a patch matrix, whose expansion writes the remainder part too; elsewhere
+  // the remainder of the input has a buffer beside it, filled as link_tf32_remainders decides. The order in which the
+  // products are summed (terms, taps, channels) decides the last bits of every statistic that calibration takes, and a
+  // threshold search turns some of those into another threshold: tap blocks, pixel pairs and row windows, which sum in
+  // another order, were a fifth faster (4.9 ms against 5.9 for ResNet-50 at batch 64) and moved one threshold in one run of
+  // twenty.
+  void setup_tf32(Interpreter &I, const std::vector<float> &filt, const std::vector<float> &bias, bool stem) {
+    conv_kernel_setup_once();
+    const ConvGeom &g = g_;
+    const int rows = g.n * g.oh * g.ow, out_cp = out_->cp;
+    act_ = do_relu_ ? 1 : 0;
+    alg_bytes = 4.0 * ((double)in_->numel() + out_->numel() + filt.size() + g.oc);
+    ConvPlan pl;
+    std::memset(&pl.p, 0, sizeof(pl.p));
+    pl.tf32 = true;
+    pl.in = (const int8_t *)in_->dev;
+    pl.ops = alg_ops;
+    ConvGemmParams &p = pl.p;
+    p.act = act_;
+    p.err = &I.ss.d_err->code;
+    p.out = (int8_t *)out_->dev;
+    p.ldc = out_cp * 4; // bytes
+    std::vector<int32_t> bias_bits(out_cp, 0);
+    for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
+    p.bias = p.mult = p.rshift = I.upload(bias_bits);
+    p.OH = g.oh; p.OW = g.ow;
+    std::vector<int8_t> w[2];
+    int taps = 1, k_bytes;
+    const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
+    if (stem) {
+      p.sh = p.sw = p.dh = p.dw = p.kh = p.kw = 1;
+      PatchArgs &a = pl.patch;
+      a = PatchArgs{g.n, g.ic, in_->cp, g.ih, g.iw, g.oh, g.ow, g.kh, g.kw, g.sh, g.sw, g.pt, g.pl, g.dh, g.dw, 0, 0, 0, g.ic,
+                    g.kh * g.kw * 4, in_->wl, in_->wphys};
+      k_bytes = a.kp * 4;
+      pl.use_patch = true;
+      pl.patch_bytes = (size_t)rows * k_bytes;
+      pl.patch_buf = (int8_t *)I.dalloc(pl.patch_bytes);
+      pl.split_lo = (float *)I.dalloc(pl.patch_bytes);
+      for (int part = 0; part < 2; ++part) w[part] = pack_patch_weights_tf32(filt.data(), g, out_cp, part);
+    } else {
+      p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
+      p.kh = g.kh; p.kw = g.kw;
+      k_bytes = in_->cp * 4;
+      taps = g.kh * g.kw;
+      p.a_mode = one ? 0 : 1;
+      // The tensor core ignores the low 13 mantissa bits of an fp32 operand, so the tensor itself serves as xh.
+      if (!in_->lo_dev) in_->lo_dev = I.dalloc(in_->bytes()); // shared by every convolution that reads this tensor
+      pl.split_src = (const float *)in_->dev;
+      pl.split_lo = (float *)in_->lo_dev;
+      pl.split_nvec = in_->bytes() / 16;
+      for (int part = 0; part < 2; ++part) w[part] = pack_conv_weights_tf32(filt.data(), g.oc, g.ic, g.kh, g.kw, out_cp, in_->cp, part);
+    }
+    finish_plan(pl, rows, taps, k_bytes, out_cp, I.sm_count);
+    p.idesc = make_idesc_tf32(128, p.BN);
+    const int8_t *part[2] = {stem ? pl.patch_buf : (const int8_t *)in_->dev, (const int8_t *)pl.split_lo};
+    for (int k = 0; k < 2; ++k) {
+      CUtensorMap *a = k ? &pl.tmA2 : &pl.tmA;
+      if (p.a_mode == 0) encode_matrix_map(a, part[k], rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
+      else encode_im2col_map(a, part[k], g, k_bytes, p.BK, a_tile_rows(p));
+      encode_weight_map(k ? &pl.tmB2 : &pl.tmB, I.upload(w[k]), out_cp, taps, k_bytes, p.BK, p.BN);
+    }
+    plans_.push_back(pl);
+  }
+  // Ungrouped layers on the tensor cores. kind: 0 INT8, 1 BF16. Two forms: row windows (wp), K blocks of a matrix or im2col
+  // map.
   void setup_tensor_core(Interpreter &I, int kind, const std::vector<float> &filt, const std::vector<float> &bias,
                          const std::vector<float> &mult, const std::vector<float> &rshift, const WindowPlan *wp) {
     conv_kernel_setup_once();
-    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4);
+    const int es = kind == 0 ? 1 : 2;
     act_ = do_relu_ ? 1 : 0;
     alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.size()) + (kind == 0 ? 12.0 : 4.0) * g_.oc;
     DenseLayer d;
@@ -633,7 +696,6 @@ public:
     ConvPlan pl;
     std::memset(&pl.p, 0, sizeof(pl.p));
     pl.bf16 = kind == 1;
-    pl.tf32 = kind == 2;
     pl.in = (const int8_t *)in_->dev;
     pl.ops = alg_ops;
     ConvGemmParams &p = pl.p;
@@ -661,16 +723,6 @@ public:
     p.kh = g.kh; p.kw = g.kw;
     if (wp) setup_window(I, pl, *wp, filt, kind);
     else setup_blocks(I, pl, d, kind);
-    if (kind == 2 && pl.q.parts > 1) { // partial sums to a workspace, bias and activation in the reducing pass
-      pl.reduce_out = (float *)p.out;
-      pl.reduce_bias = (const float *)p.bias;
-      pl.reduce_bytes = out_->bytes();
-      pl.reduce_act = p.act;
-      pl.q.part_bytes = out_->bytes();
-      p.out = (int8_t *)I.dalloc(out_->bytes() * pl.q.parts);
-      p.act = 0;
-      p.bias = I.upload(std::vector<int32_t>(d.out_cp, 0));
-    }
     I.attach_split_ws(pl);
     plans_.push_back(pl);
   }
@@ -678,7 +730,7 @@ public:
   // else a copy of its rows is made before the launch.
   void setup_window(Interpreter &I, ConvPlan &pl, const WindowPlan &wp, const std::vector<float> &filt, int kind) {
     const ConvGeom &g = g_;
-    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4);
+    const int es = kind == 0 ? 1 : 2;
     ConvGemmParams &p = pl.p;
     const void *rows = in_->dev;
     if (in_->cp * es != wp.P || in_->wl != g.pl || in_->wphys != wp.wphys) {
@@ -698,68 +750,31 @@ public:
     p.ldc_px = p.ldc;
     p.ldc *= wp.G;
     finish_plan(pl, g.n * g.oh * p.OW, g.kh, wp.win, out_->cp, I.sm_count);
-    const int w_rows = wp.G > 1 ? 128 : out_->cp, n_tiles = (out_->cp + 127) / 128;
-    if (kind == 2) {
-      finish_tf32_plan(pl, plain_tap_tiles(p, 1, p.M_total), n_tiles, I.sm_count);
-    } else if (kind == 1) {
-      p.idesc = make_idesc_bf16(128, p.BN);
-    }
-    auto weights = [&](CUtensorMap *tm, int part) {
-      encode_weight_map(tm, I.upload(pack_window_weights(filt.data(), g, wp, w_rows, p.BK, part)), w_rows, g.kh, p.BK, p.BK,
-                        p.dual ? 192 : 128);
-    };
-    weights(&pl.tmB, kind == 0 ? -2 : (kind == 1 ? -1 : 0));
-    if (kind == 2) weights(&pl.tmB2, 1);
+    const int w_rows = wp.G > 1 ? 128 : out_->cp;
+    if (kind == 1) p.idesc = make_idesc_bf16(128, p.BN);
+    encode_weight_map(&pl.tmB, I.upload(pack_window_weights(filt.data(), g, wp, w_rows, p.BK, kind == 1)), w_rows, g.kh, p.BK, p.BK,
+                      p.dual ? 192 : 128);
     encode_window_map(&pl.tmA, rows, g, wp, p.BK, a_tile_rows(p));
   }
   void setup_blocks(Interpreter &I, ConvPlan &pl, const DenseLayer &d, int kind) {
     const ConvGeom &g = d.g;
     ConvGemmParams &p = pl.p;
-    const int es = kind == 0 ? 1 : (kind == 1 ? 2 : 4), k_bytes = d.in_cp * es, rows = g.n * g.oh * g.ow;
+    const int es = kind == 0 ? 1 : 2, k_bytes = d.in_cp * es, rows = g.n * g.oh * g.ow;
     const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.oh == g.ih && g.ow == g.iw;
-    const int taps = g.kh * g.kw, n_tiles = (d.out_cp + 127) / 128;
+    const int taps = g.kh * g.kw;
     p.a_mode = one ? 0 : 1;
     finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count);
-    if (kind == 2) {
-      const int all = (k_bytes + 31) / 32;
-      TapParams q = plain_tap_tiles(p, one ? 0 : 1, rows), t;
-      double t_clocks = 0;
-      int skip = 0, keep = 1 << 20; // steps of K that tap blocks skip
-      if (d.paired && k_bytes % 64 == 0) {
-        if (g_.pl % 2) skip = all / 2;
-        if ((1 + (g_.kw - 1) * g_.dw - g_.pl) % 2 == 0) keep = all / 2;
-      }
-      const double steps = (double)g.kh * (g.kw * all - skip - std::max(all - keep, 0));
-      if (taps > 1 && choose_tap_tile(g, k_bytes, n_tiles, steps, I.sm_count, &t, &t_clocks) &&
-          t_clocks < tf32_clocks(q, 1, p.BK, (double)taps * all, n_tiles, I.sm_count)) {
-        q = t;
-        q.skip_first = skip;
-        q.keep_last = keep;
-      }
-      finish_tf32_plan(pl, q, n_tiles, I.sm_count);
-      if (q.mode == 2) encode_block_map(&pl.tmA, in_->dev, g, k_bytes, p.BK, q);
-    } else if (kind == 1) {
-      p.idesc = make_idesc_bf16(128, p.BN);
-    }
-    if (pl.q.mode != 2) {
-      if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-      else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, a_tile_rows(p));
-    }
+    if (kind == 1) p.idesc = make_idesc_bf16(128, p.BN);
+    if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
+    else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, a_tile_rows(p));
     // A tap's weights are padded to whole K blocks: rows that start off 32-byte sectors and reach past the extent arrive at
     // a third of the rate (7 x 45 x 45 pixels, 80 -> 128 channels, 5x5: 35.9 -> 28.3 us; MobileNet-v2 batch 32 426 -> 408).
-    auto weights = [&](CUtensorMap *tm, const std::vector<int8_t> &w) {
-      const size_t pitch = (size_t)p.c_chunks * p.BK, rows = (size_t)d.out_cp * taps;
-      std::vector<int8_t> v(rows * pitch, 0);
-      for (size_t i = 0; i < rows; ++i) std::memcpy(v.data() + i * pitch, w.data() + i * k_bytes, k_bytes);
-      encode_weight_map(tm, I.upload(v), d.out_cp, taps, (int)pitch, p.BK, p.dual ? 192 : 128);
-    };
-    const float *w = d.w.data();
-    if (kind == 0) weights(&pl.tmB, pack_conv_weights(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, false, 0));
-    else if (kind == 1) weights(&pl.tmB, pack_conv_weights_bf16(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp));
-    else {
-      weights(&pl.tmB, pack_conv_weights_tf32(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, 0));
-      weights(&pl.tmB2, pack_conv_weights_tf32(w, g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, 1));
-    }
+    const std::vector<int8_t> w = kind == 0 ? pack_conv_weights(d.w.data(), g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, false, 0)
+                                            : pack_conv_weights_bf16(d.w.data(), g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp);
+    const size_t pitch = (size_t)p.c_chunks * p.BK, w_rows = (size_t)d.out_cp * taps;
+    std::vector<int8_t> v(w_rows * pitch, 0);
+    for (size_t i = 0; i < w_rows; ++i) std::memcpy(v.data() + i * pitch, w.data() + i * k_bytes, k_bytes);
+    encode_weight_map(&pl.tmB, I.upload(v), d.out_cp, taps, (int)pitch, p.BK, p.dual ? 192 : 128);
   }
   // Fused leaky ReLU (tensor-core plans only): the epilogue writes the plain result to this op's tensor
   // and the activation result to `act_out`.
@@ -791,6 +806,15 @@ public:
   }
   const TensorPtr &out() const { return out_; }
   const TensorPtr &in() const { return in_; }
+  // TF32 x 3 plans (not the patch-matrix stem, whose remainder belongs to the patch matrix)
+  bool is_tf32() const { return can_write_remainder() && !plans_[0].use_patch; }
+  bool can_write_remainder() const { return !plans_.empty() && plans_[0].tf32; }
+  void set_remainder_out(void *lo) {
+    for (auto &pl : plans_) pl.p.out2 = (int8_t *)lo;
+  }
+  void skip_split() {
+    for (auto &pl : plans_) pl.split_src = nullptr;
+  }
   void invoke(cudaStream_t s) override {
     if (bf16g_) {
       ConvBf16GroupArgs a{g_.n, g_.ic, in_->cp, g_.ih, g_.iw, g_.oc, out_->cp, g_.oh, g_.ow, g_.kh, g_.kw, g_.sh, g_.sw,
@@ -833,7 +857,7 @@ public:
   int kernel_launches() const override {
     if (f32_ || dw_ || bf16g_) return 1;
     int k = 0;
-    for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack ? 1 : 0) + (pl.q.parts > 1 ? 1 : 0);
+    for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack || pl.split_src ? 1 : 0);
     return k;
   }
   bool is_tensor_core() const { return !f32_ && !dw_ && !bf16g_; }
@@ -1121,6 +1145,9 @@ public:
   }
   // INT8 two-input add that a producing convolution's epilogue can take over
   bool is_plain_i8_add() const { return out_->dtype == DT_I8 && !is_mul_ && ins_.size() == 2; }
+  // fp32 add whose result feeds a TF32 x 3 convolution: also write that convolution's remainder operand
+  bool can_write_remainder() const { return out_->dtype == DT_F32 && !is_mul_; }
+  void set_remainder_out(float *lo) { f_.lo = lo; }
   const std::vector<TensorPtr> &inputs() const { return ins_; }
   const TensorPtr &out() const { return out_; }
   const EltwiseArgs &i8_args() const { return a_; }
@@ -1167,7 +1194,7 @@ private:
   bool is_mul_;
   int do_relu_ = 0;
   EltwiseArgs a_;
-  EltwiseF32Args f_;
+  EltwiseF32Args f_ = {};
   EltwiseBf16Args b_;
 };
 
@@ -1781,6 +1808,38 @@ inline ParsedOp parse_line(const std::string &line) {
   return op;
 }
 
+// Who writes the remainder operand (x minus the upper 19 bits of x) of the fp32 tensors that TF32 x 3 convolutions read:
+// the kernel that produces the tensor when it can (an fp32 eltwise add or another TF32 x 3 convolution: 4 more bytes
+// written per value, no separate pass), else the split pass of the FIRST convolution that reads it; later readers of
+// the same tensor reuse the buffer. Ops run in program order, so the first reader always runs before the others.
+inline void Interpreter::link_tf32_remainders() {
+  for (auto &k : kernels) {
+    auto *cv = dynamic_cast<Conv2DOp *>(k.get());
+    if (!cv || !cv->is_tf32()) continue;
+    DevTensor *t = cv->in().get();
+    if (t->lo_by != 0) { // already filled by the producer or by an earlier reader
+      cv->skip_split();
+      continue;
+    }
+    OpKernel *prod = nullptr;
+    for (auto &q : kernels)
+      if (q->result.get() == t) prod = q.get();
+    if (auto *pe = dynamic_cast<EltwiseOp *>(prod)) {
+      if (pe->can_write_remainder()) {
+        pe->set_remainder_out((float *)t->lo_dev);
+        t->lo_by = 1;
+      }
+    } else if (auto *pc = dynamic_cast<Conv2DOp *>(prod)) {
+      if (pc->can_write_remainder()) {
+        pc->set_remainder_out(t->lo_dev);
+        t->lo_by = 1;
+      }
+    }
+    if (t->lo_by == 1) cv->skip_split();
+    else t->lo_by = 2; // this convolution's split pass fills it
+  }
+}
+
 // Replaces every quant(INT8->BF16) -> slope-table activation -> quant(BF16->INT8) chain whose
 // intermediates feed nothing else by one ActChainOp at the first op's position.
 inline void Interpreter::fuse_activation_chains(const std::map<std::string, int> &uses) {
@@ -2059,6 +2118,7 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
 
 inline void Interpreter::finish_module() {
   if (fuse_activations) fuse_activation_chains(uses);
+  link_tf32_remainders();
   output_details.clear();
   for (auto &k : kernels)
     if (!uses.count(k->name) && k->op_type != "input") output_details.push_back({k->name, k->result->numel() / (size_t)max_batch});

@@ -372,6 +372,7 @@ struct EltwiseF32Args {
   float coeff[4];
   int nin;
   int do_relu;
+  float *lo; // when set: also write x - (upper 19 bits of x), the remainder operand of a TF32 x 3 convolution that reads x
 };
 // One 16-byte vector per thread and step (fp32 tensors are a whole number of them: the channel pitch is a
 // multiple of 4); operand by operand, product and sum rounded separately, as the reference's loop.
@@ -396,6 +397,7 @@ __global__ void eltwise_add_f32_kernel(EltwiseF32Args a, float *__restrict__ out
       acc.w = acc.w < 0 ? 0.0f : acc.w;
     }
     reinterpret_cast<float4 *>(out)[i] = acc;
+    if (a.lo) reinterpret_cast<float4 *>(a.lo)[i] = tf32_remainder(acc);
   }
 }
 
@@ -793,6 +795,25 @@ __global__ void patch_expand_i8_kernel(const int8_t *__restrict__ in, int8_t *__
       }
     }
     out[i] = v;
+  }
+}
+
+// fp32 image stems of at most 4 channels (NHWC4): every filter tap keeps four channel slots in the patch matrix,
+// k = tap * 4 + c, so a thread copies one tap of one output pixel as one 16-byte vector and writes its TF32 remainder.
+__global__ void patch_expand_f32_kernel(const float4 *__restrict__ in, float4 *__restrict__ out, float4 *__restrict__ lo, PatchArgs a) {
+  pdl_prologue();
+  const int taps = a.kh * a.kw;
+  const size_t total = (size_t)a.n * a.oh * a.ow * taps;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int tap = (int)(i % taps);
+    const size_t pix = i / taps, t = pix / a.ow;
+    const int x = (int)(pix % a.ow), y = (int)(t % a.oh), b = (int)(t / a.oh);
+    const int s = tap % a.kw, r = tap / a.kw;
+    const int yy = y * a.sh - a.pt + r * a.dh, xx = x * a.sw - a.pl + s * a.dw;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (yy >= 0 && yy < a.ih && xx >= 0 && xx < a.iw) v = __ldg(in + ((size_t)b * a.ih + yy) * a.iw + xx);
+    out[i] = v;
+    lo[i] = tf32_remainder(v);
   }
 }
 
