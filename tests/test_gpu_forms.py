@@ -89,6 +89,7 @@ def test_row_window_conv_float(dtype, case):
     (2, 40, 136, 13, 3, 1, 2, 2), (1, 64, 130, 31, 3, 1, 1, 1), (1, 72, 80, 57, 5, 1, 1, 1),  # odd extents, ragged tiles
     (1, 512, 64, 9, 3, 1, 1, 1), (1, 256, 200, 5, 1, 1, 0, 1),  # few tiles and a long K
     (2, 80, 64, 13, 3, 2, 1, 1), (7, 72, 72, 12, 5, 1, 2, 1), (2, 144, 160, 9, 3, 1, 1, 1),  # channels off the sector grid
+    (1, 64, 256, 55, 1, 1, 0, 1), (1, 64, 256, 56, 1, 1, 0, 1),  # the last half tiles and the first whole ones (148 SMs)
     (2, 64, 96, 11, 3, 2, 1, 1)])   # a stride
 def test_conv_forms(dtype, case):
     n, ic, oc, hw, k, s, p, d = case

@@ -39,6 +39,7 @@ struct ConvGemmParams {
   int kh, kw;     // filter size (taps = kh*kw; 1 in tiled mode)
   int c_chunks;   // ceil(Cin_pad / BK)
   int BK;         // K bytes per pipeline stage: 32, 64 or 128 (= swizzle span)
+  int m_tile;     // pixels per tile: 256 in dual mode, else 128 or 64 = the tensor core's N
   int BN;         // channel tile = tensor-core M, always 128 (rows past n_valid are zero-filled)
   int n_valid;    // number of valid (padded) output channels
   int ldc;        // output row pitch in bytes
@@ -683,7 +684,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
   // starting 64 rows BEFORE the first channel, i.e. [64 zero rows][64 weight rows][64 zero rows]; rows
   // 64..191 of it ([W; 0]) times the first 128 pixels fill TMEM lanes 0..63, rows 0..127 ([0; W]) times
   // the second 128 pixels accumulate into lanes 64..127, so all 128 lanes (and all epilogue warps) work.
-  const int m_tile = p.dual ? 256 : 128;
+  const int m_tile = p.m_tile, ncols = p.dual ? 128 : m_tile;
   const int m_tiles = (p.M_total + m_tile - 1) / m_tile;
   int total_tiles = n_tiles * m_tiles; // set to 0 below when the launch is already marked as failed
   const uint32_t a_bytes = (uint32_t)m_tile * (uint32_t)p.BK;
@@ -1007,7 +1008,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           // this CTA's partial accumulator goes to the tile's block in global memory (one reduction per value,
           // 128 contiguous bytes per warp and column)
           const uint32_t lane_addr = tmem_base + (uint32_t)buf * acc_stride + ((uint32_t)(quarter * 32) << 16);
-          for (int colg = half * 32; colg < 128; colg += 32 * (kEpilogueWarps / 4)) {
+          for (int colg = half * 32; colg < ncols; colg += 32 * (kEpilogueWarps / 4)) {
             if (m0 + colg >= p.M_total) break;
             uint32_t a0[16], a1[16];
             ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, a0);
@@ -1059,21 +1060,21 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           // byte addressing: 4 bytes per channel
           const int ch = n0 + ch_base + lane;
           uint8_t *out_ch = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch) * 4;
-          if (p.act == 1) epilogue_channels_f32<true>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
-          else epilogue_channels_f32<false>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f);
+          if (p.act == 1) epilogue_channels_f32<true>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f, ncols);
+          else epilogue_channels_f32<false>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f, ncols);
         } else if (BF16) {
           // byte addressing: 2 bytes per channel, this lane's pair starts at its even channel
           const int ch = n0 + ch_base + lane;
           uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + (ch & ~1)) * 2;
-          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
-          else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f);
+          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
+          else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
         } else if constexpr (FQ) {
-          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, fq, ts, 128);
-        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128);
-        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
-        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, 128, ws_lane);
+          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, fq, ts, ncols);
+        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
+        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
+        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols);
+        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
+        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
       }
       if (SPLIT && ws_lane) continue; // split K: the accumulator buffer was handed back above
       // hand the accumulator buffer back to the MMA issuer

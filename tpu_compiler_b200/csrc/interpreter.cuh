@@ -604,7 +604,7 @@ public:
         p.kh = p.kw = 1;
         p.a_mode = 0;
         finish_plan(pl, rows, 1, a.kp, ocg_pad, I.sm_count);
-        encode_matrix_map(&pl.tmA, pl.patch_buf, rows, a.kp, a.kp, p.BK, a_tile_rows(p));
+        encode_matrix_map(&pl.tmA, pl.patch_buf, rows, a.kp, a.kp, p.BK, p.m_tile);
         encode_weight_map(&pl.tmB, d_w, ocg_pad, 1, a.kp, p.BK, p.dual ? 192 : p.BN);
       }
       if (I.selftest_lost_arrival > 0) {
@@ -669,12 +669,11 @@ public:
       for (int part = 0; part < 2; ++part) w[part] = pack_conv_weights_tf32(filt.data(), g.oc, g.ic, g.kh, g.kw, out_cp, in_->cp, part);
     }
     finish_plan(pl, rows, taps, k_bytes, out_cp, I.sm_count);
-    p.idesc = make_idesc_tf32(128, p.BN);
     const int8_t *part[2] = {stem ? pl.patch_buf : (const int8_t *)in_->dev, (const int8_t *)pl.split_lo};
     for (int k = 0; k < 2; ++k) {
       CUtensorMap *a = k ? &pl.tmA2 : &pl.tmA;
-      if (p.a_mode == 0) encode_matrix_map(a, part[k], rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-      else encode_im2col_map(a, part[k], g, k_bytes, p.BK, a_tile_rows(p));
+      if (p.a_mode == 0) encode_matrix_map(a, part[k], rows, k_bytes, k_bytes, p.BK, p.m_tile);
+      else encode_im2col_map(a, part[k], g, k_bytes, p.BK, p.m_tile);
       encode_weight_map(k ? &pl.tmB2 : &pl.tmB, I.upload(w[k]), out_cp, taps, k_bytes, p.BK, p.BN);
     }
     plans_.push_back(pl);
@@ -751,10 +750,9 @@ public:
     p.ldc *= wp.G;
     finish_plan(pl, g.n * g.oh * p.OW, g.kh, wp.win, out_->cp, I.sm_count);
     const int w_rows = wp.G > 1 ? 128 : out_->cp;
-    if (kind == 1) p.idesc = make_idesc_bf16(128, p.BN);
     encode_weight_map(&pl.tmB, I.upload(pack_window_weights(filt.data(), g, wp, w_rows, p.BK, kind == 1)), w_rows, g.kh, p.BK, p.BK,
                       p.dual ? 192 : 128);
-    encode_window_map(&pl.tmA, rows, g, wp, p.BK, a_tile_rows(p));
+    encode_window_map(&pl.tmA, rows, g, wp, p.BK, p.m_tile);
   }
   void setup_blocks(Interpreter &I, ConvPlan &pl, const DenseLayer &d, int kind) {
     const ConvGeom &g = d.g;
@@ -764,9 +762,8 @@ public:
     const int taps = g.kh * g.kw;
     p.a_mode = one ? 0 : 1;
     finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count);
-    if (kind == 1) p.idesc = make_idesc_bf16(128, p.BN);
-    if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, a_tile_rows(p));
-    else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, a_tile_rows(p));
+    if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, p.m_tile);
+    else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, p.m_tile);
     // A tap's weights are padded to whole K blocks: rows that start off 32-byte sectors and reach past the extent arrive at
     // a third of the rate (7 x 45 x 45 pixels, 80 -> 128 channels, 5x5: 35.9 -> 28.3 us; MobileNet-v2 batch 32 426 -> 408).
     const std::vector<int8_t> w = kind == 0 ? pack_conv_weights(d.w.data(), g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, false, 0)
@@ -929,9 +926,8 @@ public:
       p.act = do_relu_ ? 1 : 0;
       p.a_mode = 0;
       finish_plan(pl, m_, 1, kdev_ * 2, n_pad, I.sm_count);
-      encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_ * 2, kdev_ * 2, p.BK, a_tile_rows(p));
+      encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_ * 2, kdev_ * 2, p.BK, p.m_tile);
       encode_weight_map(&pl.tmB, d_w, n_pad, 1, kdev_ * 2, p.BK, p.dual ? 192 : p.BN);
-      p.idesc = make_idesc_bf16(128, p.BN);
       I.attach_split_ws(pl);
       plan_ = pl;
       alg_bytes = 2.0 * ((double)m_ * k_ + (double)n_ * k_ + (double)m_ * n_) + 4.0 * n_;
@@ -985,7 +981,7 @@ public:
     if (!fq.empty()) p.fq = I.upload(fq);
     p.a_mode = 0;
     finish_plan(pl, m_, 1, kdev_, n_pad, I.sm_count);
-    encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_, kdev_, p.BK, a_tile_rows(p));
+    encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_, kdev_, p.BK, p.m_tile);
     encode_weight_map(&pl.tmB, d_w, n_pad, 1, kdev_, p.BK, p.dual ? 192 : p.BN);
     I.attach_split_ws(pl);
     plan_ = pl;
