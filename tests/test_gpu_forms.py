@@ -134,3 +134,49 @@ def test_large_result_read_before_the_end(graph):
         for name in (["early", "late", "early"], ["late", "early", "p"])[i % 2]:
             assert np.array_equal(m.get_tensor(name), ref[name]), (i, name)
     m.close()
+
+
+@pytest.mark.parametrize("dtype", ["INT8", "BF16"])
+@pytest.mark.parametrize("case", [  # n, c, hw, k, stride, pad, out
+    (2, 48, 17, 3, 2, 1, 9), (1, 16, 16, 3, 2, 0, 8), (2, 40, 13, 3, 1, 1, 13), (1, 16, 5, 2, 2, 0, 3), (3, 32, 8, 2, 2, 1, 5),  # strips
+    (2, 16, 13, 13, 1, 6, 13), (1, 80, 13, 9, 1, 4, 13), (2, 64, 7, 5, 1, 2, 7), (1, 32, 28, 7, 1, 3, 28),  # planes, the last too large for one
+    (1, 32, 9, 4, 3, 1, 3), (2, 32, 6, 3, 3, 0, 2)])  # any window
+def test_max_pool_forms(dtype, case):
+    n, c, hw, k, s, p, o = case
+    rng = np.random.default_rng(60 + hw + k)
+    x = rng.integers(-128, 128, (n, c, hw, hw)).astype(np.float32) if dtype == "INT8" else graphs._bf16_np(rng.normal(0, 3, (n, c, hw, hw)))
+    text = ("input name=x shape=%d,%d,%d,%d dtype=%s\npool_max_2d name=p in=x shape=%d,%d,%d,%d dtype=%s kh=%d kw=%d sh=%d sw=%d pt=%d pb=%d "
+            "pl=%d pr=%d\n" % (n, c, hw, hw, dtype, n, c, o, o, dtype, k, k, s, s, p, p, p, p))
+    got, ref = run_model(text, {}, {"x": x}, ["p"])["p"]
+    assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("channels", [[16, 48], [32], [16] * 8, [16, 32, 16, 16, 48, 16, 16, 64, 32]])
+def test_concat_in_one_launch(channels):
+    rng = np.random.default_rng(len(channels))
+    shapes = ["input name=x%d shape=2,%d,5,7 dtype=INT8\n" % (i, c) for i, c in enumerate(channels)]
+    names = ["x%d" % i for i in range(len(channels))]
+    w = {"r": (7 * (np.arange(len(channels)) % 2)).astype(np.float32), "m": np.where(np.arange(len(channels)) % 2, 90, 1).astype(np.float32)}
+    text = "".join(shapes) + "concat name=y in=%s,-,-,r,m shape=2,%d,5,7 dtype=INT8 axis=1 do_relu=0\n" % (",".join(names), sum(channels))
+    x = {nm: rng.integers(-128, 128, (2, c, 5, 7)).astype(np.float32) for nm, c in zip(names, channels)}
+    got, ref = run_model(text, w, x, ["y"])["y"]
+    assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype", ["INT8", "BF16"])
+def test_upsample_vectors(dtype):
+    x = np.random.default_rng(2).integers(-128, 128, (2, 48, 5, 6)).astype(np.float32)
+    text = "input name=x shape=2,48,5,6 dtype=%s\nupsample name=u in=x shape=2,48,15,12 dtype=%s scale_h=3 scale_w=2\n" % (dtype, dtype)
+    got, ref = run_model(text, {}, {"x": x}, ["u"])["u"]
+    assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+def test_bf16_add_operand_counts(count):
+    rng = np.random.default_rng(count)
+    names = ["x%d" % i for i in range(count)]
+    text = "".join("input name=%s shape=3,24,9,11 dtype=BF16\n" % nm for nm in names)
+    text += "eltwise_add name=y in=%s shape=3,24,9,11 dtype=BF16 do_relu=1\n" % ",".join(names)
+    x = {nm: graphs._bf16_np(rng.normal(0, 2, (3, 24, 9, 11))) for nm in names}
+    got, ref = run_model(text, {}, x, ["y"])["y"]
+    assert np.array_equal(got, ref)

@@ -1069,7 +1069,34 @@ public:
     a_ = a;
     alg_bytes = ((double)in->numel() + out->numel()) * in->elsize();
   }
+  // max pooling of INT8 and BF16: strips of 3x3 and 2x2 windows, planes with large ones
+  bool max_pool_fast(cudaStream_t s) {
+    if (in_->dtype == DT_F32 || in_->padded_rows() || out_->padded_rows() || in_->cp != out_->cp) return false;
+    const PoolArgs &a = a_;
+    const bool bf16 = in_->dtype == DT_BF16;
+    const int vecs = in_->cp * (bf16 ? 2 : 1) / 16, vb = vecs % 2 == 0 ? 2 : 1;
+    const uint4 *src = (const uint4 *)in_->dev;
+    uint4 *dst = (uint4 *)out_->dev;
+    const size_t plane = (size_t)a.ih * a.iw * vb * 32;
+    if (a.sh == 1 && a.sw == 1 && a.oh == a.ih && a.ow == a.iw && a.kh * a.kw >= 25 && a.pt >= 0 && a.pl >= 0 && a.pt < a.kh &&
+        a.pl < a.kw && plane <= kPoolPlaneBytes) {
+      const int threads = std::min(512, (a.ih * a.iw * vb + 31) / 32 * 32), grid = a.n * (vecs / vb);
+      if (bf16) launch_k(pool_max_plane_kernel<true>, grid, threads, plane, s, src, dst, a, vecs, vb);
+      else launch_k(pool_max_plane_kernel<false>, grid, threads, plane, s, src, dst, a, vecs, vb);
+      return true;
+    }
+    auto strips = [&](auto i8, auto b16, int xs) {
+      const size_t total = (size_t)a.n * a.oh * ((a.ow + xs - 1) / xs) * vecs;
+      launch_k(bf16 ? b16 : i8, grid_for(total, 128, I_.sm_count), 128, 0, s, src, dst, a, vecs);
+      return true;
+    };
+    if (pool_strips(a, 3, 2)) return strips(pool_max_strip_kernel<false, 3, 2, 2>, pool_max_strip_kernel<true, 3, 2, 2>, 2);
+    if (pool_strips(a, 3, 1)) return strips(pool_max_strip_kernel<false, 3, 1, 4>, pool_max_strip_kernel<true, 3, 1, 4>, 4);
+    if (pool_strips(a, 2, 2)) return strips(pool_max_strip_kernel<false, 2, 2, 2>, pool_max_strip_kernel<true, 2, 2, 2>, 2);
+    return false;
+  }
   void invoke(cudaStream_t s) override {
+    if (a_.method == 0 && max_pool_fast(s)) return;
     if (in_->dtype == DT_I8) {
       size_t total = out_->pixels() * (out_->cp / 16);
       if (a_.method == 0)
@@ -1158,8 +1185,18 @@ public:
   void invoke(cudaStream_t s) override {
     if (out_->dtype == DT_BF16) {
       size_t nvec = out_->bytes() / 16;
-      if (is_mul_) launch_k(eltwise_bf16_kernel<true>, grid_for(nvec, 256, I_.sm_count), 256, 0, s, b_, (uint4 *)out_->dev, nvec);
-      else launch_k(eltwise_bf16_kernel<false>, grid_for(nvec, 256, I_.sm_count), 256, 0, s, b_, (uint4 *)out_->dev, nvec);
+      auto go = [&](auto mul, auto nin) {
+        launch_k(eltwise_bf16_kernel<decltype(mul)::value, decltype(nin)::value>, grid_for(nvec, 256, I_.sm_count), 256, 0, s, b_,
+                 (uint4 *)out_->dev, nvec);
+      };
+      auto by_count = [&](auto mul) {
+        if (b_.nin == 1) go(mul, std::integral_constant<int, 1>());
+        else if (b_.nin == 2) go(mul, std::integral_constant<int, 2>());
+        else if (b_.nin == 3) go(mul, std::integral_constant<int, 3>());
+        else go(mul, std::integral_constant<int, 4>());
+      };
+      if (is_mul_) by_count(std::true_type());
+      else by_count(std::false_type());
     } else if (out_->dtype == DT_I8) {
       size_t nvec = out_->bytes() / 16;
       if (is_mul_) launch_k(eltwise_mul_i8_kernel, grid_for(nvec, 256, I_.sm_count), 256, 0, s, a_, (int8_t *)out_->dev, nvec);
@@ -1226,26 +1263,40 @@ public:
   void invoke(cudaStream_t s) override {
     int off = 0; // in bytes of a pixel row of the output
     const int ocp = out_->cp * es_;
+    if (vectors()) { // one launch for up to eight inputs
+      for (size_t first = 0; first < ins_.size(); first += kConcatInputs) {
+        ConcatArgs a = {};
+        const size_t count = std::min<size_t>(kConcatInputs, ins_.size() - first);
+        int widest = 0;
+        for (size_t k = 0; k < count; ++k) {
+          const DevTensor &t = *ins_[first + k];
+          const int cb = t.c * es_, m = mult_[first + k], r = rsh_[first + k];
+          a.in[k] = ConcatInput{(const uint4 *)t.dev, cb / 16, t.cp * es_ / 16, off / 16, m, r, need_quant_ && !(m == 1 && r == 0)};
+          widest = std::max(widest, cb / 16);
+          off += cb;
+        }
+        const int grid = grid_for(out_->pixels() * widest, 256, I_.sm_count);
+        launch_k(concat_slice_i8_vec_kernel, dim3((unsigned)grid, (unsigned)count), 256, 0, s, a, (uint4 *)out_->dev, out_->pixels(),
+                 ocp / 16, do_relu_);
+      }
+      return;
+    }
     for (size_t i = 0; i < ins_.size(); ++i) {
       auto &t = ins_[i];
       const int cb = t->c * es_, cpb = t->cp * es_; // channel bytes: BF16 moves as two bytes per channel
-      size_t total = t->pixels() * cb;
-      int requant = need_quant_ && !(mult_[i] == 1 && rsh_[i] == 0);
-      if (cb % 16 == 0 && off % 16 == 0 && cpb % 16 == 0 && ocp % 16 == 0) {
-        size_t nvec = t->pixels() * (cb / 16);
-        launch_k(concat_slice_i8_vec_kernel, grid_for(nvec, 256, I_.sm_count), 256, 0, s, 
-            (const uint4 *)t->dev, (uint4 *)out_->dev, t->pixels(), cb / 16, cpb / 16, ocp / 16, off / 16,
-            mult_[i], rsh_[i], requant, do_relu_);
-        off += cb;
-        continue;
-      }
-      launch_k(concat_slice_i8_kernel, grid_for(total, 256, I_.sm_count), 256, 0, s, 
-          (const int8_t *)t->dev, (int8_t *)out_->dev, t->pixels(), cb, cpb, ocp, off, mult_[i], rsh_[i],
-          requant, do_relu_);
+      const int requant = need_quant_ && !(mult_[i] == 1 && rsh_[i] == 0);
+      launch_k(concat_slice_i8_kernel, grid_for(t->pixels() * cb, 256, I_.sm_count), 256, 0, s, (const int8_t *)t->dev, (int8_t *)out_->dev,
+               t->pixels(), cb, cpb, ocp, off, mult_[i], rsh_[i], requant, do_relu_);
       off += cb;
     }
   }
-  int kernel_launches() const override { return (int)ins_.size(); }
+  // every slice is whole 16-byte vectors at a 16-byte place
+  bool vectors() const {
+    bool ok = out_->cp * es_ % 16 == 0;
+    for (auto &t : ins_) ok = ok && t->c * es_ % 16 == 0 && t->cp * es_ % 16 == 0 && t->pixels() == out_->pixels();
+    return ok;
+  }
+  int kernel_launches() const override { return vectors() ? ((int)ins_.size() + kConcatInputs - 1) / kConcatInputs : (int)ins_.size(); }
 
 private:
   Interpreter &I_;
@@ -1274,6 +1325,12 @@ public:
     alg_bytes = ((double)in->numel() + out->numel()) * in->elsize();
   }
   void invoke(cudaStream_t s) override {
+    if (a_.mode == 0 && a_.icp == a_.ocp && a_.ic == a_.oc && a_.ocp * a_.es % 16 == 0) {
+      const int vecs = a_.ocp * a_.es / 16;
+      launch_k(upsample_vec_kernel, grid_for(out_->pixels() * vecs, 256, I_.sm_count), 256, 0, s, (const uint4 *)in_->dev,
+               (uint4 *)out_->dev, a_, vecs);
+      return;
+    }
     size_t total = out_->pixels() * out_->cp;
     launch_k(move_kernel, grid_for(total, 256, I_.sm_count), 256, 0, s, (const uint8_t *)in_->dev, (uint8_t *)out_->dev, a_);
   }
