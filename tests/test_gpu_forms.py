@@ -180,3 +180,21 @@ def test_bf16_add_operand_counts(count):
     x = {nm: graphs._bf16_np(rng.normal(0, 2, (3, 24, 9, 11))) for nm in names}
     got, ref = run_model(text, {}, x, ["y"])["y"]
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("relu", [0, 1])
+@pytest.mark.parametrize("case", [(1, 16, 9, 1), (2, 32, 7, 2), (32, 192, 15, 1), (40, 192, 21, 2)])  # n, c, hw, stride: one row, two rows
+@pytest.mark.parametrize("wide", [False, True])  # True: a channel outside the floating-point requantisation
+def test_depthwise_rows_and_requantisation(relu, case, wide):
+    n, c, hw, s = case
+    rng = np.random.default_rng(c + hw)
+    o = (hw - 1) // s + 1
+    w = {"f": rng.integers(-127, 128, (c, 1, 3, 3)).astype(np.float32), "b": rng.integers(-5000, 5000, c).astype(np.float32),
+         "r": rng.integers(6, 11, c).astype(np.float32), "m": (rng.integers(2 ** 23, 2 ** 24, c) * 128).astype(np.float32)}
+    if wide:
+        w["b"][3] = 2.0 ** 24
+    x = rng.integers(-128, 128, (n, c, hw, hw)).astype(np.float32)
+    text = ("input name=x shape=%d,%d,%d,%d dtype=INT8\nconv_2d name=c in=x,f,b,-,-,r,m shape=%d,%d,%d,%d dtype=INT8 kh=3 kw=3 sh=%d sw=%d "
+            "pt=1 pb=1 pl=1 pr=1 dh=1 dw=1 g=%d do_relu=%d with_bias=1\n" % (n, c, hw, hw, n, c, o, o, s, s, c, relu))
+    got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
+    assert np.array_equal(got, ref)

@@ -228,19 +228,23 @@ constexpr float kFqScale = 7.888609052210118e-31f; // 2^-100
 constexpr double kFqC = 8388608.0 + 2097152.0 - 8.0;
 
 #ifdef __CUDACC__
+// one value, and four of them packed, each with its channel's constants
+template <bool RELU> __device__ __forceinline__ int float_requant1(uint32_t a, const FloatRequant &q) {
+  float u, v;
+  asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(u) : "f"(__uint_as_float(a + q.sb)), "f"(q.m), "f"(q.d));
+  if (RELU) asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(u), "f"(q.c), "f"(q.c * -6.617444900424222e-24f)); // -2^-77: the unit 2^-149 against c's 2^-49
+  else asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(__fsub_rn(u, (float)kFqC * kFqScale)), "f"(q.c), "f"(__uint_as_float(128u)));
+  return __float_as_int(v);
+}
+template <bool RELU> __device__ __forceinline__ uint32_t float_requant_pack(int v0, int v1, int v2, int v3) {
+  if (RELU) return relu_bytes(pack_sat_s8(v1, v0, pack_sat_s8(v3, v2, 0u)));
+  return pack_sat_u8(v1, v0, pack_sat_u8(v3, v2, 0u)) ^ 0x80808080u;
+}
 // four values of one channel, packed
 template <bool RELU>
 __device__ __forceinline__ uint32_t float_requant4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const FloatRequant &q) {
-  const float e = q.c * -6.617444900424222e-24f; // -2^-77: the unit 2^-149 against c's 2^-49
-  auto one = [&](uint32_t a) {
-    float u, v;
-    asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(u) : "f"(__uint_as_float(a + q.sb)), "f"(q.m), "f"(q.d));
-    if (RELU) asm("fma.rm.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(u), "f"(q.c), "f"(e));
-    else asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(__fsub_rn(u, (float)kFqC * kFqScale)), "f"(q.c), "f"(__uint_as_float(128u)));
-    return __float_as_int(v);
-  };
-  if (RELU) return relu_bytes(pack_sat_s8(one(a1), one(a0), pack_sat_s8(one(a3), one(a2), 0u)));
-  return pack_sat_u8(one(a1), one(a0), pack_sat_u8(one(a3), one(a2), 0u)) ^ 0x80808080u;
+  return float_requant_pack<RELU>(float_requant1<RELU>(a0, q), float_requant1<RELU>(a1, q), float_requant1<RELU>(a2, q),
+                                  float_requant1<RELU>(a3, q));
 }
 #endif
 
