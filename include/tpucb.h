@@ -154,12 +154,12 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          copies, frees its tensor memory and returns, and the next tpucb_interp_sync / invoke reports it as an
  *          error status while the interpreter stays usable. With this option the INT8 convolutions of the next
  *          module never hand their accumulator back and wait only `rounds` rounds, so that exactly this happens.
- *          "fuse_residual_add" (0/1, default 0; read by the next load_module; needs fuse_activations): an INT8
+ *          "fuse_residual_add" (0 never, 1 always, 2 = default: by size; read by the next load_module; needs fuse_activations): an INT8
  *          two-input eltwise add whose later-produced operand is a tensor-core convolution that feeds nothing else
  *          (the last convolution of a residual block) runs in that convolution's epilogue, which reads the other
  *          operand and writes both the convolution's tensor and the sum; the add launches nothing. Same bits.
- *          Measured on INT8 ResNet-50 at batch 256: 1% fewer ms per step (the add kernels already run at the
- *          HBM rate and the epilogue is bound by its integer instructions), so it is off by default.
+ *          By size: results of 2.5 to 8 MB of layers that widen their input (INT8 ResNet-50 at batch 19:
+ *          2% fewer us alone, 7% with three modules in flight; at batch 1 and 256 the add is faster by itself).
  *          "fp32_tensor_cores" (0/1, default 1; read by the next load_module): fp32 convolutions with a
  *          multiple of 8 input channels run on the tensor cores as three TF32 products with fp32 accumulation
  *          (about 5e-6 of a tensor's range per layer against a double-accumulated sum, 6e-5 at the end of an

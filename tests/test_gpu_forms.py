@@ -198,3 +198,26 @@ def test_depthwise_rows_and_requantisation(relu, case, wide):
             "pt=1 pb=1 pl=1 pr=1 dh=1 dw=1 g=%d do_relu=%d with_bias=1\n" % (n, c, hw, hw, n, c, o, o, s, s, c, relu))
     got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("case", [(13, 64, 256, 30, 2), (9, 64, 200, 21, 1), (3, 128, 144, 15, 1), (40, 16, 272, 13, 1)])  # n, ic, oc, hw, mode
+def test_residual_add_with_prefetch(case):
+    """Fused adds over several tiles per CTA, ragged tiles and channel tiles that some warps have no part in."""
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, mode = case
+    rng = np.random.default_rng(oc)
+    model = graphs.single_conv_i8(n, ic, oc, hw, 1, 1, 0, relu=False, seed=77)
+    w = dict(model.weights, ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
+    shape = "shape=%d,%d,%d,%d dtype=INT8" % (n, oc, hw, hw)
+    text = "input name=res %s\n" % shape + model.text + "eltwise_add name=s in=res,conv,-,-,ar,am %s do_relu=1\n" % shape
+    x = {"x": model.meta["x"], "res": rng.integers(-128, 128, (n, oc, hw, hw)).astype(np.float32)}
+    ref = graph_runner.run(text, w, x)
+    m = module(0)
+    m.set_option("fuse_residual_add", mode)
+    m.load_text(text, w)
+    for name, v in x.items():
+        m.set_tensor(name, v)
+    for _ in range(2):
+        m.invoke()
+    assert all(np.array_equal(m.get_tensor(k), ref[k]) for k in ("conv", "s"))
+    m.close()

@@ -583,6 +583,78 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
   }
 }
 
+// The same with the fused eltwise add and the floating-point requantisation, for the two 32-pixel chunks of a warp. The
+// residual words come from memory: those of the first chunk were fetched during the tile before (`y`), those of the second
+// are fetched while the first is worked on, and then those of the next tile's first chunk, whose residual begins at `next`
+// (pixel next_m0, this lane's 4-channel group; null: none).
+// Fetched where they are needed, they cost a memory latency per chunk (batch 256 with every add fused: 190 us more than
+// without; prefetched, 30 to 100).
+// (Rows 4 k of a chunk by one wide multiply-add each; one guard for a chunk that lies inside.)
+__device__ __forceinline__ unsigned long long row_addr(const void *base, int k, int ldc) {
+  unsigned long long a;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"((uint32_t)(4 * k)), "r"((uint32_t)ldc), "l"((unsigned long long)base));
+  return a;
+}
+// `first`: the chunk's first pixel; pj: this lane's of every four
+__device__ __forceinline__ void fetch_residual(uint32_t (&y)[8], const int8_t *res, int first, int pj, const ConvGemmParams &p) {
+  if (!res) return;
+  const int8_t *at = res + (size_t)pj * p.ldc;
+  if (first + 32 <= p.M_total) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(y[k]) : "l"(row_addr(at, k, p.ldc)));
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (first + 4 * k + pj < p.M_total) y[k] = __ldg(reinterpret_cast<const uint32_t *>(at + (size_t)(4 * k) * p.ldc));
+  }
+}
+__device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4, bool ch4_ok, int m0, int half,
+                                                int lane, const FloatRequant &q, const TransposeSel &ts, int ncols, uint32_t (&y)[8],
+                                                const int8_t *next, int next_m0) {
+  const int pj = lane & 3, col0 = half * 32, col1 = col0 + 64;
+  const uint32_t mm = (uint32_t)(uint8_t)p.add_ms | ((uint32_t)(uint8_t)p.add_mr << 8);
+  const int rnd = p.add_r > 0 ? (1 << (p.add_r - 1)) : 0, r = p.add_r;
+  const bool relu = p.add_relu != 0;
+  auto chunk = [&](int colg, const uint32_t (&res)[8]) {
+    uint32_t acc0[16], acc1[16];
+    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
+    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
+    ptx::tcgen05_wait_ld();
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q);
+      w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) w[k] = transpose4x4(w[k], ts);
+    if (!ch4_ok) return;
+    int8_t *o = out4 + (size_t)(colg + pj) * p.ldc, *sp = p.out2 + (size_t)(o - p.out);
+    if (m0 + colg + 32 <= p.M_total) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) asm volatile("st.global.b32 [%0], %1;" ::"l"(row_addr(o, k, p.ldc)), "r"(w[k]) : "memory");
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t z = add4_packed(w[k], res[k], mm, rnd, r, relu);
+        asm volatile("st.global.b32 [%0], %1;" ::"l"(row_addr(sp, k, p.ldc)), "r"(z) : "memory");
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (m0 + colg + 4 * k + pj < p.M_total) {
+          *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
+          *reinterpret_cast<uint32_t *>(sp + (size_t)(4 * k) * p.ldc) = add4_packed(w[k], res[k], mm, rnd, r, relu);
+        }
+    }
+  };
+  const bool two = col1 < ncols && m0 + col1 < p.M_total;
+  uint32_t y1[8];
+  if (two) fetch_residual(y1, ch4_ok ? p.res + (out4 - p.out) + (size_t)col1 * p.ldc : nullptr, m0 + col1, pj, p);
+  if (col0 < ncols && m0 + col0 < p.M_total) chunk(col0, y);
+  fetch_residual(y, next ? next + (size_t)col0 * p.ldc : nullptr, next_m0 + col0, pj, p);
+  if (two) chunk(col1, y1);
+}
+
 // Epilogue of a BF16 convolution (core/conv.cpp:90-98: fp32 result + fp32 bias, ReLU, BF16 rounding). The
 // accumulators are fp32; a thread rounds two neighbouring pixels of its channel into one word, exchanges
 // words with the lane of the neighbouring channel and stores two channels of one pixel (a warp writes
@@ -958,6 +1030,16 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     int t = 0;
     bool ok = true;
     int tm = walk_m0, tn = walk_n0;
+    // fused add: the residual of a tile (tm, tn), counted from this lane's 4-channel group; null where it has none
+    uint32_t res_words[8];
+    auto residual_at = [&](int item, int m, int n) -> const int8_t * {
+      const int ch = n * p.BN + quarter * 32 + (lane >> 2) * 4;
+      return item < total_items && ch < p.n_valid ? p.res + (size_t)m * m_tile * p.ldc + p.c_off + ch : nullptr;
+    };
+    if constexpr (ACTSEL == 103) {
+      const int8_t *r = residual_at(blockIdx.x, tm, tn);
+      fetch_residual(res_words, r ? r + (size_t)(half * 32) * p.ldc : nullptr, tm * m_tile + half * 32, lane & 3, p);
+    }
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++t) {
       int tile = item;
       if (split_k > 1) {
@@ -1068,6 +1150,9 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + (ch & ~1)) * 2;
           if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
           else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
+        } else if constexpr (ACTSEL == 103) {
+          epilogue_add_fq(p, lane_addr, out4, ch4_ok, m0, half, lane, fq, ts, ncols, res_words,
+                          residual_at(item + gridDim.x, tm, tn), tm * m_tile);
         } else if constexpr (FQ) {
           epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, fq, ts, ncols);
         } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
@@ -1075,6 +1160,12 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols);
         else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
         else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
+      }
+      if constexpr (ACTSEL == 103) {
+        if (n0 + ch_base >= p.n_valid) { // no outputs here: the next tile's residual all the same
+          const int8_t *r = residual_at(item + gridDim.x, tm, tn);
+          fetch_residual(res_words, r ? r + (size_t)(half * 32) * p.ldc : nullptr, tm * m_tile + half * 32, lane & 3, p);
+        }
       }
       if (SPLIT && ws_lane) continue; // split K: the accumulator buffer was handed back above
       // hand the accumulator buffer back to the MMA issuer

@@ -252,7 +252,7 @@ public:
     split_ws.push_back({pl.p.ws_count, cbytes});
   }
   bool fuse_activations = true; // set before load_module
-  bool fuse_residual_add = false; // set before load_module: eltwise adds run in the producing convolution's epilogue
+  int fuse_residual_add = 2; // set before load_module: eltwise adds in the producing convolution's epilogue: 0 never, 1 always, 2 by size
   bool fp32_tensor_cores = true; // set before load_module: fp32 convolutions as three TF32 products
   void link_tf32_remainders();
   void fuse_activation_chains(const std::map<std::string, int> &uses);
@@ -790,7 +790,7 @@ public:
   // Fused eltwise add (tensor-core INT8 plans without an activation of their own): the epilogue also forms
   // sat8(relu?((conv * ms + residual * mr + 2^(r-1)) >> r)) into `sum_out`; this op's own tensor is still written.
   bool can_fuse_add() const {
-    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1;
+    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1 && !plans_[0].p.dual;
   }
   void set_residual_add(const int8_t *residual, int8_t *sum_out, int ms, int mr, int rshift, int relu) {
     for (auto &pl : plans_) {
@@ -1958,6 +1958,12 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     const int self = pos[0] > pos[1] ? 0 : 1, other = 1 - self;
     auto *cv = dynamic_cast<Conv2DOp *>(kernels[pos[self]].get());
     if (!cv || !cv->can_fuse_add() || !single_use(cv->name)) continue;
+    // By size: layers that widen their input, results of 2.5 to 8 MB. There the launch that goes and the operand that is not
+    // read again count (ResNet-50 batch 19: 496 -> 485 us, three modules in flight 305 -> 284). Smaller ones lengthen the
+    // epilogue of a launch that is nothing but latency (batch 1 320 -> 329, batch 3 346 -> 352), larger ones are bound by the
+    // epilogue's instructions where the add itself runs at the rate of memory (batch 256: 2588 -> 2689), and layers with a
+    // long K and a short result gain alone and lose in flight (MobileNet-v2 batch 32: 394 -> 379 and 259 -> 266).
+    if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19 || cv->out()->bytes() > 8u << 20)) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
         r->padded_rows() || o->padded_rows() || a->cp % 4 != 0)
