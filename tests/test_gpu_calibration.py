@@ -319,3 +319,29 @@ def test_histogram_bins_at_the_rounding_boundaries():
         ref, _ = np.histogram(idx, bins=bins, range=(0, bins - 1))
         assert np.array_equal(hist.cpu().numpy()[0], ref.astype(np.int64)), float(am)
     m.close()
+
+
+@pytest.mark.parametrize("count", [1, 2, 3])
+def test_last_batch_read_from_the_tensors(count):
+    """run and run_multi take the last batch's histograms from the module's tensors; the separate passes, between which
+    anybody may use the module, do not: the same statistics, histograms and thresholds."""
+    from tpu_compiler_b200 import module
+    from tpu_compiler_b200.calibration import ActivationCalibrator
+    model = small_fp32_model(4)
+    rng = np.random.default_rng(80)
+    data = [np.clip(rng.normal(0, 1 + i, (4, 3, 24, 24)), -3, 3).astype(np.float32) for i in range(count)]
+    m = module(0)
+    m.load_text(model.text, model.weights)
+    a = ActivationCalibrator(m, lambda: iter(data))
+    stats = a.find_min_max_abs()
+    m.run(data[0] * 0)  # in between
+    hist = a.calc_histograms(stats)
+    thr = {k: float(v) for k, v in a.find_threshold(hist, stats).items()}
+    for gb in (None, 0):
+        b = ActivationCalibrator(m, lambda: iter(data), keep_activations_gb=gb)
+        got, _ = b.run()
+        assert {k: float(v) for k, v in got.items()} == thr
+        assert np.array_equal(b.histograms.cpu().numpy(), hist.cpu().numpy())
+    multi, _ = ActivationCalibrator(m, lambda: iter(data)).run_multi([1024, 2048])
+    assert {k: float(v) for k, v in multi[2048].items()} == thr
+    m.close()

@@ -59,6 +59,8 @@ class ActivationCalibrator:
         self.keep_activations_gb = keep_activations_gb   # None: 60% of the free device memory; 0: keep nothing
         self._kept = []          # per cached batch: (uint8 device buffer, images)
         self._kept_offsets = None
+        self._one_run = False    # inside run / run_multi: nobody else uses the module between the two passes
+        self._live = None        # (index, images) of the batch whose activations the module's tensors hold
         self._plan = None         # (bytes per batch, budget), see _keep_plan
         self._local_images = -1   # images this rank saw in pass 1
         self._pinned = None
@@ -96,12 +98,26 @@ class ActivationCalibrator:
         self._kept = []
         per_batch, budget = self._keep_plan()
         self.pass1_host_s = {k: 0.0 for k in self.pass1_host_s}
-        for batch in self.batches():
+        self._live = None
+        batches = iter(self.batches())
+        batch = next(batches, None)
+        index = 0
+        while batch is not None:
             self._upload(batch)
             t_enq = time.perf_counter()
             self.model.launch()
+            images = batch.shape[0]
+            if self._one_run:   # the last batch of a run is not copied: its histograms are taken from the tensors themselves
+                                # (two batches of 64 ResNet-50 images: 17.8 -> 17.0 ms)
+                self.pass1_host_s["enqueue"] += time.perf_counter() - t_enq
+                batch = next(batches, None)
+                t_enq = time.perf_counter()
+                if batch is None and per_batch:
+                    self._live = (index, images)
             keep = None
-            if self._reserved:
+            if self._live is not None:
+                pass
+            elif self._reserved:
                 keep = self._reserved.pop()
             elif per_batch and (len(self._kept) + 1) * per_batch <= budget:
                 try:
@@ -118,9 +134,12 @@ class ActivationCalibrator:
             if keep is not None:
                 # torch allocated `keep` on its own stream and the kernels above ran on the module's: the buffer is not
                 # handed back to torch before the module's stream has been synchronised (end of this pass and of pass 2)
-                self._kept.append((keep, batch.shape[0]))
-            n_img += batch.shape[0]
+                self._kept.append((keep, images))
+            n_img += images
             self.pass1_host_s["enqueue"] += time.perf_counter() - t_enq
+            if not self._one_run:
+                batch = next(batches, None)
+            index += 1
         t_sync = time.perf_counter()
         self.model.sync()
         self.pass1_host_s["final_sync"] += time.perf_counter() - t_sync
@@ -220,14 +239,19 @@ class ActivationCalibrator:
         kept = self._kept
         if release:
             self._kept = []   # this was the cache's last histogram pass
+        live = self._live if self._one_run else None
         absmax = (C.c_float * T)(*[float(activations_statistics[n][2]) for n in self.names])
         for keep, _ in kept:
             vals = (C.c_void_p * T)(*[keep.data_ptr() + o for o in self._kept_offsets])
             check(self._lib.tpucb_calib_hist_all(self.model._h, self._name_array(), T, vals, absmax, self.bin_num,
                                                  C.c_void_p(hist.data_ptr())))
-        for i, batch in enumerate(self.batches() if self._needs_recompute(kept) else ()):
-            if i < len(kept):
-                continue   # this batch's activations were read from the cache
+        if live is not None:
+            check(self._lib.tpucb_calib_hist_all(self.model._h, self._name_array(), T, None, absmax, self.bin_num,
+                                                 C.c_void_p(hist.data_ptr())))
+        for i, batch in enumerate(self.batches() if self._needs_recompute(kept, live) else ()):
+            if i < len(kept) or (live is not None and i == live[0]):
+                continue   # this batch's activations were read from the cache, or from the tensors
+            self._live = None
             self._upload(batch)
             self.model.launch()
             check(self._lib.tpucb_calib_hist_all(self.model._h, self._name_array(), T, None, absmax, self.bin_num,
@@ -236,9 +260,10 @@ class ActivationCalibrator:
         del kept
         return hist
 
-    def _needs_recompute(self, kept):
-        """False when every batch of pass 1 is in the cache (then pass 2 does not even ask for the images again)."""
-        return sum(n for _, n in kept) < self._local_images
+    def _needs_recompute(self, kept, live):
+        """False when every batch of pass 1 is in the cache or in the tensors (then pass 2 does not even ask for the images
+        again)."""
+        return sum(n for _, n in kept) + (live[1] if live else 0) < self._local_images
 
     def _check_ranks_agree(self):
         """Every rank must calibrate the same tensors in the same order, or the all-reduces below would combine
@@ -316,20 +341,28 @@ class ActivationCalibrator:
         (kld_calibrator.py:298-336): per bin count one histogram launch per cached batch and one KLD search. Returns
         ({bin count: {name: threshold}} in the order given, statistics). Bin counts are limited to 4096 by the
         histogram kernels (shared-memory tables); the reference's larger candidates (8192 .. 32768) are not covered."""
-        stats = self.find_min_max_abs()
         out = {}
         bin_nums = list(bin_nums)
         keep = self.bin_num
-        for i, bins in enumerate(bin_nums):
-            self.bin_num = int(bins)
-            hist = self.calc_histograms(stats, release=(i == len(bin_nums) - 1))
-            out[int(bins)] = self.find_threshold(hist, stats)
-        self.bin_num = keep
+        self._one_run = True
+        try:
+            stats = self.find_min_max_abs()
+            for i, bins in enumerate(bin_nums):
+                self.bin_num = int(bins)
+                hist = self.calc_histograms(stats, release=(i == len(bin_nums) - 1))
+                out[int(bins)] = self.find_threshold(hist, stats)
+        finally:
+            self._one_run = False
+            self.bin_num = keep
         return out, stats
 
     def run(self, output_calibration_table=None):
-        stats = self.find_min_max_abs()
-        hist = self.calc_histograms(stats)
+        self._one_run = True
+        try:
+            stats = self.find_min_max_abs()
+            hist = self.calc_histograms(stats)
+        finally:
+            self._one_run = False
         thresholds = self.find_threshold(hist, stats)
         self.histograms = hist
         if output_calibration_table and (self.dist is None or self.dist.get_rank() == 0):

@@ -100,6 +100,20 @@ __device__ __forceinline__ float4 tf32_remainder(const float4 &x) {
   return l;
 }
 
+// n / d and n % d of an element index: 32-bit arithmetic while it fits, which is always but for tensors of tens of
+// gigabytes (a 64-bit division is a call of some forty instructions).
+__device__ __forceinline__ unsigned div_rem(size_t &n, unsigned d) {
+  if ((n >> 32) == 0) {
+    const unsigned a = (unsigned)n, q = a / d;
+    n = q;
+    return a - q * d;
+  }
+  const size_t q = n / d;
+  const unsigned r = (unsigned)(n - q * d);
+  n = q;
+  return r;
+}
+
 // Programmatic dependent launch (kernels launched through launch_k with the stream-serialisation attribute): a kernel
 // lets its successor in the stream be scheduled early (pdl_trigger) and waits for its predecessor's memory operations
 // before its own first global access (pdl_wait). Both are no-ops in a kernel launched the ordinary way.

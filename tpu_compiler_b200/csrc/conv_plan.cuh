@@ -353,7 +353,9 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   // activations, which halves the bytes that have to reach shared memory per MAC. Larger weight
   // sets would force one CTA per SM, which measured slower than re-fetching the weights from L2.
   const int ctas_per_sm = 2;
-  const size_t budget = 113 * 1024;
+  // (An fp32 launch of at most one CTA per SM takes all of the shared memory: ResNet-50 at batch 30 3654 -> 3591 us. For INT8
+  // and BF16 launches it is a loss: those of other streams no longer fit beside them.)
+  const size_t budget = (pl.tf32 && total_tiles <= sm_count ? 220 : 113) * 1024;
   // (Pixel groups have small activation tiles: up to 60 KB of weights leave them four stages.)
   p.w_resident = (!pl.tf32 && total_tiles >= 2LL * n_tiles && w_all <= (p.group > 1 ? 60 : 48) * 1024 &&
                   budget - kSmemHeader - 1024 - w_all >= (p.group > 1 ? 4 : 3) * a_bytes) ? 1 : 0;
