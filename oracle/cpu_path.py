@@ -37,14 +37,8 @@ def _requant(acc, bias, rshift, mult, relu):
         R.ref_requant_per_channel(_p(out), _p(acc), _p(bias), int(relu), C.c_int64(n), C.c_int64(oc), C.c_int64(isz),
                                   _p(rs), _p(mu))
         return out
-    v = acc.astype(np.int64) + bias.astype(np.int64).reshape(1, oc, *([1] * (acc.ndim - 2)))
-    L = O.lib()
-    flat = v.reshape(n, oc, -1)
-    res = np.empty(flat.shape, np.float32)
-    for c in range(oc):
-        res[:, c] = [L.orc_qdm_i32(int(x), int(rs[c]), int(mu[c])) for x in flat[:, c].reshape(-1)]
-    res = res.reshape(acc.shape)
-    return np.maximum(res, 0) if relu else res
+    O.lib().orc_qdm_channels(_p(acc), _p(bias), _p(rs), _p(mu), _p(out), C.c_int64(n), C.c_int64(oc), C.c_int64(isz), int(relu))
+    return out
 
 
 def run(text, weights, inputs, keep_all=False):

@@ -60,6 +60,20 @@ int orc_qdm_i32(int32_t v, uint32_t rshift, uint32_t multiplier) {
   return sat8f((float)q);
 }
 
+// The same over a convolution's fp32 results [n][oc][isz], per channel: quantizeActivationInt8PerChannelMultiplierAndRShift,
+// QuantizationArithmetic.cpp:849-871.
+void orc_qdm_channels(const float *acc, const float *bias, const float *rshift, const float *multiplier, float *out, int64_t n,
+                      int64_t oc, int64_t isz, int do_relu) {
+#pragma omp parallel for
+  for (int64_t p = 0; p < n * oc; ++p) {
+    const int64_t o = p % oc;
+    for (int64_t i = p * isz; i < (p + 1) * isz; ++i) {
+      const int q = orc_qdm_i32((int32_t)acc[i] + (int32_t)bias[o], (uint32_t)rshift[o], (uint32_t)multiplier[o]);
+      out[i] = (float)(do_relu && q < 0 ? 0 : q);
+    }
+  }
+}
+
 // float overload, qdm=true: QuantizationArithmetic.cpp:518-527 ((int32_t)v cast).
 int orc_qdm_f32(float v, uint32_t rshift, uint32_t multiplier) {
   return orc_qdm_i32((int32_t)v, rshift, multiplier);
