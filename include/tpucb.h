@@ -230,7 +230,9 @@ int tpucb_calib_kld(tpucb_interp *it, const int64_t *d_hist, const float *widths
 /* ---- threshold auto-tuner (python/cvi_toolkit/calibration/kld_calibrator.py:113-201) ------ */
 
 /* Device-to-device copy of one tensor between two interpreters on the same GPU; the two
- * tensors must agree in type, shape and device layout. It stands in for the get_tensor ->
+ * tensors must agree in type and shape, and neither may have the padded rows of an image stem's input
+ * unless both have the same (the channel pitch, which depends on the ops that read a tensor, may differ).
+ * It stands in for the get_tensor ->
  * set_data round trip through numpy with which the reference's tuner would move an activation
  * between two loaded modules (bindings/python/pytuner.cpp:252-288). Returns after the copy. */
 int tpucb_interp_copy_tensor(tpucb_interp *dst, const char *dst_name, tpucb_interp *src,

@@ -148,3 +148,39 @@ def test_distance_entry_point_against_numpy():
             m3.copy_tensor_from("y2", m2, "z")
         for m in (m1, m2, m3):
             m.close()
+
+
+@pytest.mark.parametrize("c", [17, 48, 80])
+def test_copy_tensor_between_channel_pitches(c):
+    """A tensor that a convolution of several taps reads starts its pixels on 32-byte sectors, the same tensor elsewhere on
+    16-byte vectors: copies go both ways, values and zero padding intact."""
+    from tpu_compiler_b200 import graphs, module
+    rng = np.random.default_rng(c)
+    shape = (2, c, 9, 7)
+    line = "input name=x shape=%d,%d,%d,%d dtype=INT8\n" % shape
+    conv = graphs.single_conv_i8(2, c, 24, 9, 3, 1, 1, seed=77)
+    conv_text = line.replace("name=x", "name=x0") + line + conv.text.splitlines()[-1].replace("2,24,9,9", "2,24,9,7") + "\n"
+    reader, plain = module(0), module(0)
+    reader.load_text(conv_text, conv.weights)
+    plain.load_text(line, {})
+    assert reader.tensor_device("x")["pitch"] == (c + 31) // 32 * 32
+    assert plain.tensor_device("x")["pitch"] == reader.tensor_device("x0")["pitch"] == (c + 15) // 16 * 16
+    a, b = (rng.integers(-128, 128, shape).astype(np.float32) for _ in range(2))
+    reader.set_tensor("x", a)
+    reader.invoke()
+    want = reader.get_tensor("conv")
+    reader.set_tensor("x", b)
+    plain.set_tensor("x", a)
+    reader.copy_tensor_from("x", plain, "x")   # to the wider pitch
+    np.testing.assert_array_equal(reader.get_tensor("x"), a)
+    reader.invoke()
+    np.testing.assert_array_equal(reader.get_tensor("conv"), want)
+    plain.set_tensor("x", b)
+    plain.copy_tensor_from("x", reader, "x")   # and back
+    np.testing.assert_array_equal(plain.get_tensor("x"), a)
+    reader.copy_tensor_from("x0", reader, "x")
+    np.testing.assert_array_equal(reader.get_tensor("x0"), a)
+    with pytest.raises(RuntimeError):
+        plain.copy_tensor_from("x", reader, "conv")
+    reader.close()
+    plain.close()

@@ -457,12 +457,17 @@ int tpucb_interp_copy_tensor(tpucb_interp *dst, const char *dst_name, tpucb_inte
   TPUCB_CHECK(D.device() == S.device(), "tpucb_interp_copy_tensor: the two interpreters live on different devices");
   auto d = D.tensor(dst_name);
   auto s = S.tensor(src_name);
-  TPUCB_CHECK(d->dtype == s->dtype && d->n == s->n && d->c == s->c && d->h == s->h && d->w == s->w && d->cp == s->cp &&
-                  d->wl == s->wl && d->wphys == s->wphys,
+  const bool same = d->cp == s->cp && d->wl == s->wl && d->wphys == s->wphys;
+  TPUCB_CHECK(d->dtype == s->dtype && d->n == s->n && d->c == s->c && d->h == s->h && d->w == s->w &&
+                  (same || (!d->padded_rows() && !s->padded_rows())),
               "tpucb_interp_copy_tensor: %s and %s differ in type, shape or device layout", dst_name, src_name);
   D.bind();
   TPUCB_CUDA(cudaStreamSynchronize(S.stream)); // the source's producers have finished
-  TPUCB_CUDA(cudaMemcpyAsync(d->dev, s->dev, s->bytes(), cudaMemcpyDeviceToDevice, D.stream));
+  if (same)
+    TPUCB_CUDA(cudaMemcpyAsync(d->dev, s->dev, s->bytes(), cudaMemcpyDeviceToDevice, D.stream));
+  else // the pitch depends on who reads a tensor in its module (load_module): the channels are copied, the padding of d stays zero
+    TPUCB_CUDA(cudaMemcpy2DAsync(d->dev, d->cp * d->elsize(), s->dev, s->cp * s->elsize(), s->c * s->elsize(), s->pixels(),
+                                 cudaMemcpyDeviceToDevice, D.stream));
   TPUCB_CUDA(cudaStreamSynchronize(D.stream)); // the source may be overwritten once this returns
   TPUCB_API_END
 }

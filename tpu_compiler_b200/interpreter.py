@@ -297,7 +297,7 @@ class module:
     # ---- tuner helpers ---------------------------------------------------------------
     def copy_tensor_from(self, name, other, other_name):
         """Device-to-device copy of ``other_name`` of module ``other`` into this module's ``name``
-        (same GPU, same type, shape and device layout)."""
+        (same GPU, type and shape; the channel pitches may differ, the padded rows of a stem's input may not)."""
         check(self._lib.tpucb_interp_copy_tensor(self._h, name.encode(), other._h, other_name.encode()))
 
     def tuner_distance(self, name, ref, ref_name, scale):

@@ -152,8 +152,8 @@ class SimpleTuner:
 
     @staticmethod
     def _move(dst, dst_name, src, src_name):
-        """Device-to-device when the two tensors share a device layout; a few-channel tensor that a
-        stem convolution wants with padded rows is staged through the host instead."""
+        """Device-to-device, whatever the channel pitches; only a few-channel tensor that a stem convolution wants with
+        padded rows is staged through the host instead."""
         try:
             dst.copy_tensor_from(dst_name, src, src_name)
         except RuntimeError as e:
