@@ -26,6 +26,7 @@
 // leaves through the common tear-down (TMEM freed, in-flight copies drained).
 #pragma once
 #include "common.cuh"
+#include <type_traits>
 #include <cuda.h>
 
 namespace tpucb {
@@ -974,47 +975,55 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         }
         const uint32_t d_tmem = tmem_base + (uint32_t)buf * acc_stride;
         uint32_t wres_lo = desc_w_lo; // weight-resident mode: descriptor (low word) of K block `kit`
-        for (int kit = k_begin; kit < k_end; ++kit, ++it) {
-          if (!ptx::mbar_try_wait(m_full, mph) && !ptx::mbar_wait_bounded(m_full, mph, abort_flag, wait_rounds)) {
-            if (!*abort_flag) report_error(p.err, kErrFullWait);
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
-          ptx::tcgen05_fence_after();
-          // transposed product: weights are the A operand (M = channels), activations B (N = pixels)
-          const uint32_t w_lo = p.w_resident ? wres_lo : ring_lo + a_step;
-          const uint32_t acc_first = kit > k_begin ? 1u : 0u;
-          if (!p.dual) {
-            if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-            else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-            else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-            else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-          } else {
-            // dual mode: sub-tile 0 uses weight rows 64..191 ([W; 0]), sub-tile 1 rows 0..127 ([0; W])
-            for (int sub = 0; sub < 2; ++sub) {
-              const uint32_t a_lo = w_lo + (sub == 0 ? dual_step : 0u);
-              const uint32_t b_lo = ring_lo + (uint32_t)sub * sub_step;
-              const uint32_t first = (kit > k_begin || sub > 0) ? 1u : 0u;
-              if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-              else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-              else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-              else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+        // The loop over K blocks twice: for whole blocks of plain tiles, and for blocks with a padded tail and dual mode. One
+        // loop that chose between one and four MMAs inside cost every K block 23 ns (3x3, 512 channels, 7x7, N = 1 unsplit,
+        // 36 blocks: 15.4 -> 13.9 us; ResNet-50 batch 1 318 -> 292 us, batch 256 2560 -> 2530).
+        auto k_loop = [&](auto whole) {
+          for (int kit = k_begin; kit < k_end; ++kit, ++it) {
+            if (!ptx::mbar_try_wait(m_full, mph) && !ptx::mbar_wait_bounded(m_full, mph, abort_flag, wait_rounds)) {
+              if (!*abort_flag) report_error(p.err, kErrFullWait);
+              *abort_flag = 1;
+              ok = false;
+              break;
+            }
+            ptx::tcgen05_fence_after();
+            // transposed product: weights are the A operand (M = channels), activations B (N = pixels)
+            const uint32_t w_lo = p.w_resident ? wres_lo : ring_lo + a_step;
+            const uint32_t acc_first = kit > k_begin ? 1u : 0u;
+            if constexpr (decltype(whole)::value) {
+              ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+            } else if (!p.dual) {
+              if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+              else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+              else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+            } else {
+              // dual mode: sub-tile 0 uses weight rows 64..191 ([W; 0]), sub-tile 1 rows 0..127 ([0; W])
+              for (int sub = 0; sub < 2; ++sub) {
+                const uint32_t a_lo = w_lo + (sub == 0 ? dual_step : 0u);
+                const uint32_t b_lo = ring_lo + (uint32_t)sub * sub_step;
+                const uint32_t first = (kit > k_begin || sub > 0) ? 1u : 0u;
+                if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+              }
+            }
+            ptx::tcgen05_commit(m_empty); // frees the stage when the MMAs retire
+            wres_lo += w_step;
+            m_full += 8;
+            m_empty += 8;
+            ring_lo += stage_step;
+            if (++ms == p.stages) {
+              ms = 0;
+              mph ^= 1u;
+              m_full = bar_full;
+              m_empty = bar_empty;
+              ring_lo = desc_ring_lo;
             }
           }
-          ptx::tcgen05_commit(m_empty); // frees the stage when the MMAs retire
-          wres_lo += w_step;
-          m_full += 8;
-          m_empty += 8;
-          ring_lo += stage_step;
-          if (++ms == p.stages) {
-            ms = 0;
-            mph ^= 1u;
-            m_full = bar_full;
-            m_empty = bar_empty;
-            ring_lo = desc_ring_lo;
-          }
-        }
+        };
+        if (ksteps == 4 && !p.dual) k_loop(std::true_type{});
+        else k_loop(std::false_type{});
         if (ok) ptx::tcgen05_commit(bar_acc_full + 8 * buf);
       }
     }
