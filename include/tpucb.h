@@ -174,7 +174,9 @@ int tpucb_interp_time_launches(tpucb_interp *it, int iters, float *ms_total);
 int tpucb_interp_kernel_count(tpucb_interp *it, int *count);
 
 /* Device pointer, byte size and channel pitch of a tensor's NHWC storage (for the
- * calibration statistics entry points below and for torch.distributed collectives). */
+ * calibration statistics entry points below and for torch.distributed collectives). The storage is the
+ * start of an allocation of cudaMalloc: cudaIpcGetMemHandle takes it, and cudaDeviceEnablePeerAccess
+ * makes it readable to other GPUs. It belongs to the module until the next load or destroy. */
 int tpucb_interp_tensor_device(tpucb_interp *it, const char *name, void **dev, size_t *bytes,
                                int *channels, int *channel_pitch, int *dtype);
 

@@ -207,3 +207,49 @@ def test_command_line_round_trip(tmp_path):
     assert list(out) == ["prob"] and set(allt) == set(ref)
     for n, v in allt.items():
         assert v.shape == ref[n].shape and np.abs(v - ref[n]).max() <= 1e-4 * max(np.abs(ref[n]).max(), 1e-6), n
+
+
+IPC_CHILD = """
+import ctypes as C, sys
+cu = C.CDLL("libcuda.so.1")
+class Handle(C.Structure):
+    _fields_ = [("bytes", C.c_char * 64)]
+ctx, ptr, n = C.c_void_p(), C.c_uint64(), int(sys.argv[2])
+assert cu.cuInit(0) == 0 and cu.cuDevicePrimaryCtxRetain(C.byref(ctx), 0) == 0 and cu.cuCtxSetCurrent(ctx) == 0
+h = Handle.from_buffer_copy(bytes.fromhex(sys.argv[1]))
+cu.cuIpcOpenMemHandle_v2.argtypes = [C.c_void_p, Handle, C.c_uint]
+assert cu.cuIpcOpenMemHandle_v2(C.byref(ptr), h, 1) == 0
+out = (C.c_char * n)()
+assert cu.cuMemcpyDtoH_v2(out, ptr, C.c_size_t(n)) == 0 and cu.cuIpcCloseMemHandle(ptr) == 0
+sys.stdout.write(bytes(out).hex())
+"""
+
+
+@pytest.mark.parametrize("hw", [5, 300])  # part of a driver page, and an allocation of several
+def test_tensor_storage_opens_in_another_process(hw):
+    """tensor_device gives an allocation of its own: another process opens it by its IPC handle and reads the values, also in
+    a module that has taken over the storage of a closed one."""
+    import ctypes as C
+    import subprocess
+    import sys
+    from tpu_compiler_b200 import module
+    cu = C.CDLL("libcuda.so.1")
+    keeper = module(0)
+    keeper.load_text("input name=k shape=1,16,2,2 dtype=INT8\n", {})
+    for seed in (1, 2):
+        m = module(0)
+        m.load_text("input name=x shape=1,16,%d,%d dtype=INT8\n" % (hw, hw), {})
+        x = np.random.default_rng(seed).integers(-128, 128, (1, 16, hw, hw)).astype(np.float32)
+        m.set_tensor("x", x)
+        m.sync()
+        t = m.tensor_device("x")
+        handle = (C.c_char * 64)()
+        cu.cuIpcGetMemHandle.argtypes = [C.c_void_p, C.c_uint64]
+        assert cu.cuIpcGetMemHandle(handle, t["ptr"]) == 0
+        p = subprocess.run([sys.executable, "-c", IPC_CHILD, bytes(handle).hex(), str(t["bytes"])], capture_output=True,
+                           text=True, timeout=120)
+        assert p.returncode == 0, p.stderr
+        got = np.frombuffer(bytes.fromhex(p.stdout), np.int8).reshape(1, hw, hw, 16)
+        np.testing.assert_array_equal(got.transpose(0, 3, 1, 2), x)
+        m.close()
+    keeper.close()

@@ -4,16 +4,21 @@
 // cudaMalloc / cudaFree each of them costs a driver call that also waits for the whole device, and
 // cudaGetDeviceProperties and the stream and event calls cost milliseconds more: the auto-tuner, which loads one small
 // module per tuned op, spent 95% of its time there (102 ms for 17 modules of a few ops; 5 ms per module).
-// Buffers therefore come from a stream-ordered memory pool of this library's own (cudaMallocFromPoolAsync), and the
-// streams and events of a destroyed interpreter are handed to the next one.
+// Weights, tables and staging therefore come from a stream-ordered memory pool of this library's own
+// (cudaMallocFromPoolAsync), and the streams and events of a destroyed interpreter are handed to the next one. Tensors,
+// whose addresses callers ask for (tpucb_interp_tensor_device), are blocks of cudaMalloc, which other processes can open
+// (cudaIpcGetMemHandle) and peers can read; the blocks of a destroyed module are kept for the next one.
 //
-// Both are bounded and given back: when a module goes, free memory above kPoolKeepBytes returns to the driver, at most
-// kPoolKeepStreams idle stream sets are kept, and when the last interpreter of a GPU goes, everything goes.
-// Several threads may use it at once (one mutex around the lists; the pool calls are thread-safe themselves). A buffer is
-// allocated and freed on its interpreter's stream, which is idle when the interpreter is destroyed.
+// All are bounded and given back: when a module goes, free memory above kPoolKeepBytes returns to the driver (so much of
+// either kind), at most kPoolKeepStreams idle stream sets are kept, and when the last interpreter of a GPU goes, everything
+// goes. Several threads may use it at once (one mutex around the lists; the pool calls are thread-safe themselves). A pool
+// buffer is allocated and freed on its interpreter's stream, which is idle when the interpreter is destroyed; a block is
+// given back only when nothing uses it any more, so the next owner need not wait for the former one's stream.
 #pragma once
 #include "host_common.h"
 
+#include <algorithm>
+#include <iterator>
 #include <mutex>
 
 namespace tpucb {
@@ -108,7 +113,10 @@ public:
       cudaStreamDestroy(d.stream);
       idle_.pop_back();
     }
-    if (live_ == 0) cudaMemPoolTrimTo(mem_, 0);
+    if (live_ == 0) {
+      drop_blocks(0);
+      cudaMemPoolTrimTo(mem_, 0);
+    }
   }
 
   void *alloc(size_t bytes, cudaStream_t stream) {
@@ -117,7 +125,41 @@ public:
     return p;
   }
 
-  cudaMemPool_t handle() const { return mem_; }
+  // A tensor's storage: a free block of at most a quarter more, or a new one (a block of 1 MB and more costs the driver 0.3 ms
+  // to allocate and as much to free).
+  void *alloc_block(size_t bytes) {
+    const size_t need = (std::max<size_t>(bytes, 16) + 511) / 512 * 512;
+    std::lock_guard<std::mutex> lock(m_);
+    auto it = free_blocks_.lower_bound(need);
+    if (it != free_blocks_.end() && it->first <= need + need / 4) {
+      void *p = it->second;
+      free_bytes_ -= it->first;
+      blocks_[p] = it->first;
+      free_blocks_.erase(it);
+      return p;
+    }
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, need);
+    if (e == cudaErrorMemoryAllocation) { // what lies free here may make room
+      cudaGetLastError();
+      drop_blocks(0);
+      cudaMemPoolTrimTo(mem_, 0);
+      e = cudaMalloc(&p, need);
+    }
+    TPUCB_CUDA(e);
+    blocks_[p] = need;
+    return p;
+  }
+  // Nothing on the device may still use the block.
+  void free_block(void *p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(m_);
+    auto it = blocks_.find(p);
+    free_blocks_.insert({it->second, p});
+    free_bytes_ += it->second;
+    blocks_.erase(it);
+    drop_blocks(kPoolKeepBytes);
+  }
 
   // Gives the driver back what lies free above kPoolKeepBytes. Called where a module's buffers have been freed; in between
   // the pool holds on to what it has (its release threshold counts the memory in use too, so with any finite threshold
@@ -129,6 +171,16 @@ public:
   }
 
 private:
+  // Gives free blocks back to the driver, the largest first, until no more than `keep` bytes are left.
+  void drop_blocks(size_t keep) {
+    while (free_bytes_ > keep) {
+      auto it = std::prev(free_blocks_.end());
+      cudaFree(it->second);
+      free_bytes_ -= it->first;
+      free_blocks_.erase(it);
+    }
+  }
+
   explicit DevicePool(int device) {
     int major = 0, minor = 0;
     TPUCB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
@@ -147,6 +199,9 @@ private:
   std::mutex m_;
   cudaMemPool_t mem_ = nullptr;
   std::vector<StreamSet> idle_;
+  std::multimap<size_t, void *> free_blocks_; // by size
+  std::map<void *, size_t> blocks_;           // in use
+  size_t free_bytes_ = 0;
   int live_ = 0;
 };
 

@@ -98,8 +98,7 @@ public:
     cudaDeviceSynchronize(); // as cudaFree would: nobody's kernels still read a tensor of this module
     invalidate_graph();
     kernels.clear();
-    for (auto &kv : tensors)
-      if (kv.second->owns) dfree(kv.second->dev);
+    free_tensors();
     for (void *p : allocations) dfree(p);
     dfree(staging);
     for (int i = 0; i < 2; ++i) dfree(async_staging[i]);
@@ -123,6 +122,11 @@ public:
   }
   void dfree(void *p) {
     if (p) cudaFreeAsync(p, stream);
+  }
+  void free_tensors() { // the device is idle
+    for (auto &kv : tensors)
+      if (kv.second->owns) pool->free_block(kv.second->dev);
+    tensors.clear();
   }
   template <class T> T *upload(const std::vector<T> &v) {
     T *p = (T *)dalloc(v.size() * sizeof(T));
@@ -171,7 +175,7 @@ public:
       t->wl = lr->second.wl;
       t->wphys = lr->second.wphys;
     }
-    t->dev = pool->alloc(t->bytes(), stream);
+    t->dev = pool->alloc_block(t->bytes());
     TPUCB_CUDA(cudaMemsetAsync(t->dev, 0, t->bytes(), stream));
     return t;
   }
@@ -2019,14 +2023,12 @@ inline void Interpreter::reset_module() {
   TPUCB_CUDA(cudaDeviceSynchronize());
   kernels.clear();
   quants_disabled = 0;
-  for (auto &kv : tensors)
-    if (kv.second->owns) dfree(kv.second->dev);
+  free_tensors();
   for (void *p : allocations) dfree(p);
   allocations.clear();
   split_ws.clear();
   TPUCB_CUDA(cudaStreamSynchronize(stream));
   pool->trim();
-  tensors.clear();
   tensor_order.clear();
   input_details.clear();
   output_details.clear();
@@ -2096,6 +2098,15 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
       return -1;
     }
     out = make_tensor(op.name, op.shape, dt);
+    struct Refused { // an op that is refused below leaves no tensor behind
+      Interpreter *I;
+      void *dev;
+      ~Refused() {
+        if (!dev) return;
+        cudaStreamSynchronize(I->stream);
+        I->pool->free_block(dev);
+      }
+    } refused{this, out->dev};
     if (op.type == "input") {
       k.reset(new InputOp());
       input_details.push_back({op.name, out->numel() / (size_t)max_batch});
@@ -2177,7 +2188,6 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
     } else if (op.type == "softmax") {
       k.reset(new SoftmaxOp(*this, op, opd(0), out));
     } else {
-      dfree(out->dev);
       throw Error(strfmt("op type '%s' (%s) is not implemented by the B200 backend", op.type.c_str(), op.name.c_str()));
     }
     k->name = op.name;
@@ -2186,6 +2196,7 @@ inline int Interpreter::add_op(const ParsedOp &op_in) {
     k->datatype = dt;
     k->result = out;
     tensors[op.name] = out;
+    refused.dev = nullptr;
     tensor_order.push_back(op.name);
     producer_type[op.name] = op.type;
     k->line = op_in.line;
@@ -2269,18 +2280,6 @@ inline void Interpreter::load_module(const std::string &text) {
       rl.cp = round_up((int)op.shape[1], 32); rl.wphys = (int)op.shape[3];
       layout_requests[op.name] = rl;
     }
-  }
-  // The pool grows once, by about what the tensors of a large module need, instead of tensor by tensor.
-  size_t need = 0;
-  for (const ParsedOp &op : parsed) {
-    size_t v = (size_t)max_batch * (op.dtype == "INT8" ? 1 : (op.dtype == "BF16" ? 2 : 4));
-    for (int64_t d : op.shape) v *= (size_t)std::max<int64_t>(d, 1);
-    if (op.type != "reshape") need += v;
-  }
-  if (need >= (64u << 20)) {
-    void *p = nullptr; // (a request that is too large by its rounding is no error: the tensors will tell)
-    if (cudaMallocFromPoolAsync(&p, need, pool->handle(), stream) == cudaSuccess) dfree(p);
-    else cudaGetLastError();
   }
   for (const ParsedOp &op : parsed) add_op(op);
   finish_module();
