@@ -221,3 +221,20 @@ def test_residual_add_with_prefetch(case):
         m.invoke()
     assert all(np.array_equal(m.get_tensor(k), ref[k]) for k in ("conv", "s"))
     m.close()
+
+
+@pytest.mark.parametrize("dtype", ["INT8", "BF16", "FP32"])
+@pytest.mark.parametrize("shape", [
+    (1, 1, 1, 1), (3, 1001, 1, 1), (5, 3, 17, 23), (2, 70, 9, 5),        # value by value, small results into pinned memory
+    (1, 32, 181, 181), (1, 32, 181, 182), (1, 31, 190, 190), (2, 33, 130, 130), (1, 2048, 23, 23),  # both sides of 2^20 values, 32 channels
+    (1, 4194305, 1, 1)])                                               # more channels than a grid has rows of tiles
+def test_download_forms(dtype, shape):
+    from tpu_compiler_b200 import module
+    if dtype != "INT8" and shape[1] > 10 ** 6:
+        pytest.skip("one type is enough")
+    m = module(0)
+    m.load_text("input name=x shape=%d,%d,%d,%d dtype=%s\n" % (shape + (dtype,)), {})
+    x = np.random.default_rng(sum(shape)).integers(-128, 128, shape).astype(np.float32)
+    m.set_tensor("x", x)
+    assert np.array_equal(m.get_tensor("x"), x)
+    m.close()

@@ -2503,10 +2503,12 @@ inline void Interpreter::get_tensor(const std::string &name, float *out, size_t 
         on = copy_stream;
         TPUCB_CUDA(cudaStreamWaitEvent(on, p.done, 0));
       }
-  const dim3 grid((unsigned)((v.g.n * (size_t)v.g.h * v.g.w + 63) / 64), (unsigned)((v.g.c + 63) / 64));
-  if (t->dtype == DT_I8) launch_k(dev_to_nchw_f32_kernel<DT_I8>, grid, 256, 0, on, v.dev, stg, v.g);
-  else if (t->dtype == DT_BF16) launch_k(dev_to_nchw_f32_kernel<DT_BF16>, grid, 256, 0, on, v.dev, stg, v.g);
-  else launch_k(dev_to_nchw_f32_kernel<DT_F32>, grid, 256, 0, on, v.dev, stg, v.g);
+  const bool tiles = download_in_tiles(v.g);
+  const dim3 grid = tiles ? dim3((unsigned)((v.g.n * (size_t)v.g.h * v.g.w + 63) / 64), (unsigned)((v.g.c + 63) / 64))
+                          : dim3(grid_for(numel, 256, sm_count));
+  if (t->dtype == DT_I8) launch_k(tiles ? dev_to_nchw_f32_tile_kernel<DT_I8> : dev_to_nchw_f32_kernel<DT_I8>, grid, 256, 0, on, v.dev, stg, v.g);
+  else if (t->dtype == DT_BF16) launch_k(tiles ? dev_to_nchw_f32_tile_kernel<DT_BF16> : dev_to_nchw_f32_kernel<DT_BF16>, grid, 256, 0, on, v.dev, stg, v.g);
+  else launch_k(tiles ? dev_to_nchw_f32_tile_kernel<DT_F32> : dev_to_nchw_f32_kernel<DT_F32>, grid, 256, 0, on, v.dev, stg, v.g);
   TPUCB_CUDA(cudaGetLastError());
   if (!direct) TPUCB_CUDA(cudaMemcpyAsync(out, stg, numel * sizeof(float), cudaMemcpyDeviceToHost, on));
   TPUCB_CUDA(cudaStreamSynchronize(on));

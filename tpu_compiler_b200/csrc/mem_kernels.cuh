@@ -110,10 +110,29 @@ __device__ __forceinline__ float load_as_f32(const void *p, int dt, size_t i) {
   return reinterpret_cast<const float *>(p)[i];
 }
 
-// download: device NHWC -> fp32 NCHW, a tile of 64 pixels by 64 channels per block (256 threads) through shared memory:
-// reads run along the channels, writes along the pixels of one channel.
+// download: device NHWC -> fp32 NCHW. One value per thread, in the order of the result: all stores are contiguous, and the
+// reads are too where a pixel has one or few channels or an image one pixel. (256 x 1000 x 1 x 1: 4.2 us, in tiles 10.3;
+// 8 x 3 x 224 x 224: 8.3, 37; 1 x 64 x 56 x 56: 4.2, 8.3.)
 template <int DT>
 __global__ void __launch_bounds__(256) dev_to_nchw_f32_kernel(const void *__restrict__ src, float *__restrict__ dst, TensorGeom g) {
+  pdl_prologue();
+  const size_t total = (size_t)g.n * g.c * g.h * g.w;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    size_t t = i;
+    const unsigned x = div_rem(t, g.w), y = div_rem(t, g.h), c = div_rem(t, g.c);
+    dst[i] = load_as_f32(src, DT, ((t * g.h + y) * g.wphys + g.wl + x) * g.cp + c);
+  }
+}
+
+// ... and through a tile of 64 pixels by 64 channels in shared memory, whose reads run along the channels and whose writes
+// along the pixels of one channel: for results that fill the chip with such tiles, where the strided reads above fetch a
+// sector per value (64 x 2048 x 7 x 7: 28.8 -> 20.5 us, 8 x 255 x 52 x 52: 26.7 -> 18.5; 8 x 255 x 26 x 26, 1.4 M values:
+// 10.3 -> 9.8; but 8 x 2048 x 7 x 7, 0.8 M: 6.4 -> 8.3, and 24 channels, 2.4 M: 13.0 -> 14.5).
+inline bool download_in_tiles(const TensorGeom &g) {
+  return g.c >= 32 && g.c <= 64 * 65535 && (size_t)g.n * g.c * g.h * g.w >= (1u << 20);
+}
+template <int DT>
+__global__ void __launch_bounds__(256) dev_to_nchw_f32_tile_kernel(const void *__restrict__ src, float *__restrict__ dst, TensorGeom g) {
   pdl_prologue();
   __shared__ float s_v[64][65];
   const size_t hw = (size_t)g.h * g.w, pixels = g.n * hw, p0 = blockIdx.x * (size_t)64;
