@@ -293,7 +293,6 @@ public:
     async_staging_bytes[k] = bytes;
   }
   void upload_pageable(void *staging, const void *data, size_t bytes);
-  int upload_next = 0;    // upload slot of the next piece
   int quants_disabled = 0; // quant ops that set_tensor_async_i8 has switched off
   void set_tensor_async(const std::string &name, const float *pinned, size_t numel);
   void set_tensor_async_i8(const std::string &name, const int8_t *pinned, size_t numel);
@@ -2338,20 +2337,19 @@ inline void Interpreter::upload_pageable(void *staging, const void *data, size_t
     TPUCB_CUDA(cudaMemcpyAsync(staging, data, bytes, cudaMemcpyHostToDevice, stream));
     return;
   }
-  if (!ss.upload) {
-    TPUCB_CUDA(cudaHostAlloc((void **)&ss.upload, kUploadSlot * kUploadSlots, cudaHostAllocDefault));
-    for (cudaEvent_t &e : ss.upload_read) TPUCB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  }
   constexpr size_t kBlock = 64u << 10;
   constexpr int kPiece = 4; // blocks
-  constexpr int kMaxPieces = (int)(kUploadSlot / (kBlock * kPiece));
+  constexpr int kMaxPieces = 4;
   const bool parallel = bytes >= (1u << 20);
-  for (size_t at = 0; at < bytes; at += kUploadSlot) {
-    const size_t len = std::min(kUploadSlot, bytes - at);
-    const int blocks = (int)((len + kBlock - 1) / kBlock), pieces = (blocks + kPiece - 1) / kPiece, slot = upload_next;
-    upload_next = (upload_next + 1) % kUploadSlots;
-    TPUCB_CUDA(cudaEventSynchronize(ss.upload_read[slot]));
-    uint8_t *pinned = ss.upload + (size_t)slot * kUploadSlot;
+  UploadRing &ring = bytes < kLargeUpload ? ss.small : ss.large;
+  for (size_t at = 0; at < bytes; at += ring.slot_bytes) {
+    const size_t len = std::min(ring.slot_bytes, bytes - at);
+    const int blocks = (int)((len + kBlock - 1) / kBlock), pieces = (blocks + kPiece - 1) / kPiece, slot = ring.next;
+    ring.next = (ring.next + 1) % ring.slots;
+    if (!ring.read[slot]) TPUCB_CUDA(cudaEventCreateWithFlags(&ring.read[slot], cudaEventDisableTiming));
+    if (!ring.mem[slot]) TPUCB_CUDA(cudaHostAlloc((void **)&ring.mem[slot], ring.slot_bytes, cudaHostAllocDefault));
+    TPUCB_CUDA(cudaEventSynchronize(ring.read[slot]));
+    uint8_t *pinned = ring.mem[slot];
     const uint8_t *src = (const uint8_t *)data + at;
     std::atomic<int> done[kMaxPieces];
     for (auto &d : done) d.store(0, std::memory_order_relaxed);
@@ -2374,7 +2372,7 @@ inline void Interpreter::upload_pageable(void *staging, const void *data, size_t
           return sent == pieces;
         });
     TPUCB_CUDA(e);
-    TPUCB_CUDA(cudaEventRecord(ss.upload_read[slot], stream));
+    TPUCB_CUDA(cudaEventRecord(ring.read[slot], stream));
   }
 }
 
