@@ -113,21 +113,28 @@ inline int pick_bk(int k_bytes) {
   return best;
 }
 
+// One output channel's filter, [channels][taps] -> [taps][pitch] of T: converted in one sweep (which the compiler
+// vectorises), then the taps are told apart; `line` holds channels * taps values.
+template <class T, class Convert>
+inline void pack_filter(const float *w, int channels, int taps, T *out, size_t pitch, T *line, Convert convert) {
+  T *to = taps == 1 ? out : line;
+  const size_t n = (size_t)channels * taps;
+  for (size_t i = 0; i < n; ++i) to[i] = convert(w[i]);
+  if (taps > 1)
+    for (int t = 0; t < taps; ++t)
+      for (int c = 0; c < channels; ++c) out[t * pitch + c] = line[(size_t)c * taps + t];
+}
+
 // Pack OIHW fp32 weights (integer-valued) to int8 [oc_pad][taps][cin_pad] for the im2col
 // path, or [oc_pad][1][kp] with K order (r, s, c) for the patch path. For grouped
 // convolution the caller passes one group's slice.
 inline std::vector<int8_t> pack_conv_weights(const float *w, int oc, int icg, int kh, int kw,
                                              int oc_pad, int cin_pad, bool patch, int kp) {
   const int taps = kh * kw;
-  std::vector<int8_t> out((size_t)oc_pad * (patch ? kp : taps * cin_pad), 0);
+  const size_t row = patch ? kp : (size_t)taps * cin_pad, pitch = patch ? icg : cin_pad;
+  std::vector<int8_t> out(oc_pad * row, 0), line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    for (int c = 0; c < icg; ++c)
-      for (int r = 0; r < kh; ++r)
-        for (int s = 0; s < kw; ++s) {
-          int8_t v = (int8_t)(int)w[(((size_t)o * icg + c) * kh + r) * kw + s];
-          if (patch) out[(size_t)o * kp + (size_t)(r * kw + s) * icg + c] = v;
-          else out[((size_t)o * taps + (r * kw + s)) * cin_pad + c] = v;
-        }
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, out.data() + o * row, pitch, line.data(), [](float v) { return (int8_t)(int)v; });
   return out;
 }
 
@@ -136,15 +143,12 @@ inline std::vector<int8_t> pack_conv_weights(const float *w, int oc, int icg, in
 inline std::vector<int8_t> pack_conv_weights_bf16(const float *w, int oc, int icg, int kh, int kw, int oc_pad,
                                                   int cin_pad) {
   const int taps = kh * kw;
-  std::vector<uint16_t> out((size_t)oc_pad * taps * cin_pad, 0);
+  const size_t row = (size_t)taps * cin_pad;
+  std::vector<int8_t> bytes(oc_pad * row * 2, 0);
+  std::vector<uint16_t> line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    for (int c = 0; c < icg; ++c)
-      for (int r = 0; r < kh; ++r)
-        for (int s = 0; s < kw; ++s)
-          out[((size_t)o * taps + (r * kw + s)) * cin_pad + c] =
-              (uint16_t)(f32_bits(w[(((size_t)o * icg + c) * kh + r) * kw + s]) >> 16);
-  std::vector<int8_t> bytes(out.size() * 2);
-  std::memcpy(bytes.data(), out.data(), bytes.size());
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, reinterpret_cast<uint16_t *>(bytes.data()) + o * row, cin_pad, line.data(),
+                [](float v) { return (uint16_t)(f32_bits(v) >> 16); });
   return bytes;
 }
 
@@ -427,7 +431,9 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
 struct DenseLayer {
   ConvGeom g; // g.ic = in_cp and g.oc = out_cp once paired
   int in_cp, out_cp;
-  std::vector<float> w, bias, mult, rshift; // OIHW; per channel
+  const float *w;         // OIHW: the caller's filter, or `own` once paired
+  std::vector<float> own;
+  std::vector<float> bias, mult, rshift; // per channel
   bool paired = false;
 };
 inline bool pair_applies(const ConvGeom &g, int in_cp, int out_cp, int es) {
@@ -461,7 +467,8 @@ inline void pair_layer(DenseLayer &d) {
     twice(d.mult);
     twice(d.rshift);
   }
-  d.w = std::move(w);
+  d.own = std::move(w);
+  d.w = d.own.data();
   d.g.ic = ic2; d.g.oc = oc2; d.g.iw /= 2; d.g.ow /= 2; d.g.kw = kw2; d.g.dw = 1; d.g.pl = pl2;
   d.g.pr = d.g.ow - d.g.iw - pl2 + kw2 - 1;
   d.in_cp = ic2;

@@ -334,16 +334,16 @@ inline int requant_fast_flags(const std::vector<float> &rshift, const std::vecto
 }
 
 // Constants of the floating-point requantisation (FloatRequant) for the channels of a layer, padded to `pad_to`; empty when
-// a channel's sums may leave its range. filt: [oc][per_channel] integer-valued weights; |activation| <= 128.
-inline std::vector<FloatRequant> float_requant(const std::vector<float> &filt, const std::vector<float> &bias,
+// a channel's sums may leave its range. filt: [oc][per] integer-valued weights; |activation| <= 128.
+inline std::vector<FloatRequant> float_requant(const float *filt, size_t per, const std::vector<float> &bias,
                                                const std::vector<float> &mult, const std::vector<float> &rshift, bool relu,
                                                int pad_to) {
-  const size_t oc = bias.size(), per = filt.size() / oc;
+  const size_t oc = bias.size();
   std::vector<FloatRequant> out(std::max<size_t>(oc, pad_to), FloatRequant{0u, 0.0f, 0.0f, 0.0f});
   const double scale = kFqScale;
   for (size_t o = 0; o < oc; ++o) {
     // sum of |w| in sixteen lanes: integers that stay exact in a float (2^24 / 128 weights and more per lane)
-    const float *w = filt.data() + o * per;
+    const float *w = filt + o * per;
     float lane[16] = {};
     double sum = 0;
     for (size_t i = 0; i < per; i += 16 << 16) {
@@ -538,7 +538,7 @@ public:
     d_bias_ = I.upload(to_i32(bias, oc_pad));
     d_mult_ = I.upload(to_i32(mult, oc_pad, true));
     d_rsh_ = I.upload(to_i32(rshift, oc_pad, true));
-    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, mult, rshift, do_relu_ != 0, oc_pad);
+    const std::vector<FloatRequant> fq = float_requant(filt.data.data(), filt.data.size() / bias.size(), bias, mult, rshift, do_relu_ != 0, oc_pad);
     const FloatRequant *d_fq = fq.empty() ? nullptr : I.upload(fq);
 
     if (g.g == g.ic && g.g == g.oc && g.g > 1 && g.ins_h == 0 && g.ins_w == 0) {
@@ -692,7 +692,7 @@ public:
     alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.size()) + (kind == 0 ? 12.0 : 4.0) * g_.oc;
     DenseLayer d;
     d.g = g_; d.in_cp = in_->cp; d.out_cp = out_->cp;
-    d.w = filt; d.bias = bias; d.mult = mult; d.rshift = rshift;
+    d.w = filt.data(); d.bias = bias; d.mult = mult; d.rshift = rshift;
     // (1x1 layers of 16 or 32 channels twice)
     while (!wp && pair_applies(d.g, d.in_cp, d.out_cp, es) && (g_.kw == 1 || !d.paired)) pair_layer(d);
     const ConvGeom &g = d.g;
@@ -711,7 +711,7 @@ public:
       p.bias = I.upload(to_i32(d.bias, d.out_cp));
       p.mult = I.upload(to_i32(d.mult, d.out_cp, true));
       p.rshift = I.upload(to_i32(d.rshift, d.out_cp, true));
-      const std::vector<FloatRequant> fq = float_requant(d.w, d.bias, d.mult, d.rshift, do_relu_ != 0, d.out_cp);
+      const std::vector<FloatRequant> fq = float_requant(d.w, (size_t)g.ic * g.kh * g.kw, d.bias, d.mult, d.rshift, do_relu_ != 0, d.out_cp);
       if (!fq.empty()) p.fq = I.upload(fq);
       if (I.selftest_lost_arrival > 0) {
         p.wait_rounds = I.selftest_lost_arrival;
@@ -770,12 +770,10 @@ public:
     else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, p.m_tile);
     // A tap's weights are padded to whole K blocks: rows that start off 32-byte sectors and reach past the extent arrive at
     // a third of the rate (7 x 45 x 45 pixels, 80 -> 128 channels, 5x5: 35.9 -> 28.3 us; MobileNet-v2 batch 32 426 -> 408).
-    const std::vector<int8_t> w = kind == 0 ? pack_conv_weights(d.w.data(), g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp, false, 0)
-                                            : pack_conv_weights_bf16(d.w.data(), g.oc, g.ic, g.kh, g.kw, d.out_cp, d.in_cp);
-    const size_t pitch = (size_t)p.c_chunks * p.BK, w_rows = (size_t)d.out_cp * taps;
-    std::vector<int8_t> v(w_rows * pitch, 0);
-    for (size_t i = 0; i < w_rows; ++i) std::memcpy(v.data() + i * pitch, w.data() + i * k_bytes, k_bytes);
-    encode_weight_map(&pl.tmB, I.upload(v), d.out_cp, taps, (int)pitch, p.BK, p.dual ? 192 : 128);
+    const int pitch = p.c_chunks * p.BK;
+    const int8_t *d_w = I.upload(kind == 0 ? pack_conv_weights(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch, false, 0)
+                                           : pack_conv_weights_bf16(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch / 2));
+    encode_weight_map(&pl.tmB, d_w, d.out_cp, taps, pitch, p.BK, p.dual ? 192 : 128);
   }
   // Fused leaky ReLU (tensor-core plans only): the epilogue writes the plain result to this op's tensor
   // and the activation result to `act_out`.
@@ -1000,7 +998,7 @@ public:
     // multiplier the two orders give the same int8 result.
     p.act = do_relu_ ? 1 : 0;
     p.fastq = requant_fast_flags(rs, bias, k_);
-    const std::vector<FloatRequant> fq = float_requant(filt.data, bias, mu, rs, do_relu_ != 0, n_pad);
+    const std::vector<FloatRequant> fq = float_requant(filt.data.data(), filt.data.size() / bias.size(), bias, mu, rs, do_relu_ != 0, n_pad);
     if (!fq.empty()) p.fq = I.upload(fq);
     p.a_mode = 0;
     finish_plan(pl, m_, 1, kdev_, n_pad, I.sm_count);
