@@ -345,3 +345,65 @@ def test_last_batch_read_from_the_tensors(count):
     multi, _ = ActivationCalibrator(m, lambda: iter(data)).run_multi([1024, 2048])
     assert {k: float(v) for k, v in multi[2048].items()} == thr
     m.close()
+
+
+class _Lying:
+    """An iterator that says after every item that nothing is left."""
+
+    def __init__(self, items):
+        self._it = iter(items)
+
+    def __iter__(self):
+        return self
+
+    def __next__(self):
+        return next(self._it)
+
+    def __length_hint__(self):
+        return 0
+
+
+@pytest.mark.parametrize("kind", ["list", "list_iterator", "generator", "lying"])
+def test_loader_is_asked_after_the_statistics_are_enqueued(kind):
+    """A loader slower than the forward pass must find every batch's work enqueued when it is asked for the next, whatever
+    it says about its length, and the results do not depend on that."""
+    from tpu_compiler_b200 import module
+    from tpu_compiler_b200.calibration import ActivationCalibrator
+    model = small_fp32_model(4)
+    rng = np.random.default_rng(81)
+    data = [np.clip(rng.normal(0, 1 + i, (4, 3, 24, 24)), -3, 3).astype(np.float32) for i in range(3)]
+    m = module(0)
+    m.load_text(model.text, model.weights)
+    want = {k: float(v) for k, v in ActivationCalibrator(m, lambda: (b for b in data), keep_activations_gb=0).run()[0].items()}
+    order = []
+
+    class Recorded(list):   # the batches, noting when each is taken
+        def __iter__(self):
+            for b in list.__iter__(self):
+                order.append("batch")
+                yield b
+
+    def batches():
+        if kind == "list":
+            return Recorded(data)
+        if kind == "list_iterator":
+            return iter(data)
+        return _Lying(Recorded(data)) if kind == "lying" else (b for b in Recorded(data))
+
+    cal = ActivationCalibrator(m, batches)
+
+    class Lib:
+        def __getattr__(self, name):
+            if name == "tpucb_calib_minmax_all":
+                order.append("statistics")
+            return getattr(lib, name)
+
+    lib, cal._lib = cal._lib, Lib()
+    got, _ = cal.run()
+    assert {k: float(v) for k, v in got.items()} == want
+    if kind == "list_iterator":
+        assert order == ["statistics"] * 3
+    else:
+        assert order[:6] == ["batch", "statistics"] * 3
+    assert cal.num_samples == 12
+    m.close()

@@ -18,6 +18,7 @@ Batches beyond the budget are recomputed as before. The values read are the same
 """
 import ctypes as C
 import datetime
+import operator
 import time
 
 import numpy as np
@@ -99,7 +100,8 @@ class ActivationCalibrator:
         per_batch, budget = self._keep_plan()
         self.pass1_host_s = {k: 0.0 for k in self.pass1_host_s}
         self._live = None
-        batches = iter(self.batches())
+        loader = self.batches()
+        batches = iter(loader)
         batch = next(batches, None)
         index = 0
         while batch is not None:
@@ -107,17 +109,13 @@ class ActivationCalibrator:
             t_enq = time.perf_counter()
             self.model.launch()
             images = batch.shape[0]
-            if self._one_run:   # the last batch of a run is not copied: its histograms are taken from the tensors themselves
-                                # (two batches of 64 ResNet-50 images: 17.8 -> 17.0 ms)
-                self.pass1_host_s["enqueue"] += time.perf_counter() - t_enq
-                batch = next(batches, None)
-                t_enq = time.perf_counter()
-                if batch is None and per_batch:
-                    self._live = (index, images)
+            # the last batch of a run is not copied: its histograms are taken from the tensors themselves
+            if self._one_run and per_batch and self._is_last(loader, batches, index):
+                self._live = (index, images)
             keep = None
             if self._live is not None:
                 pass
-            elif self._reserved:
+            elif self._reserved and budget:
                 keep = self._reserved.pop()
             elif per_batch and (len(self._kept) + 1) * per_batch <= budget:
                 try:
@@ -137,14 +135,28 @@ class ActivationCalibrator:
                 self._kept.append((keep, images))
             n_img += images
             self.pass1_host_s["enqueue"] += time.perf_counter() - t_enq
-            if not self._one_run:
-                batch = next(batches, None)
+            batch = next(batches, None)  # all of this batch's work is enqueued: a slow loader keeps nothing waiting
+            if batch is not None and self._live is not None:
+                self._live = None   # not the last one after all: it is recomputed, and so are those behind it, because
+                budget = 0          # the cache holds the first batches without a gap
             index += 1
         t_sync = time.perf_counter()
         self.model.sync()
         self.pass1_host_s["final_sync"] += time.perf_counter() - t_sync
         self._local_images = n_img
         return stats, n_img
+
+    @staticmethod
+    def _is_last(loader, batches, index):
+        """Whether batch ``index``, just taken from ``batches``, is the last one, as far as can be told without asking for
+        the next: from the loader's length, or from what the iterator says is left (a list's iterator knows, a
+        generator does not). A wrong yes costs a recomputation, a wrong no a copy."""
+        try:
+            if loader is not batches and hasattr(loader, "__len__"):
+                return len(loader) == index + 1
+            return operator.length_hint(batches, -1) == 0
+        except TypeError:   # a DataLoader over an iterable data set has the method, but no length
+            return False
 
     def _name_array(self):
         if getattr(self, "_names_c", None) is None:
