@@ -407,3 +407,46 @@ def test_loader_is_asked_after_the_statistics_are_enqueued(kind):
         assert order[:6] == ["batch", "statistics"] * 3
     assert cal.num_samples == 12
     m.close()
+
+
+def test_pinned_batches_live_until_their_copies_have_left():
+    """A loader that drops its pinned batches: none of them may be freed (and its memory handed to the next batch) before
+    the copy out of it is known to be over."""
+    import weakref
+    import torch
+    from tpu_compiler_b200 import module
+    from tpu_compiler_b200.calibration import ActivationCalibrator
+    model = small_fp32_model(4)
+    m = module(0)
+    m.load_text(model.text, model.weights)
+    pending, early = {}, []
+
+    class Model:
+        def __getattr__(self, name):
+            return getattr(m, name)
+
+        def set_tensor_async(self, name, ptr, numel):
+            pending[ptr.value] = True
+            m.set_tensor_async(name, ptr, numel)
+
+        def wait_uploads(self):
+            m.wait_uploads()
+            pending.clear()
+
+        def sync(self):
+            m.sync()
+            pending.clear()
+
+    def batches():
+        g = torch.Generator().manual_seed(3)
+        for _ in range(7):
+            b = torch.randn(4, 3, 24, 24, generator=g).clamp_(-3, 3).pin_memory()
+            weakref.finalize(b, lambda p=b.data_ptr(): early.append(p) if p in pending else None)
+            yield b
+            del b
+
+    cal = ActivationCalibrator(Model(), batches, keep_activations_gb=0)
+    cal.run()
+    assert not early and cal.num_samples == 28
+    del cal
+    m.close()

@@ -67,6 +67,7 @@ class ActivationCalibrator:
         self._pinned = None
         self._pinned_numel = 0
         self._pinned_next = 0
+        self._in_flight = ()     # pinned batches of the caller's whose copies may still read them
         self._reserved = []      # cache buffers allocated ahead of pass 1
         # host seconds of this rank's last pass 1 by part: copying batches into pinned memory, waiting for earlier
         # uploads to leave their buffer, enqueueing (module launch + statistics launch), the final synchronisation
@@ -192,12 +193,18 @@ class ActivationCalibrator:
         with set_tensor_async, so the host-side copy and the transfer of batch i + 1 run while batch i is computed."""
         if (isinstance(batch, torch.Tensor) and batch.device.type == "cpu" and batch.dtype == torch.float32 and
                 batch.is_contiguous() and batch.is_pinned()):
-            # already in page-locked memory (a loader with pin_memory=True): sent from where it lies; the two most
-            # recent batches are kept alive until their copies have left the host
+            # already in page-locked memory (a loader with pin_memory=True): sent from where it lies, and kept alive until
+            # its copy has left the host (this thread enqueues far faster than batches are computed, and the loader may
+            # take the memory of a batch that nobody holds for another one)
             t0 = time.perf_counter()
+            if len(self._in_flight) >= 2:
+                self.model.wait_uploads()
+                self._in_flight = ()
+            t1 = time.perf_counter()
             self.model.set_tensor_async(self.input_name, C.c_void_p(batch.data_ptr()), batch.numel())
-            self._in_flight = (getattr(self, "_in_flight", ()) + (batch,))[-2:]
-            self.pass1_host_s["enqueue"] += time.perf_counter() - t0
+            self._in_flight += (batch,)
+            self.pass1_host_s["wait_uploads"] += t1 - t0
+            self.pass1_host_s["enqueue"] += time.perf_counter() - t1
             return
         if isinstance(batch, torch.Tensor):
             batch = batch.numpy()
