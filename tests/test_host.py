@@ -127,3 +127,73 @@ def test_concurrent_builds(tmp_path):
     assert got == [b"half-written-library"] * 2
     assert open(log_path).read().count("compiled") == 1
     assert [f for f in os.listdir(tmp_path) if f.endswith(".tmp")] == []
+
+
+COPY_HELPERS = r"""
+#include "host_copy.h"
+#include <cerrno>
+#include <cstdio>
+#include <cstdlib>
+#include <dlfcn.h>
+#include <pthread.h>
+#include <sys/wait.h>
+#include <vector>
+
+static std::atomic<int> may_start{1 << 30}; // threads that may still be created
+extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *x) {
+  if (may_start.fetch_sub(1) <= 0) return EAGAIN;
+  static auto real = (int (*)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *))dlsym(RTLD_NEXT, "pthread_create");
+  return real(t, a, f, x);
+}
+
+static bool copies(unsigned seed, int rounds) {
+  const size_t block = 64u << 10;
+  std::vector<uint8_t> src(37 * block + 4321);
+  uint8_t *dst = (uint8_t *)aligned_alloc(64, 38 * block);
+  bool good = true;
+  for (int r = 0; r < rounds; ++r) {
+    const int n = 1 + (r * 7 + seed) % 38;
+    const size_t len = n == 38 ? src.size() : n * block;
+    for (size_t i = 0; i < len; i += 97) src[i] = (uint8_t)(i * 31 + r + seed);
+    std::atomic<int> done{0};
+    int calls = 0;
+    tpucb::CopyHelpers::run(
+        n, true,
+        [&](int i) {
+          tpucb::stream_copy(dst + i * block, src.data() + i * block, std::min(block, len - i * block));
+          done.fetch_add(1);
+        },
+        [&] { ++calls; return done.load() == n; });
+    good = good && calls >= 1 && done.load() == n && std::memcmp(dst, src.data(), len) == 0;
+  }
+  free(dst);
+  return good;
+}
+
+int main(int argc, char **argv) {
+  if (argc > 1) may_start = atoi(argv[1]);
+  if (!copies(0, 50)) return 1;
+  if (argc > 1) return 0;
+  std::atomic<int> bad{0};
+  std::vector<std::thread> users;
+  for (unsigned t = 1; t <= 4; ++t) users.emplace_back([&, t] { if (!copies(t, 200)) ++bad; });
+  for (auto &u : users) u.join();
+  const pid_t child = fork();
+  if (child == 0) _exit(copies(9, 50) ? 0 : 1); // the helpers of the parent are not there
+  int status = 1;
+  waitpid(child, &status, 0);
+  return bad || status || !copies(10, 50);
+}
+"""
+
+
+def test_copy_helpers_threads_fork_and_thread_limit(tmp_path):
+    """The copies of set_tensor on several host threads: four threads at once, a forked child, and a process that may start
+    no helper, one or two."""
+    import subprocess
+    src, exe = tmp_path / "t.cpp", str(tmp_path / "t")
+    src.write_text("#include <algorithm>\n#include <cstdint>\n" + COPY_HELPERS)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-I", os.path.join(ROOT, "tpu_compiler_b200", "csrc"), str(src), "-o", exe,
+                    "-ldl"], check=True)
+    for args in ([], ["0"], ["1"], ["2"]):
+        assert subprocess.run([exe] + args, timeout=120).returncode == 0, args

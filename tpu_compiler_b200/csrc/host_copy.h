@@ -99,7 +99,10 @@ private:
   CopyHelpers() {
     const unsigned cores = std::thread::hardware_concurrency();
     const int helpers = cores >= 8 ? 3 : (cores >= 4 ? 1 : 0);
-    for (int i = 0; i < helpers; ++i) std::thread([this] { loop(); }).detach();
+    try {
+      for (int i = 0; i < helpers; ++i) std::thread([this] { loop(); }).detach();
+    } catch (...) { // no more threads to be had: those that run are enough, and none are, too
+    }
   }
   static void pause() {
 #if defined(__x86_64__)
