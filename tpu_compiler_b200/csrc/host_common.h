@@ -91,6 +91,11 @@ inline int &pdl_mode() {
   static thread_local int v = 1;
   return v;
 }
+// SMs of the device that this thread launches on (set with the flags above)
+inline int &launch_sm_count() {
+  static thread_local int v = 148;
+  return v;
+}
 // While one lives, launch_k marks launches when the mode includes the convolution class; afterwards as before.
 struct PdlConvScope {
   bool before;
@@ -118,7 +123,7 @@ inline void launch_k(void (*kernel)(KArgs...), G grid, B block, size_t smem, cud
   // cannot be placed badly by the order in which its predecessor's blocks leave, and its scheduling is most of what it
   // costs (MobileNet-v2 batch 1 227 -> 218 us, 12 307 -> 296; YOLOv4-style batch 1 1181 -> 1160; twice the threads: a loss).
   const bool pdl = launch_pdl_flag() || (pdl_mode() == 1 && (size_t)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z *
-                                             cfg.blockDim.x * cfg.blockDim.y * cfg.blockDim.z <= 148 * 256);
+                                             cfg.blockDim.x * cfg.blockDim.y * cfg.blockDim.z <= (size_t)launch_sm_count() * 256);
   // The arguments are converted to the kernel's own parameter types and passed by address; without the attribute the
   // launch goes through the classic entry point.
   auto go = [&](KArgs... a) {

@@ -110,6 +110,7 @@ public:
     TPUCB_CUDA(cudaSetDevice(device_));
     pdl_mode() = use_pdl;
     launch_pdl_flag() = use_pdl >= 2;
+    launch_sm_count() = sm_count;
     conv_split_k_enabled() = split_k && selftest_lost_arrival == 0; // the self-test needs tiles that follow one another in a CTA
   }
   int device() const { return device_; }
