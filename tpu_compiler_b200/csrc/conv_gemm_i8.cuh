@@ -152,14 +152,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *tmap, uint
       "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *tmap, uint32_t bar, int x,
-                                            int y, int z, int w) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
-      "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
 __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const void *tmap, uint32_t bar,
                                                    int c, int w, int h, int n, uint16_t off_w,
                                                    uint16_t off_h) {
@@ -317,7 +309,6 @@ __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr, int BK)
 constexpr int kEpilogueWarps = 8;
 constexpr int kConvThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kMaxStages = 8;
-constexpr int kMaxBN = 256;
 constexpr int kSmemHeader = 8192; // barriers + staged per-channel parameters
 
 // Records why a launch gave up, in the device word that later CTAs and kernels look at and in the host's own memory, whose
@@ -475,7 +466,7 @@ __device__ __forceinline__ uint32_t transpose4x4(uint32_t w, const TransposeSel 
 //   lane_addr  TMEM address of the warp's lane quarter in the buffer
 //   out4       output address of (pixel m0, this lane's 4-channel group)
 //   ch4_ok     the 4-channel group lies inside the valid channels
-//   ncols      pixel columns of the accumulator buffer (128; 256 for the two-SM tile)
+//   ncols      pixel columns of the accumulator buffer that the tile fills (128, or 64 for half tiles)
 //   FORM       of the requantisation: 0 requant_one, 1 requant_fast, 2 requant_fast with every rshift >= 1, 3 float_requant4
 template <int ACT, int FORM, bool FROM_WS = false, class Consts = ChanConst>
 __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4,

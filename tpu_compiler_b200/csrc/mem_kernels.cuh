@@ -843,23 +843,23 @@ dwconv3x3_dp4a_kernel(const uint32_t *__restrict__ in, uint32_t *__restrict__ ou
         const uint32_t wa[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-        const int w0 = (int)wa[k], w1 = (int)(wa[k] << 8); // taps on bytes 0..2, or on bytes 1..3
-        const uint32_t t0 = tch[0][k], t1 = tch[1][k], t2 = tch[2][k];
-        if (S == 1) {
-          acc[o][0][k] = __dp4a((int)t0, w0, acc[o][0][k]);                                 // columns 0..2
-          acc[o][1][k] = __dp4a((int)t0, w1, acc[o][1][k]);                                 // 1..3
-          acc[o][2][k] = __dp4a((int)__funnelshift_r(t0, t1, 16), w0, acc[o][2][k]);        // 2..4
-          acc[o][3][k] = __dp4a((int)__funnelshift_r(t0, t1, 24), w0, acc[o][3][k]);        // 3..5
-          acc[o][4][k] = __dp4a((int)t1, w0, acc[o][4][k]);                                 // 4..6
-          acc[o][5][k] = __dp4a((int)t1, w1, acc[o][5][k]);                                 // 5..7
-          acc[o][6][k] = __dp4a((int)__funnelshift_r(t1, t2, 16), w0, acc[o][6][k]);        // 6..8
-          acc[o][7][k] = __dp4a((int)__funnelshift_r(t1, t2, 24), w0, acc[o][7][k]);        // 7..9
-        } else {
-          acc[o][0][k] = __dp4a((int)t0, w0, acc[o][0][k]);                                 // columns 0..2
-          acc[o][1][k] = __dp4a((int)__funnelshift_r(t0, t1, 16), w0, acc[o][1][k]);        // 2..4
-          acc[o][2][k] = __dp4a((int)t1, w0, acc[o][2][k]);                                 // 4..6
-          acc[o][3][k] = __dp4a((int)__funnelshift_r(t1, t2, 16), w0, acc[o][3][k]);        // 6..8
-        }
+          const int w0 = (int)wa[k], w1 = (int)(wa[k] << 8); // taps on bytes 0..2, or on bytes 1..3
+          const uint32_t t0 = tch[0][k], t1 = tch[1][k], t2 = tch[2][k];
+          if (S == 1) {
+            acc[o][0][k] = __dp4a((int)t0, w0, acc[o][0][k]);                                 // columns 0..2
+            acc[o][1][k] = __dp4a((int)t0, w1, acc[o][1][k]);                                 // 1..3
+            acc[o][2][k] = __dp4a((int)__funnelshift_r(t0, t1, 16), w0, acc[o][2][k]);        // 2..4
+            acc[o][3][k] = __dp4a((int)__funnelshift_r(t0, t1, 24), w0, acc[o][3][k]);        // 3..5
+            acc[o][4][k] = __dp4a((int)t1, w0, acc[o][4][k]);                                 // 4..6
+            acc[o][5][k] = __dp4a((int)t1, w1, acc[o][5][k]);                                 // 5..7
+            acc[o][6][k] = __dp4a((int)__funnelshift_r(t1, t2, 16), w0, acc[o][6][k]);        // 6..8
+            acc[o][7][k] = __dp4a((int)__funnelshift_r(t1, t2, 24), w0, acc[o][7][k]);        // 7..9
+          } else {
+            acc[o][0][k] = __dp4a((int)t0, w0, acc[o][0][k]);                                 // columns 0..2
+            acc[o][1][k] = __dp4a((int)__funnelshift_r(t0, t1, 16), w0, acc[o][1][k]);        // 2..4
+            acc[o][2][k] = __dp4a((int)t1, w0, acc[o][2][k]);                                 // 4..6
+            acc[o][3][k] = __dp4a((int)__funnelshift_r(t1, t2, 16), w0, acc[o][3][k]);        // 6..8
+          }
         }
       }
     }
