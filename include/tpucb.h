@@ -143,8 +143,9 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          global access. 1 gives the attribute to the tensor-core convolution kernels, the activation chains and
  *          launches too small to fill the chip, which measured faster than none and than all (on large memory-bound
  *          kernels it costs 1-5%).
- *          "split_k" (0/1, default 1; read by the next load_module): INT8 convolutions and inner products with few
- *          tiles and 24 K blocks or more share each tile among several CTAs (exact: int32 partial sums).
+ *          "split_k" (0/1, default 1; read by the next load_module): INT8 convolutions and inner products with at most
+ *          half as many tiles as SMs and a K that is long enough to pay for the exchange (from about 24 K blocks for
+ *          a few tiles to 48 for many) share each tile among several CTAs (exact: int32 partial sums).
  *          "fuse_activations" (0/1, default 1; read by the next load_module): run each
  *          quant(INT8->BF16) -> slope-table activation -> quant(BF16->INT8) chain as one launch
  *          that still writes all three tensors.
@@ -158,8 +159,8 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          two-input eltwise add whose later-produced operand is a tensor-core convolution that feeds nothing else
  *          (the last convolution of a residual block) runs in that convolution's epilogue, which reads the other
  *          operand and writes both the convolution's tensor and the sum; the add launches nothing. Same bits.
- *          By size: results of 2.5 to 8 MB of layers that widen their input (INT8 ResNet-50 at batch 19:
- *          2% fewer us alone, 7% with three modules in flight; at batch 1 and 256 the add is faster by itself).
+ *          By size: results of 2.5 to 8 MiB of layers that widen their input (INT8 ResNet-50 at batch 19:
+ *          3% fewer us alone, 5% with three modules in flight; at batch 1 and 256 the add is faster by itself).
  *          "fp32_tensor_cores" (0/1, default 1; read by the next load_module): fp32 convolutions with a
  *          multiple of 8 input channels run on the tensor cores as three TF32 products with fp32 accumulation
  *          (about 5e-6 of a tensor's range per layer against a double-accumulated sum, 6e-5 at the end of an

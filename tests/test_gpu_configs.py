@@ -79,7 +79,7 @@ def test_conv_sweep_point_full_rshift_range(relu):
 
 @pytest.mark.parametrize("n,c,hw,relu", [(1, 512, 7, True), (2, 1024, 5, False), (3, 384, 9, True)])
 def test_split_k_layers(n, c, hw, relu):
-    """Launches with few tiles and 24 K blocks or more share each tile among several CTAs (int32 partial sums added in
+    """Launches with few tiles and a long K share each tile among several CTAs (int32 partial sums added in
     global memory, the CTA that completes a tile runs the epilogue). Exact against the oracle, equal to the unsplit
     launch, and the same again on every graph replay (the workspace is left zero)."""
     from tpu_compiler_b200 import module

@@ -238,3 +238,22 @@ def test_download_forms(dtype, shape):
     m.set_tensor("x", x)
     assert np.array_equal(m.get_tensor("x"), x)
     m.close()
+
+
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, k: most tiles that are still split in three, in two, and fewest that are not
+    (12, 512, 512, 7, 3), (8, 128, 512, 10, 7), (1, 64, 128, 33, 5), (16, 512, 512, 7, 3)])
+def test_split_rule_edges(case):
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, k = case
+    model = graphs.single_conv_i8(n, ic, oc, hw, k, 1, k // 2, seed=3300 + k)
+    got = []
+    for split in (1, 0):
+        m = module(0)
+        m.set_option("split_k", split)
+        m.load_text(model.text, model.weights)
+        m.set_tensor("x", model.meta["x"])
+        for _ in range(2):
+            m.invoke()
+            got.append(m.get_tensor("conv"))
+        m.close()
+    assert all(np.array_equal(g, got[-1]) for g in got)

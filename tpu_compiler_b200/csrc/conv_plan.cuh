@@ -341,9 +341,11 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   const int k_iters = taps * p.c_chunks;
   const int n_tiles = (oc_pad + bn - 1) / bn;
   // A launch of few tiles takes half tiles: twice the CTAs, each with half the epilogue and three quarters of the bytes per K
-  // block (ResNet-50 batch 1 334 -> 318 us, BF16 batch 8 722 -> 669, YOLOv4-style batch 1 1166 -> 1012). Up to a third of the
-  // SMs: with more, launches of other streams that would have run beside this one no longer fit (19 x 14 x 14, 256 -> 256
-  // channels, 60 tiles: 10.3 us against 10.8 alone, but 4.3 against 4.0 with three streams). Quarter tiles gained nothing more.
+  // block (us alone and with three modules in flight: ResNet-50 batch 1 313 / 128 -> 292 / 116, BF16 batch 8 657 / 295 -> 594 /
+  // 285, YOLOv4-style batch 1 1069 / 446 -> 905 / 397; 8 x 14 x 14, 256 channels, 26 tiles: 9.3 / 4.7 -> 8.7 / 4.1). Up to a
+  // third of the SMs: with more, launches of other streams that would have run beside this one no longer fit (half tiles
+  // throughout: ResNet-50 batch 19 465 / 330 against 458 / 274, BF16 batch 8 582 / 319; 19 x 14 x 14, 256 channels, 60 tiles:
+  // 9.0 us against 10.2 alone, but 4.4 against 4.2). Quarter tiles gained nothing more.
   p.m_tile = p.dual ? 256 : 128;
   if (!p.dual && (rows + 127) / 128 * n_tiles * 3 <= sm_count) p.m_tile = 64;
   const int m_tiles = (rows + p.m_tile - 1) / p.m_tile;
@@ -357,8 +359,9 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   // activations, which halves the bytes that have to reach shared memory per MAC. Larger weight
   // sets would force one CTA per SM, which measured slower than re-fetching the weights from L2.
   const int ctas_per_sm = 2;
-  // (An fp32 launch of at most one CTA per SM takes all of the shared memory: ResNet-50 at batch 30 3654 -> 3591 us. For INT8
-  // and BF16 launches it is a loss: those of other streams no longer fit beside them.)
+  // (An fp32 launch of at most one CTA per SM takes all of the shared memory: ResNet-50 at batch 30 alone, as calibration and
+  // the tuner run it, 3455 -> 3377 us. Launches of other streams no longer fit beside it, three modules in flight 2474 ->
+  // 2653, which is why INT8 and BF16 launches leave half.)
   const size_t budget = (pl.tf32 && total_tiles <= sm_count ? 220 : 113) * 1024;
   // (Pixel groups have small activation tiles: up to 60 KB of weights leave them four stages.)
   p.w_resident = (!pl.tf32 && total_tiles >= 2LL * n_tiles && w_all <= (p.group > 1 ? 60 : 48) * 1024 &&

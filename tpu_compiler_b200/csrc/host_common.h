@@ -74,7 +74,7 @@ struct HostWeight {
 };
 
 // Whether launch_k marks its launches for programmatic dependent launch. Set per launch: the interpreter's option
-// "pdl" says which class of kernels gets the mark (pdl_mode: 0 none, 1 the tensor-core convolution kernels and others with set-up worth overlapping, 2 all), and
+// "pdl" says which class of kernels gets the mark (pdl_mode: 0 none, 1 the tensor-core convolution kernels, others with set-up worth overlapping and small launches, 2 all), and
 // the code that launches a kernel of the convolution class says so with PdlConvScope.
 inline bool &launch_pdl_flag() {
   static thread_local bool on = true;

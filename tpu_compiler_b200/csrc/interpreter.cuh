@@ -1960,11 +1960,18 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     const int self = pos[0] > pos[1] ? 0 : 1, other = 1 - self;
     auto *cv = dynamic_cast<Conv2DOp *>(kernels[pos[self]].get());
     if (!cv || !cv->can_fuse_add() || !single_use(cv->name)) continue;
-    // By size: layers that widen their input, results of 2.5 to 8 MB. There the launch that goes and the operand that is not
-    // read again count (ResNet-50 batch 19: 496 -> 485 us, three modules in flight 305 -> 284). Smaller ones lengthen the
-    // epilogue of a launch that is nothing but latency (batch 1 320 -> 329, batch 3 346 -> 352), larger ones are bound by the
-    // epilogue's instructions where the add itself runs at the rate of memory (batch 256: 2588 -> 2689), and layers with a
-    // long K and a short result gain alone and lose in flight (MobileNet-v2 batch 32: 394 -> 379 and 259 -> 266).
+    // By size: layers that widen their input, results of 2.5 to 8 MiB. There the launch that goes and the operand that is not
+    // read again count. Measured stage by stage on ResNet-50, all adds of one stage fused, us per step alone and with three
+    // modules in flight against none fused, by the stage's result:
+    //   below: 0.77 MiB +2 / +3 (res2, batch 1) and +7 / +14 (res4, batch 4), 1.5 MiB +2.7 / -1.5 and +2.2 / -7.7, 2.3 MiB
+    //   +3.7 / -10.7: a longer epilogue in launches that are nothing but latency;
+    //   inside: 3.06 MiB -1.9 / -4.7, +5.3 / -9.7 and +4.1 / -10.9, 4.2 -6.5 / -11.7, 6.1 -5.0 / -0.9 and +2.2 / -9.1, 7.3 -5.8 /
+    //   +0.6, 7.7 -4.5 / -3.3;
+    //   above: 8.4 -4.6 / +2.9, 9.2 -8.6 / +3.5 and -7.4 / +2.3, 12.3 -3.3 / +13, 24.5 +13 / +31, 98 +28 / -3: bound by the
+    //   epilogue's instructions, where the add by itself runs at the rate of memory.
+    // The window as a whole: batch 8 -6.9 / -3.5, 16 -0.3 / -14, 19 -14 / -13, 22 -7 / -14, 32 +4 / -21, 40 -8 / -14, 64 -1 / -3,
+    // nothing at 1, 96 and above. Layers with a long K and a short result gain alone and lose in flight (MobileNet-v2 batch
+    // 32: 394 -> 379 and 259 -> 266).
     if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19 || cv->out()->bytes() > 8u << 20)) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
@@ -2259,9 +2266,10 @@ inline void Interpreter::load_module(const std::string &text) {
       }
     }
     // An INT8 tensor that goes from an input or a convolution to convolutions only, one of them of several taps, starts
-    // each pixel on a 32-byte sector (7 x 45 x 45, 5x5 to 128 channels: 80 channels 28.3 -> 18.6 us at a pitch of 96, 48
-    // channels 19.3 -> 16.1 at 64). Tensors of other ops keep the pitch that their partners have, and those of 1x1 layers
-    // gain less from sectors than the wider pixels cost (MobileNet-v2 batch 32 408 -> 421).
+    // each pixel on a 32-byte sector (7 x 45 x 45, 5x5 to 128 channels, alone / with three streams: 80 channels 23.0 / 10.5 ->
+    // 16.3 / 6.6 us at a pitch of 96, 48 channels 17.7 / 6.9 -> 12.2 / 5.7 at 64). Tensors of other ops keep the pitch that
+    // their partners have, and those of 1x1 layers gain less from sectors than the wider pixels cost (MobileNet-v2 batch 32
+    // 408 -> 421).
     std::map<std::string, int> taps_of; // by source: filter taps of its largest consumer; -1: not convolutions only
     for (auto &op : parsed)
       for (size_t i = 0; i < op.in.size(); ++i) {
