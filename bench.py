@@ -722,17 +722,15 @@ def main():
         achieved = conv_ops / (conv_ms * 1e-3) / 1e12
         i8_tops = C.c_double(0.0)  # this library's own tcgen05 kind::i8 issue microbenchmark, live on this GPU
         check(L.tpucb_measure_i8_mma_peak(local_rank, 128, C.byref(i8_tops)))
-        # DRAM bytes per conv launch from the committed ncu capture of one step at batch 64
-        # (profiles/resnet50_int8_b64_dram_traffic.md: 10.09 MB read per launch, writes still dirty in L2 when the
-        # kernel ends), scaled by the images per launch; null for the workloads that have no capture.
         # DRAM traffic per launch: not captured in this run (a profiler capture of this size is out of bounds). The read
-        # side is the ncu figure of a whole step at batch 64 (10.09 MB of dram__bytes_read per tensor-core launch)
-        # scaled by the images per launch; ncu attributes no write-back to these kernels (their outputs are still
-        # dirty in L2 when they end), so the write side is the algorithmic output bytes.
+        # side is the ncu figure of a whole step at batch 64 (profiles/launch_lists.md: 10.49 MB of dram__bytes_read per
+        # tensor-core launch) scaled by the images per launch; ncu attributes no write-back to these kernels (their outputs
+        # are still dirty in L2 when they end), so the write side is the algorithmic output bytes. Null for the workloads
+        # that have no capture.
         traffic = None
         if args.workload == "resnet50":
             out_bytes = sum(float(np.prod(i["shape"])) for i in m.op_info if i["bound"] == "tensor") / max(n_conv, 1)
-            traffic = 10.09e6 * B / 64.0 + out_bytes
+            traffic = 10.49e6 * B / 64.0 + out_bytes
         if args.workload == "resnet50_bf16":
             # BF16 graph: the same pipeline with kind::f16 MMAs; the denominator is the measured bf16 rate itself
             roofline = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
@@ -750,8 +748,9 @@ def main():
                                         "batch / 64, plus the algorithmic output bytes (ncu attributes no write-back to "
                                         "the kernel); not captured in this run. Algorithmic bytes per launch: %.1f MB"
                                         % (conv_bytes / max(n_conv, 1) / 1e6),
-                        "kernel": "conv_gemm_i8_fq_kernel<0> / <1>: the tcgen05 kind::i8 implicit GEMM of "
-                                  "conv_gemm_i8.cuh in its ReLU and plain instantiations, %d launches per step" % n_conv,
+                        "kernel": "conv_gemm_i8_fq_kernel<0> / <1> and conv_gemm_i8_kernel: the tcgen05 kind::i8 implicit GEMM "
+                                  "of conv_gemm_i8.cuh with the floating-point and the integer requantisation, %d launches "
+                                  "per step" % n_conv,
                         "peak_source": "2 x bf16_tflops_sustained of %s peaks (no INT8 figure is measured; the 8-bit "
                                        "rate of the same tensor pipe is twice the 16-bit rate)" % peaks["source"],
                         "avg_launch_us": conv_ms * 1e3 / max(n_conv, 1),
