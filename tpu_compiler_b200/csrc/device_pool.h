@@ -9,8 +9,8 @@
 // whose addresses callers ask for (tpucb_interp_tensor_device), are blocks of cudaMalloc, which other processes can open
 // (cudaIpcGetMemHandle) and peers can read; the blocks of a destroyed module are kept for the next one.
 //
-// All are bounded and given back: when a module goes, free memory above kPoolKeepBytes returns to the driver (so much of
-// either kind), at most kPoolKeepStreams idle stream sets are kept, and when the last interpreter of a GPU goes, everything
+// All are bounded and given back: when a module goes, free memory above kPoolKeepBytes (the pool) and kBlockKeepBytes (the
+// blocks, a hundredth of the GPU's memory) returns to the driver, at most kPoolKeepStreams idle stream sets are kept, and when the last interpreter of a GPU goes, everything
 // goes. Several threads may use it at once (one mutex around the lists; the pool calls are thread-safe themselves). A pool
 // buffer is allocated and freed on its interpreter's stream, which is idle when the interpreter is destroyed; a block is
 // given back only when nothing uses it any more, so the next owner need not wait for the former one's stream.
@@ -24,6 +24,7 @@
 namespace tpucb {
 
 constexpr size_t kPoolKeepBytes = 256u << 20;
+constexpr size_t kBlockKeepBytes = 2048ull << 20;
 constexpr size_t kPoolKeepStreams = 8;
 
 // The error word of an interpreter: kernels that give up write their code here and, through `host`, into pinned host
@@ -145,6 +146,7 @@ public:
     std::lock_guard<std::mutex> lock(m_);
     auto it = free_blocks_.lower_bound(need);
     if (it != free_blocks_.end() && it->first <= need + need / 4) {
+      it = std::prev(free_blocks_.upper_bound(it->first)); // of its size the one freed last: L2 and TLB may still hold it
       void *p = it->second;
       free_bytes_ -= it->first;
       blocks_[p] = it->first;
@@ -171,7 +173,7 @@ public:
     free_blocks_.insert({it->second, p});
     free_bytes_ += it->second;
     blocks_.erase(it);
-    drop_blocks(kPoolKeepBytes);
+    drop_blocks(kBlockKeepBytes);
   }
 
   // Gives the driver back what lies free above kPoolKeepBytes. Called where a module's buffers have been freed; in between
