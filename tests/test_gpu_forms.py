@@ -257,3 +257,19 @@ def test_split_rule_edges(case):
             got.append(m.get_tensor("conv"))
         m.close()
     assert all(np.array_equal(g, got[-1]) for g in got)
+
+
+@pytest.mark.parametrize("relu", [0, 1])
+def test_bf16_results_past_the_largest_finite(relu):
+    """Sums that overflow or round past the largest BF16 become +0x7f7f for either sign; ReLU makes negative ones zero. Every
+    product is exact; channels and pixels leave remainders of a 32 x 32 block."""
+    rng = np.random.default_rng(11)
+    n, ic, oc, hw = 2, 32, 40, 9
+    f = np.zeros((oc, ic, 1, 1), np.float32)
+    f[np.arange(oc), np.arange(oc) % ic, 0, 0] = np.where(np.arange(oc) % 3 == 2, -1, 1) * np.float32(2.0) ** np.where(np.arange(oc) % 2, 64, 0)
+    x = np.float32(2.0) ** 63 * rng.choice([-3.0, -1.9921875, -1.0, 0.0, 1.0, 1.9921875, 3.0], (n, ic, hw, hw)).astype(np.float32)
+    b = np.where(np.arange(oc) % 5 == 0, 2.0 ** 119, 0.0).astype(np.float32)  # half of the last place of the largest finite value
+    text = "input name=x shape=%d,%d,%d,%d dtype=BF16\n" % (n, ic, hw, hw) + conv_text("BF16", n, ic, oc, hw, 1, 1, 0, 1, relu)
+    got, ref = run_model(text, {"f": f, "b": b}, {"x": x}, ["c"])["c"]
+    assert (ref == graphs._bf16_np(np.float32(3.39e38))).any()
+    assert np.array_equal(got, ref)

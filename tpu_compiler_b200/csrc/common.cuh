@@ -254,11 +254,35 @@ template <bool RELU> __device__ __forceinline__ uint32_t float_requant_pack(int 
   if (RELU) return relu_bytes(pack_sat_s8(v1, v0, pack_sat_s8(v3, v2, 0u)));
   return pack_sat_u8(v1, v0, pack_sat_u8(v3, v2, 0u)) ^ 0x80808080u;
 }
+// two 32-bit values as a register pair
+__device__ __forceinline__ unsigned long long pack_b32x2(uint32_t lo, uint32_t hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) { return pack_b32x2(__float_as_uint(lo), __float_as_uint(hi)); }
+// Two values of one channel: the packed multiply-adds round each half as the single ones do and take one issue slot for two.
+template <bool RELU> __device__ __forceinline__ void float_requant2(uint32_t a0, uint32_t a1, const FloatRequant &q, int &v0, int &v1) {
+  unsigned long long f = pack_b32x2(a0 + q.sb, a1 + q.sb);
+  asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(pack_f32x2(q.m, q.m)), "l"(pack_f32x2(q.d, q.d)));
+  const unsigned long long c = pack_f32x2(q.c, q.c);
+  if (RELU) {
+    const float e = q.c * -6.617444900424222e-24f; // as above
+    asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(c), "l"(pack_f32x2(e, e)));
+  } else {
+    const float k = -(float)kFqC * kFqScale;
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(pack_f32x2(k, k)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(c), "l"(pack_b32x2(128u, 128u)));
+  }
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(v0), "=r"(v1) : "l"(f));
+}
 // four values of one channel, packed
 template <bool RELU>
 __device__ __forceinline__ uint32_t float_requant4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const FloatRequant &q) {
-  return float_requant_pack<RELU>(float_requant1<RELU>(a0, q), float_requant1<RELU>(a1, q), float_requant1<RELU>(a2, q),
-                                  float_requant1<RELU>(a3, q));
+  int v0, v1, v2, v3;
+  float_requant2<RELU>(a0, a1, q, v0, v1);
+  float_requant2<RELU>(a2, a3, q, v2, v3);
+  return float_requant_pack<RELU>(v0, v1, v2, v3);
 }
 #endif
 

@@ -15,9 +15,8 @@
 // accumulate in int32 in tensor memory (tcgen05.mma kind::i8). With channels on the TMEM
 // lanes every epilogue thread owns ONE output channel, so its bias / multiplier / rshift
 // constants sit in registers instead of being re-read per value; the epilogue requantises,
-// saturates, applies ReLU, transposes 4 channels x 4 pixels between neighbouring lanes with
-// byte permutes and two shuffles, and stores 4 channels of one pixel per lane (a warp
-// writes whole 32-byte sectors of the NHWC output).
+// saturates, applies ReLU, transposes through shared memory with transposing matrix stores, and
+// stores 8 channels of one pixel per lane (a warp writes whole 32-byte sectors of the NHWC output).
 //
 // Warp roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA
 // issuer, warps 2..9 = epilogue (two warps per TMEM lane quarter, alternating
@@ -309,7 +308,7 @@ __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr, int BK)
 constexpr int kEpilogueWarps = 8;
 constexpr int kConvThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kMaxStages = 8;
-constexpr int kSmemHeader = 8192; // barriers + staged per-channel parameters
+constexpr int kSmemHeader = 1024 + 8 * 1024; // barriers, then kStageBytes for each epilogue warp
 
 // Records why a launch gave up, in the device word that later CTAs and kernels look at and in the host's own memory, whose
 // address stands 8 bytes behind the device word (ErrWord).
@@ -443,35 +442,68 @@ __device__ __forceinline__ int leaky_of(int v, const ConvGemmParams &p) {
   return mul_rshift_sat8(v, p.leaky_mn, p.leaky_rn);
 }
 
-// Byte-permute selectors of the 4x4 transpose between the four lanes of a group (lane & 3): two exchange steps
-// (lane ^ 1, then lane ^ 2); each lane sends its whole word and picks two of its own bytes and two of its
-// partner's with one permute per step.
-struct TransposeSel {
-  uint32_t merge1, merge2;
+// Channel of a 32-channel block that sits on TMEM lane `lane` of its quarter, and the row of the packed weights that puts it
+// there. Lanes 4i + j hold channels 8j + i: the transposing matrix store below then leaves runs of eight channels.
+TPUCB_HD int lane_channel(int lane) { return 8 * (lane & 3) + (lane >> 2); }
+TPUCB_HD int packed_row(int channel) { return (channel & ~31) | (4 * (channel & 7) + ((channel & 31) >> 3)); }
+
+// A warp's kStageBytes of shared memory, through which the epilogue turns "one channel, several pixels" per lane into "one
+// pixel, eight channels": matrix stores that transpose (rows of 16 bytes, `put` is this lane's), 16-byte loads from `get`.
+// Per 32 channels x 32 pixels two stores and two loads (INT8); exchanged between lanes by shuffles and byte permutes it was
+// 32 instructions, and 16 for the stores and their addresses instead of 8. ResNet-50, us alone before and after: INT8 batch 256
+// 2555 -> 2470 (64 -> 256 channels, 1x1, 56 x 56: 82 -> 76), batch 19 465 -> 442; BF16 batch 128 2459 -> 2276 (72 -> 47).
+constexpr int kStageBytes = 1024;
+struct StageLane {
+  uint32_t put, get;
+  int px; // the first pixel that this lane gets
 };
-__device__ __forceinline__ TransposeSel make_transpose_sel(int lane) {
-  TransposeSel t;
-  t.merge1 = (lane & 1) ? 0x3715u : 0x6240u;
-  t.merge2 = (lane & 2) ? 0x3276u : 0x5410u;
-  return t;
+// PX_PER_WORD: pixels that a lane packs into one word before the transposition (4 of one byte, 2 of two)
+template <int PX_PER_WORD> __device__ __forceinline__ StageLane make_stage_lane(uint32_t warp_stage, int lane) {
+  const int pair = lane >> 3, h = (lane >> 2) & 1;
+  return StageLane{warp_stage + lane * 16, warp_stage + pair * 128 + (2 * (lane & 3) + h) * 16, (PX_PER_WORD * pair) + h};
 }
-// In: lane i of a 4-lane group holds bytes (pixel 0..3) of channel i. Out: lane j holds bytes
-// (channel 0..3) of pixel j.
-__device__ __forceinline__ uint32_t transpose4x4(uint32_t w, const TransposeSel &t) {
-  const uint32_t z = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 1), t.merge1);
-  return __byte_perm(z, __shfl_xor_sync(0xffffffffu, z, 2), t.merge2);
+__device__ __forceinline__ void lds128(uint32_t at, uint32_t (&v)[4]) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
+}
+// INT8. In: byte b of w[k] is pixel 4k + b of this lane's channel. Out: u[2i], u[2i + 1] hold channels 8 (lane & 3) .. + 7 of
+// pixel st.px + stage_step8(i).
+__device__ __forceinline__ constexpr int stage_step8(int i) { return 2 * (i & 1) + 16 * (i >> 1); }
+__device__ __forceinline__ void transpose_i8(const uint32_t (&w)[8], uint32_t (&u)[8], const StageLane &st) {
+  __syncwarp(); // the previous chunk has been read
+  asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};" ::"r"(st.put), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]) : "memory");
+  asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};" ::"r"(st.put + 512u), "r"(w[4]), "r"(w[5]),
+               "r"(w[6]), "r"(w[7]) : "memory");
+  __syncwarp();
+  uint32_t a[4], b[4];
+  lds128(st.get, a);
+  lds128(st.get + 512u, b);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    u[i] = a[i];
+    u[4 + i] = b[i];
+  }
+}
+// address of pixel `px` from `base`, by one wide multiply-add (the multiply-add pipe has room, the integer ALU has not)
+__device__ __forceinline__ unsigned long long px_addr(const void *base, int px, int pitch) {
+  unsigned long long a;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"((uint32_t)px), "r"((uint32_t)pitch), "l"((unsigned long long)base));
+  return a;
+}
+__device__ __forceinline__ void stg64(unsigned long long at, uint32_t x, uint32_t y) {
+  asm volatile("st.global.v2.b32 [%0], {%1, %2};" ::"l"(at), "r"(x), "r"(y) : "memory");
 }
 
 // Epilogue of one accumulator buffer for the 32 channels (TMEM lanes) of this warp.
 //   lane_addr  TMEM address of the warp's lane quarter in the buffer
-//   out4       output address of (pixel m0, this lane's 4-channel group)
-//   ch4_ok     the 4-channel group lies inside the valid channels
+//   out8       output address of (pixel m0, this lane's group of eight channels)
+//   ch8_ok     that group lies inside the valid channels
 //   ncols      pixel columns of the accumulator buffer that the tile fills (128, or 64 for half tiles)
 //   FORM       of the requantisation: 0 requant_one, 1 requant_fast, 2 requant_fast with every rshift >= 1, 3 float_requant4
 template <int ACT, int FORM, bool FROM_WS = false, class Consts = ChanConst>
-__device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4,
-                                                       bool ch4_ok, int m0, int half, int halves, int lane,
-                                                       const Consts &cc, const TransposeSel &ts, int ncols,
+__device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out8,
+                                                       bool ch8_ok, int m0, int half, int halves, int lane,
+                                                       const Consts &cc, const StageLane &st, int ncols,
                                                        int32_t *ws_lane = nullptr) {
   constexpr int QACT = ACT == 3 ? 0 : ACT; // the fused add works on the plain (no activation) int8 result
   // four pixels of this lane's channel, packed
@@ -487,23 +519,23 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
       return FORM != 0 && ACT == 1 ? relu_bytes(w) : w; // the multiply-high form leaves the ReLU clamp to the packed bytes
     }
   };
-  const int pj = lane & 3;
   // (Software-pipelining these loads in 16-column pieces made the epilogue alone 14% faster and the whole
   // kernel 4% slower, so the two loads of a chunk are simply issued together.)
   for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
     if (m0 + colg >= p.M_total) break;
-    const bool whole = m0 + colg + 32 <= p.M_total; // whole chunk in range: one guard for the eight stores
-    int8_t *o = out4 + (size_t)(colg + pj) * p.ldc;
-    uint32_t y[8];
+    const bool whole = m0 + colg + 32 <= p.M_total; // whole chunk in range: one guard for the stores
+    const int first = m0 + colg + st.px;            // this lane's first pixel
+    int8_t *o = out8 + (size_t)(colg + st.px) * p.ldc;
+    uint2 y[4];
     if (ACT == 3) {
       // the residual words of the fused eltwise add sit where the results go (same geometry): fetched first, so
       // that their latency passes under the accumulator loads and the requantisation
       const int8_t *rp = p.res + (size_t)(o - p.out);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        y[k] = 0u;
-        if (ch4_ok && (whole || m0 + colg + 4 * k + pj < p.M_total))
-          y[k] = __ldg(reinterpret_cast<const uint32_t *>(rp + (size_t)(4 * k) * p.ldc));
+      for (int i = 0; i < 4; ++i) {
+        y[i] = make_uint2(0u, 0u);
+        if (ch8_ok && (whole || first + stage_step8(i) < p.M_total))
+          y[i] = __ldg(reinterpret_cast<const uint2 *>(rp + (size_t)stage_step8(i) * p.ldc));
       }
     }
     uint32_t acc0[16], acc1[16];
@@ -523,54 +555,37 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
       ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
       ptx::tcgen05_wait_ld();
     }
-    uint32_t w[8];
+    uint32_t w[8], u[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       w[k] = rq4(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3]);
       w[4 + k] = rq4(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3]);
     }
+    transpose_i8(w, u, st);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) w[k] = transpose4x4(w[k], ts);
-    if (ACT == 3) {
-      // fused eltwise add: both tensors are written
-      int8_t *sp = p.out2 + (size_t)(o - p.out);
-      const uint32_t mm = (uint32_t)(uint8_t)p.add_ms | ((uint32_t)(uint8_t)p.add_mr << 8);
-      const int rnd = p.add_r > 0 ? (1 << (p.add_r - 1)) : 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (ch4_ok && (whole || m0 + colg + 4 * k + pj < p.M_total)) {
-          *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
-          *reinterpret_cast<uint32_t *>(sp + (size_t)(4 * k) * p.ldc) = add4_packed(w[k], y[k], mm, rnd, p.add_r, p.add_relu != 0);
-        }
-    } else if (ACT == 2) {
-      // fused leaky ReLU: the activation works on the packed, saturated values after the transpose (four
-      // channels of one pixel per word); the plain result goes to `out` when the graph keeps that tensor
-      uint32_t l[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        l[k] = pack4_sat(leaky_of(sext_byte<0>(w[k]), p), leaky_of(sext_byte<1>(w[k]), p), leaky_of(sext_byte<2>(w[k]), p),
-                         leaky_of(sext_byte<3>(w[k]), p));
-      int8_t *o2 = (p.out2 ? p.out2 + (out4 - p.out) : out4) + (size_t)(colg + pj) * p.ldc;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (ch4_ok && (whole || m0 + colg + 4 * k + pj < p.M_total)) {
-          if (p.out2) *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
-          *reinterpret_cast<uint32_t *>(o2 + (size_t)(4 * k) * p.ldc) = l[k];
-        }
-    } else if (whole) {
-      if (ch4_ok) {
-        // row addresses by one wide multiply-add each (the multiply-add pipe has room, the integer ALU has not)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          unsigned long long addr;
-          asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(addr) : "r"((uint32_t)(4 * k)), "r"((uint32_t)p.ldc), "l"((unsigned long long)o));
-          asm volatile("st.global.b32 [%0], %1;" ::"l"(addr), "r"(w[k]) : "memory");
-        }
+    for (int i = 0; i < 4; ++i) {
+      if (!ch8_ok || (!whole && first + stage_step8(i) >= p.M_total)) continue;
+      const unsigned long long at = px_addr(o, stage_step8(i), p.ldc);
+      const uint32_t a = u[2 * i], b = u[2 * i + 1];
+      if (ACT == 3) {
+        // fused eltwise add: both tensors are written
+        const uint32_t mm = (uint32_t)(uint8_t)p.add_ms | ((uint32_t)(uint8_t)p.add_mr << 8);
+        const int rnd = p.add_r > 0 ? (1 << (p.add_r - 1)) : 0;
+        stg64(at, a, b);
+        stg64(at + (unsigned long long)(p.out2 - p.out), add4_packed(a, y[i].x, mm, rnd, p.add_r, p.add_relu != 0),
+              add4_packed(b, y[i].y, mm, rnd, p.add_r, p.add_relu != 0));
+      } else if (ACT == 2) {
+        // fused leaky ReLU: the activation works on the packed, saturated values (eight channels of one pixel); the plain
+        // result goes to `out` when the graph keeps that tensor
+        auto leaky = [&](uint32_t v) {
+          return pack4_sat(leaky_of(sext_byte<0>(v), p), leaky_of(sext_byte<1>(v), p), leaky_of(sext_byte<2>(v), p),
+                           leaky_of(sext_byte<3>(v), p));
+        };
+        if (p.out2) stg64(at, a, b);
+        stg64(p.out2 ? at + (unsigned long long)(p.out2 - p.out) : at, leaky(a), leaky(b));
+      } else {
+        stg64(at, a, b);
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (ch4_ok && m0 + colg + 4 * k + pj < p.M_total) *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
     }
   }
 }
@@ -578,106 +593,112 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
 // The same with the fused eltwise add and the floating-point requantisation, for the two 32-pixel chunks of a warp. The
 // residual words come from memory: those of the first chunk were fetched during the tile before (`y`), those of the second
 // are fetched while the first is worked on, and then those of the next tile's first chunk, whose residual begins at `next`
-// (pixel next_m0, this lane's 4-channel group; null: none).
+// (pixel next_m0, this lane's group of eight channels; null: none).
 // Fetched where they are needed, they cost a memory latency per chunk (batch 256 with every add fused: 190 us more than
 // without; prefetched, 30 to 100).
-// (Rows 4 k of a chunk by one wide multiply-add each; one guard for a chunk that lies inside.)
-__device__ __forceinline__ unsigned long long row_addr(const void *base, int k, int ldc) {
-  unsigned long long a;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"((uint32_t)(4 * k)), "r"((uint32_t)ldc), "l"((unsigned long long)base));
-  return a;
-}
-// `first`: the chunk's first pixel; pj: this lane's of every four
-__device__ __forceinline__ void fetch_residual(uint32_t (&y)[8], const int8_t *res, int first, int pj, const ConvGemmParams &p) {
+// `res`: this lane's first pixel of the chunk, whose number is `first`
+__device__ __forceinline__ void fetch_residual(uint2 (&y)[4], const int8_t *res, int first, const ConvGemmParams &p) {
   if (!res) return;
-  const int8_t *at = res + (size_t)pj * p.ldc;
-  if (first + 32 <= p.M_total) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(y[k]) : "l"(row_addr(at, k, p.ldc)));
-  } else {
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (first + 4 * k + pj < p.M_total) y[k] = __ldg(reinterpret_cast<const uint32_t *>(at + (size_t)(4 * k) * p.ldc));
-  }
+  for (int i = 0; i < 4; ++i)
+    if (first + stage_step8(i) < p.M_total)
+      asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(y[i].x), "=r"(y[i].y) : "l"(px_addr(res, stage_step8(i), p.ldc)));
 }
-__device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out4, bool ch4_ok, int m0, int half,
-                                                int lane, const FloatRequant &q, const TransposeSel &ts, int ncols, uint32_t (&y)[8],
+__device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out8, bool ch8_ok, int m0, int half,
+                                                const FloatRequant &q, const StageLane &st, int ncols, uint2 (&y)[4],
                                                 const int8_t *next, int next_m0) {
-  const int pj = lane & 3, col0 = half * 32, col1 = col0 + 64;
+  const int col0 = half * 32, col1 = col0 + 64;
   const uint32_t mm = (uint32_t)(uint8_t)p.add_ms | ((uint32_t)(uint8_t)p.add_mr << 8);
   const int rnd = p.add_r > 0 ? (1 << (p.add_r - 1)) : 0, r = p.add_r;
   const bool relu = p.add_relu != 0;
-  auto chunk = [&](int colg, const uint32_t (&res)[8]) {
+  auto chunk = [&](int colg, const uint2 (&res)[4]) {
     uint32_t acc0[16], acc1[16];
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
     ptx::tcgen05_wait_ld();
-    uint32_t w[8];
+    uint32_t w[8], u[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q);
       w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q);
     }
+    transpose_i8(w, u, st);
+    const int8_t *o = out8 + (size_t)(colg + st.px) * p.ldc;
+    const unsigned long long to_sum = (unsigned long long)(p.out2 - p.out);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) w[k] = transpose4x4(w[k], ts);
-    if (!ch4_ok) return;
-    int8_t *o = out4 + (size_t)(colg + pj) * p.ldc, *sp = p.out2 + (size_t)(o - p.out);
-    if (m0 + colg + 32 <= p.M_total) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) asm volatile("st.global.b32 [%0], %1;" ::"l"(row_addr(o, k, p.ldc)), "r"(w[k]) : "memory");
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t z = add4_packed(w[k], res[k], mm, rnd, r, relu);
-        asm volatile("st.global.b32 [%0], %1;" ::"l"(row_addr(sp, k, p.ldc)), "r"(z) : "memory");
+    for (int i = 0; i < 4; ++i)
+      if (ch8_ok && m0 + colg + st.px + stage_step8(i) < p.M_total) {
+        const unsigned long long at = px_addr(o, stage_step8(i), p.ldc);
+        stg64(at, u[2 * i], u[2 * i + 1]);
+        stg64(at + to_sum, add4_packed(u[2 * i], res[i].x, mm, rnd, r, relu), add4_packed(u[2 * i + 1], res[i].y, mm, rnd, r, relu));
       }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (m0 + colg + 4 * k + pj < p.M_total) {
-          *reinterpret_cast<uint32_t *>(o + (size_t)(4 * k) * p.ldc) = w[k];
-          *reinterpret_cast<uint32_t *>(sp + (size_t)(4 * k) * p.ldc) = add4_packed(w[k], res[k], mm, rnd, r, relu);
-        }
-    }
   };
   const bool two = col1 < ncols && m0 + col1 < p.M_total;
-  uint32_t y1[8];
-  if (two) fetch_residual(y1, ch4_ok ? p.res + (out4 - p.out) + (size_t)col1 * p.ldc : nullptr, m0 + col1, pj, p);
+  uint2 y1[4];
+  if (two) fetch_residual(y1, ch8_ok ? p.res + (out8 - p.out) + (size_t)(col1 + st.px) * p.ldc : nullptr, m0 + col1 + st.px, p);
   if (col0 < ncols && m0 + col0 < p.M_total) chunk(col0, y);
-  fetch_residual(y, next ? next + (size_t)col0 * p.ldc : nullptr, next_m0 + col0, pj, p);
+  fetch_residual(y, next ? next + (size_t)(col0 + st.px) * p.ldc : nullptr, next_m0 + col0 + st.px, p);
   if (two) chunk(col1, y1);
 }
 
 // Epilogue of a BF16 convolution (core/conv.cpp:90-98: fp32 result + fp32 bias, ReLU, BF16 rounding). The
-// accumulators are fp32; a thread rounds two neighbouring pixels of its channel into one word, exchanges
-// words with the lane of the neighbouring channel and stores two channels of one pixel (a warp writes
-// 64 contiguous bytes per pixel). `out_pair` addresses (pixel m0, the even channel of this lane's pair);
-// `pitch` is the output row pitch in bytes.
+// accumulators are fp32; a thread rounds two neighbouring pixels of its channel into one word, and the words are transposed
+// through shared memory (see StageLane): a lane stores eight channels (16 bytes) of one pixel. `out8` addresses (pixel m0,
+// this lane's group of eight channels); `ldc` is in bytes. The rounding is the hardware's; a multiply-add by zero carries
+// every result that it made infinite or NaN into `odd`, and a chunk that holds one is rounded again by the bit rule.
 template <bool RELU>
-__device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out_pair,
-                                                       bool ch_ok, int m0, int half, int halves, int lane, float bias,
+__device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out8,
+                                                       bool ch_ok, int m0, int half, int halves, float bias, const StageLane &st,
                                                        int ncols = 128) {
-  const int odd = lane & 1;
-  const size_t pitch = (size_t)p.ldc;
+  const unsigned long long bias2 = pack_f32x2(bias, bias);
   for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
     if (m0 + colg >= p.M_total) break;
     uint32_t acc0[16], acc1[16];
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
     ptx::tcgen05_wait_ld();
+    uint32_t w[16], odd = 0u;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const uint32_t b0 = j < 8 ? acc0[2 * j] : acc1[2 * j - 16], b1 = j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15];
-      float v0 = __fadd_rn(bits_f32(b0), bias), v1 = __fadd_rn(bits_f32(b1), bias);
-      if (RELU) {
-        v0 = v0 > 0.0f ? v0 : 0.0f;
-        v1 = v1 > 0.0f ? v1 : 0.0f;
+      unsigned long long v = pack_b32x2(j < 8 ? acc0[2 * j] : acc1[2 * j - 16], j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15]);
+      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(bias2));
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+      if (RELU) asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(w[j]) : "f"(hi), "f"(lo));
+      else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[j]) : "f"(hi), "f"(lo));
+      asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(odd) : "r"(w[j]), "r"(0u));
+    }
+    if (odd & 0x7fff7fffu) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float lo = __fadd_rn(bits_f32(j < 8 ? acc0[2 * j] : acc1[2 * j - 16]), bias);
+        float hi = __fadd_rn(bits_f32(j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15]), bias);
+        if (RELU) {
+          lo = lo > 0.0f ? lo : 0.0f;
+          hi = hi > 0.0f ? hi : 0.0f;
+        }
+        w[j] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
       }
-      const uint32_t w = bf16x2_round_bits(v0, v1); // low half: pixel 2j, high half: pixel 2j + 1
-      const uint32_t o = __shfl_xor_sync(0xffffffffu, w, 1);
-      // even lane: channels (c, c+1) of pixel 2j; odd lane: channels (c-1, c) of pixel 2j + 1
-      const uint32_t y = odd ? __byte_perm(o, w, 0x7632) : __byte_perm(w, o, 0x5410);
-      const int pix = colg + 2 * j + odd;
-      if (ch_ok && m0 + pix < p.M_total) *reinterpret_cast<uint32_t *>(out_pair + (size_t)pix * pitch) = y;
+    }
+    const bool whole = m0 + colg + 32 <= p.M_total;
+#pragma unroll
+    for (int part = 0; part < 2; ++part) { // 16 pixels each: 1 KB
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(st.put + 512u * k),
+                     "r"(w[8 * part + 4 * k]), "r"(w[8 * part + 4 * k + 1]), "r"(w[8 * part + 4 * k + 2]), "r"(w[8 * part + 4 * k + 3])
+                     : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int px = colg + 16 * part + 8 * k + st.px;
+        uint32_t v[4];
+        lds128(st.get + 512u * k, v);
+        if (ch_ok && (whole || m0 + px < p.M_total))
+          asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(px_addr(out8, px, p.ldc)), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                       "r"(v[3]) : "memory");
+      }
     }
   }
 }
@@ -1022,7 +1043,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;     // TMEM lanes (= channels of the tile) this warp may read
     const int half = (warp - 2) >> 2; // which alternate 32-pixel column groups it takes
-    const TransposeSel ts = make_transpose_sel(lane);
+    const StageLane st = make_stage_lane<BF16 ? 2 : 4>(base + 1024u + (uint32_t)((warp - 2) * kStageBytes), lane);
     ChanConst cc = {};
     FloatRequant fq = {};
     float bias_f = 0.0f;
@@ -1030,15 +1051,15 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     int t = 0;
     bool ok = true;
     int tm = walk_m0, tn = walk_n0;
-    // fused add: the residual of a tile (tm, tn), counted from this lane's 4-channel group; null where it has none
-    uint32_t res_words[8];
+    // fused add: the residual of a tile (tm, tn), counted from this lane's group of eight channels; null where it has none
+    uint2 res_words[4];
     auto residual_at = [&](int item, int m, int n) -> const int8_t * {
-      const int ch = n * p.BN + quarter * 32 + (lane >> 2) * 4;
+      const int ch = n * p.BN + quarter * 32 + (lane & 3) * 8;
       return item < total_items && ch < p.n_valid ? p.res + (size_t)m * m_tile * p.ldc + p.c_off + ch : nullptr;
     };
     if constexpr (ACTSEL == 103) {
       const int8_t *r = residual_at(blockIdx.x, tm, tn);
-      fetch_residual(res_words, r ? r + (size_t)(half * 32) * p.ldc : nullptr, tm * m_tile + half * 32, lane & 3, p);
+      fetch_residual(res_words, r ? r + (size_t)(half * 32 + st.px) * p.ldc : nullptr, tm * m_tile + half * 32 + st.px, p);
     }
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++t) {
       int tile = item;
@@ -1061,14 +1082,14 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const int buf = t & 1;
       if (n0 != staged_n0) {
         if (BF16 || TF32) {
-          const int ch = n0 + ch_base + lane;
+          const int ch = n0 + ch_base + lane_channel(lane);
           bias_f = ch < p.n_valid ? __int_as_float(p.bias[ch]) : 0.0f; // fp32 bias bits in the int32 array
         } else if (FQ) {
-          const int ch = n0 + ch_base + lane;
+          const int ch = n0 + ch_base + lane_channel(lane);
           const uint4 c = ch < p.n_valid ? __ldg(reinterpret_cast<const uint4 *>(p.fq) + ch) : make_uint4(0u, 0u, 0u, 0u);
           fq = FloatRequant{c.x, __uint_as_float(c.y), __uint_as_float(c.z), __uint_as_float(c.w)};
         } else {
-          cc = load_chan_const(p, n0 + ch_base + lane);
+          cc = load_chan_const(p, n0 + ch_base + lane_channel(lane));
         }
         staged_n0 = n0;
       }
@@ -1082,7 +1103,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const bool split_item = SPLIT && split_k > 1;
       if (!ok && !split_item) break; // (a split item still passes its two barriers, see below)
       ptx::tcgen05_fence_after();
-      const int ch4 = n0 + ch_base + (lane >> 2) * 4;
+      const int ch8 = n0 + ch_base + (lane & 3) * 8;
       int32_t *ws_lane = nullptr; // split K: this lane's channel column of the tile's partial-sum block
       if (split_item) {
         ws_lane = p.ws + (size_t)tile * (128 * 128) + quarter * 32 + lane;
@@ -1136,35 +1157,34 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       if (n0 + ch_base < p.n_valid && m0 < p.M_total) { // warp-uniform: this lane quarter holds real outputs
         const uint32_t lane_addr = tmem_base + (uint32_t)buf * acc_stride + ((uint32_t)(quarter * 32) << 16);
         const size_t out_m0 = (size_t)m0 * p.ldc + (p.group > 1 ? (quarter * 32 * p.group >> 7) * p.ldc_px : 0); // bytes
-        int8_t *out4 = p.out + out_m0 + p.c_off + ch4;
-        const bool ch4_ok = ch4 < p.n_valid;
+        int8_t *out8 = p.out + out_m0 + p.c_off + ch8;
+        const bool ch8_ok = ch8 < p.n_valid;
         if (TF32) {
           // byte addressing: 4 bytes per channel
-          const int ch = n0 + ch_base + lane;
+          const int ch = n0 + ch_base + lane_channel(lane);
           uint8_t *out_ch = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch) * 4;
           if (p.act == 1) epilogue_channels_f32<true>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f, ncols);
           else epilogue_channels_f32<false>(p, lane_addr, out_ch, ch < p.n_valid, m0, half, kEpilogueWarps / 4, bias_f, ncols);
         } else if (BF16) {
-          // byte addressing: 2 bytes per channel, this lane's pair starts at its even channel
-          const int ch = n0 + ch_base + lane;
-          uint8_t *out_pair = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + (ch & ~1)) * 2;
-          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
-          else epilogue_channels_bf16<false>(p, lane_addr, out_pair, ch < p.n_valid, m0, half, kEpilogueWarps / 4, lane, bias_f, ncols);
+          // byte addressing: 2 bytes per channel
+          uint8_t *out16 = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch8) * 2;
+          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias_f, st, ncols);
+          else epilogue_channels_bf16<false>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias_f, st, ncols);
         } else if constexpr (ACTSEL == 103) {
-          epilogue_add_fq(p, lane_addr, out4, ch4_ok, m0, half, lane, fq, ts, ncols, res_words,
+          epilogue_add_fq(p, lane_addr, out8, ch8_ok, m0, half, fq, st, ncols, res_words,
                           residual_at(item + gridDim.x, tm, tn), tm * m_tile);
         } else if constexpr (FQ) {
-          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, fq, ts, ncols);
-        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
-        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
-        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols);
-        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
-        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out4, ch4_ok, m0, half, kEpilogueWarps / 4, lane, cc, ts, ncols, ws_lane);
+          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, fq, st, ncols);
+        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
+        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
+        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols);
+        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
+        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
       }
       if constexpr (ACTSEL == 103) {
         if (n0 + ch_base >= p.n_valid) { // no outputs here: the next tile's residual all the same
           const int8_t *r = residual_at(item + gridDim.x, tm, tn);
-          fetch_residual(res_words, r ? r + (size_t)(half * 32) * p.ldc : nullptr, tm * m_tile + half * 32, lane & 3, p);
+          fetch_residual(res_words, r ? r + (size_t)(half * 32 + st.px) * p.ldc : nullptr, tm * m_tile + half * 32 + st.px, p);
         }
       }
       if (SPLIT && ws_lane) continue; // split K: the accumulator buffer was handed back above

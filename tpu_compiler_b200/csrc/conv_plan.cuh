@@ -125,46 +125,49 @@ inline void pack_filter(const float *w, int channels, int taps, T *out, size_t p
       for (int c = 0; c < channels; ++c) out[t * pitch + c] = line[(size_t)c * taps + t];
 }
 
-// Pack OIHW fp32 weights (integer-valued) to int8 [oc_pad][taps][cin_pad] for the im2col
-// path, or [oc_pad][1][kp] with K order (r, s, c) for the patch path. For grouped
+// Rows of the packed weights: whole blocks of 32 channels, in the order of packed_row.
+inline size_t packed_rows(int oc_pad) { return (size_t)(oc_pad + 31) / 32 * 32; }
+
+// Pack OIHW fp32 weights (integer-valued) to int8 [rows][taps][cin_pad] for the im2col
+// path, or [rows][1][kp] with K order (r, s, c) for the patch path. For grouped
 // convolution the caller passes one group's slice.
 inline std::vector<int8_t> pack_conv_weights(const float *w, int oc, int icg, int kh, int kw,
                                              int oc_pad, int cin_pad, bool patch, int kp) {
   const int taps = kh * kw;
   const size_t row = patch ? kp : (size_t)taps * cin_pad, pitch = patch ? icg : cin_pad;
-  std::vector<int8_t> out(oc_pad * row, 0), line((size_t)icg * taps);
+  std::vector<int8_t> out(packed_rows(oc_pad) * row, 0), line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    pack_filter(w + (size_t)o * icg * taps, icg, taps, out.data() + o * row, pitch, line.data(), [](float v) { return (int8_t)(int)v; });
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, out.data() + packed_row(o) * row, pitch, line.data(), [](float v) { return (int8_t)(int)v; });
   return out;
 }
 
-// BF16 weights [oc_pad][tap][cin_pad] as 16-bit patterns (the values of a BF16 graph's filter are
+// BF16 weights [rows][tap][cin_pad] as 16-bit patterns (the values of a BF16 graph's filter are
 // BF16-representable floats: the upper 16 bits are the value), returned as bytes
 inline std::vector<int8_t> pack_conv_weights_bf16(const float *w, int oc, int icg, int kh, int kw, int oc_pad,
                                                   int cin_pad) {
   const int taps = kh * kw;
   const size_t row = (size_t)taps * cin_pad;
-  std::vector<int8_t> bytes(oc_pad * row * 2, 0);
+  std::vector<int8_t> bytes(packed_rows(oc_pad) * row * 2, 0);
   std::vector<uint16_t> line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    pack_filter(w + (size_t)o * icg * taps, icg, taps, reinterpret_cast<uint16_t *>(bytes.data()) + o * row, cin_pad, line.data(),
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, reinterpret_cast<uint16_t *>(bytes.data()) + packed_row(o) * row, cin_pad, line.data(),
                 [](float v) { return (uint16_t)(f32_bits(v) >> 16); });
   return bytes;
 }
 
-// fp32 weights for the TF32 x 3 convolution, K-major [oc_pad][tap][cin_pad] as bytes: part 0 = the upper 19 bits of
+// fp32 weights for the TF32 x 3 convolution, K-major [rows][tap][cin_pad] as bytes: part 0 = the upper 19 bits of
 // every word, part 1 = the exact remainder.
 inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int icg, int kh, int kw, int oc_pad, int cin_pad,
                                                   int part) {
   const int taps = kh * kw;
-  std::vector<float> out((size_t)oc_pad * taps * cin_pad, 0.0f);
+  std::vector<float> out(packed_rows(oc_pad) * taps * cin_pad, 0.0f);
   for (int o = 0; o < oc; ++o)
     for (int c = 0; c < icg; ++c)
       for (int r = 0; r < kh; ++r)
         for (int s = 0; s < kw; ++s) {
           const float v = w[(((size_t)o * icg + c) * kh + r) * kw + s];
           const float hi = bits_f32(f32_bits(v) & 0xffffe000u);
-          out[((size_t)o * taps + (r * kw + s)) * cin_pad + c] = part == 0 ? hi : v - hi;
+          out[((size_t)packed_row(o) * taps + (r * kw + s)) * cin_pad + c] = part == 0 ? hi : v - hi;
         }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
@@ -174,12 +177,12 @@ inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int ic
 // the same for the patch matrix of an fp32 image stem: four channel slots per tap, k = tap * 4 + c
 inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeom &g, int oc_pad, int part) {
   const int kp = g.kh * g.kw * 4;
-  std::vector<float> out((size_t)oc_pad * kp, 0.0f);
+  std::vector<float> out(packed_rows(oc_pad) * kp, 0.0f);
   for (int o = 0; o < g.oc; ++o)
     for (int c = 0; c < g.ic; ++c)
       for (int t = 0; t < g.kh * g.kw; ++t) {
         const float v = w[((size_t)o * g.ic + c) * g.kh * g.kw + t], hi = bits_f32(f32_bits(v) & 0xffffe000u);
-        out[(size_t)o * kp + t * 4 + c] = part == 0 ? hi : v - hi;
+        out[(size_t)packed_row(o) * kp + t * 4 + c] = part == 0 ? hi : v - hi;
       }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
@@ -188,7 +191,7 @@ inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeo
 
 inline void encode_weight_map(CUtensorMap *tm, const int8_t *d_w, int oc_pad, int taps, int k_inner,
                               int BK, int BN) {
-  cuuint64_t dims[3] = {(cuuint64_t)k_inner, (cuuint64_t)taps, (cuuint64_t)oc_pad};
+  cuuint64_t dims[3] = {(cuuint64_t)k_inner, (cuuint64_t)taps, (cuuint64_t)packed_rows(oc_pad)};
   cuuint64_t strides[2] = {(cuuint64_t)k_inner, (cuuint64_t)k_inner * taps};
   cuuint32_t box[3] = {(cuuint32_t)BK, 1, (cuuint32_t)BN};
   cuuint32_t es[3] = {1, 1, 1};
@@ -287,7 +290,7 @@ inline std::vector<int8_t> pack_window_weights(const float *w, const ConvGeom &g
         for (int r = 0; r < g.kh; ++r)
           for (int s = 0; s < g.kw; ++s) {
             const float v = w[(((size_t)o * g.ic + c) * g.kh + r) * g.kw + s];
-            int8_t *at = out.data() + ((size_t)(j * slot + o) * g.kh + r) * BK + (size_t)(j * g.sw + s * g.dw) * wp.P + c * es;
+            int8_t *at = out.data() + ((size_t)packed_row(j * slot + o) * g.kh + r) * BK + (size_t)(j * g.sw + s * g.dw) * wp.P + c * es;
             if (bf16) {
               const uint16_t h = (uint16_t)(f32_bits(v) >> 16);
               std::memcpy(at, &h, 2);

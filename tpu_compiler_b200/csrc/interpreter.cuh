@@ -769,7 +769,7 @@ public:
     p.ldc_px = p.ldc;
     p.ldc *= wp.G;
     finish_plan(pl, g.n * g.oh * p.OW, g.kh, wp.win, out_->cp, I.sm_count);
-    const int w_rows = wp.G > 1 ? 128 : out_->cp;
+    const int w_rows = wp.G > 1 ? 128 : (int)packed_rows(out_->cp);
     encode_weight_map(&pl.tmB, I.upload(pack_window_weights(filt.data(), g, wp, w_rows, p.BK, kind == 1)), w_rows, g.kh, p.BK, p.BK,
                       p.dual ? 192 : 128);
     encode_window_map(&pl.tmA, rows, g, wp, p.BK, p.m_tile);
@@ -939,11 +939,11 @@ public:
       conv_kernel_setup_once();
       const int n_pad = out->cp;
       kdev_ = hw * in->cp;
-      std::vector<uint16_t> w((size_t)n_pad * kdev_, 0);
+      std::vector<uint16_t> w(packed_rows(n_pad) * kdev_, 0);
       for (int j = 0; j < n_; ++j)
         for (int c = 0; c < in->c; ++c)
           for (int p = 0; p < hw; ++p)
-            w[(size_t)j * kdev_ + (size_t)p * in->cp + c] = (uint16_t)(f32_bits(filt.data[(size_t)j * k_ + (size_t)c * hw + p]) >> 16);
+            w[(size_t)packed_row(j) * kdev_ + (size_t)p * in->cp + c] = (uint16_t)(f32_bits(filt.data[(size_t)j * k_ + (size_t)c * hw + p]) >> 16);
       std::vector<int8_t> wb(w.size() * 2);
       std::memcpy(wb.data(), w.data(), wb.size());
       const int8_t *d_w = I.upload(wb);
@@ -990,11 +990,11 @@ public:
     conv_kernel_setup_once();
     const int n_pad = out->cp;
     kdev_ = hw * in->cp;
-    std::vector<int8_t> w((size_t)n_pad * kdev_, 0);
+    std::vector<int8_t> w(packed_rows(n_pad) * kdev_, 0);
     for (int j = 0; j < n_; ++j)
       for (int c = 0; c < in->c; ++c)
         for (int p = 0; p < hw; ++p)
-          w[(size_t)j * kdev_ + (size_t)p * in->cp + c] = (int8_t)(int)filt.data[(size_t)j * k_ + (size_t)c * hw + p];
+          w[(size_t)packed_row(j) * kdev_ + (size_t)p * in->cp + c] = (int8_t)(int)filt.data[(size_t)j * k_ + (size_t)c * hw + p];
     const int8_t *d_w = I.upload(w);
     // one (rshift, multiplier) pair per batch slice (fullyconnected.cpp:78-88) -> broadcast per column
     std::vector<float> rs(n_, I.weight(op.in[5]).data.at(0)), mu(n_, I.weight(op.in[6]).data.at(0));
