@@ -262,26 +262,50 @@ __device__ __forceinline__ unsigned long long pack_b32x2(uint32_t lo, uint32_t h
 }
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) { return pack_b32x2(__float_as_uint(lo), __float_as_uint(hi)); }
 // Two values of one channel: the packed multiply-adds round each half as the single ones do and take one issue slot for two.
-template <bool RELU> __device__ __forceinline__ void float_requant2(uint32_t a0, uint32_t a1, const FloatRequant &q, int &v0, int &v1) {
+// The constants are held as pairs whose making the compiler may not repeat (it did, before some uses).
+__device__ __forceinline__ unsigned long long hold_pair(float v) {
+  unsigned long long d;
+  asm volatile("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+  return d;
+}
+struct FloatRequantShared { // what the channels share without ReLU
+  unsigned long long k, h;
+  __device__ __forceinline__ void set() {
+    k = hold_pair(-(float)kFqC * kFqScale);
+    h = hold_pair(__uint_as_float(128u));
+  }
+};
+template <bool RELU> struct FloatRequantPairs {
+  uint32_t sb;
+  unsigned long long m, d, c, e; // e: ReLU the last addend, else unused
+  __device__ __forceinline__ void set(const FloatRequant &q) {
+    sb = q.sb;
+    m = hold_pair(q.m);
+    d = hold_pair(q.d);
+    c = hold_pair(q.c);
+    if (RELU) e = hold_pair(q.c * -6.617444900424222e-24f); // as above
+  }
+};
+template <bool RELU>
+__device__ __forceinline__ void float_requant2(uint32_t a0, uint32_t a1, const FloatRequantPairs<RELU> &q, const FloatRequantShared &s, int &v0,
+                                               int &v1) {
   unsigned long long f = pack_b32x2(a0 + q.sb, a1 + q.sb);
-  asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(pack_f32x2(q.m, q.m)), "l"(pack_f32x2(q.d, q.d)));
-  const unsigned long long c = pack_f32x2(q.c, q.c);
+  asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(q.m), "l"(q.d));
   if (RELU) {
-    const float e = q.c * -6.617444900424222e-24f; // as above
-    asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(c), "l"(pack_f32x2(e, e)));
+    asm("fma.rm.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(q.c), "l"(q.e));
   } else {
-    const float k = -(float)kFqC * kFqScale;
-    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(pack_f32x2(k, k)));
-    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(c), "l"(pack_b32x2(128u, 128u)));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(s.k));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(q.c), "l"(s.h));
   }
   asm("mov.b64 {%0, %1}, %2;" : "=r"(v0), "=r"(v1) : "l"(f));
 }
 // four values of one channel, packed
 template <bool RELU>
-__device__ __forceinline__ uint32_t float_requant4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const FloatRequant &q) {
+__device__ __forceinline__ uint32_t float_requant4(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, const FloatRequantPairs<RELU> &q,
+                                                   const FloatRequantShared &s) {
   int v0, v1, v2, v3;
-  float_requant2<RELU>(a0, a1, q, v0, v1);
-  float_requant2<RELU>(a2, a3, q, v2, v3);
+  float_requant2<RELU>(a0, a1, q, s, v0, v1);
+  float_requant2<RELU>(a2, a3, q, s, v2, v3);
   return float_requant_pack<RELU>(v0, v1, v2, v3);
 }
 #endif

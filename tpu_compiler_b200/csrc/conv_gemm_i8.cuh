@@ -90,6 +90,13 @@ namespace ptx {
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
+// True in one lane of a converged warp. The compiler knows that a branch on it holds one thread: copies and MMAs, whose
+// operands are registers of the whole warp, are then issued once, not in a loop over the lanes that might be active.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
@@ -134,6 +141,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     if (*abort_flag) return false;
   }
   return false;
+}
+// The same by a whole warp, whose lanes get one answer: the loops of the copying and issuing warps are then uniform, and what
+// they compute stays in the registers that the copies and MMAs take (by one lane of a branch, every operand was moved there
+// for every instruction).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int rounds) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, rounds));
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, uint32_t bar, int x,
                                             int y) {
@@ -503,13 +517,13 @@ __device__ __forceinline__ void stg64(unsigned long long at, uint32_t x, uint32_
 template <int ACT, int FORM, bool FROM_WS = false, class Consts = ChanConst>
 __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out8,
                                                        bool ch8_ok, int m0, int half, int halves, int lane,
-                                                       const Consts &cc, const StageLane &st, int ncols,
+                                                       const Consts &cc, const FloatRequantShared &fs, const StageLane &st, int ncols,
                                                        int32_t *ws_lane = nullptr) {
   constexpr int QACT = ACT == 3 ? 0 : ACT; // the fused add works on the plain (no activation) int8 result
   // four pixels of this lane's channel, packed
   auto rq4 = [&](uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) -> uint32_t {
     if constexpr (FORM == 3) {
-      return float_requant4<QACT == 1>(a0, a1, a2, a3, cc);
+      return float_requant4<QACT == 1>(a0, a1, a2, a3, cc, fs);
     } else {
       auto rq = [&](uint32_t a) {
         if constexpr (FORM == 0) return requant_one<QACT>((int32_t)a, cc, p);
@@ -521,21 +535,19 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
   };
   // (Software-pipelining these loads in 16-column pieces made the epilogue alone 14% faster and the whole
   // kernel 4% slower, so the two loads of a chunk are simply issued together.)
-  for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
-    if (m0 + colg >= p.M_total) break;
-    const bool whole = m0 + colg + 32 <= p.M_total; // whole chunk in range: one guard for the stores
-    const int first = m0 + colg + st.px;            // this lane's first pixel
-    int8_t *o = out8 + (size_t)(colg + st.px) * p.ldc;
+  const int cols = min(ncols, p.M_total - m0);
+  int left = ch8_ok ? p.M_total - m0 - half * 32 - st.px : 0; // pixels in range from this lane's first one of the chunk
+  unsigned long long o = px_addr(out8, half * 32 + st.px, p.ldc);
+  for (int colg = half * 32; colg < cols; colg += 32 * halves, left -= 32 * halves, o = px_addr((const void *)o, 32 * halves, p.ldc)) {
     uint2 y[4];
     if (ACT == 3) {
       // the residual words of the fused eltwise add sit where the results go (same geometry): fetched first, so
       // that their latency passes under the accumulator loads and the requantisation
-      const int8_t *rp = p.res + (size_t)(o - p.out);
+      const int8_t *rp = p.res + (o - (unsigned long long)p.out);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         y[i] = make_uint2(0u, 0u);
-        if (ch8_ok && (whole || first + stage_step8(i) < p.M_total))
-          y[i] = __ldg(reinterpret_cast<const uint2 *>(rp + (size_t)stage_step8(i) * p.ldc));
+        if (stage_step8(i) < left) y[i] = __ldg(reinterpret_cast<const uint2 *>(rp + (size_t)stage_step8(i) * p.ldc));
       }
     }
     uint32_t acc0[16], acc1[16];
@@ -564,8 +576,8 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
     transpose_i8(w, u, st);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      if (!ch8_ok || (!whole && first + stage_step8(i) >= p.M_total)) continue;
-      const unsigned long long at = px_addr(o, stage_step8(i), p.ldc);
+      if (stage_step8(i) >= left) continue;
+      const unsigned long long at = px_addr((const void *)o, stage_step8(i), p.ldc);
       const uint32_t a = u[2 * i], b = u[2 * i + 1];
       if (ACT == 3) {
         // fused eltwise add: both tensors are written
@@ -605,7 +617,7 @@ __device__ __forceinline__ void fetch_residual(uint2 (&y)[4], const int8_t *res,
       asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(y[i].x), "=r"(y[i].y) : "l"(px_addr(res, stage_step8(i), p.ldc)));
 }
 __device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out8, bool ch8_ok, int m0, int half,
-                                                const FloatRequant &q, const StageLane &st, int ncols, uint2 (&y)[4],
+                                                const FloatRequantPairs<false> &q, const FloatRequantShared &fs, const StageLane &st, int ncols, uint2 (&y)[4],
                                                 const int8_t *next, int next_m0) {
   const int col0 = half * 32, col1 = col0 + 64;
   const uint32_t mm = (uint32_t)(uint8_t)p.add_ms | ((uint32_t)(uint8_t)p.add_mr << 8);
@@ -619,8 +631,8 @@ __device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_
     uint32_t w[8], u[8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q);
-      w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q);
+      w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q, fs);
+      w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q, fs);
     }
     transpose_i8(w, u, st);
     const int8_t *o = out8 + (size_t)(colg + st.px) * p.ldc;
@@ -641,18 +653,37 @@ __device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_
   if (two) chunk(col1, y1);
 }
 
+// Two BF16 roundings (and ReLU) by the hardware; a multiply-add by zero carries every result that it made infinite or NaN into
+// `odd`, and a caller that finds one there rounds again by the reference's bit rule (bf16_pack_rule).
+template <bool RELU> __device__ __forceinline__ uint32_t bf16_pack_relu(unsigned long long v, uint32_t &odd) {
+  float lo, hi;
+  uint32_t w;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  if (RELU) asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+  else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+  asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(odd) : "r"(w), "r"(0u));
+  return w;
+}
+template <bool RELU> __device__ __forceinline__ uint32_t bf16_pack_rule(uint32_t a0, uint32_t a1, float bias) {
+  float lo = __fadd_rn(bits_f32(a0), bias), hi = __fadd_rn(bits_f32(a1), bias);
+  if (RELU) {
+    lo = lo > 0.0f ? lo : 0.0f;
+    hi = hi > 0.0f ? hi : 0.0f;
+  }
+  return (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+}
 // Epilogue of a BF16 convolution (core/conv.cpp:90-98: fp32 result + fp32 bias, ReLU, BF16 rounding). The
 // accumulators are fp32; a thread rounds two neighbouring pixels of its channel into one word, and the words are transposed
 // through shared memory (see StageLane): a lane stores eight channels (16 bytes) of one pixel. `out8` addresses (pixel m0,
-// this lane's group of eight channels); `ldc` is in bytes. The rounding is the hardware's; a multiply-add by zero carries
-// every result that it made infinite or NaN into `odd`, and a chunk that holds one is rounded again by the bit rule.
+// this lane's group of eight channels); `ldc` is in bytes.
 template <bool RELU>
 __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out8,
-                                                       bool ch_ok, int m0, int half, int halves, float bias, const StageLane &st,
+                                                       bool ch_ok, int m0, int half, int halves, unsigned long long bias2, const StageLane &st,
                                                        int ncols = 128) {
-  const unsigned long long bias2 = pack_f32x2(bias, bias);
-  for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
-    if (m0 + colg >= p.M_total) break;
+  const int cols = min(ncols, p.M_total - m0);
+  int left = ch_ok ? p.M_total - m0 - half * 32 - st.px : 0; // pixels in range from this lane's first one of the chunk
+  unsigned long long o = px_addr(out8, half * 32 + st.px, p.ldc);
+  for (int colg = half * 32; colg < cols; colg += 32 * halves, left -= 32 * halves, o = px_addr((const void *)o, 32 * halves, p.ldc)) {
     uint32_t acc0[16], acc1[16];
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
@@ -662,25 +693,13 @@ __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, 
     for (int j = 0; j < 16; ++j) {
       unsigned long long v = pack_b32x2(j < 8 ? acc0[2 * j] : acc1[2 * j - 16], j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15]);
       asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(bias2));
-      float lo, hi;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-      if (RELU) asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(w[j]) : "f"(hi), "f"(lo));
-      else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[j]) : "f"(hi), "f"(lo));
-      asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(odd) : "r"(w[j]), "r"(0u));
+      w[j] = bf16_pack_relu<RELU>(v, odd);
     }
     if (odd & 0x7fff7fffu) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        float lo = __fadd_rn(bits_f32(j < 8 ? acc0[2 * j] : acc1[2 * j - 16]), bias);
-        float hi = __fadd_rn(bits_f32(j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15]), bias);
-        if (RELU) {
-          lo = lo > 0.0f ? lo : 0.0f;
-          hi = hi > 0.0f ? hi : 0.0f;
-        }
-        w[j] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
-      }
+      for (int j = 0; j < 16; ++j)
+        w[j] = bf16_pack_rule<RELU>(j < 8 ? acc0[2 * j] : acc1[2 * j - 16], j < 8 ? acc0[2 * j + 1] : acc1[2 * j - 15], __uint_as_float((uint32_t)bias2));
     }
-    const bool whole = m0 + colg + 32 <= p.M_total;
 #pragma unroll
     for (int part = 0; part < 2; ++part) { // 16 pixels each: 1 KB
       __syncwarp();
@@ -692,12 +711,11 @@ __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, 
       __syncwarp();
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const int px = colg + 16 * part + 8 * k + st.px;
         uint32_t v[4];
         lds128(st.get + 512u * k, v);
-        if (ch_ok && (whole || m0 + px < p.M_total))
-          asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(px_addr(out8, px, p.ldc)), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-                       "r"(v[3]) : "memory");
+        if (16 * part + 8 * k < left)
+          asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(px_addr((const void *)o, 16 * part + 8 * k, p.ldc)), "r"(v[0]),
+                       "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
       }
     }
   }
@@ -709,10 +727,11 @@ __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, 
 template <bool RELU>
 __device__ __forceinline__ void epilogue_channels_f32(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out_ch, bool ch_ok,
                                                       int m0, int half, int halves, float bias, int ncols = 128) {
-  const size_t pitch = (size_t)p.ldc;
-  uint8_t *lo_ch = p.out2 ? reinterpret_cast<uint8_t *>(p.out2) + (out_ch - reinterpret_cast<uint8_t *>(p.out)) : nullptr;
-  for (int colg = half * 32; colg < ncols; colg += 32 * halves) {
-    if (m0 + colg >= p.M_total) break;
+  const int cols = min(ncols, p.M_total - m0);
+  int left = ch_ok ? p.M_total - m0 - half * 32 : 0; // pixels in range from the chunk's first one
+  unsigned long long o = px_addr(out_ch, half * 32, p.ldc);
+  const unsigned long long to_lo = (unsigned long long)(reinterpret_cast<uint8_t *>(p.out2) - reinterpret_cast<uint8_t *>(p.out));
+  for (int colg = half * 32; colg < cols; colg += 32 * halves, left -= 32 * halves, o = px_addr((const void *)o, 32 * halves, p.ldc)) {
     uint32_t acc0[16], acc1[16];
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
     ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
@@ -721,10 +740,12 @@ __device__ __forceinline__ void epilogue_channels_f32(const ConvGemmParams &p, u
     for (int j = 0; j < 32; ++j) {
       float v = __fadd_rn(bits_f32(j < 16 ? acc0[j & 15] : acc1[j & 15]), bias);
       if (RELU) v = v > 0.0f ? v : 0.0f;
-      if (ch_ok && m0 + colg + j < p.M_total) {
-        *reinterpret_cast<float *>(out_ch + (size_t)(colg + j) * pitch) = v;
+      if (j < left) {
+        const unsigned long long at = px_addr((const void *)o, j, p.ldc);
+        asm volatile("st.global.f32 [%0], %1;" ::"l"(at), "f"(v) : "memory");
         // the remainder operand of a TF32 x 3 convolution that reads this result, when one does
-        if (lo_ch) *reinterpret_cast<float *>(lo_ch + (size_t)(colg + j) * pitch) = __fsub_rn(v, __uint_as_float(__float_as_uint(v) & 0xffffe000u));
+        if (p.out2)
+          asm volatile("st.global.f32 [%0], %1;" ::"l"(at + to_lo), "f"(__fsub_rn(v, __uint_as_float(__float_as_uint(v) & 0xffffe000u))) : "memory");
       }
     }
   }
@@ -762,7 +783,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 172);
   volatile int *split_last = reinterpret_cast<volatile int *>(smem + 176); // split K: this CTA completes its tile
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int n_tiles = (p.n_valid + p.BN - 1) / p.BN;
   // Dual mode (<= 64 output channels): a tile covers 256 pixels. The weight tile is fetched as 192 rows
@@ -819,12 +840,12 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
   ptx::tcgen05_fence_before();
   __syncthreads();
   ptx::tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   if (*abort_flag != 0) total_tiles = 0;
   const int total_items = total_tiles * split_k;
   // What does not depend on the previous kernel is started before the wait for it: the tensor maps are fetched and a
   // CTA that keeps its weights resident starts their copies (weights are written at load time only).
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && ptx::elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmB) : "memory");
     if (p.w_resident && (int)blockIdx.x < total_tiles) {
@@ -840,7 +861,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
 
   if (warp == 0) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0) {
+    {
       int it = 0; // k-iterations issued so far, across tiles
       int ps = 0;        // ring stage of iteration `it`
       uint32_t pph = 0;  // its phase bit
@@ -884,28 +905,27 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         for (int kit = k_begin; kit < k_end; ++kit, ++it) {
           const CUtensorMap *mapA = (TF32 && term == 0) ? &tmA2 : &tmA;
           const CUtensorMap *mapB = (TF32 && term == 1) ? &tmB2 : &tmB;
-          if (it >= p.stages) {
-            if (!ptx::mbar_wait_bounded(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
-              if (!*abort_flag) report_error(p.err, kErrEmptyWait);
-              *abort_flag = 1;
-              ok = false;
-              break;
-            }
+          if (it >= p.stages && !ptx::mbar_wait_warp(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
+            if (lane == 0 && !*abort_flag) report_error(p.err, kErrEmptyWait);
+            *abort_flag = 1;
+            ok = false;
+            break;
           }
           const int c0 = chunk * p.BK;
           const uint32_t a_dst = tiles + (uint32_t)ps * stage_bytes;
           const uint32_t b_dst = a_dst + a_bytes;
           const uint32_t fb = bar_full + 8 * ps;
-          ptx::mbar_expect_tx(fb, stage_bytes);
-          if (p.a_mode == 1) {
-            // one copy per tile, also in dual mode (the map's pixel count per copy is the tile's: every copy costs
-            // its issuing thread about 430 cycles whatever its size)
-            ptx::tma_load_im2col_4d(a_dst, mapA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
-                                    (uint16_t)(tr * p.dh));
-          } else {
-            ptx::tma_load_2d(a_dst, mapA, fb, c0, m0);
+          if (ptx::elect_one()) {
+            ptx::mbar_expect_tx(fb, stage_bytes);
+            if (p.a_mode == 1) {
+              // one copy per tile, also in dual mode (the map's pixel count per copy is the tile's)
+              ptx::tma_load_im2col_4d(a_dst, mapA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
+                                      (uint16_t)(tr * p.dh));
+            } else {
+              ptx::tma_load_2d(a_dst, mapA, fb, c0, m0);
+            }
+            if (!p.w_resident) ptx::tma_load_3d(b_dst, mapB, fb, c0, tap, n0);
           }
-          if (!p.w_resident) ptx::tma_load_3d(b_dst, mapB, fb, c0, tap, n0);
           if (++chunk == p.c_chunks) {
             chunk = 0;
             ++tap;
@@ -943,7 +963,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       int it = 0, t = 0;
       int ms = 0;        // ring stage of iteration `it`
       uint32_t mph = 0;  // its phase bit
@@ -962,8 +982,8 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       uint32_t m_full = bar_full, m_empty = bar_empty, ring_lo = desc_ring_lo;
       const int ksteps = p.ksteps;
       if (p.w_resident && (int)blockIdx.x < total_tiles) {
-        if (!ptx::mbar_wait_bounded(bar_w, 0u, abort_flag, wait_rounds)) {
-          if (!*abort_flag) report_error(p.err, kErrFullWait);
+        if (!ptx::mbar_wait_warp(bar_w, 0u, abort_flag, wait_rounds)) {
+          if (lane == 0 && !*abort_flag) report_error(p.err, kErrFullWait);
           *abort_flag = 1;
           ok = false;
         }
@@ -977,8 +997,8 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         const int buf = t & 1;
         if (t >= 2) {
           // the epilogue must have drained this accumulator buffer (its previous use)
-          if (!ptx::mbar_wait_bounded(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
-            if (!*abort_flag) report_error(p.err, kErrAccWait);
+          if (!ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
+            if (lane == 0 && !*abort_flag) report_error(p.err, kErrAccWait);
             *abort_flag = 1;
             ok = false;
             break;
@@ -992,8 +1012,8 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         // 36 blocks: 15.4 -> 13.9 us; ResNet-50 batch 1 318 -> 292 us, batch 256 2560 -> 2530).
         auto k_loop = [&](auto whole) {
           for (int kit = k_begin; kit < k_end; ++kit, ++it) {
-            if (!ptx::mbar_try_wait(m_full, mph) && !ptx::mbar_wait_bounded(m_full, mph, abort_flag, wait_rounds)) {
-              if (!*abort_flag) report_error(p.err, kErrFullWait);
+            if (!ptx::mbar_wait_warp(m_full, mph, abort_flag, wait_rounds)) {
+              if (lane == 0 && !*abort_flag) report_error(p.err, kErrFullWait);
               *abort_flag = 1;
               ok = false;
               break;
@@ -1002,25 +1022,27 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
             // transposed product: weights are the A operand (M = channels), activations B (N = pixels)
             const uint32_t w_lo = p.w_resident ? wres_lo : ring_lo + a_step;
             const uint32_t acc_first = kit > k_begin ? 1u : 0u;
-            if constexpr (decltype(whole)::value) {
-              ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-            } else if (!p.dual) {
-              if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-              else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-              else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
-            } else {
-              // dual mode: sub-tile 0 uses weight rows 64..191 ([W; 0]), sub-tile 1 rows 0..127 ([0; W])
-              for (int sub = 0; sub < 2; ++sub) {
-                const uint32_t a_lo = w_lo + (sub == 0 ? dual_step : 0u);
-                const uint32_t b_lo = ring_lo + (uint32_t)sub * sub_step;
-                const uint32_t first = (kit > k_begin || sub > 0) ? 1u : 0u;
-                if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-                else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-                else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
-                else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+            if (ptx::elect_one()) {
+              if constexpr (decltype(whole)::value) {
+                ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+              } else if (!p.dual) {
+                if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+                else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+                else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, w_lo, ring_lo, desc_hi, p.idesc, acc_first);
+              } else {
+                // dual mode: sub-tile 0 uses weight rows 64..191 ([W; 0]), sub-tile 1 rows 0..127 ([0; W])
+                for (int sub = 0; sub < 2; ++sub) {
+                  const uint32_t a_lo = w_lo + (sub == 0 ? dual_step : 0u);
+                  const uint32_t b_lo = ring_lo + (uint32_t)sub * sub_step;
+                  const uint32_t first = (kit > k_begin || sub > 0) ? 1u : 0u;
+                  if (ksteps == 4) ptx::tcgen05_mma_i8_kblock<4, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                  else if (ksteps == 3) ptx::tcgen05_mma_i8_kblock<3, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                  else if (ksteps == 2) ptx::tcgen05_mma_i8_kblock<2, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                  else ptx::tcgen05_mma_i8_kblock<1, KIND>(d_tmem, a_lo, b_lo, desc_hi, p.idesc, first);
+                }
               }
+              ptx::tcgen05_commit(m_empty); // frees the stage when the MMAs retire
             }
-            ptx::tcgen05_commit(m_empty); // frees the stage when the MMAs retire
             wres_lo += w_step;
             m_full += 8;
             m_empty += 8;
@@ -1036,7 +1058,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         };
         if (ksteps == 4 && !p.dual) k_loop(std::true_type{});
         else k_loop(std::false_type{});
-        if (ok) ptx::tcgen05_commit(bar_acc_full + 8 * buf);
+        if (ok && ptx::elect_one()) ptx::tcgen05_commit(bar_acc_full + 8 * buf);
       }
     }
   } else {
@@ -1045,8 +1067,11 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     const int half = (warp - 2) >> 2; // which alternate 32-pixel column groups it takes
     const StageLane st = make_stage_lane<BF16 ? 2 : 4>(base + 1024u + (uint32_t)((warp - 2) * kStageBytes), lane);
     ChanConst cc = {};
-    FloatRequant fq = {};
+    FloatRequantPairs<ACTSEL == 101> fq = {};
+    FloatRequantShared fshared = {};
+    if constexpr (FQ && ACTSEL != 101) fshared.set();
     float bias_f = 0.0f;
+    unsigned long long bias2 = 0;
     int staged_n0 = -1;
     int t = 0;
     bool ok = true;
@@ -1084,10 +1109,11 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         if (BF16 || TF32) {
           const int ch = n0 + ch_base + lane_channel(lane);
           bias_f = ch < p.n_valid ? __int_as_float(p.bias[ch]) : 0.0f; // fp32 bias bits in the int32 array
+          if (BF16) bias2 = hold_pair(bias_f);
         } else if (FQ) {
           const int ch = n0 + ch_base + lane_channel(lane);
           const uint4 c = ch < p.n_valid ? __ldg(reinterpret_cast<const uint4 *>(p.fq) + ch) : make_uint4(0u, 0u, 0u, 0u);
-          fq = FloatRequant{c.x, __uint_as_float(c.y), __uint_as_float(c.z), __uint_as_float(c.w)};
+          fq.set(FloatRequant{c.x, __uint_as_float(c.y), __uint_as_float(c.z), __uint_as_float(c.w)});
         } else {
           cc = load_chan_const(p, n0 + ch_base + lane_channel(lane));
         }
@@ -1168,18 +1194,18 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         } else if (BF16) {
           // byte addressing: 2 bytes per channel
           uint8_t *out16 = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch8) * 2;
-          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias_f, st, ncols);
-          else epilogue_channels_bf16<false>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias_f, st, ncols);
+          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
+          else epilogue_channels_bf16<false>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
         } else if constexpr (ACTSEL == 103) {
-          epilogue_add_fq(p, lane_addr, out8, ch8_ok, m0, half, fq, st, ncols, res_words,
+          epilogue_add_fq(p, lane_addr, out8, ch8_ok, m0, half, fq, fshared, st, ncols, res_words,
                           residual_at(item + gridDim.x, tm, tn), tm * m_tile);
         } else if constexpr (FQ) {
-          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, fq, st, ncols);
-        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
-        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
-        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols);
-        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
-        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, st, ncols, ws_lane);
+          epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, fq, fshared, st, ncols);
+        } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
+        else if (p.act == 2) epilogue_channels_impl<2, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
+        else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols);
+        else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
+        else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
       }
       if constexpr (ACTSEL == 103) {
         if (n0 + ch_base >= p.n_valid) { // no outputs here: the next tile's residual all the same
