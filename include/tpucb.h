@@ -146,6 +146,9 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          "split_k" (0/1, default 1; read by the next load_module): INT8 convolutions and inner products with at most
  *          half as many tiles as SMs and a K that is long enough to pay for the exchange (from about 24 K blocks for
  *          a few tiles to 48 for many) share each tile among several CTAs (exact: int32 partial sums).
+ *          "big_tiles" (0 never, 1 = default: by size, else 1000 * CTAs (1, 2) + pixels (32 .. 256, a multiple of 32): every
+ *          layer that can, in this form; read by the next load_module): tensor-core convolutions that fill the GPU and have a
+ *          long K run tiles of up to 256 pixels, one CTA per SM, or two SMs per tile.
  *          "fuse_activations" (0/1, default 1; read by the next load_module): run each
  *          quant(INT8->BF16) -> slope-table activation -> quant(BF16->INT8) chain as one launch
  *          that still writes all three tensors.

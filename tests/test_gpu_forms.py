@@ -273,3 +273,38 @@ def test_bf16_results_past_the_largest_finite(relu):
     got, ref = run_model(text, {"f": f, "b": b}, {"x": x}, ["c"])["c"]
     assert (ref == graphs._bf16_np(np.float32(3.39e38))).any()
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype", ["INT8", "BF16", "FP32"])
+@pytest.mark.parametrize("form", [1256, 1096, 2256, 2192, 2032])  # 1000 CTAs per tile + pixels per tile
+@pytest.mark.parametrize("case", [
+    # n, ic, oc, hw, k, stride, pad, dilation, ReLU
+    (3, 64, 256, 20, 1, 1, 0, 1, 0),    # one short K block, the last tile's second half past the last pixel
+    (2, 96, 136, 13, 3, 1, 1, 1, 1),    # channels that end inside a tile, K blocks with a tail
+    (5, 160, 300, 9, 3, 2, 1, 1, 0),    # a stride, images inside a tile
+    (1, 1040, 520, 5, 1, 1, 0, 1, 1),   # fewer pixels than a tile, a long K, a channel tile that one CTA of a pair has alone
+    (23, 80, 144, 41, 3, 1, 1, 1, 0)])  # several tiles per CTA
+def test_big_tiles(dtype, form, case):
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, k, s, p, d, relu = case
+    if dtype == "INT8":
+        model = graphs.single_conv_i8(n, ic, oc, hw, k, s, p, d, relu=bool(relu), seed=6200 + ic + k)
+        text, w, x, name = model.text, model.weights, model.meta["x"], "conv"
+    else:
+        rng = np.random.default_rng(47 + ic + k)
+        cut = graphs._bf16_np if dtype == "BF16" else (lambda v: np.asarray(v, np.float32))
+        w = {"f": cut(rng.normal(0, (2.0 / (ic * k * k)) ** 0.5, (oc, ic, k, k))), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+        x, name = cut(rng.normal(0, 1, (n, ic, hw, hw))), "c"
+        text = "input name=x shape=%d,%d,%d,%d dtype=%s\n" % (n, ic, hw, hw, dtype) + conv_text(dtype, n, ic, oc, hw, k, s, p, d, relu)
+    got = []
+    for mode in (0, form):
+        m = module(0)
+        m.set_option("big_tiles", mode)
+        m.load_text(text, w)
+        m.set_tensor("x", x)
+        for _ in range(2):
+            m.invoke()
+        got.append(m.get_tensor(name))
+        m.close()
+    # the products of an output value are summed in the same order: every bit is the same
+    assert np.array_equal(got[0], got[1])

@@ -3,7 +3,7 @@
 // (lib/Dialect/TPU/IR/TPUOperationSupport.cpp:366-428): four independent pads, the
 // output size taken from the result type, dilation, optional input zero-insertion.
 #pragma once
-#include "conv_gemm_i8.cuh"
+#include "conv_big.cuh"
 #include "host_common.h"
 #include "mem_kernels.cuh"
 
@@ -84,6 +84,9 @@ struct ConvPlan {
   int ws_tiles = 0;  // split K: tiles of the partial-sum workspace (p.ws, p.ws_count), allocated by the op that owns the plan
   bool bf16 = false; // runs conv_gemm_bf16_kernel (K sizes and pitches in bytes, 2 per element)
   bool tf32 = false; // runs conv_gemm_tf32x3_kernel (fp32 operands, 4 bytes per element; three K passes)
+  int ctas = 0;      // runs the kernels of conv_big.cuh with this many CTAs per tile (0: those of conv_gemm_i8.cuh)
+  CUtensorMap tmO, tmO2; // ctas > 0: the results, and those of the fused activation or the remainder operand
+  int box_px() const { return ctas > 1 ? p.m_tile / ctas : p.m_tile; } // pixels per copy of the activations
   CUtensorMap tmA2, tmB2;           // tf32: remainder parts of the activations and of the weights
   const float *split_src = nullptr; // tf32: the fp32 input, whose remainder is written to split_lo before the launch
   float *split_lo = nullptr;
@@ -125,32 +128,32 @@ inline void pack_filter(const float *w, int channels, int taps, T *out, size_t p
       for (int c = 0; c < channels; ++c) out[t * pitch + c] = line[(size_t)c * taps + t];
 }
 
-// Rows of the packed weights: whole blocks of 32 channels, in the order of packed_row.
+// Rows of the packed weights: whole blocks of 32 channels, in the order of packed_row (`natural`: of the channels, for conv_big.cuh).
 inline size_t packed_rows(int oc_pad) { return (size_t)(oc_pad + 31) / 32 * 32; }
 
 // Pack OIHW fp32 weights (integer-valued) to int8 [rows][taps][cin_pad] for the im2col
 // path, or [rows][1][kp] with K order (r, s, c) for the patch path. For grouped
 // convolution the caller passes one group's slice.
 inline std::vector<int8_t> pack_conv_weights(const float *w, int oc, int icg, int kh, int kw,
-                                             int oc_pad, int cin_pad, bool patch, int kp) {
+                                             int oc_pad, int cin_pad, bool patch, int kp, bool natural = false) {
   const int taps = kh * kw;
   const size_t row = patch ? kp : (size_t)taps * cin_pad, pitch = patch ? icg : cin_pad;
   std::vector<int8_t> out(packed_rows(oc_pad) * row, 0), line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    pack_filter(w + (size_t)o * icg * taps, icg, taps, out.data() + packed_row(o) * row, pitch, line.data(), [](float v) { return (int8_t)(int)v; });
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, out.data() + (natural ? o : packed_row(o)) * row, pitch, line.data(), [](float v) { return (int8_t)(int)v; });
   return out;
 }
 
 // BF16 weights [rows][tap][cin_pad] as 16-bit patterns (the values of a BF16 graph's filter are
 // BF16-representable floats: the upper 16 bits are the value), returned as bytes
 inline std::vector<int8_t> pack_conv_weights_bf16(const float *w, int oc, int icg, int kh, int kw, int oc_pad,
-                                                  int cin_pad) {
+                                                  int cin_pad, bool natural) {
   const int taps = kh * kw;
   const size_t row = (size_t)taps * cin_pad;
   std::vector<int8_t> bytes(packed_rows(oc_pad) * row * 2, 0);
   std::vector<uint16_t> line((size_t)icg * taps);
   for (int o = 0; o < oc; ++o)
-    pack_filter(w + (size_t)o * icg * taps, icg, taps, reinterpret_cast<uint16_t *>(bytes.data()) + packed_row(o) * row, cin_pad, line.data(),
+    pack_filter(w + (size_t)o * icg * taps, icg, taps, reinterpret_cast<uint16_t *>(bytes.data()) + (natural ? o : packed_row(o)) * row, cin_pad, line.data(),
                 [](float v) { return (uint16_t)(f32_bits(v) >> 16); });
   return bytes;
 }
@@ -158,7 +161,7 @@ inline std::vector<int8_t> pack_conv_weights_bf16(const float *w, int oc, int ic
 // fp32 weights for the TF32 x 3 convolution, K-major [rows][tap][cin_pad] as bytes: part 0 = the upper 19 bits of
 // every word, part 1 = the exact remainder.
 inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int icg, int kh, int kw, int oc_pad, int cin_pad,
-                                                  int part) {
+                                                  int part, bool natural) {
   const int taps = kh * kw;
   std::vector<float> out(packed_rows(oc_pad) * taps * cin_pad, 0.0f);
   for (int o = 0; o < oc; ++o)
@@ -167,7 +170,7 @@ inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int ic
         for (int s = 0; s < kw; ++s) {
           const float v = w[(((size_t)o * icg + c) * kh + r) * kw + s];
           const float hi = bits_f32(f32_bits(v) & 0xffffe000u);
-          out[((size_t)packed_row(o) * taps + (r * kw + s)) * cin_pad + c] = part == 0 ? hi : v - hi;
+          out[((size_t)(natural ? o : packed_row(o)) * taps + (r * kw + s)) * cin_pad + c] = part == 0 ? hi : v - hi;
         }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
@@ -175,14 +178,14 @@ inline std::vector<int8_t> pack_conv_weights_tf32(const float *w, int oc, int ic
 }
 
 // the same for the patch matrix of an fp32 image stem: four channel slots per tap, k = tap * 4 + c
-inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeom &g, int oc_pad, int part) {
+inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeom &g, int oc_pad, int part, bool natural) {
   const int kp = g.kh * g.kw * 4;
   std::vector<float> out(packed_rows(oc_pad) * kp, 0.0f);
   for (int o = 0; o < g.oc; ++o)
     for (int c = 0; c < g.ic; ++c)
       for (int t = 0; t < g.kh * g.kw; ++t) {
         const float v = w[((size_t)o * g.ic + c) * g.kh * g.kw + t], hi = bits_f32(f32_bits(v) & 0xffffe000u);
-        out[(size_t)packed_row(o) * kp + t * 4 + c] = part == 0 ? hi : v - hi;
+        out[(size_t)(natural ? o : packed_row(o)) * kp + t * 4 + c] = part == 0 ? hi : v - hi;
       }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
@@ -314,16 +317,99 @@ inline void encode_window_map(CUtensorMap *tm, const void *d_in, const ConvGeom 
   fix_small_im2col_map(tm, (size_t)row * g.ih * g.n);
 }
 
+// Maps of the tensors that the kernels of conv_big.cuh write: 32 pixels x 128 bytes per store, clipped to the valid
+// channels and the last pixel.
+inline void encode_out_maps(ConvPlan &pl) {
+  if (pl.ctas == 0) return;
+  const int es = pl.tf32 ? 4 : (pl.bf16 ? 2 : 1);
+  for (int k = 0; k < 2; ++k) {
+    int8_t *to = k ? pl.p.out2 : pl.p.out;
+    cuuint64_t dims[2] = {(cuuint64_t)pl.p.n_valid * es, (cuuint64_t)pl.p.M_total};
+    cuuint64_t strides[1] = {(cuuint64_t)pl.p.ldc};
+    cuuint32_t box[2] = {128, 32}, one[2] = {1, 1};
+    CUresult r = tma_api().tiled(k ? &pl.tmO2 : &pl.tmO, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, to ? to : pl.p.out, dims, strides, box, one,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, pl.tf32 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    TPUCB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(results) failed: %d", (int)r);
+  }
+}
+
+// Whether a plan runs on the kernels of conv_big.cuh, and in which form: CTAs per tile (one: 128 channels, two: 256) and
+// pixels per tile.
+inline bool finish_big_plan(ConvPlan &pl, int rows, int taps, int oc_pad, int sm_count) {
+  ConvGemmParams &p = pl.p;
+  const int mode = conv_big_mode(), kind = pl.tf32 ? 2 : (pl.bf16 ? 1 : 0);
+  if (mode == 0 || p.group > 1 || p.c_off || oc_pad % 16 || (kind == 0 && !p.fq && !(p.fastq & 1))) return false;
+  const int k_iters = taps * p.c_chunks * (kind == 2 ? 3 : 1);
+  int ctas = mode > 1 ? mode / 1000 : 0, px = mode % 1000;
+  auto tiles_of = [&](int c, int n) { return (long long)((rows + n - 1) / n) * ((oc_pad + 128 * c - 1) / (128 * c)); };
+  if (mode == 1 && kind < 2) {
+    // Launches of 1.3 tiles of 128 x 256 per SM and more, whose K is long enough that its loop counts and not the epilogue, which
+    // the kernels of conv_gemm_i8.cuh do better (INT8 from 8 K blocks, BF16 from 2); pairs where the loop is nearly everything.
+    // us alone / with three launches in flight, there -> here:
+    //   INT8, 256 images: 3x3 256 channels 14x14 25.4 / 24.6 -> 22.4 / 21.3 (pair), 128 at 28x28 27.3 / 28.0 -> 24.3 / 25.4, 512 at
+    //     7x7 28.6 / 22.6 -> 25.9 / 20.1, 64 at 56x56 52.0 / 50.5 -> 46.4 / 45.1; 1x1 1024 -> 256 14.2 / 15.7 -> 13.0 / 15.0;
+    //     large ones: 32 x 512 x 56 x 56 183 / 180 -> 158 / 155 (single), 140 / 141 (pair);
+    //     not: 1x1 512 -> 2048 (4 blocks) 18.1 / 16.6 against 20.1 / 17.9, 64 -> 256 58 / 53 against 62 / 59;
+    //   BF16, 128 images: 3x3 256 at 14x14 28.7 / 23.6 -> 27.2 / 21.5, 512 at 7x7 30.3 / 22.5 -> 26.5 / 20.0; 1x1 256 -> 1024 18.6 /
+    //     18.4 -> 16.9 / 16.3, 128 -> 512 25.3 / 24.6 -> 24.1 / 23.0; not 64 -> 256 43.7 / 40.4 against 45.6 / 39.5;
+    //   fewer tiles: INT8, 64 images, 128 at 28x28 (196) 10.9 / 8.5 against 11.0 / 8.6, 256 at 14x14 (98) 10.9 / 6.7 against 10.5 /
+    //     6.7; tiles of 192 pixels 9.2 / 8.0: faster alone, slower in flight.
+    if (oc_pad <= 64 || tiles_of(1, 256) * 10 < 13LL * sm_count || k_iters < (kind == 0 ? 8 : 2)) return false;
+    px = 256;
+    ctas = oc_pad > 128 && k_iters >= 16 && tiles_of(2, 256) >= sm_count ? 2 : 1;
+  } else if (mode == 1) {
+    // fp32 runs alone (calibration, the tuner), so whole waves count: clocks per K block of a wave, as measured (3x3 256
+    // channels at 14x14 and 128 at 28x28, 64 images: 85.6 -> 66.2 us and 79.0 -> 70.8; 1x1 1024 -> 256 55.9 -> 46.1, 256 -> 1024
+    // 40.5 -> 35.8; not: 3x3 512 at 7x7, one tile per SM there, 106 against 118).
+    if (oc_pad <= 64) return false;
+    const long long there = (tiles_of(1, 128) + sm_count - 1) / sm_count;
+    double best = there <= 1 ? 466.0 : 376.0 * there;
+    for (int c = 1; c <= (k_iters >= 16 ? 2 : 1); ++c)
+      for (int n = 128; n <= 256; n += 64) {
+        const long long slots = sm_count / c, waves = (tiles_of(c, n) + slots - 1) / slots;
+        const double cost = waves * (c == 1 ? std::max(520.0, 2.5 * n) : std::max(530.0, 2.37 * n));
+        if (cost > 0.97 * best && (ctas == 0 || cost > best)) continue;
+        best = cost;
+        ctas = c;
+        px = n;
+      }
+    if (ctas == 0) return false;
+  }
+  const size_t stage = (size_t)(128 + px / ctas) * p.BK, fixed = 1024 + kBigHeader + kBigStaging[kind];
+  int stages = (int)std::min<size_t>(kMaxStages, (227 * 1024 - fixed) / stage);
+  if (stages < 2) return false;
+  pl.ctas = ctas;
+  p.dual = 0;
+  p.w_resident = 0;
+  p.split_k = 1;
+  p.k_per = taps * p.c_chunks;
+  p.BN = 128;
+  p.n_valid = oc_pad;
+  p.tmem_cols = 512;
+  p.m_tile = px;
+  p.stages = stages;
+  const int M = 128 * ctas;
+  p.idesc = kind == 2 ? make_idesc_tf32(M, px) : (kind == 1 ? make_idesc_bf16(M, px) : make_idesc_i8(M, px));
+  const long long tiles = (long long)((rows + px - 1) / px) * ((oc_pad + M - 1) / M);
+  pl.grid = dim3((unsigned)(ctas * std::min<long long>(tiles, sm_count / ctas)), 1, 1);
+  // (More than half of an SM's shared memory in any case: two CTAs of these kernels on one SM would wait for each other's
+  // tensor memory.)
+  pl.smem = std::max<size_t>(fixed + stages * stage, 120 * 1024);
+  return true;
+}
+
 // Build the launch plan for one GEMM-shaped problem.
 //   rows       implicit-GEMM M
 //   k_inner    K bytes per tap (padded input channels, or the whole K in matrix mode)
 //   oc_pad     padded output channels (multiple of 16)
-inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pad, int sm_count) {
+inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pad, int sm_count, bool may_be_big = false) {
   ConvGemmParams &p = pl.p;
   p.M_total = rows;
   p.BK = pick_bk(k_inner);
   p.c_chunks = (k_inner + p.BK - 1) / p.BK;
   p.ksteps = p.c_chunks == 1 ? (k_inner + 31) / 32 : p.BK / 32;
+  if (may_be_big && finish_big_plan(pl, rows, taps, oc_pad, sm_count)) return;
   // Dual mode: layers with at most 64 output channels would leave half of the TMEM lanes (and half of
   // the epilogue warps) idle; they run 256-pixel tiles instead (see the kernel). Not combined with
   // pixel groups, which fill them.
@@ -482,6 +568,41 @@ inline void pair_layer(DenseLayer &d) {
   d.paired = true;
 }
 
+// The kernel of a plan on conv_big.cuh. `use` gets it as a function pointer and says whether it is one of the fp32 form, which
+// takes two more maps.
+template <class Use> inline void with_big_kernel(int ctas, int kind, int act, bool fq, Use use) {
+  auto by_ctas = [&](auto c) {
+    constexpr int C = decltype(c)::value;
+    if (kind == 2) {
+      if (act == 1) use(conv_big_tf32x3_kernel<C, 1>);
+      else use(conv_big_tf32x3_kernel<C, 0>);
+    } else if (kind == 1) {
+      if (act == 1) use(conv_big_kernel<C, 1, 1, 0>);
+      else use(conv_big_kernel<C, 1, 0, 0>);
+    } else if (fq) {
+      if (act == 1) use(conv_big_kernel<C, 0, 1, 3>);
+      else if (act == 2) use(conv_big_kernel<C, 0, 2, 3>);
+      else use(conv_big_kernel<C, 0, 0, 3>);
+    } else {
+      if (act == 1) use(conv_big_kernel<C, 0, 1, 1>);
+      else if (act == 2) use(conv_big_kernel<C, 0, 2, 1>);
+      else use(conv_big_kernel<C, 0, 0, 1>);
+    }
+  };
+  if (ctas == 2) by_ctas(std::integral_constant<int, 2>());
+  else by_ctas(std::integral_constant<int, 1>());
+}
+inline void launch_big_plan(const ConvPlan &pl, cudaStream_t stream, int sm_count) {
+  if (pl.tf32 && pl.split_src)
+    launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
+             reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
+  with_big_kernel(pl.ctas, pl.tf32 ? 2 : (pl.bf16 ? 1 : 0), pl.p.act, pl.p.fq != nullptr, [&](auto kernel) {
+    if constexpr (std::is_invocable_v<decltype(kernel), CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ConvGemmParams>)
+      launch_k(kernel, pl.grid, kBigThreads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmO, pl.tmO2, pl.p);
+    else launch_k(kernel, pl.grid, kBigThreads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.tmO, pl.tmO2, pl.p);
+  });
+}
+
 inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_count) {
   if (pl.use_patch && pl.tf32)
     launch_k(patch_expand_f32_kernel, grid_for((size_t)pl.p.M_total * pl.patch.kp / 4, 256, sm_count), 256, 0, stream,
@@ -496,7 +617,8 @@ inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_cou
   }
   const int threads = kConvThreads;
   PdlConvScope conv_class; // the tensor-core kernel and its helper passes may start while the predecessor finishes
-  if (pl.tf32) {
+  if (pl.ctas > 0) launch_big_plan(pl, stream, sm_count);
+  else if (pl.tf32) {
     if (pl.split_src)
       launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
                reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
@@ -529,6 +651,12 @@ inline void conv_kernel_setup_once() {
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    for (int ctas = 1; ctas <= 2; ++ctas)
+      for (int form = 0; form < 4; ++form) // INT8 twice (requantisation), BF16, fp32
+        for (int act = 0; act < (form < 2 ? 3 : 2); ++act)
+          with_big_kernel(ctas, std::max(0, form - 1), act, form == 1, [](auto kernel) {
+            TPUCB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+          });
     return true;
   }();
   (void)done;

@@ -87,6 +87,13 @@ inline bool &conv_split_k_enabled() {
   return on;
 }
 
+// Which launch plans take the kernels for launches that fill the GPU (conv_big.cuh; option "big_tiles"): 0 none, 1 by size,
+// else 1000 times the CTAs of a tile + its pixels: every layer that can, in this form.
+inline int &conv_big_mode() {
+  static thread_local int v = 1;
+  return v;
+}
+
 inline int &pdl_mode() {
   static thread_local int v = 1;
   return v;

@@ -111,6 +111,7 @@ public:
     pdl_mode() = use_pdl;
     launch_pdl_flag() = use_pdl >= 2;
     launch_sm_count() = sm_count;
+    conv_big_mode() = selftest_lost_arrival ? 0 : big_tiles;
     conv_split_k_enabled() = split_k && selftest_lost_arrival == 0; // the self-test needs tiles that follow one another in a CTA
   }
   int device() const { return device_; }
@@ -270,6 +271,7 @@ public:
     split_ws.push_back({pl.p.ws_count, cbytes});
   }
   bool fuse_activations = true; // set before load_module
+  int big_tiles = 1; // set before load_module: see conv_big_mode
   int fuse_residual_add = 2; // set before load_module: eltwise adds in the producing convolution's epilogue: 0 never, 1 always, 2 by size
   bool fp32_tensor_cores = true; // set before load_module: fp32 convolutions as three TF32 products
   void link_tf32_remainders();
@@ -661,7 +663,6 @@ public:
     for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
     p.bias = p.mult = p.rshift = I.upload(bias_bits);
     p.OH = g.oh; p.OW = g.ow;
-    std::vector<int8_t> w[2];
     int taps = 1, k_bytes;
     const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
     if (stem) {
@@ -674,7 +675,6 @@ public:
       pl.patch_bytes = (size_t)rows * k_bytes;
       pl.patch_buf = (int8_t *)I.dalloc(pl.patch_bytes);
       pl.split_lo = (float *)I.dalloc(pl.patch_bytes);
-      for (int part = 0; part < 2; ++part) w[part] = pack_patch_weights_tf32(filt.data(), g, out_cp, part);
     } else {
       p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
       p.kh = g.kh; p.kw = g.kw;
@@ -686,16 +686,18 @@ public:
       pl.split_src = (const float *)in_->dev;
       pl.split_lo = (float *)in_->lo_dev;
       pl.split_nvec = in_->bytes() / 16;
-      for (int part = 0; part < 2; ++part) w[part] = pack_conv_weights_tf32(filt.data(), g.oc, g.ic, g.kh, g.kw, out_cp, in_->cp, part);
     }
-    finish_plan(pl, rows, taps, k_bytes, out_cp, I.sm_count);
+    finish_plan(pl, rows, taps, k_bytes, out_cp, I.sm_count, true);
     const int8_t *part[2] = {stem ? pl.patch_buf : (const int8_t *)in_->dev, (const int8_t *)pl.split_lo};
     for (int k = 0; k < 2; ++k) {
       CUtensorMap *a = k ? &pl.tmA2 : &pl.tmA;
-      if (p.a_mode == 0) encode_matrix_map(a, part[k], rows, k_bytes, k_bytes, p.BK, p.m_tile);
-      else encode_im2col_map(a, part[k], g, k_bytes, p.BK, p.m_tile);
-      encode_weight_map(k ? &pl.tmB2 : &pl.tmB, I.upload(w[k]), out_cp, taps, k_bytes, p.BK, p.BN);
+      if (p.a_mode == 0) encode_matrix_map(a, part[k], rows, k_bytes, k_bytes, p.BK, pl.box_px());
+      else encode_im2col_map(a, part[k], g, k_bytes, p.BK, pl.box_px());
+      const std::vector<int8_t> w = stem ? pack_patch_weights_tf32(filt.data(), g, out_cp, k, pl.ctas > 0)
+                                         : pack_conv_weights_tf32(filt.data(), g.oc, g.ic, g.kh, g.kw, out_cp, in_->cp, k, pl.ctas > 0);
+      encode_weight_map(k ? &pl.tmB2 : &pl.tmB, I.upload(w), out_cp, taps, k_bytes, p.BK, 128);
     }
+    encode_out_maps(pl);
     plans_.push_back(pl);
   }
   // Ungrouped layers on the tensor cores. kind: 0 INT8, 1 BF16. Two forms: row windows (wp), K blocks of a matrix or im2col
@@ -781,14 +783,15 @@ public:
     const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.oh == g.ih && g.ow == g.iw;
     const int taps = g.kh * g.kw;
     p.a_mode = one ? 0 : 1;
-    finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count);
-    if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, p.m_tile);
-    else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, p.m_tile);
+    finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count, true);
+    if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, pl.box_px());
+    else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, pl.box_px());
+    encode_out_maps(pl);
     // A tap's weights are padded to whole K blocks: rows that start off 32-byte sectors and reach past the extent arrive at
     // a third of the rate (7 x 45 x 45 pixels, 80 -> 128 channels, 5x5: 35.9 -> 28.3 us; MobileNet-v2 batch 32 426 -> 408).
     const int pitch = p.c_chunks * p.BK;
-    const int8_t *d_w = I.upload(kind == 0 ? pack_conv_weights(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch, false, 0)
-                                           : pack_conv_weights_bf16(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch / 2));
+    const int8_t *d_w = I.upload(kind == 0 ? pack_conv_weights(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch, false, 0, pl.ctas > 0)
+                                           : pack_conv_weights_bf16(d.w, g.oc, g.ic, g.kh, g.kw, d.out_cp, pitch / 2, pl.ctas > 0));
     encode_weight_map(&pl.tmB, d_w, d.out_cp, taps, pitch, p.BK, p.dual ? 192 : 128);
   }
   // Fused leaky ReLU (tensor-core plans only): the epilogue writes the plain result to this op's tensor
@@ -801,13 +804,14 @@ public:
       pl.p.act = 2;
       pl.p.leaky_mp = mp; pl.p.leaky_rp = rp; pl.p.leaky_mn = mn; pl.p.leaky_rn = rn;
       pl.p.out2 = act_out;
+      encode_out_maps(pl);
     }
     act_ = 2;
   }
   // Fused eltwise add (tensor-core INT8 plans without an activation of their own): the epilogue also forms
   // sat8(relu?((conv * ms + residual * mr + 2^(r-1)) >> r)) into `sum_out`; this op's own tensor is still written.
   bool can_fuse_add() const {
-    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1 && !plans_[0].p.dual;
+    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1 && !plans_[0].p.dual && plans_[0].ctas == 0;
   }
   void set_residual_add(const int8_t *residual, int8_t *sum_out, int ms, int mr, int rshift, int relu) {
     for (auto &pl : plans_) {
@@ -825,7 +829,10 @@ public:
   bool is_tf32() const { return can_write_remainder() && !plans_[0].use_patch; }
   bool can_write_remainder() const { return !plans_.empty() && plans_[0].tf32; }
   void set_remainder_out(void *lo) {
-    for (auto &pl : plans_) pl.p.out2 = (int8_t *)lo;
+    for (auto &pl : plans_) {
+      pl.p.out2 = (int8_t *)lo;
+      encode_out_maps(pl);
+    }
   }
   void skip_split() {
     for (auto &pl : plans_) pl.split_src = nullptr;

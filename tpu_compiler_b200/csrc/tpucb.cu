@@ -376,6 +376,11 @@ int tpucb_interp_set_option(tpucb_interp *it, const char *key, int value) {
     it->impl.selftest_lost_arrival = value; // takes effect at the next load_module
   } else if (k == "split_k") {
     it->impl.split_k = value != 0; // takes effect at the next load_module
+  } else if (k == "big_tiles") {
+    const int px = value % 1000;
+    TPUCB_CHECK(value == 0 || value == 1 || ((value / 1000 == 1 || value / 1000 == 2) && px >= 32 && px <= 256 && px % 32 == 0),
+                "big_tiles: 0 (never), 1 (by size, the default) or 1000 * CTAs (1, 2) + pixels (32 .. 256, a multiple of 32)");
+    it->impl.big_tiles = value; // takes effect at the next load_module
   } else if (k == "fuse_activations") {
     it->impl.fuse_activations = value != 0; // takes effect at the next load_module
   } else if (k == "fuse_residual_add") {
