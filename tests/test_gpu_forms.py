@@ -308,3 +308,21 @@ def test_big_tiles(dtype, form, case):
         m.close()
     # the products of an output value are summed in the same order: every bit is the same
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("relu", [0, 1])
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, k, stride, pad, dilation: the patches built in shared memory
+    (1, 3, 16, 9, 3, 1, 1, 1),      # fewer tiles than SMs, an odd number of taps
+    (3, 3, 64, 65, 7, 2, 3, 1),     # ragged last tile
+    (2, 4, 40, 64, 6, 3, 2, 1),     # an even number of taps, four channels, channels that end inside a quarter
+    (5, 1, 64, 96, 7, 1, 6, 2),     # several tiles per SM, a dilation, taps outside the image
+    (1, 3, 64, 30, 8, 2, 3, 1), (1, 3, 72, 30, 7, 2, 3, 1)])  # too many taps, too many channels: the patch matrix
+def test_fp32_stem_patches(case, relu):
+    n, ic, oc, hw, k, s, p, d = case
+    rng = np.random.default_rng(53 + oc + k)
+    w = {"f": rng.normal(0, (2.0 / (ic * k * k)) ** 0.5, (oc, ic, k, k)).astype(np.float32), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+    x = rng.normal(0, 1, (n, ic, hw, hw)).astype(np.float32)
+    text = "input name=x shape=%d,%d,%d,%d dtype=FP32\n" % (n, ic, hw, hw) + conv_text("FP32", n, ic, oc, hw, k, s, p, d, relu)
+    got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
+    # three products leave 2^-22 of each term; the tensor core cuts each of the 25 partial sums of a term at 2^-23 of the sum
+    assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()

@@ -4,6 +4,7 @@
 // output size taken from the result type, dilation, optional input zero-insertion.
 #pragma once
 #include "conv_big.cuh"
+#include "conv_stem_f32.cuh"
 #include "host_common.h"
 #include "mem_kernels.cuh"
 
@@ -86,6 +87,8 @@ struct ConvPlan {
   bool tf32 = false; // runs conv_gemm_tf32x3_kernel (fp32 operands, 4 bytes per element; three K passes)
   int ctas = 0;      // runs the kernels of conv_big.cuh with this many CTAs per tile (0: those of conv_gemm_i8.cuh)
   CUtensorMap tmO, tmO2; // ctas > 0: the results, and those of the fused activation or the remainder operand
+  bool stem = false; // runs conv_stem_tf32x3_kernel
+  StemArgs stem_args;
   int box_px() const { return ctas > 1 ? p.m_tile / ctas : p.m_tile; } // pixels per copy of the activations
   CUtensorMap tmA2, tmB2;           // tf32: remainder parts of the activations and of the weights
   const float *split_src = nullptr; // tf32: the fp32 input, whose remainder is written to split_lo before the launch
@@ -186,6 +189,22 @@ inline std::vector<int8_t> pack_patch_weights_tf32(const float *w, const ConvGeo
       for (int t = 0; t < g.kh * g.kw; ++t) {
         const float v = w[((size_t)o * g.ic + c) * g.kh * g.kw + t], hi = bits_f32(f32_bits(v) & 0xffffe000u);
         out[(size_t)(natural ? o : packed_row(o)) * kp + t * 4 + c] = part == 0 ? hi : v - hi;
+      }
+  std::vector<int8_t> bytes(out.size() * 4);
+  std::memcpy(bytes.data(), out.data(), bytes.size());
+  return bytes;
+}
+
+// and for the stem kernel: [high parts, remainders][taps, even][64 channels][4]
+inline std::vector<int8_t> pack_stem_weights_tf32(const float *w, const ConvGeom &g) {
+  const int taps = g.kh * g.kw, taps2 = (taps + 1) / 2 * 2;
+  std::vector<float> out((size_t)2 * taps2 * 64 * 4, 0.0f);
+  for (int o = 0; o < g.oc; ++o)
+    for (int c = 0; c < g.ic; ++c)
+      for (int t = 0; t < taps; ++t) {
+        const float v = w[((size_t)o * g.ic + c) * taps + t], hi = bits_f32(f32_bits(v) & 0xffffe000u);
+        out[((size_t)t * 64 + o) * 4 + c] = hi;
+        out[((size_t)(taps2 + t) * 64 + o) * 4 + c] = v - hi;
       }
   std::vector<int8_t> bytes(out.size() * 4);
   std::memcpy(bytes.data(), out.data(), bytes.size());
@@ -617,7 +636,10 @@ inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_cou
   }
   const int threads = kConvThreads;
   PdlConvScope conv_class; // the tensor-core kernel and its helper passes may start while the predecessor finishes
-  if (pl.ctas > 0) launch_big_plan(pl, stream, sm_count);
+  if (pl.stem) {
+    if (pl.p.act == 1) launch_k(conv_stem_tf32x3_kernel<true>, pl.grid, kStemThreads, pl.smem, stream, pl.stem_args, pl.p);
+    else launch_k(conv_stem_tf32x3_kernel<false>, pl.grid, kStemThreads, pl.smem, stream, pl.stem_args, pl.p);
+  } else if (pl.ctas > 0) launch_big_plan(pl, stream, sm_count);
   else if (pl.tf32) {
     if (pl.split_src)
       launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
@@ -651,6 +673,8 @@ inline void conv_kernel_setup_once() {
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_tf32x3_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_tf32x3_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     for (int ctas = 1; ctas <= 2; ++ctas)
       for (int form = 0; form < 4; ++form) // INT8 twice (requantisation), BF16, fp32
         for (int act = 0; act < (form < 2 ? 3 : 2); ++act)

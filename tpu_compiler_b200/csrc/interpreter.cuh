@@ -663,6 +663,19 @@ public:
     for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
     p.bias = p.mult = p.rshift = I.upload(bias_bits);
     p.OH = g.oh; p.OW = g.ow;
+    if (stem && out_cp <= 64 && g.kh * g.kw <= kStemMaxTaps && (g.kh - 1) * g.dh < 32768 && (g.kw - 1) * g.dw < 65536) {
+      p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
+      p.kh = g.kh; p.kw = g.kw;
+      p.M_total = rows;
+      p.n_valid = out_cp;
+      p.idesc = make_idesc_tf32(128, kStemPx);
+      pl.stem = true;
+      pl.stem_args = StemArgs{(const float4 *)in_->dev, (const uint8_t *)I.upload(pack_stem_weights_tf32(filt.data(), g)), g.ih, g.iw, g.kh * g.kw};
+      pl.grid = dim3((unsigned)std::min((rows + kStemPx - 1) / kStemPx, I.sm_count));
+      pl.smem = stem_smem(g.kh * g.kw);
+      plans_.push_back(pl);
+      return;
+    }
     int taps = 1, k_bytes;
     const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.pb == 0 && g.pr == 0;
     if (stem) {
@@ -825,8 +838,8 @@ public:
   }
   const TensorPtr &out() const { return out_; }
   const TensorPtr &in() const { return in_; }
-  // TF32 x 3 plans (not the patch-matrix stem, whose remainder belongs to the patch matrix)
-  bool is_tf32() const { return can_write_remainder() && !plans_[0].use_patch; }
+  // TF32 x 3 plans that read a remainder operand of their input tensor (stems form their own)
+  bool is_tf32() const { return can_write_remainder() && !plans_[0].use_patch && !plans_[0].stem; }
   bool can_write_remainder() const { return !plans_.empty() && plans_[0].tf32; }
   void set_remainder_out(void *lo) {
     for (auto &pl : plans_) {
