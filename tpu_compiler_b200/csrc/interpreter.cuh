@@ -1995,19 +1995,14 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     const int self = pos[0] > pos[1] ? 0 : 1, other = 1 - self;
     auto *cv = dynamic_cast<Conv2DOp *>(kernels[pos[self]].get());
     if (!cv || !cv->can_fuse_add() || !single_use(cv->name)) continue;
-    // By size: layers that widen their input, results of 2.5 to 8 MiB. There the launch that goes and the operand that is not
-    // read again count. Measured stage by stage on ResNet-50, all adds of one stage fused, us per step alone and with three
-    // modules in flight against none fused, by the stage's result:
-    //   below: 0.77 MiB +2 / +3 (res2, batch 1) and +7 / +14 (res4, batch 4), 1.5 MiB +2.7 / -1.5 and +2.2 / -7.7, 2.3 MiB
-    //   +3.7 / -10.7: a longer epilogue in launches that are nothing but latency;
-    //   inside: 3.06 MiB -1.9 / -4.7, +5.3 / -9.7 and +4.1 / -10.9, 4.2 -6.5 / -11.7, 6.1 -5.0 / -0.9 and +2.2 / -9.1, 7.3 -5.8 /
-    //   +0.6, 7.7 -4.5 / -3.3;
-    //   above: 8.4 -4.6 / +2.9, 9.2 -8.6 / +3.5 and -7.4 / +2.3, 12.3 -3.3 / +13, 24.5 +13 / +31, 98 +28 / -3: bound by the
-    //   epilogue's instructions, where the add by itself runs at the rate of memory.
-    // The window as a whole: batch 8 -6.9 / -3.5, 16 -0.3 / -14, 19 -14 / -13, 22 -7 / -14, 32 +4 / -21, 40 -8 / -14, 64 -1 / -3,
-    // nothing at 1, 96 and above. Layers with a long K and a short result gain alone and lose in flight (MobileNet-v2 batch
-    // 32: 394 -> 379 and 259 -> 266).
-    if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19 || cv->out()->bytes() > 8u << 20)) continue;
+    // By size: layers that widen their input, results of 2.5 MiB and more. The launch that goes and the operand that is not read
+    // again count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
+    // modules in flight, none fused -> by this rule: batch 8 331 / 166 -> 321 / 159, 16 404 / 232 -> 393 / 218, 19 419 / 257 -> 395 /
+    // 242, 24 445 / 300 -> 411 / 286, 32 515 / 362 -> 499 / 350, 48 606 / 495 -> 572 / 482, 64 741 / 626 -> 720 / 606, 96 946 / 905 ->
+    // 924 / 868, 128 1238 / 1176 -> 1221 / 1113, 256 2381 / 2271 -> 2314 / 2113. Smaller results gain too, a little (every add
+    // fused: batch 3 278 / 117 -> 272 / 109, 8 323 / 147). Layers with a long K and a short result gain alone and not in flight
+    // (MobileNet-v2 batch 32: 357 / 234 -> 336 / 234, 128: 860 / 712 -> 848 / 716).
+    if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19)) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
         r->padded_rows() || o->padded_rows() || a->cp % 4 != 0)
