@@ -159,11 +159,11 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          error status while the interpreter stays usable. With this option the INT8 convolutions of the next
  *          module never hand their accumulator back and wait only `rounds` rounds, so that exactly this happens.
  *          "fuse_residual_add" (0 never, 1 always, 2 = default: by size; read by the next load_module; needs fuse_activations): an INT8
- *          two-input eltwise add whose later-produced operand is a tensor-core convolution that feeds nothing else
+ *          two-input eltwise add (or a BF16 one with ReLU) whose later-produced operand is a tensor-core convolution that feeds nothing else
  *          (the last convolution of a residual block) runs in that convolution's epilogue, which reads the other
  *          operand and writes both the convolution's tensor and the sum; the add launches nothing. Same bits.
- *          By size: results of 2.5 to 8 MiB of layers that widen their input (INT8 ResNet-50 at batch 19:
- *          3% fewer us alone, 5% with three modules in flight; at batch 1 and 256 the add is faster by itself).
+ *          By size: results of 2.5 MiB and more of layers that widen their input (INT8 ResNet-50 at batch 19:
+ *          6% fewer us, at batch 256 3% alone and 7% with three modules in flight; BF16 at batch 128 3% and 12%).
  *          "fp32_tensor_cores" (0/1, default 1; read by the next load_module): fp32 convolutions with a
  *          multiple of 8 input channels run on the tensor cores as three TF32 products with fp32 accumulation
  *          (about 5e-6 of a tensor's range per layer against a double-accumulated sum, 6e-5 at the end of an

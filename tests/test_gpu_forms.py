@@ -326,3 +326,32 @@ def test_fp32_stem_patches(case, relu):
     got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
     # three products leave 2^-22 of each term; the tensor core cuts each of the 25 partial sums of a term at 2^-23 of the sum
     assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("case", [(13, 64, 256, 30, 1), (9, 64, 200, 21, 1), (3, 128, 144, 15, 1), (40, 16, 272, 13, 1), (64, 64, 256, 20, 2)])  # n, ic, oc, hw, mode
+def test_bf16_residual_add_with_prefetch(case):
+    """The BF16 add in the convolution's epilogue: several tiles per CTA, ragged tiles, channel tiles that some warps have no part
+    in, sums that overflow. Both tensors equal those of the add by itself."""
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, mode = case
+    rng = np.random.default_rng(oc)
+    shape = "shape=%d,%d,%d,%d dtype=BF16" % (n, oc, hw, hw)
+    text = ("input name=res %s\n" % shape + "input name=x shape=%d,%d,%d,%d dtype=BF16\n" % (n, ic, hw, hw) +
+            conv_text("BF16", n, ic, oc, hw, 1, 1, 0, 1, 0) + "eltwise_add name=s in=res,c %s do_relu=1\n" % shape)
+    w = {"f": graphs._bf16_np(rng.normal(0, 0.2, (oc, ic, 1, 1))), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+    x = {"x": graphs._bf16_np(rng.normal(0, 1, (n, ic, hw, hw))), "res": graphs._bf16_np(rng.normal(0, 1, (n, oc, hw, hw)) * 2.0 ** rng.integers(-20, 20, (n, oc, hw, hw)))}
+    x["x"][0, :, 0, 0] *= np.float32(2.0) ** 124  # sums past the largest finite value
+    x["res"][0, :, 0, 0] = 3.38e38
+    got = []
+    for fuse in (0, mode):
+        m = module(0)
+        m.set_option("fuse_residual_add", fuse)
+        m.load_text(text, w)
+        for name, v in x.items():
+            m.set_tensor(name, v)
+        for _ in range(2):
+            m.invoke()
+        got.append([m.get_tensor(k) for k in ("c", "s")] + [m.kernel_count()])
+        m.close()
+    assert got[1][2] == got[0][2] - 1
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])

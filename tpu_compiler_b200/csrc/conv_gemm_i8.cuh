@@ -727,6 +727,86 @@ __device__ __forceinline__ void epilogue_channels_bf16(const ConvGemmParams &p, 
   }
 }
 
+// The same with the BF16 eltwise add (two operands, ReLU) that consumes this convolution (core/eltwise.cpp:41-52): both tensors
+// are written. The sum of two BF16 values rounded once is what the reference's fp32 sum rounded to BF16 is: where the exponents
+// are so far apart that the fp32 sum is inexact, the smaller operand moves neither. Residual words a chunk ahead, as in
+// epilogue_add_fq. `left`: pixels in range from this lane's first one (0: the lane has no channels).
+__device__ __forceinline__ void fetch_residual16(uint4 (&y)[4], const uint8_t *res, int left, int pitch) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (8 * i < left)
+      asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(y[i].x), "=r"(y[i].y), "=r"(y[i].z), "=r"(y[i].w) : "l"(px_addr(res, 8 * i, pitch)));
+}
+__device__ __forceinline__ uint32_t add_relu_bf16x2(uint32_t x, uint32_t y, uint32_t &odd) {
+  uint32_t s;
+  asm("fma.rn.relu.bf16x2 %0, %1, %2, %3;" : "=r"(s) : "r"(x), "r"(0x3f803f80u), "r"(y));
+  asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(odd) : "r"(s), "r"(0u));
+  return s;
+}
+__device__ __forceinline__ uint32_t add_relu_bf16x2_rule(uint32_t x, uint32_t y) {
+  float lo = __fadd_rn(bits_f32(x << 16), bits_f32(y << 16)), hi = __fadd_rn(bits_f32(x & 0xffff0000u), bits_f32(y & 0xffff0000u));
+  lo = lo > 0.0f ? lo : 0.0f;
+  hi = hi > 0.0f ? hi : 0.0f;
+  return (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+}
+__device__ __forceinline__ void epilogue_add_bf16(const ConvGemmParams &p, uint32_t lane_addr, uint8_t *out8, int left, int half,
+                                                  unsigned long long bias2, const StageLane &st, int cols, uint4 (&y)[4], const uint8_t *next,
+                                                  int next_left) {
+  const int col0 = half * 32, col1 = col0 + 64;
+  const unsigned long long to_sum = (unsigned long long)(p.out2 - p.out);
+  auto chunk = [&](int colg, const uint4 (&res)[4]) {
+    const unsigned long long o = px_addr(out8, colg, p.ldc);
+    // sixteen pixels at a time: with all 32 accumulators of the chunk beside the residual words of two, registers spilled
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      uint32_t acc[16], w[8], odd = 0u;
+      ptx::tcgen05_ld_x16(lane_addr + (uint32_t)(colg + 16 * part), acc);
+      ptx::tcgen05_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        unsigned long long v = pack_b32x2(acc[2 * j], acc[2 * j + 1]);
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(bias2));
+        w[j] = bf16_pack_relu<false>(v, odd);
+      }
+      if (odd & 0x7fff7fffu) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = bf16_pack_rule<false>(acc[2 * j], acc[2 * j + 1], __uint_as_float((uint32_t)bias2));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(st.put + 512u * k), "r"(w[4 * k]),
+                     "r"(w[4 * k + 1]), "r"(w[4 * k + 2]), "r"(w[4 * k + 3]) : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        uint32_t v[4];
+        lds128(st.get + 512u * k, v);
+        const int i = 2 * part + k;
+        if (8 * i < left - colg) {
+          const unsigned long long at = px_addr((const void *)o, 8 * i, p.ldc);
+          asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+          const uint32_t r[4] = {res[i].x, res[i].y, res[i].z, res[i].w};
+          uint32_t s[4], far = 0u;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[j] = add_relu_bf16x2(v[j], r[j], far);
+          if (far & 0x7fff7fffu) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[j] = add_relu_bf16x2_rule(v[j], r[j]);
+          }
+          asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(at + to_sum), "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]) : "memory");
+        }
+      }
+    }
+  };
+  uint4 y1[4];
+  const uint8_t *res = reinterpret_cast<const uint8_t *>(p.res) + (out8 - reinterpret_cast<uint8_t *>(p.out));
+  if (col1 < cols) fetch_residual16(y1, res + (size_t)col1 * p.ldc, left - col1, p.ldc);
+  if (col0 < cols) chunk(col0, y);
+  fetch_residual16(y, next + (size_t)col0 * p.ldc, next_left - col0, p.ldc);
+  if (col1 < cols) chunk(col1, y1);
+}
+
 // Epilogue of an fp32 convolution computed as three TF32 products (calibration forward; core/conv.cpp:80-89): fp32
 // accumulator + fp32 bias, ReLU, stored as fp32. A lane owns a channel: for every pixel the warp writes 32 consecutive
 // channels (128 contiguous bytes). `out_ch` addresses (pixel m0, this lane's channel); `pitch` is the row pitch in bytes.
@@ -1088,6 +1168,14 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const int ch = n * p.BN + quarter * 32 + (lane & 3) * 8;
       return item < total_items && ch < p.n_valid ? p.res + (size_t)m * m_tile * p.ldc + p.c_off + ch : nullptr;
     };
+    uint4 res16[4]; // the same for the BF16 add; this lane's first pixel of tile (m, n) and the pixels in range from there
+    auto left_of = [&](int item, int m, int n) {
+      return item < total_items && n * p.BN + quarter * 32 + (lane & 3) * 8 < p.n_valid ? p.M_total - m * m_tile - st.px : 0;
+    };
+    auto res16_at = [&](int m, int n) {
+      return reinterpret_cast<const uint8_t *>(p.res) + ((size_t)m * m_tile + st.px) * p.ldc + (size_t)(n * p.BN + quarter * 32 + (lane & 3) * 8) * 2;
+    };
+    if constexpr (BF16 && ACTSEL == 3) fetch_residual16(res16, res16_at(tm, tn) + (size_t)(half * 32) * p.ldc, left_of(blockIdx.x, tm, tn) - half * 32, p.ldc);
     if constexpr (ACTSEL == 103) {
       const int8_t *r = residual_at(blockIdx.x, tm, tn);
       fetch_residual(res_words, r ? r + (size_t)(half * 32 + st.px) * p.ldc : nullptr, tm * m_tile + half * 32 + st.px, p);
@@ -1200,7 +1288,10 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         } else if (BF16) {
           // byte addressing: 2 bytes per channel
           uint8_t *out16 = reinterpret_cast<uint8_t *>(p.out) + out_m0 + (size_t)(p.c_off + ch8) * 2;
-          if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
+          if constexpr (ACTSEL == 3)
+            epilogue_add_bf16(p, lane_addr, out16 + (size_t)st.px * p.ldc, ch8_ok ? p.M_total - m0 - st.px : 0, half, bias2, st,
+                              min(ncols, p.M_total - m0), res16, res16_at(tm, tn), left_of(item + gridDim.x, tm, tn));
+          else if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
           else epilogue_channels_bf16<false>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
         } else if constexpr (ACTSEL == 103) {
           epilogue_add_fq(p, lane_addr, out8, ch8_ok, m0, half, fq, fshared, st, ncols, res_words,
@@ -1212,6 +1303,10 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         else if (p.act == 3) epilogue_channels_impl<3, FAST ? 1 : 0>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols);
         else if (FAST && (p.fastq & 2)) epilogue_channels_impl<0, FAST ? 2 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
         else epilogue_channels_impl<0, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
+      }
+      if constexpr (BF16 && ACTSEL == 3) {
+        if (n0 + ch_base >= p.n_valid)
+          fetch_residual16(res16, res16_at(tm, tn) + (size_t)(half * 32) * p.ldc, left_of(item + gridDim.x, tm, tn) - half * 32, p.ldc);
       }
       if constexpr (ACTSEL == 103) {
         if (n0 + ch_base >= p.n_valid) { // no outputs here: the next tile's residual all the same
@@ -1271,6 +1366,12 @@ __global__ void __launch_bounds__(kConvThreads, 2)
 conv_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const ConvGemmParams p) {
   conv_gemm_body<true, false>(tmA, tmB, p, tmA, tmB);
+}
+// ... with the residual add that consumes it (ConvGemmParams::act 3)
+__global__ void __launch_bounds__(kConvThreads, 2)
+conv_gemm_bf16_add_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                          const ConvGemmParams p) {
+  conv_gemm_body<true, false, false, false, 3>(tmA, tmB, p, tmA, tmB);
 }
 
 // fp32 convolution on the tensor cores as three TF32 products (see conv_gemm_body): tmA / tmA2 are the upper and

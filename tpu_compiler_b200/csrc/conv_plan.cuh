@@ -645,7 +645,8 @@ inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_cou
       launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
                reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
     launch_k(conv_gemm_tf32x3_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.p);
-  } else if (pl.bf16) launch_k(conv_gemm_bf16_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  } else if (pl.bf16 && pl.p.act == 3) launch_k(conv_gemm_bf16_add_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
+  else if (pl.bf16) launch_k(conv_gemm_bf16_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1 && (pl.p.fastq & 1)) launch_k(conv_gemm_i8_split_kernel<true>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.split_k > 1) launch_k(conv_gemm_i8_split_kernel<false>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
   else if (pl.p.fq && pl.p.act == 1) launch_k(conv_gemm_i8_fq_kernel<1>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
@@ -670,6 +671,7 @@ inline void conv_kernel_setup_once() {
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
+    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_bf16_add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
     TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));

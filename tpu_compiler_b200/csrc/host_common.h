@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <set>
 #include <memory>
 #include <stdexcept>
 #include <string>

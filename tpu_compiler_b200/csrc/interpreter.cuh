@@ -165,6 +165,7 @@ public:
     int cp = 0, wl = 0, wphys = 0;
   };
   std::map<std::string, RowLayout> layout_requests;
+  std::set<std::string> add_tails; // BF16 convolutions whose result goes to one residual add only (load_module): planned so that it can be fused
 
   TensorPtr make_tensor(const std::string &name, const std::vector<int64_t> &shape, int dtype) {
     auto t = std::make_shared<DevTensor>();
@@ -756,7 +757,7 @@ public:
     p.OH = g.oh; p.OW = g.ow; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
     p.kh = g.kh; p.kw = g.kw;
     if (wp) setup_window(I, pl, *wp, filt, kind);
-    else setup_blocks(I, pl, d, kind);
+    else setup_blocks(I, pl, d, kind, !I.add_tails.count(out_->name));
     I.attach_split_ws(pl);
     plans_.push_back(pl);
   }
@@ -789,14 +790,14 @@ public:
                       p.dual ? 192 : 128);
     encode_window_map(&pl.tmA, rows, g, wp, p.BK, p.m_tile);
   }
-  void setup_blocks(Interpreter &I, ConvPlan &pl, const DenseLayer &d, int kind) {
+  void setup_blocks(Interpreter &I, ConvPlan &pl, const DenseLayer &d, int kind, bool may_be_big) {
     const ConvGeom &g = d.g;
     ConvGemmParams &p = pl.p;
     const int es = kind == 0 ? 1 : 2, k_bytes = d.in_cp * es, rows = g.n * g.oh * g.ow;
     const bool one = g.kh == 1 && g.kw == 1 && g.sh == 1 && g.sw == 1 && g.pt == 0 && g.pl == 0 && g.oh == g.ih && g.ow == g.iw;
     const int taps = g.kh * g.kw;
     p.a_mode = one ? 0 : 1;
-    finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count, true);
+    finish_plan(pl, rows, taps, k_bytes, d.out_cp, I.sm_count, may_be_big);
     if (one) encode_matrix_map(&pl.tmA, (const int8_t *)in_->dev, rows, k_bytes, k_bytes, p.BK, pl.box_px());
     else encode_im2col_map(&pl.tmA, (const int8_t *)in_->dev, g, k_bytes, p.BK, pl.box_px());
     encode_out_maps(pl);
@@ -824,7 +825,7 @@ public:
   // Fused eltwise add (tensor-core INT8 plans without an activation of their own): the epilogue also forms
   // sat8(relu?((conv * ms + residual * mr + 2^(r-1)) >> r)) into `sum_out`; this op's own tensor is still written.
   bool can_fuse_add() const {
-    return can_fuse_leaky() && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1 && !plans_[0].p.dual && plans_[0].ctas == 0;
+    return !(f32_ || dw_ || bf16g_ || act_ != 0 || plans_.empty()) && (in_->dtype == DT_I8 || plans_[0].bf16) && plans_.size() == 1 && plans_[0].p.split_k <= 1 && plans_[0].p.group <= 1 && !plans_[0].p.dual && plans_[0].ctas == 0;
   }
   void set_residual_add(const int8_t *residual, int8_t *sum_out, int ms, int mr, int rshift, int relu) {
     for (auto &pl : plans_) {
@@ -834,7 +835,7 @@ public:
       pl.p.add_ms = ms; pl.p.add_mr = mr; pl.p.add_r = rshift; pl.p.add_relu = relu;
     }
     act_ = 3;
-    alg_bytes += 2.0 * out_->numel(); // the residual read and the sum written
+    alg_bytes += 2.0 * out_->numel() * out_->elsize(); // the residual read and the sum written
   }
   const TensorPtr &out() const { return out_; }
   const TensorPtr &in() const { return in_; }
@@ -1223,8 +1224,11 @@ public:
       parse_coeff(op, f_.coeff, nin);
     }
   }
-  // INT8 two-input add that a producing convolution's epilogue can take over
-  bool is_plain_i8_add() const { return out_->dtype == DT_I8 && !is_mul_ && ins_.size() == 2; }
+  // two-input add that a producing convolution's epilogue can take over
+  bool is_plain_add() const {
+    return !is_mul_ && ins_.size() == 2 &&
+           (out_->dtype == DT_I8 || (out_->dtype == DT_BF16 && do_relu_ && b_.coeff[0] == 1.0f && b_.coeff[1] == 1.0f));
+  }
   // fp32 add whose result feeds a TF32 x 3 convolution: also write that convolution's remainder operand
   bool can_write_remainder() const { return out_->dtype == DT_F32 && !is_mul_; }
   void set_remainder_out(float *lo) { f_.lo = lo; }
@@ -1984,7 +1988,7 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
   // (EltwiseAddOpKernel::i8_invoke, core/eltwise.cpp:52-85, on top of Conv2DOpKernel::invoke, core/conv.cpp:80-104).
   for (size_t j = 0; j < n && fuse_residual_add; ++j) {
     auto *ad = dynamic_cast<EltwiseOp *>(kernels[j].get());
-    if (!ad || !ad->is_plain_i8_add()) continue;
+    if (!ad || !ad->is_plain_add()) continue;
     const auto &ins = ad->inputs();
     // the producers' positions; the later one must be the convolution
     int pos[2] = {-1, -1};
@@ -2002,13 +2006,18 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     // 924 / 868, 128 1238 / 1176 -> 1221 / 1113, 256 2381 / 2271 -> 2314 / 2113. Smaller results gain too, a little (every add
     // fused: batch 3 278 / 117 -> 272 / 109, 8 323 / 147). Layers with a long K and a short result gain alone and not in flight
     // (MobileNet-v2 batch 32: 357 / 234 -> 336 / 234, 128: 860 / 712 -> 848 / 716).
+    // BF16 (two operands, ReLU): batch 8 498 / 233 -> 488 / 215, 32 804 / 604 -> 802 / 542, 128 2234 / 2117 -> 2157 / 1866.
     if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19)) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
         r->padded_rows() || o->padded_rows() || a->cp % 4 != 0)
       continue;
-    const EltwiseArgs &ea = ad->i8_args();
-    cv->set_residual_add((const int8_t *)r->dev, (int8_t *)o->dev, ea.mult[self], ea.mult[other], ea.rshift, ea.do_relu);
+    if (a->dtype == DT_BF16) {
+      cv->set_residual_add((const int8_t *)r->dev, (int8_t *)o->dev, 1, 1, 0, 1);
+    } else {
+      const EltwiseArgs &ea = ad->i8_args();
+      cv->set_residual_add((const int8_t *)r->dev, (int8_t *)o->dev, ea.mult[self], ea.mult[other], ea.rshift, ea.do_relu);
+    }
     std::unique_ptr<OpKernel> away(new FusedAwayOp());
     away->name = ad->name; away->op_type = ad->op_type; away->shape = ad->shape; away->datatype = ad->datatype;
     away->result = ad->result; away->line = ad->line; away->dirty = ad->dirty;
@@ -2266,12 +2275,22 @@ inline void Interpreter::load_module(const std::string &text) {
   // Pre-pass: a few-channel convolution whose input is produced by an input or quant op and has no
   // other consumer asks for that tensor to be stored in its window layout (WindowPlan).
   layout_requests.clear();
+  add_tails.clear();
   {
     std::map<std::string, const ParsedOp *> by_name;
     std::map<std::string, int> n_uses;
     for (auto &op : parsed) {
       by_name[op.name] = &op;
       for (auto &nm : op.in) n_uses[nm]++;
+    }
+    for (auto &op : parsed) {
+      if (!fuse_activations || !fuse_residual_add || op.type != "eltwise_add" || op.dtype != "BF16" || op.in.size() < 2) continue;
+      const ParsedOp *late = nullptr;
+      for (int k = 0; k < 2; ++k) {
+        auto it = by_name.find(op.in[k]);
+        if (it != by_name.end() && (!late || it->second > late)) late = it->second;
+      }
+      if (late && late->type == "conv_2d" && n_uses[late->name] == 1) add_tails.insert(late->name);
     }
     for (auto &op : parsed) {
       if (op.type != "conv_2d" || (op.dtype != "INT8" && op.dtype != "BF16") || op.in.empty()) continue;
