@@ -1512,7 +1512,8 @@ public:
   ActChainOp(Interpreter &I, const QuantOp &q0, const LutOp &lut, const QuantOp &q1)
       : I_(I), in_(q0.in()), deq_(q0.out()), act_(lut.out()), out_(q1.out()) {
     alg_bytes = 6.0 * out_->numel();
-    table_ = (uint2 *)I.dalloc(256 * sizeof(uint2));
+    table_ = (uint32_t *)I.dalloc(256 * sizeof(uint32_t));
+    scale_ = bf16_round(q0.scale());
     act_table_kernel<<<1, 256, 0, I.stream>>>(table_, q0.scale(), lut.scale(), lut.base_table(), lut.slope_table(), q1.scale());
     TPUCB_CUDA(cudaGetLastError());
   }
@@ -1521,13 +1522,14 @@ public:
     const int grid = (int)std::min<size_t>((nvec + 255) / 256, (size_t)I_.sm_count * 8);
     PdlConvScope pdl; // stands behind a convolution: its table is in place when the convolution ends
     launch_k(act_chain_i8_kernel, grid, 256, 0, s, (const uint2 *)in_->dev, (uint4 *)deq_->dev, (uint4 *)act_->dev,
-             (uint2 *)out_->dev, nvec, table_);
+             (uint2 *)out_->dev, nvec, table_, scale_);
   }
 
 private:
   Interpreter &I_;
   TensorPtr in_, deq_, act_, out_;
-  uint2 *table_ = nullptr;
+  uint32_t *table_ = nullptr;
+  float scale_ = 0;
 };
 
 class FusedAwayOp : public OpKernel {
@@ -2025,7 +2027,8 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
   }
   for (size_t i = 0; i < n; ++i) {
     auto *q0 = dynamic_cast<QuantOp *>(kernels[i].get());
-    if (!q0 || q0->kind() != 3 || !single_use(q0->name)) continue;
+    // (a scale whose products could leave the finite BF16 values keeps the ops by themselves: the pass rounds without that check)
+    if (!q0 || q0->kind() != 3 || !single_use(q0->name) || !(std::fabs(q0->scale()) < 1e30f)) continue;
     size_t j = n, k = n;
     for (size_t t = i + 1; t < n && j == n; ++t) {
       auto *l = dynamic_cast<LutOp *>(kernels[t].get());

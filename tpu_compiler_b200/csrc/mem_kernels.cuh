@@ -1166,9 +1166,10 @@ __global__ void lut_bf16_slope_kernel(const uint16_t *__restrict__ in, uint16_t 
 
 // The chain the reference's mixed-precision graphs use around a BF16 activation,
 //   quant INT8->BF16  ->  slope-table activation (BF16)  ->  quant BF16->INT8,
-// as one lookup: its three results are functions of one byte. act_table_kernel forms them for all 256 bytes when the module
-// is loaded, with the arithmetic of the three ops; an entry is (BF16 dequantised | BF16 activation << 16, int8 result).
-__global__ void act_table_kernel(uint2 *__restrict__ table, float scale_in, float lut_scale, const float *__restrict__ base,
+// in one pass. The last two results are functions of one byte, looked up: act_table_kernel forms them for all 256 bytes when
+// the module is loaded, with the arithmetic of the ops; an entry is BF16 activation | int8 result << 16. The first is one
+// multiplication and one rounding.
+__global__ void act_table_kernel(uint32_t *__restrict__ table, float scale_in, float lut_scale, const float *__restrict__ base,
                                  const float *__restrict__ slope, float scale_out) {
   __shared__ float2 s_t[256];
   const int i = threadIdx.x;
@@ -1177,33 +1178,48 @@ __global__ void act_table_kernel(uint2 *__restrict__ table, float scale_in, floa
   uint32_t d0, d1;
   dequant_word_bf16((uint32_t)i, bf16_round(scale_in), d0, d1);
   const uint32_t a = lut_slope_pair(d0, lut_scale, s_t);
-  table[i] = make_uint2((d0 & 0xffffu) | (a << 16), quant_bf16x4_to_i8(a, a, bf16_round(scale_out)) & 0xffu);
+  table[i] = (a & 0xffffu) | (quant_bf16x4_to_i8(a, a, bf16_round(scale_out)) & 0xffu) << 16;
 }
-// The pass: 1 byte read and 5 written per value, all three tensors stay fetchable. The arithmetic took 23 instructions per
-// value and kept it at 3.3 TB/s; a value is now one 8-byte shared-memory read and four instructions (4.5 to 4.9 TB/s, 8 x 64
-// x 208 x 208: 41 -> 30 us). The table does not depend on the kernel before, so it is filled while that one ends, and the
-// launch carries the programmatic mark: a detector's batch of one went from 1387 to 1153 us, of eight from 2165 to 1863.
-// Two copies side by side, for odd and even lanes, halve the lanes that meet in a bank; more copies cost more to fill than
-// they gave (one 1947, two 1913, four 1919, sixteen 1950 us at a batch of eight, without the mark). Eight values per
-// thread and step: every access of a warp is one contiguous run.
+// The pass: 1 byte read and 5 written per value, all three tensors stay fetchable. The table does not depend on the kernel
+// before, so it is filled while that one ends, and the launch carries the programmatic mark. What bounds it beside memory are
+// the lanes of a warp that meet in a bank: entries of four bytes, four copies side by side, one for every fourth lane (entries of
+// eight bytes with the dequantised value in them, two copies, 8 x 64 x 208 x 208: 30 us, now 26.7, 5.0 TB/s; YOLOv4-style batch 8
+// 1507 -> 1475 us). Eight values per thread and step: every access of a
+// warp is one contiguous run.
 __global__ void __launch_bounds__(256) act_chain_i8_kernel(const uint2 *__restrict__ in, uint4 *__restrict__ deq, uint4 *__restrict__ act,
-                                                           uint2 *__restrict__ out, size_t nvec, const uint2 *__restrict__ table) {
+                                                           uint2 *__restrict__ out, size_t nvec, const uint32_t *__restrict__ table,
+                                                           float scale) {
   pdl_trigger();
-  __shared__ __align__(16) uint2 s_t[256 * 2];
-  const uint2 e = __ldg(table + threadIdx.x);
-  reinterpret_cast<uint4 *>(s_t)[threadIdx.x] = make_uint4(e.x, e.y, e.x, e.y);
+  __shared__ __align__(16) uint32_t s_t[256 * 4];
+  const uint32_t e = __ldg(table + threadIdx.x);
+  reinterpret_cast<uint4 *>(s_t)[threadIdx.x] = make_uint4(e, e, e, e);
   pdl_wait();
   __syncthreads();
-  const uint32_t lane_off = (threadIdx.x & 1u) * 8u;
+  const uint32_t lane_off = (threadIdx.x & 3u) * 4u;
   const uint8_t *t = reinterpret_cast<const uint8_t *>(s_t);
+  const unsigned long long sb = hold_pair(scale), off = hold_pair(-8388736.0f); // -(2^23 + 128)
+  // BF16 of two bytes' values times the scale: b ^ 0x80 in the low byte of 2^23 is 2^23 + 128 + b
+  auto deq2 = [&](uint32_t x, int j) {
+    unsigned long long f = pack_b32x2(__byte_perm(x, 0x4B000000u, 0x7650u | j), __byte_perm(x, 0x4B000000u, 0x7651u | j));
+    float lo, hi;
+    uint32_t d;
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(off));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(sb));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(f));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+  };
   auto word = [&](uint32_t w, uint32_t &d0, uint32_t &d1, uint32_t &a0, uint32_t &a1) { // four values
-    const uint2 e0 = *reinterpret_cast<const uint2 *>(t + ((w & 0xffu) * 16u + lane_off));
-    const uint2 e1 = *reinterpret_cast<const uint2 *>(t + (((w >> 8) & 0xffu) * 16u + lane_off));
-    const uint2 e2 = *reinterpret_cast<const uint2 *>(t + (((w >> 16) & 0xffu) * 16u + lane_off));
-    const uint2 e3 = *reinterpret_cast<const uint2 *>(t + ((w >> 24) * 16u + lane_off));
-    d0 = __byte_perm(e0.x, e1.x, 0x5410); a0 = __byte_perm(e0.x, e1.x, 0x7632);
-    d1 = __byte_perm(e2.x, e3.x, 0x5410); a1 = __byte_perm(e2.x, e3.x, 0x7632);
-    return __byte_perm(__byte_perm(e0.y, e1.y, 0x0040), __byte_perm(e2.y, e3.y, 0x0040), 0x5410);
+    const uint32_t e0 = *reinterpret_cast<const uint32_t *>(t + (((w << 4) & 0xff0u) | lane_off));
+    const uint32_t e1 = *reinterpret_cast<const uint32_t *>(t + (((w >> 4) & 0xff0u) | lane_off));
+    const uint32_t e2 = *reinterpret_cast<const uint32_t *>(t + (((w >> 12) & 0xff0u) | lane_off));
+    const uint32_t e3 = *reinterpret_cast<const uint32_t *>(t + (((w >> 20) & 0xff0u) | lane_off));
+    const uint32_t x = w ^ 0x80808080u;
+    d0 = deq2(x, 0);
+    d1 = deq2(x, 2);
+    a0 = __byte_perm(e0, e1, 0x5410);
+    a1 = __byte_perm(e2, e3, 0x5410);
+    return __byte_perm(__byte_perm(e0, e1, 0x0062), __byte_perm(e2, e3, 0x0062), 0x5410);
   };
   auto put = [&](size_t i, const uint2 &v) {
     uint4 d, a;
