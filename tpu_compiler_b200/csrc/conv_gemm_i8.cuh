@@ -609,53 +609,80 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
   }
 }
 
-// The same with the fused eltwise add and the floating-point requantisation, for the two 32-pixel chunks of a warp. The
-// residual words come from memory: those of the first chunk were fetched during the tile before (`y`), those of the second
-// are fetched while the first is worked on, and then those of the next tile's first chunk, whose residual begins at `next`
-// (pixel next_m0, this lane's group of eight channels; null: none).
-// Fetched where they are needed, they cost a memory latency per chunk (batch 256 with every add fused: 190 us more than
-// without; prefetched, 30 to 100).
-// `res`: this lane's first pixel of the chunk, whose number is `first`
-__device__ __forceinline__ void fetch_residual(uint2 (&y)[4], const int8_t *res, int first, const ConvGemmParams &p) {
-  if (!res) return;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (first + stage_step8(i) < p.M_total)
-      asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(y[i].x), "=r"(y[i].y) : "l"(px_addr(res, stage_step8(i), p.ldc)));
+// The same with the fused eltwise add and the floating-point requantisation, for the two 32-pixel chunks of a warp. With three
+// tensors in every chunk the accesses to memory count: the four warps that hold the channels of the same pixels exchange their
+// results through shared memory, and each handles 8 pixels x 128 channels, 16 bytes a lane, four pixels per access (of its own 32
+// channels it was 8 bytes a lane and 8 pixels, twice the accesses of twice the lines each, and the
+// load/store pipe 60% busy: ResNet-50 batch 256 2336 us against 2210, with three modules in flight 2127 / 2003, batch 64 605 / 573).
+// The residual words are fetched a chunk ahead, across tiles: those of the first chunk during the tile before (`y`), those of the
+// second while the first is worked on. Fetched where they are needed, they cost a memory latency per chunk.
+struct AddLane {
+  uint32_t put, get; // this lane's row of its warp's matrix stores; its 8 channels in the exchange, the next 8 are 32 bytes on
+  int px, ch;        // its first pixel of a chunk (the second is 4 on) and its first channel of a tile
+};
+constexpr int kAddQuarter = kStageBytes + 32; // 32 bytes more: a lane group's eight accesses meet in a bank two by two, not four by four
+__device__ __forceinline__ AddLane make_add_lane(uint32_t stage, int half, int quarter, int lane) {
+  const uint32_t at = stage + (uint32_t)(half * 4 * kAddQuarter);
+  const int c16 = lane & 7, h = (lane >> 3) & 1, pos = lane >> 4;
+  return AddLane{at + (uint32_t)(quarter * kAddQuarter + lane * 16),
+                 at + (uint32_t)((c16 >> 1) * kAddQuarter + (quarter >> 1) * 512 + (quarter & 1) * 256 + (4 * (c16 & 1) + h) * 16 + pos * 8),
+                 8 * quarter + (lane >> 3), 16 * c16};
 }
-__device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out8, bool ch8_ok, int m0, int half,
-                                                const FloatRequantPairs<false> &q, const FloatRequantShared &fs, const StageLane &st, int ncols, uint2 (&y)[4],
-                                                const int8_t *next, int next_m0) {
+// `at`: this lane's first pixel of the chunk; left: pixels in range from there (0: the lane has no channels)
+__device__ __forceinline__ void fetch_residual(uint4 (&y)[2], const int8_t *at, int left, int pitch) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (4 * i < left)
+      asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(y[i].x), "=r"(y[i].y), "=r"(y[i].z), "=r"(y[i].w) : "l"(px_addr(at, 4 * i, pitch)));
+}
+// out16: this lane's first pixel of the tile; mine: the warp's accumulators hold channels of the layer
+__device__ __forceinline__ void epilogue_add_fq(const ConvGemmParams &p, uint32_t lane_addr, int8_t *out16, int left, bool mine, int m0, int half,
+                                                const FloatRequantPairs<false> &q, const FloatRequantShared &fs, const AddLane &al, int ncols,
+                                                uint4 (&y)[2], const int8_t *next, int next_left) {
   const int col0 = half * 32, col1 = col0 + 64;
   const AddConsts ac = make_add_consts(p);
-  const int left = ch8_ok ? p.M_total - m0 - st.px : 0; // pixels in range from this lane's first one of the tile
   const unsigned long long to_sum = (unsigned long long)(p.out2 - p.out);
-  auto chunk = [&](int colg, const uint2 (&res)[4]) {
-    uint32_t acc0[16], acc1[16];
-    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
-    ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
-    ptx::tcgen05_wait_ld();
-    uint32_t w[8], u[8];
+  auto meet = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); };
+  auto chunk = [&](int colg, const uint4 (&res)[2]) {
+    uint32_t w[8];
+    if (mine) {
+      uint32_t acc0[16], acc1[16];
+      ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg, acc0);
+      ptx::tcgen05_ld_x16(lane_addr + (uint32_t)colg + 16u, acc1);
+      ptx::tcgen05_wait_ld();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q, fs);
-      w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q, fs);
-    }
-    transpose_i8(w, u, st);
-    const unsigned long long o = px_addr(out8, colg + st.px, p.ldc);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (stage_step8(i) < left - colg) {
-        const unsigned long long at = px_addr((const void *)o, stage_step8(i), p.ldc);
-        stg64(at, u[2 * i], u[2 * i + 1]);
-        stg64(at + to_sum, add4_packed(u[2 * i], res[i].x, ac), add4_packed(u[2 * i + 1], res[i].y, ac));
+      for (int k = 0; k < 4; ++k) {
+        w[k] = float_requant4<false>(acc0[4 * k + 0], acc0[4 * k + 1], acc0[4 * k + 2], acc0[4 * k + 3], q, fs);
+        w[4 + k] = float_requant4<false>(acc1[4 * k + 0], acc1[4 * k + 1], acc1[4 * k + 2], acc1[4 * k + 3], q, fs);
       }
+    }
+    meet(); // the chunk before has been read
+    if (mine) {
+      asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};" ::"r"(al.put), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                   "r"(w[3]) : "memory");
+      asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};" ::"r"(al.put + 512u), "r"(w[4]), "r"(w[5]),
+                   "r"(w[6]), "r"(w[7]) : "memory");
+    }
+    meet();
+    const unsigned long long o = px_addr(out16, colg, p.ldc);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t u[4];
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(u[0]), "=r"(u[1]) : "r"(al.get + 128u * i) : "memory");
+      asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(u[2]), "=r"(u[3]) : "r"(al.get + 128u * i + 32u) : "memory");
+      if (4 * i < left - colg) {
+        const unsigned long long at = px_addr((const void *)o, 4 * i, p.ldc);
+        asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(at), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
+        asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(at + to_sum), "r"(add4_packed(u[0], res[i].x, ac)),
+                     "r"(add4_packed(u[1], res[i].y, ac)), "r"(add4_packed(u[2], res[i].z, ac)), "r"(add4_packed(u[3], res[i].w, ac)) : "memory");
+      }
+    }
   };
+  uint4 y1[2];
   const bool two = col1 < ncols && m0 + col1 < p.M_total;
-  uint2 y1[4];
-  if (two) fetch_residual(y1, ch8_ok ? p.res + (out8 - p.out) + (size_t)(col1 + st.px) * p.ldc : nullptr, m0 + col1 + st.px, p);
+  if (two) fetch_residual(y1, p.res + (out16 - p.out) + (size_t)col1 * p.ldc, left - col1, p.ldc);
   if (col0 < ncols && m0 + col0 < p.M_total) chunk(col0, y);
-  fetch_residual(y, next ? next + (size_t)(col0 + st.px) * p.ldc : nullptr, next_m0 + col0 + st.px, p);
+  fetch_residual(y, next + (size_t)col0 * p.ldc, next_left - col0, p.ldc);
   if (two) chunk(col1, y1);
 }
 
@@ -1162,12 +1189,14 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     int t = 0;
     bool ok = true;
     int tm = walk_m0, tn = walk_n0;
-    // fused add: the residual of a tile (tm, tn), counted from this lane's group of eight channels; null where it has none
-    uint2 res_words[4];
-    auto residual_at = [&](int item, int m, int n) -> const int8_t * {
-      const int ch = n * p.BN + quarter * 32 + (lane & 3) * 8;
-      return item < total_items && ch < p.n_valid ? p.res + (size_t)m * m_tile * p.ldc + p.c_off + ch : nullptr;
+    // fused add (INT8): this lane's first pixel of tile (m, n) in the residual, and the pixels in range from there
+    uint4 res_words[2];
+    const AddLane al = make_add_lane(base + 256u, half, quarter, lane);
+    auto residual_at = [&](int m, int n) { return p.res + ((size_t)m * m_tile + al.px) * p.ldc + p.c_off + n * p.BN + al.ch; };
+    auto residual_left = [&](int item, int m, int n) {
+      return item < total_items && n * p.BN + al.ch < p.n_valid ? p.M_total - m * m_tile - al.px : 0;
     };
+    bool live = true; // INT8 add: false once a wait has run out; the warp then does no work but comes to every barrier
     uint4 res16[4]; // the same for the BF16 add; this lane's first pixel of tile (m, n) and the pixels in range from there
     auto left_of = [&](int item, int m, int n) {
       return item < total_items && n * p.BN + quarter * 32 + (lane & 3) * 8 < p.n_valid ? p.M_total - m * m_tile - st.px : 0;
@@ -1177,8 +1206,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
     };
     if constexpr (BF16 && ACTSEL == 3) fetch_residual16(res16, res16_at(tm, tn) + (size_t)(half * 32) * p.ldc, left_of(blockIdx.x, tm, tn) - half * 32, p.ldc);
     if constexpr (ACTSEL == 103) {
-      const int8_t *r = residual_at(blockIdx.x, tm, tn);
-      fetch_residual(res_words, r ? r + (size_t)(half * 32 + st.px) * p.ldc : nullptr, tm * m_tile + half * 32 + st.px, p);
+      fetch_residual(res_words, residual_at(tm, tn) + (size_t)(half * 32) * p.ldc, residual_left(blockIdx.x, tm, tn) - half * 32, p.ldc);
     }
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x, ++t) {
       int tile = item;
@@ -1213,13 +1241,17 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         }
         staged_n0 = n0;
       }
-      ok = ptx::mbar_wait_bounded(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds);
+      ok = live && ptx::mbar_wait_bounded(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds);
       if (!ok && !*abort_flag) {
         report_error(p.err, kErrAccWait);
         *abort_flag = 1;
       }
       // the wait result may differ between lanes only on the error path; make it uniform
       ok = __all_sync(0xffffffffu, ok);
+      if constexpr (ACTSEL == 103) {
+        live = ok;
+        ok = true;
+      }
       const bool split_item = SPLIT && split_k > 1;
       if (!ok && !split_item) break; // (a split item still passes its two barriers, see below)
       ptx::tcgen05_fence_after();
@@ -1274,7 +1306,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         if (verdict == 0) continue;
         __threadfence();
       }
-      if (n0 + ch_base < p.n_valid && m0 < p.M_total) { // warp-uniform: this lane quarter holds real outputs
+      if ((ACTSEL == 103 || n0 + ch_base < p.n_valid) && m0 < p.M_total) { // warp-uniform: this lane quarter holds real outputs
         const uint32_t lane_addr = tmem_base + (uint32_t)buf * acc_stride + ((uint32_t)(quarter * 32) << 16);
         const size_t out_m0 = (size_t)m0 * p.ldc + (p.group > 1 ? (quarter * 32 * p.group >> 7) * p.ldc_px : 0); // bytes
         int8_t *out8 = p.out + out_m0 + p.c_off + ch8;
@@ -1294,8 +1326,9 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           else if (p.act == 1) epilogue_channels_bf16<true>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
           else epilogue_channels_bf16<false>(p, lane_addr, out16, ch8_ok, m0, half, kEpilogueWarps / 4, bias2, st, ncols);
         } else if constexpr (ACTSEL == 103) {
-          epilogue_add_fq(p, lane_addr, out8, ch8_ok, m0, half, fq, fshared, st, ncols, res_words,
-                          residual_at(item + gridDim.x, tm, tn), tm * m_tile);
+          epilogue_add_fq(p, lane_addr, p.out + (size_t)(m0 + al.px) * p.ldc + p.c_off + n0 + al.ch,
+                          live && n0 + al.ch < p.n_valid ? p.M_total - m0 - al.px : 0, live && n0 + ch_base < p.n_valid, m0, half, fq, fshared, al,
+                          ncols, res_words, residual_at(tm, tn), residual_left(item + gridDim.x, tm, tn));
         } else if constexpr (FQ) {
           epilogue_channels_impl<ACTSEL - 100, 3>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, fq, fshared, st, ncols);
         } else if (p.act == 1) epilogue_channels_impl<1, FAST ? 1 : 0, SPLIT>(p, lane_addr, out8, ch8_ok, m0, half, kEpilogueWarps / 4, lane, cc, fshared, st, ncols, ws_lane);
@@ -1307,12 +1340,6 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       if constexpr (BF16 && ACTSEL == 3) {
         if (n0 + ch_base >= p.n_valid)
           fetch_residual16(res16, res16_at(tm, tn) + (size_t)(half * 32) * p.ldc, left_of(item + gridDim.x, tm, tn) - half * 32, p.ldc);
-      }
-      if constexpr (ACTSEL == 103) {
-        if (n0 + ch_base >= p.n_valid) { // no outputs here: the next tile's residual all the same
-          const int8_t *r = residual_at(item + gridDim.x, tm, tn);
-          fetch_residual(res_words, r ? r + (size_t)(half * 32 + st.px) * p.ldc : nullptr, tm * m_tile + half * 32 + st.px, p);
-        }
       }
       if (SPLIT && ws_lane) continue; // split K: the accumulator buffer was handed back above
       // hand the accumulator buffer back to the MMA issuer

@@ -2003,16 +2003,16 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     if (!cv || !cv->can_fuse_add() || !single_use(cv->name)) continue;
     // By size: layers that widen their input, results of 2.5 MiB and more. The launch that goes and the operand that is not read
     // again count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
-    // modules in flight, none fused -> by this rule: batch 8 331 / 166 -> 321 / 159, 16 404 / 232 -> 393 / 218, 19 419 / 257 -> 395 /
-    // 242, 24 445 / 300 -> 411 / 286, 32 515 / 362 -> 499 / 350, 48 606 / 495 -> 572 / 482, 64 741 / 626 -> 720 / 606, 96 946 / 905 ->
-    // 924 / 868, 128 1238 / 1176 -> 1221 / 1113, 256 2381 / 2271 -> 2314 / 2113. Smaller results gain too, a little (every add
-    // fused: batch 3 278 / 117 -> 272 / 109, 8 323 / 147). Layers with a long K and a short result gain alone and not in flight
-    // (MobileNet-v2 batch 32: 357 / 234 -> 336 / 234, 128: 860 / 712 -> 848 / 716).
-    // BF16 (two operands, ReLU): batch 8 498 / 233 -> 488 / 215, 32 804 / 604 -> 802 / 542, 128 2234 / 2117 -> 2157 / 1866.
-    if (fuse_residual_add == 2 && (cv->out()->cp <= cv->in()->cp || cv->out()->bytes() < 5u << 19)) continue;
+    // modules in flight, none fused -> by this rule: INT8 batch 8 332 / 166 -> 319 / 158, 19 421 / 257 -> 393 / 236, 64 740 / 627 ->
+    // 693 / 573, 256 2423 / 2280 -> 2210 / 2011; smaller results gain too, a little (every add fused: batch 3 278 / 117 -> 272 /
+    // 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 498 / 233 -> 488 / 215, 32 804 / 604 -> 802 / 542, 128 2234 / 2117 ->
+    // 2157 / 1866. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
+    // fused: batch 1 182 / 65 -> 167 / 62, 7 217 / 104 -> 203 / 103, 32 357 / 235 -> 338 / 234, but 128 864 / 713 -> 851 / 719).
+    const bool widens = cv->out()->cp > cv->in()->cp;
+    if (fuse_residual_add == 2 && (widens ? cv->out()->bytes() < 5u << 19 : cv->out()->bytes() > 4u << 20)) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
-        r->padded_rows() || o->padded_rows() || a->cp % 4 != 0)
+        r->padded_rows() || o->padded_rows() || a->cp % 16 != 0)
       continue;
     if (a->dtype == DT_BF16) {
       cv->set_residual_add((const int8_t *)r->dev, (int8_t *)o->dev, 1, 1, 0, 1);
