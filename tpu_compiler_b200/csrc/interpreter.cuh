@@ -2005,8 +2005,8 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     // again count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
     // modules in flight, none fused -> by this rule: INT8 batch 8 332 / 166 -> 319 / 158, 19 421 / 257 -> 393 / 236, 64 740 / 627 ->
     // 693 / 573, 256 2423 / 2280 -> 2210 / 2011; smaller results gain too, a little (every add fused: batch 3 278 / 117 -> 272 /
-    // 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 498 / 233 -> 488 / 215, 32 804 / 604 -> 802 / 542, 128 2234 / 2117 ->
-    // 2157 / 1866. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
+    // 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 499 / 233 -> 486 / 213, 32 803 / 602 -> 776 / 525, 128 2231 / 2174 ->
+    // 2088 / 1791. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
     // fused: batch 1 182 / 65 -> 167 / 62, 7 217 / 104 -> 203 / 103, 32 357 / 235 -> 338 / 234, but 128 864 / 713 -> 851 / 719).
     const bool widens = cv->out()->cp > cv->in()->cp;
     if (fuse_residual_add == 2 && (widens ? cv->out()->bytes() < 5u << 19 : cv->out()->bytes() > 4u << 20)) continue;
