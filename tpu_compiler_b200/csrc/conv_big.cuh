@@ -417,9 +417,7 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
           if (ACT != 2 || p.out2) send(&tmO);
           if (ACT == 2) { // leaky ReLU on the packed, saturated values
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              w[k] = pack4_sat(leaky_of(sext_byte<0>(w[k]), p), leaky_of(sext_byte<1>(w[k]), p), leaky_of(sext_byte<2>(w[k]), p),
-                               leaky_of(sext_byte<3>(w[k]), p));
+            for (int k = 0; k < 8; ++k) w[k] = leaky4(w[k], p);
             send(&tmO2);
           }
         } else {

@@ -459,10 +459,18 @@ __device__ __forceinline__ uint32_t add4_packed(uint32_t x, uint32_t y, const Ad
                                __dp4a(b, c.m23, c.rnd) >> c.r);
   return c.relu ? relu_bytes(w) : w;
 }
-// INT8 leaky ReLU of a saturated convolution result (core/activation.cpp:126-153).
-__device__ __forceinline__ int leaky_of(int v, const ConvGemmParams &p) {
-  if (v > 0) return p.leaky_mp != 0 ? mul_rshift_sat8(v, p.leaky_mp, p.leaky_rp) : v;
-  return mul_rshift_sat8(v, p.leaky_mn, p.leaky_rn);
+// INT8 leaky ReLU of four packed convolution results (core/activation.cpp:126-153): (v * m + rnd) >> r with the multiplier of
+// the value's sign, positive values unchanged where their multiplier is 0; the pack saturates.
+__device__ __forceinline__ uint32_t leaky4(uint32_t w, const ConvGemmParams &p) {
+  const int rp = p.leaky_mp != 0 ? p.leaky_rp : 0, rn = p.leaky_rn;
+  const int ap = rp > 0 ? 1 << (rp - 1) : 0, an = rn > 0 ? 1 << (rn - 1) : 0, mp = p.leaky_mp != 0 ? p.leaky_mp : 1, mn = p.leaky_mn;
+  auto one = [&](int v) {
+    const bool pos = v > 0;
+    return (v * (pos ? mp : mn) + (pos ? ap : an)) >> (pos ? rp : rn);
+  };
+  auto below = [&](int v) { return v > 0 ? v : (v * mn + an) >> rn; };
+  if (p.leaky_mp != 0) return pack4_sat(one(sext_byte<0>(w)), one(sext_byte<1>(w)), one(sext_byte<2>(w)), one(sext_byte<3>(w)));
+  return pack4_sat(below(sext_byte<0>(w)), below(sext_byte<1>(w)), below(sext_byte<2>(w)), below(sext_byte<3>(w)));
 }
 
 // Channel of a 32-channel block that sits on TMEM lane `lane` of its quarter, and the row of the packed weights that puts it
@@ -596,12 +604,8 @@ __device__ __forceinline__ void epilogue_channels_impl(const ConvGemmParams &p, 
       } else if (ACT == 2) {
         // fused leaky ReLU: the activation works on the packed, saturated values (eight channels of one pixel); the plain
         // result goes to `out` when the graph keeps that tensor
-        auto leaky = [&](uint32_t v) {
-          return pack4_sat(leaky_of(sext_byte<0>(v), p), leaky_of(sext_byte<1>(v), p), leaky_of(sext_byte<2>(v), p),
-                           leaky_of(sext_byte<3>(v), p));
-        };
         if (p.out2) stg64(at, a, b);
-        stg64(p.out2 ? at + (unsigned long long)(p.out2 - p.out) : at, leaky(a), leaky(b));
+        stg64(p.out2 ? at + (unsigned long long)(p.out2 - p.out) : at, leaky4(a, p), leaky4(b, p));
       } else {
         stg64(at, a, b);
       }
