@@ -355,3 +355,27 @@ def test_bf16_residual_add_with_prefetch(case):
         m.close()
     assert got[1][2] == got[0][2] - 1
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("shape", [(1, 1024, 96, 8, 1), (2, 144, 160, 9, 3), (1, 48, 200, 40, 5)])  # n, ic, oc, hw, k
+def test_float_requantisation_past_its_range(relu, shape):
+    """Sums far past the range in which the floating-point form is exact, of both signs, beside small ones: every shift for which
+    the ends of the range are saturated and those just past, the smallest and largest normalised multipliers."""
+    n, ic, oc, hw, k = shape
+    rng = np.random.default_rng(17 + oc + relu)
+    f = rng.integers(-127, 128, (oc, ic, k, k)).astype(np.float32)
+    f[::3] = np.sign(f[::3]) * 127          # the largest sums
+    f[1::3] = np.where(rng.random(f[1::3].shape) < 0.03, f[1::3], 0)
+    r = (np.arange(oc) % 16).astype(np.float32)
+    r[oc // 2:] = rng.integers(7, 14, oc - oc // 2)
+    m = (rng.integers(2 ** 23, 2 ** 24, oc) * 128).astype(np.float32)
+    m[::7], m[3::7] = 2.0 ** 30, 2.0 ** 31 - 128
+    b = rng.integers(-2 ** 20, 2 ** 20, oc).astype(np.float32)
+    b[::11] = rng.choice([-1, 1], b[::11].shape) * np.float32(2.0) ** 27
+    x = rng.integers(-128, 128, (n, ic, hw, hw)).astype(np.float32)
+    x[0, :, : hw // 2] = np.sign(f[0, :, :1, :1] + 0.5) * 127  # in step with the first filter
+    for top in (16, 14):  # with a shift that keeps the layer on the integer form, and without
+        text = "input name=x shape=%d,%d,%d,%d dtype=INT8\n" % (n, ic, hw, hw) + conv_text("INT8", n, ic, oc, hw, k, 1, k // 2, 1, int(relu), True)
+        got, ref = run_model(text, {"f": f, "b": b, "r": np.where(r < top, r, 9), "m": m}, {"x": x}, ["c"])["c"]
+        assert np.array_equal(got, ref)

@@ -232,8 +232,8 @@ __device__ __forceinline__ uint32_t relu_bytes(uint32_t w) {
 //   v = fma.rn(h, c, 128), c = 2^-r (1 + 2^-23): the factor moves exact ties away from zero and nothing else across one
 // The products are scaled so that v's unit is 2^-149, the smallest subnormal: the bits of v ARE the integer (the sign bit
 // makes negative ones very negative integers, which saturate), and the packing instruction takes them as they are.
-// float_requant (host) checks per channel, from the sum of |weights|, that s and hi stay in range and that d is a float;
-// a layer that fails keeps the integer forms.
+// float_requant (host) checks per channel, from the sum of |weights|, that s and hi stay in range, or that results are saturated
+// where they do not, and that d is a float; a layer that fails keeps the integer forms.
 struct FloatRequant {
   uint32_t sb; // bias + bits of A
   float m, d, c;

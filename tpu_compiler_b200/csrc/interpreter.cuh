@@ -378,15 +378,20 @@ inline std::vector<FloatRequant> float_requant(const float *filt, size_t per, co
     }
     const double bound = std::fabs((double)bias[o]) + 128.0 * sum;
     const double m = std::ldexp((double)mult[o], -31), r = rshift[o], rnd = r > 0 ? std::ldexp(1.0, (int)r - 1) : 0.0;
+    // Sums past the range in which every step is exact are fine where the ends of it give saturated results: every step is
+    // monotone, the sum's bits as a float (finite while |s| < 2^29) among them, so what lies beyond is saturated as well.
+    auto saturated = [&](double hi) { return std::ldexp(hi, -(int)r) >= 127.6; };
     double d, c = std::ldexp(1.0, -49 - (int)r);
     bool ok = r >= 0;
     FloatRequant &q = out[o];
     if (relu) {
-      ok = ok && r <= 22 && bound < 8388608.0 && bound * m + rnd + 1.0 <= 8388608.0;
+      ok = ok && r <= 22 && ((bound < 8388608.0 && bound * m + rnd + 1.0 <= 8388608.0) ||
+                             (bound < 536870912.0 && (m == 0 || (saturated(8388607.0 * m - 1.0) && saturated(8388608.0 - rnd - 2.0)))));
       q.sb = 0x4B000000u + (uint32_t)(int32_t)bias[o];
       d = 8388608.0 + rnd + 0.5 - 8388608.0 * m;
     } else {
-      ok = ok && r <= 31 && bound < 4194304.0 && bound * m < 2097152.0 - 16.0;
+      ok = ok && r <= 31 && ((bound < 4194304.0 && bound * m < 2097152.0 - 16.0) ||
+                             (bound < 536870912.0 && (m == 0 || (saturated(4194303.0 * m - 1.0) && saturated(2097152.0 - 16.0)))));
       q.sb = 0x4B400000u + (uint32_t)(int32_t)bias[o];
       d = kFqC + 0.5 - 12582912.0 * m;
       c *= 1.0 + std::ldexp(1.0, -23);
