@@ -69,3 +69,44 @@ def test_malformed_modules_are_refused_with_a_status():
     out = m.run(model.meta["x"])["conv"]
     assert np.array_equal(out, graph_runner.run(model.text, model.weights, {"x": model.meta["x"]})["conv"])
     m.close()
+
+
+@pytest.mark.parametrize("form", ["big_tiles 1256", "big_tiles 2256", "fused add"])
+def test_bounded_wait_runs_out_in_the_other_forms(form):
+    """The kernels whose epilogue warps meet at barriers: after the MMA issuer's wait and then theirs have run out, every warp (and
+    both CTAs of a pair) still leaves, and the interpreter stays usable."""
+    from tpu_compiler_b200 import TpucbError, module
+    k, hw = (1, 56) if form == "fused add" else (3, 28)
+    model = graphs.single_conv_i8(64, 64, 256, hw, k, 1, k // 2, relu=False, seed=37)  # more than two tiles per CTA
+    text, w, x, names = model.text, dict(model.weights), {"x": model.meta["x"]}, ["conv"]
+    if form == "fused add":
+        shape = "shape=64,256,%d,%d dtype=INT8" % (hw, hw)
+        text = "input name=res %s\n" % shape + text + "eltwise_add name=s in=res,conv,-,-,ar,am %s do_relu=1\n" % shape
+        w.update(ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
+        x["res"], names = np.random.default_rng(3).integers(-128, 128, (64, 256, hw, hw)).astype(np.float32), ["conv", "s"]
+    got = []
+    m = module(0)
+    for rounds in (4, 0):
+        m.set_option("selftest_lost_arrival", rounds)
+        if form == "fused add":
+            m.set_option("fuse_residual_add", 1 if rounds else 0)
+        else:
+            m.set_option("big_tiles", int(form.split()[1]) if rounds else 0)
+        m.load_text(text, w)
+        for name, v in x.items():
+            m.set_tensor(name, v)
+        if rounds:
+            for _ in range(2):
+                with pytest.raises(TpucbError, match="bounded wait"):
+                    m.invoke()
+        else:
+            m.invoke()
+            got.append([m.get_tensor(n) for n in names])
+    m.set_option("fuse_residual_add", 1)
+    m.set_option("big_tiles", 1 if form == "fused add" else int(form.split()[1]))
+    m.load_text(text, w)
+    for name, v in x.items():
+        m.set_tensor(name, v)
+    m.invoke()
+    assert all(np.array_equal(a, m.get_tensor(n)) for a, n in zip(got[0], names))
+    m.close()

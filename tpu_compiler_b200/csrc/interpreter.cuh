@@ -111,7 +111,7 @@ public:
     pdl_mode() = use_pdl;
     launch_pdl_flag() = use_pdl >= 2;
     launch_sm_count() = sm_count;
-    conv_big_mode() = selftest_lost_arrival ? 0 : big_tiles;
+    conv_big_mode() = selftest_lost_arrival && big_tiles == 1 ? 0 : big_tiles;
     conv_split_k_enabled() = split_k && selftest_lost_arrival == 0; // the self-test needs tiles that follow one another in a CTA
   }
   int device() const { return device_; }
@@ -361,37 +361,39 @@ inline std::vector<FloatRequant> float_requant(const float *filt, size_t per, co
   std::vector<FloatRequant> out(std::max<size_t>(oc, pad_to), FloatRequant{0u, 0.0f, 0.0f, 0.0f});
   const double scale = kFqScale;
   for (size_t o = 0; o < oc; ++o) {
-    // sum of |w| in sixteen lanes: integers that stay exact in a float (2^24 / 128 weights and more per lane)
-    const float *w = filt + o * per;
-    float lane[16] = {};
-    double sum = 0;
-    for (size_t i = 0; i < per; i += 16 << 16) {
-      const size_t end = std::min(per, i + (16u << 16));
-      size_t j = i;
-      for (; j + 16 <= end; j += 16)
-        for (int l = 0; l < 16; ++l) lane[l] += std::fabs(w[j + l]);
-      for (; j < end; ++j) lane[0] += std::fabs(w[j]);
-      for (float &l : lane) {
-        sum += l;
-        l = 0.0f;
-      }
-    }
-    const double bound = std::fabs((double)bias[o]) + 128.0 * sum;
     const double m = std::ldexp((double)mult[o], -31), r = rshift[o], rnd = r > 0 ? std::ldexp(1.0, (int)r - 1) : 0.0;
     // Sums past the range in which every step is exact are fine where the ends of it give saturated results: every step is
     // monotone, the sum's bits as a float (finite while |s| < 2^29) among them, so what lies beyond is saturated as well.
     auto saturated = [&](double hi) { return std::ldexp(hi, -(int)r) >= 127.6; };
+    const bool at_ends = m == 0 || (relu ? saturated(8388607.0 * m - 1.0) && saturated(8388608.0 - rnd - 2.0)
+                                         : saturated(4194303.0 * m - 1.0) && saturated(2097152.0 - 16.0));
+    bool ok = r >= 0 && r <= (relu ? 22 : 31);
+    if (!(at_ends && std::fabs((double)bias[o]) + 128.0 * 128.0 * per < 536870912.0)) {
+      // sum of |w| in sixteen lanes: integers that stay exact in a float (2^24 / 128 weights and more per lane)
+      const float *w = filt + o * per;
+      float lane[16] = {};
+      double sum = 0;
+      for (size_t i = 0; i < per; i += 16 << 16) {
+        const size_t end = std::min(per, i + (16u << 16));
+        size_t j = i;
+        for (; j + 16 <= end; j += 16)
+          for (int l = 0; l < 16; ++l) lane[l] += std::fabs(w[j + l]);
+        for (; j < end; ++j) lane[0] += std::fabs(w[j]);
+        for (float &l : lane) {
+          sum += l;
+          l = 0.0f;
+        }
+      }
+      const double bound = std::fabs((double)bias[o]) + 128.0 * sum;
+      ok = ok && ((at_ends && bound < 536870912.0) || (relu ? bound < 8388608.0 && bound * m + rnd + 1.0 <= 8388608.0
+                                                            : bound < 4194304.0 && bound * m < 2097152.0 - 16.0));
+    }
     double d, c = std::ldexp(1.0, -49 - (int)r);
-    bool ok = r >= 0;
     FloatRequant &q = out[o];
     if (relu) {
-      ok = ok && r <= 22 && ((bound < 8388608.0 && bound * m + rnd + 1.0 <= 8388608.0) ||
-                             (bound < 536870912.0 && (m == 0 || (saturated(8388607.0 * m - 1.0) && saturated(8388608.0 - rnd - 2.0)))));
       q.sb = 0x4B000000u + (uint32_t)(int32_t)bias[o];
       d = 8388608.0 + rnd + 0.5 - 8388608.0 * m;
     } else {
-      ok = ok && r <= 31 && ((bound < 4194304.0 && bound * m < 2097152.0 - 16.0) ||
-                             (bound < 536870912.0 && (m == 0 || (saturated(4194303.0 * m - 1.0) && saturated(2097152.0 - 16.0)))));
       q.sb = 0x4B400000u + (uint32_t)(int32_t)bias[o];
       d = kFqC + 0.5 - 12582912.0 * m;
       c *= 1.0 + std::ldexp(1.0, -23);
