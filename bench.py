@@ -723,14 +723,15 @@ def main():
         i8_tops = C.c_double(0.0)  # this library's own tcgen05 kind::i8 issue microbenchmark, live on this GPU
         check(L.tpucb_measure_i8_mma_peak(local_rank, 128, C.byref(i8_tops)))
         # DRAM traffic per launch: not captured in this run (a profiler capture of this size is out of bounds). The read
-        # side is the ncu figure of a whole step at batch 64 (profiles/launch_lists.md: 10.49 MB of dram__bytes_read per
-        # tensor-core launch) scaled by the images per launch; ncu attributes no write-back to these kernels (their outputs
+        # side is the ncu figure of a whole step at batch 64 (profiles/launch_lists.md: 16.66 MB of dram__bytes_read per
+        # tensor-core launch, residuals of the fused adds among them) scaled by the images per launch; ncu attributes no write-back to these kernels (their outputs
         # are still dirty in L2 when they end), so the write side is the algorithmic output bytes. Null for the workloads
         # that have no capture.
         traffic = None
         if args.workload == "resnet50":
-            out_bytes = sum(float(np.prod(i["shape"])) for i in m.op_info if i["bound"] == "tensor") / max(n_conv, 1)
-            traffic = 10.49e6 * B / 64.0 + out_bytes
+            out_bytes = sum(float(np.prod(i["shape"])) for i in m.op_info  # an add of no bytes of its own is in a convolution's launch
+                            if i["bound"] == "tensor" or (i["type"] == "eltwise_add" and i["bytes"] == 0)) / max(n_conv, 1)
+            traffic = 16.66e6 * B / 64.0 + out_bytes
         if args.workload == "resnet50_bf16":
             # BF16 graph: the same pipeline with kind::f16 MMAs; the denominator is the measured bf16 rate itself
             roofline = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",

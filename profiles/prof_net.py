@@ -2,6 +2,7 @@
 
     python profiles/prof_net.py <graph of tpu_compiler_b200.graphs> <batch>
     python profiles/prof_net.py conv <batch> <c_in> <c_out> <hw> <k> <relu>
+    python profiles/prof_net.py conv_add <batch> <c_in> <c_out> <hw>   (a 1x1 layer and the INT8 residual add behind it)
     python profiles/prof_net.py calibration <batch>          (two batches of the fp32 ResNet-50)
 """
 import os
@@ -26,6 +27,14 @@ kind, batch = sys.argv[1], int(sys.argv[2])
 if kind == "conv":
     c_in, c_out, hw, k, relu = (int(v) for v in sys.argv[3:8])
     model = graphs.single_conv_i8(1, c_in, c_out, hw, k, 1, k // 2, relu=bool(relu))
+elif kind == "conv_add":
+    c_in, c_out, hw = (int(v) for v in sys.argv[3:6])
+    model = graphs.single_conv_i8(1, c_in, c_out, hw, 1, 1, 0, relu=False)
+    shape = "shape=1,%d,%d,%d dtype=INT8" % (c_out, hw, hw)
+    model.text = "%sinput name=res %s\neltwise_add name=sum in=res,conv,-,-,ar,am %s do_relu=1\n" % (model.text, shape, shape)
+    lines = model.text.splitlines()
+    model.text = "\n".join([lines[-2]] + lines[:-2] + [lines[-1]]) + "\n"  # the residual is there before the convolution
+    model.weights.update(ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
 elif kind == "calibration":
     model = graphs.resnet50_fp32(1)
 else:
@@ -39,9 +48,9 @@ if kind == "calibration":
     profiled(cal.run)
 else:
     m.set_option("cuda_graph", 0)
-    name = m.get_input_details()[0]
+    name = "x" if kind == "conv_add" else m.get_input_details()[0]
     x = np.random.default_rng(0).uniform(-1, 1, m.get_tensor_shape(name)).astype(np.float32)
-    m.set_tensor(name, np.rint(x * 127) if kind == "conv" else x)
+    m.set_tensor(name, np.rint(x * 127) if kind.startswith("conv") else x)
     m.launch()
     m.launch()
     m.sync()
