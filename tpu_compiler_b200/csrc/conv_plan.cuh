@@ -486,15 +486,14 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
     if (grid < n_tiles) grid = n_tiles;
   }
   // Split K: a launch with fewer tiles than SMs and a long K gives each tile to several CTAs (ConvGemmParams::split_k): at
-  // least six K blocks per CTA, at most sixteen CTAs per tile, no more CTAs than SMs. A K block takes 0.30 us of a CTA that
-  // has its SM to itself (0.33 for a tile of 128 pixels). The exchange through global memory (reductions, fence, count, read
+  // least six K blocks per CTA, at most sixteen CTAs per tile, no more CTAs than SMs. A K block takes 0.21 us of a CTA that
+  // has its SM to itself (0.25 for a tile of 128 pixels). The exchange through global memory (reductions, fence, count, read
   // back) takes 3.4 us for a few CTAs and 4.9 from 75 on (tiles of 128 pixels: 8.5 from 100 on, twice the partial sums).
   // Split where that pays by half a microsecond; us alone and with three streams in flight, unsplit -> split:
-  //   3x3, 512 channels, 7x7: N = 1 13.8 / 5.5 -> 8.4 / 4.1 (6 parts), 8 14.1 / 6.1 -> 10.4 / 4.8 (5), 12 14.7 / 6.2 -> 11.7 /
-  //   5.5 (3); not split: 16 14.4 / 6.2 against 13.5 / 6.2 (2), 19 14.3 / 6.2 against 13.6 / 6.3, 32 (128 pixels) 15.8 / 6.2
-  //   against 18.1 / 7.3;
-  //   3x3, 256 channels, 14x14: N = 1 8.6 / 4.1 against 8.5 / 4.1 (3), 4 8.7 / 4.1 against 9.7 / 4.5: not split;
-  //   3x3, 1024 channels, 5x5: N = 2 24.9 / 9.6 -> 9.3 / 4.9 (12), 8 25.1 / 9.6 -> 13.5 / 6.2 (4).
+  //   3x3, 512 channels, 7x7: N = 1 10.6 / 4.9 -> 8.0 / 4.1 (6 parts), 4 10.7 / 4.9 -> 9.3 / 4.5, 8 10.8 / 4.9 -> 10.0 / 4.9 (5); not
+  //   split: 12 11.2 / 4.9 against 10.8 / 5.0 (3);
+  //   3x3, 512 -> 1024 channels, 13x13: N = 1 10.8 / 4.9 -> 9.8 / 4.9 (6); not split: 2 11.1 / 4.9 against 10.9 / 5.5 (3);
+  //   3x3, 1024 channels, 5x5: N = 2 18.4 / 7.6 -> 9.2 / 4.5 (12), 8 18.5 / 7.6 -> 12.3 / 5.6 (4).
   // Two CTAs per SM were a loss wherever other work fills the gaps (5x5, 64 -> 128 channels, 7 x 45 x 45, 222 CTAs: 16.1 us
   // against 12.7 unsplit, three streams at once 9.8 against 5.3). The weights are then not kept resident (a CTA needs only
   // its own K range once).
@@ -505,7 +504,7 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
     if (want >= 2) {
       const int per = (k_iters + want - 1) / want, parts = (k_iters + per - 1) / per;
       const double ctas = (double)total_tiles * parts;
-      const double block = p.m_tile == 64 ? 0.30 : 0.33;
+      const double block = p.m_tile == 64 ? 0.21 : 0.25;
       const double exchange = 3.4 + (p.m_tile == 64 ? 0.02 * std::min(ctas, 75.0) : 0.051 * std::min(ctas, 100.0));
       if (block * (k_iters - per) > exchange + 0.5) {
         p.k_per = per;
