@@ -586,38 +586,57 @@ inline void pair_layer(DenseLayer &d) {
   d.paired = true;
 }
 
-// The kernel of a plan on conv_big.cuh. `use` gets it as a function pointer and says whether it is one of the fp32 form, which
-// takes two more maps.
-template <class Use> inline void with_big_kernel(int ctas, int kind, int act, bool fq, Use use) {
-  auto by_ctas = [&](auto c) {
-    constexpr int C = decltype(c)::value;
-    if (kind == 2) {
-      if (act == 1) use(conv_big_tf32x3_kernel<C, 1>);
-      else use(conv_big_tf32x3_kernel<C, 0>);
-    } else if (kind == 1) {
-      if (act == 1) use(conv_big_kernel<C, 1, 1, 0>);
-      else use(conv_big_kernel<C, 1, 0, 0>);
-    } else if (fq) {
-      if (act == 1) use(conv_big_kernel<C, 0, 1, 3>);
-      else if (act == 2) use(conv_big_kernel<C, 0, 2, 3>);
-      else use(conv_big_kernel<C, 0, 0, 3>);
-    } else {
-      if (act == 1) use(conv_big_kernel<C, 0, 1, 1>);
-      else if (act == 2) use(conv_big_kernel<C, 0, 2, 1>);
-      else use(conv_big_kernel<C, 0, 0, 1>);
-    }
-  };
-  if (ctas == 2) by_ctas(std::integral_constant<int, 2>());
-  else by_ctas(std::integral_constant<int, 1>());
+// The tensor-core kernel of a plan, as a constant that `use` gets.
+template <auto K> struct KernelConstant {
+  static constexpr auto value = K;
+};
+template <class Use> inline void with_conv_kernel(const ConvPlan &pl, Use use) {
+  const ConvGemmParams &p = pl.p;
+  if (pl.stem) {
+    if (p.act == 1) use(KernelConstant<conv_stem_tf32x3_kernel<true>>());
+    else use(KernelConstant<conv_stem_tf32x3_kernel<false>>());
+  } else if (pl.ctas > 0) {
+    auto by_ctas = [&](auto c) {
+      constexpr int C = decltype(c)::value;
+      if (pl.tf32) {
+        if (p.act == 1) use(KernelConstant<conv_big_tf32x3_kernel<C, 1>>());
+        else use(KernelConstant<conv_big_tf32x3_kernel<C, 0>>());
+      } else if (pl.bf16) {
+        if (p.act == 1) use(KernelConstant<conv_big_kernel<C, 1, 1, 0>>());
+        else use(KernelConstant<conv_big_kernel<C, 1, 0, 0>>());
+      } else if (p.fq) {
+        if (p.act == 1) use(KernelConstant<conv_big_kernel<C, 0, 1, 3>>());
+        else if (p.act == 2) use(KernelConstant<conv_big_kernel<C, 0, 2, 3>>());
+        else use(KernelConstant<conv_big_kernel<C, 0, 0, 3>>());
+      } else {
+        if (p.act == 1) use(KernelConstant<conv_big_kernel<C, 0, 1, 1>>());
+        else if (p.act == 2) use(KernelConstant<conv_big_kernel<C, 0, 2, 1>>());
+        else use(KernelConstant<conv_big_kernel<C, 0, 0, 1>>());
+      }
+    };
+    if (pl.ctas == 2) by_ctas(std::integral_constant<int, 2>());
+    else by_ctas(std::integral_constant<int, 1>());
+  } else if (pl.tf32) use(KernelConstant<conv_gemm_tf32x3_kernel>());
+  else if (pl.bf16 && p.act == 3) use(KernelConstant<conv_gemm_bf16_add_kernel>());
+  else if (pl.bf16) use(KernelConstant<conv_gemm_bf16_kernel>());
+  else if (p.split_k > 1 && (p.fastq & 1)) use(KernelConstant<conv_gemm_i8_split_kernel<true>>());
+  else if (p.split_k > 1) use(KernelConstant<conv_gemm_i8_split_kernel<false>>());
+  else if (p.fq && p.act == 1) use(KernelConstant<conv_gemm_i8_fq_kernel<1>>());
+  else if (p.fq && p.act == 0) use(KernelConstant<conv_gemm_i8_fq_kernel<0>>());
+  else if (p.fq && p.act == 2) use(KernelConstant<conv_gemm_i8_fq_kernel<2>>());
+  else if (p.fq) use(KernelConstant<conv_gemm_i8_fq_kernel<3>>());
+  else if (!(p.fastq & 1)) use(KernelConstant<conv_gemm_i8_wide_kernel>());
+  else use(KernelConstant<conv_gemm_i8_kernel>());
 }
-inline void launch_big_plan(const ConvPlan &pl, cudaStream_t stream, int sm_count) {
-  if (pl.tf32 && pl.split_src)
-    launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
-             reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
-  with_big_kernel(pl.ctas, pl.tf32 ? 2 : (pl.bf16 ? 1 : 0), pl.p.act, pl.p.fq != nullptr, [&](auto kernel) {
-    if constexpr (std::is_invocable_v<decltype(kernel), CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ConvGemmParams>)
-      launch_k(kernel, pl.grid, kBigThreads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmO, pl.tmO2, pl.p);
-    else launch_k(kernel, pl.grid, kBigThreads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.tmO, pl.tmO2, pl.p);
+// To be called at load for every plan, and again when its activation changes. Only the kernels that are used are set up: the
+// driver loads a kernel when its attribute is set, which takes half a millisecond each.
+inline void conv_kernel_ready(const ConvPlan &pl) {
+  with_conv_kernel(pl, [](auto k) {
+    static const bool done = [] {
+      TPUCB_CUDA(cudaFuncSetAttribute(decltype(k)::value, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+      return true;
+    }();
+    (void)done;
   });
 }
 
@@ -633,58 +652,22 @@ inline void launch_conv_plan(const ConvPlan &pl, cudaStream_t stream, int sm_cou
     if (a.es == 1) launch_k(window_repack_kernel<uint8_t>, grid, 256, 0, stream, a);
     else launch_k(window_repack_kernel<uint16_t>, grid, 256, 0, stream, a);
   }
-  const int threads = kConvThreads;
   PdlConvScope conv_class; // the tensor-core kernel and its helper passes may start while the predecessor finishes
-  if (pl.stem) {
-    if (pl.p.act == 1) launch_k(conv_stem_tf32x3_kernel<true>, pl.grid, kStemThreads, pl.smem, stream, pl.stem_args, pl.p);
-    else launch_k(conv_stem_tf32x3_kernel<false>, pl.grid, kStemThreads, pl.smem, stream, pl.stem_args, pl.p);
-  } else if (pl.ctas > 0) launch_big_plan(pl, stream, sm_count);
-  else if (pl.tf32) {
-    if (pl.split_src)
-      launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
-               reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
-    launch_k(conv_gemm_tf32x3_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.p);
-  } else if (pl.bf16 && pl.p.act == 3) launch_k(conv_gemm_bf16_add_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.bf16) launch_k(conv_gemm_bf16_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.split_k > 1 && (pl.p.fastq & 1)) launch_k(conv_gemm_i8_split_kernel<true>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.split_k > 1) launch_k(conv_gemm_i8_split_kernel<false>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.fq && pl.p.act == 1) launch_k(conv_gemm_i8_fq_kernel<1>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.fq && pl.p.act == 0) launch_k(conv_gemm_i8_fq_kernel<0>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.fq && pl.p.act == 2) launch_k(conv_gemm_i8_fq_kernel<2>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (pl.p.fq) launch_k(conv_gemm_i8_fq_kernel<3>, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else if (!(pl.p.fastq & 1)) launch_k(conv_gemm_i8_wide_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-  else launch_k(conv_gemm_i8_kernel, pl.grid, threads, pl.smem, stream, pl.tmA, pl.tmB, pl.p);
-}
-
-inline void conv_kernel_setup_once() {
-  static bool done = [] {
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_fq_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_split_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_bf16_add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_i8_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_gemm_tf32x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_tf32x3_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    TPUCB_CUDA(cudaFuncSetAttribute(conv_stem_tf32x3_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    for (int ctas = 1; ctas <= 2; ++ctas)
-      for (int form = 0; form < 4; ++form) // INT8 twice (requantisation), BF16, fp32
-        for (int act = 0; act < (form < 2 ? 3 : 2); ++act)
-          with_big_kernel(ctas, std::max(0, form - 1), act, form == 1, [](auto kernel) {
-            TPUCB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-          });
-    return true;
-  }();
-  (void)done;
+  if (pl.tf32 && !pl.stem && pl.split_src)
+    launch_k(tf32_split_kernel, grid_for(pl.split_nvec, 256, sm_count), 256, 0, stream, reinterpret_cast<const float4 *>(pl.split_src),
+             reinterpret_cast<float4 *>(pl.split_lo), pl.split_nvec);
+  const int threads = pl.stem ? kStemThreads : (pl.ctas > 0 ? kBigThreads : kConvThreads);
+  with_conv_kernel(pl, [&](auto k) {
+    constexpr auto kernel = decltype(k)::value;
+    typedef std::remove_const_t<decltype(kernel)> Kernel;
+    using Map = CUtensorMap;
+    auto go = [&](auto &&...args) { launch_k(kernel, pl.grid, threads, pl.smem, stream, args..., pl.p); };
+    if constexpr (std::is_invocable_v<Kernel, StemArgs, ConvGemmParams>) go(pl.stem_args);
+    else if constexpr (std::is_invocable_v<Kernel, Map, Map, ConvGemmParams>) go(pl.tmA, pl.tmB);
+    else if constexpr (std::is_invocable_v<Kernel, Map, Map, Map, Map, Map, Map, ConvGemmParams>) go(pl.tmA, pl.tmB, pl.tmA2, pl.tmB2, pl.tmO, pl.tmO2);
+    else if (pl.ctas > 0) go(pl.tmA, pl.tmB, pl.tmO, pl.tmO2);
+    else go(pl.tmA, pl.tmB, pl.tmA2, pl.tmB2);
+  });
 }
 
 } // namespace tpucb

@@ -597,7 +597,7 @@ public:
       return;
     }
 
-    conv_kernel_setup_once(); // grouped layers, input insertion: one launch per group over an expanded patch matrix
+    // grouped layers, input insertion: one launch per group over an expanded patch matrix
     const int groups = g.g;
     for (int grp = 0; grp < groups; ++grp) {
       ConvPlan pl;
@@ -642,6 +642,7 @@ public:
         pl.p.lose_arrival = 1;
       }
       I.attach_split_ws(pl);
+      conv_kernel_ready(pl);
       plans_.push_back(pl);
     }
   }
@@ -652,7 +653,6 @@ public:
   // another order, were a fifth faster (4.9 ms against 5.9 for ResNet-50 at batch 64) and moved one threshold in one run of
   // twenty.
   void setup_tf32(Interpreter &I, const std::vector<float> &filt, const std::vector<float> &bias, bool stem) {
-    conv_kernel_setup_once();
     const ConvGeom &g = g_;
     const int rows = g.n * g.oh * g.ow, out_cp = out_->cp;
     act_ = do_relu_ ? 1 : 0;
@@ -681,6 +681,7 @@ public:
       pl.stem_args = StemArgs{(const float4 *)in_->dev, (const uint8_t *)I.upload(pack_stem_weights_tf32(filt.data(), g)), g.ih, g.iw, g.kh * g.kw};
       pl.grid = dim3((unsigned)std::min((rows + kStemPx - 1) / kStemPx, I.sm_count));
       pl.smem = stem_smem(g.kh * g.kw);
+      conv_kernel_ready(pl);
       plans_.push_back(pl);
       return;
     }
@@ -719,13 +720,13 @@ public:
       encode_weight_map(k ? &pl.tmB2 : &pl.tmB, I.upload(w), out_cp, taps, k_bytes, p.BK, 128);
     }
     encode_out_maps(pl);
+    conv_kernel_ready(pl);
     plans_.push_back(pl);
   }
   // Ungrouped layers on the tensor cores. kind: 0 INT8, 1 BF16. Two forms: row windows (wp), K blocks of a matrix or im2col
   // map.
   void setup_tensor_core(Interpreter &I, int kind, const std::vector<float> &filt, const std::vector<float> &bias,
                          const std::vector<float> &mult, const std::vector<float> &rshift, const WindowPlan *wp) {
-    conv_kernel_setup_once();
     const int es = kind == 0 ? 1 : 2;
     act_ = do_relu_ ? 1 : 0;
     alg_bytes = (double)es * ((double)in_->numel() + out_->numel() + filt.size()) + (kind == 0 ? 12.0 : 4.0) * g_.oc;
@@ -766,6 +767,7 @@ public:
     if (wp) setup_window(I, pl, *wp, filt, kind);
     else setup_blocks(I, pl, d, kind, !I.add_tails.count(out_->name));
     I.attach_split_ws(pl);
+    conv_kernel_ready(pl);
     plans_.push_back(pl);
   }
   // The row-window form (WindowPlan). The input tensor has the window layout when it was asked for at load and granted;
@@ -826,6 +828,7 @@ public:
       pl.p.leaky_mp = mp; pl.p.leaky_rp = rp; pl.p.leaky_mn = mn; pl.p.leaky_rn = rn;
       pl.p.out2 = act_out;
       encode_out_maps(pl);
+      conv_kernel_ready(pl);
     }
     act_ = 2;
   }
@@ -840,6 +843,7 @@ public:
       pl.p.res = residual;
       pl.p.out2 = sum_out;
       pl.p.add_ms = ms; pl.p.add_mr = mr; pl.p.add_r = rshift; pl.p.add_relu = relu;
+      conv_kernel_ready(pl);
     }
     act_ = 3;
     alg_bytes += 2.0 * out_->numel() * out_->elsize(); // the residual read and the sum written
@@ -964,7 +968,6 @@ public:
       // BF16 inner product (core/fullyconnected.cpp:44-91 with the BF16 rounding of the result): the tensor-core
       // pipeline with BF16 operands, fp32 accumulators and fp32 bias; K sizes and pitches in bytes.
       TPUCB_CHECK(in->dtype == DT_BF16, "fc %s: a BF16 inner product needs a BF16 input", op.name.c_str());
-      conv_kernel_setup_once();
       const int n_pad = out->cp;
       kdev_ = hw * in->cp;
       std::vector<uint16_t> w(packed_rows(n_pad) * kdev_, 0);
@@ -994,6 +997,7 @@ public:
       encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_ * 2, kdev_ * 2, p.BK, p.m_tile);
       encode_weight_map(&pl.tmB, d_w, n_pad, 1, kdev_ * 2, p.BK, p.dual ? 192 : p.BN);
       I.attach_split_ws(pl);
+      conv_kernel_ready(pl);
       plan_ = pl;
       alg_bytes = 2.0 * ((double)m_ * k_ + (double)n_ * k_ + (double)m_ * n_) + 4.0 * n_;
       return;
@@ -1015,7 +1019,6 @@ public:
     TPUCB_CHECK(in->dtype == DT_I8, "fc %s: INT8 needs an INT8 input", op.name.c_str());
     TPUCB_CHECK(op.in.size() >= 7 && I.has_weight(op.in[5]) && I.has_weight(op.in[6]),
                 "fc %s: INT8 needs rshift and multiplier operands", op.name.c_str());
-    conv_kernel_setup_once();
     const int n_pad = out->cp;
     kdev_ = hw * in->cp;
     std::vector<int8_t> w(packed_rows(n_pad) * kdev_, 0);
@@ -1049,6 +1052,7 @@ public:
     encode_matrix_map(&pl.tmA, (const int8_t *)in->dev, m_, kdev_, kdev_, p.BK, p.m_tile);
     encode_weight_map(&pl.tmB, d_w, n_pad, 1, kdev_, p.BK, p.dual ? 192 : p.BN);
     I.attach_split_ws(pl);
+    conv_kernel_ready(pl);
     plan_ = pl;
     alg_bytes = (double)m_ * k_ + (double)n_ * k_ + (double)m_ * n_ + 4.0 * n_ + 8;
   }
