@@ -207,12 +207,12 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
           const int c0 = chunk * p.BK;
           const uint32_t fb = lead_full + 8 * ps;
           if (ptx::elect_one()) {
-          if (rank == 0) ptx::mbar_expect_tx(bar_full + 8 * ps, CTAS * bytes);
-          if (!acts) ptx::big_load_3d<CTAS>(dst, (TF32 && term == 1) ? &tmB2 : &tmB, fb, c0, tap, n0);
-          else if (p.a_mode == 1)
-            ptx::big_load_im2col<CTAS>(dst, (TF32 && term == 0) ? &tmA2 : &tmA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
-                                       (uint16_t)(tr * p.dh));
-          else ptx::big_load_2d<CTAS>(dst, (TF32 && term == 0) ? &tmA2 : &tmA, fb, c0, m0);
+            if (rank == 0) ptx::mbar_expect_tx(bar_full + 8 * ps, CTAS * bytes);
+            if (!acts) ptx::big_load_3d<CTAS>(dst, (TF32 && term == 1) ? &tmB2 : &tmB, fb, c0, tap, n0);
+            else if (p.a_mode == 1)
+              ptx::big_load_im2col<CTAS>(dst, (TF32 && term == 0) ? &tmA2 : &tmA, fb, c0, w_base, h_base, n_img, (uint16_t)(ts * p.dw),
+                                         (uint16_t)(tr * p.dh));
+            else ptx::big_load_2d<CTAS>(dst, (TF32 && term == 0) ? &tmA2 : &tmA, fb, c0, m0);
           }
           if (++chunk == p.c_chunks) {
             chunk = 0;
@@ -276,14 +276,14 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
             ptx::tcgen05_fence_after();
             const uint32_t w_lo = lo + w_at;
             if (ptx::elect_one()) {
-            if constexpr (decltype(whole)::value) {
-              ptx::big_mma<CTAS, KIND>(d, w_lo, lo, hi, p.idesc, kit > 0 ? 1u : 0u);
+              if constexpr (decltype(whole)::value) {
+                ptx::big_mma<CTAS, KIND>(d, w_lo, lo, hi, p.idesc, kit > 0 ? 1u : 0u);
 #pragma unroll
-              for (int k = 1; k < 4; ++k) ptx::big_mma<CTAS, KIND>(d, w_lo + 2 * k, lo + 2 * k, hi, p.idesc, 1u);
-            } else {
-              for (int k = 0; k < ksteps; ++k) ptx::big_mma<CTAS, KIND>(d, w_lo + 2 * k, lo + 2 * k, hi, p.idesc, kit + k > 0 ? 1u : 0u);
-            }
-            ptx::big_commit<CTAS>(m_empty);
+                for (int k = 1; k < 4; ++k) ptx::big_mma<CTAS, KIND>(d, w_lo + 2 * k, lo + 2 * k, hi, p.idesc, 1u);
+              } else {
+                for (int k = 0; k < ksteps; ++k) ptx::big_mma<CTAS, KIND>(d, w_lo + 2 * k, lo + 2 * k, hi, p.idesc, kit + k > 0 ? 1u : 0u);
+              }
+              ptx::big_commit<CTAS>(m_empty);
             }
             m_full += 8;
             m_empty += 8;
