@@ -197,3 +197,69 @@ def test_copy_helpers_threads_fork_and_thread_limit(tmp_path):
                     "-ldl"], check=True)
     for args in ([], ["0"], ["1"], ["2"]):
         assert subprocess.run([exe] + args, timeout=120).returncode == 0, args
+
+
+KERNELS_READY = r"""
+#include <cuda_runtime.h>
+#include <cudaTypedefs.h>
+#include <map>
+#include <mutex>
+#include <thread>
+static thread_local int current_device = 0;
+static std::mutex m;
+static std::map<std::pair<int, const void *>, int> set_up;
+static int failing = 0; // calls that report an error yet
+static cudaError_t fake_get_device(int *d) { *d = current_device; return cudaSuccess; }
+template <class Kernel> cudaError_t fake_set_attribute(Kernel k, cudaFuncAttribute, int) {
+  std::lock_guard<std::mutex> g(m);
+  if (failing > 0 && failing--) return cudaErrorInvalidValue;
+  ++set_up[{current_device, (const void *)k}];
+  return cudaSuccess;
+}
+#define cudaGetDevice fake_get_device
+#define cudaFuncSetAttribute fake_set_attribute
+#include "conv_plan.cuh"
+
+int main() {
+  tpucb::ConvPlan i8, tf32;
+  std::memset(&i8.p, 0, sizeof(i8.p));
+  i8.p.fastq = 1;
+  std::memset(&tf32.p, 0, sizeof(tf32.p));
+  tf32.tf32 = true;
+  for (int device : {0, 1, 0, 1}) { // as a module on the first device and then one on the second would
+    current_device = device;
+    tpucb::conv_kernel_ready(i8);
+    tpucb::conv_kernel_ready(tf32);
+  }
+  if (set_up.size() != 4) return 1;
+  current_device = 2;
+  failing = 1;
+  try { // an error of the driver leaves the device to the next caller
+    tpucb::conv_kernel_ready(i8);
+    return 2;
+  } catch (const tpucb::Error &) {
+  }
+  tpucb::conv_kernel_ready(i8);
+  std::vector<std::thread> users;
+  for (int t = 0; t < 8; ++t)
+    users.emplace_back([&] {
+      current_device = 3;
+      tpucb::conv_kernel_ready(i8);
+    });
+  for (auto &u : users) u.join();
+  for (auto &k : set_up)
+    if (k.second != 1) return 3;
+  return set_up.size() == 6 ? 0 : 4;
+}
+"""
+
+
+def test_kernels_are_set_up_on_every_device(tmp_path):
+    """A kernel's limit of shared memory belongs to a device: what plans call at load sets it once on each (the driver's calls
+    are replaced here), again after an error, and once for several threads."""
+    import subprocess
+    from tpu_compiler_b200 import build as b
+    src, exe = tmp_path / "t.cu", str(tmp_path / "t")
+    src.write_text(KERNELS_READY)
+    subprocess.run([b._nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "-O0", "-I", b.CSRC, str(src), "-o", exe], check=True)
+    assert subprocess.run([exe], timeout=120).returncode == 0

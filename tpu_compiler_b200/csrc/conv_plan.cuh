@@ -7,6 +7,7 @@
 #include "conv_stem_f32.cuh"
 #include "host_common.h"
 #include "mem_kernels.cuh"
+#include "per_device.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -628,15 +629,15 @@ template <class Use> inline void with_conv_kernel(const ConvPlan &pl, Use use) {
   else if (!(p.fastq & 1)) use(KernelConstant<conv_gemm_i8_wide_kernel>());
   else use(KernelConstant<conv_gemm_i8_kernel>());
 }
-// To be called at load for every plan, and again when its activation changes. Only the kernels that are used are set up: the
-// driver loads a kernel when its attribute is set, which takes half a millisecond each.
+// To be called at load for every plan, and again when its activation changes, on the device that will run it: the limit of
+// shared memory belongs to a kernel on a device. Only the kernels that are used are set up: the driver loads a kernel when its
+// attribute is set, which takes half a millisecond each.
 inline void conv_kernel_ready(const ConvPlan &pl) {
-  with_conv_kernel(pl, [](auto k) {
-    static const bool done = [] {
-      TPUCB_CUDA(cudaFuncSetAttribute(decltype(k)::value, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-      return true;
-    }();
-    (void)done;
+  int device = 0;
+  TPUCB_CUDA(cudaGetDevice(&device));
+  with_conv_kernel(pl, [&](auto k) {
+    static OncePerDevice ready; // one of each kernel
+    ready.run(device, [] { TPUCB_CUDA(cudaFuncSetAttribute(decltype(k)::value, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)); });
   });
 }
 
