@@ -162,6 +162,8 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          two-input eltwise add (or a BF16 one with ReLU) whose later-produced operand is a tensor-core convolution that feeds nothing else
  *          (the last convolution of a residual block) runs in that convolution's epilogue, which reads the other
  *          operand and writes both the convolution's tensor and the sum; the add launches nothing. Same bits.
+ *          Always: whatever "big_tiles" says of that convolution, but not in the forms whose epilogue has no add: tiles that are
+ *          split ("split_k"), image stems as row windows, layers of at most 64 channels on pairs of pixel tiles.
  *          By size: results of 2.5 MiB and more of layers that widen their input (INT8 ResNet-50 at batch 19:
  *          6% fewer us, at batch 256 3% alone and 7% with three modules in flight; BF16 at batch 128 3% and 12%).
  *          "fp32_tensor_cores" (0/1, default 1; read by the next load_module): fp32 convolutions with a

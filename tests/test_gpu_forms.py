@@ -223,6 +223,34 @@ def test_residual_add_with_prefetch(case):
     m.close()
 
 
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, big_tiles: by size (196 tiles of 256 pixels, 9 K blocks) and forced on a small one
+    (16, 64, 128, 56, 1), (2, 96, 136, 13, 1256), (2, 96, 136, 13, 2192)])
+def test_every_add_is_fused_when_asked(case):
+    """fuse_residual_add = 1 on layers that would run large tiles: the add launches nothing, both tensors keep their bits."""
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, big = case
+    model = graphs.single_conv_i8(1, ic, oc, hw, 3, 1, 1, relu=False, seed=78)
+    w = dict(model.weights, ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
+    shape = "shape=%d,%d,%d,%d dtype=INT8" % (n, oc, hw, hw)
+    text = ("input name=res %s\n" % shape + model.text.replace("shape=1,", "shape=%d," % n) +
+            "eltwise_add name=s in=res,conv,-,-,ar,am %s do_relu=1\n" % shape)
+    rng = np.random.default_rng(oc)
+    x = {"x": rng.integers(-128, 128, (n, ic, hw, hw)).astype(np.float32), "res": rng.integers(-128, 128, (n, oc, hw, hw)).astype(np.float32)}
+    got = []
+    for fuse in (0, 1):
+        m = module(0)
+        m.set_option("fuse_residual_add", fuse)
+        m.set_option("big_tiles", big)
+        m.load_text(text, w)
+        for name, v in x.items():
+            m.set_tensor(name, v)
+        m.invoke()
+        got.append([m.get_tensor(k) for k in ("conv", "s")] + [m.kernel_count()])
+        m.close()
+    assert got[1][2] == got[0][2] - 1
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("dtype", ["INT8", "BF16", "FP32"])
 @pytest.mark.parametrize("shape", [
     (1, 1, 1, 1), (3, 1001, 1, 1), (5, 3, 17, 23), (2, 70, 9, 5),        # value by value, small results into pinned memory

@@ -165,7 +165,9 @@ public:
     int cp = 0, wl = 0, wphys = 0;
   };
   std::map<std::string, RowLayout> layout_requests;
-  std::set<std::string> add_tails; // BF16 convolutions whose result goes to one residual add only (load_module): planned so that it can be fused
+  // Convolutions whose result goes to one residual add only (load_module), planned without the large tiles, whose epilogue has no
+  // add: BF16 ones, and INT8 ones when every add is to be fused (by size, an INT8 layer that takes the large tiles keeps them).
+  std::set<std::string> add_tails;
 
   TensorPtr make_tensor(const std::string &name, const std::vector<int64_t> &shape, int dtype) {
     auto t = std::make_shared<DevTensor>();
@@ -2298,13 +2300,14 @@ inline void Interpreter::load_module(const std::string &text) {
       for (auto &nm : op.in) n_uses[nm]++;
     }
     for (auto &op : parsed) {
-      if (!fuse_activations || !fuse_residual_add || op.type != "eltwise_add" || op.dtype != "BF16" || op.in.size() < 2) continue;
+      if (!fuse_activations || !fuse_residual_add || op.type != "eltwise_add" || op.in.size() < 2) continue;
+      if (!(op.dtype == "BF16" || (op.dtype == "INT8" && fuse_residual_add == 1))) continue;
       const ParsedOp *late = nullptr;
       for (int k = 0; k < 2; ++k) {
         auto it = by_name.find(op.in[k]);
         if (it != by_name.end() && (!late || it->second > late)) late = it->second;
       }
-      if (late && late->type == "conv_2d" && n_uses[late->name] == 1) add_tails.insert(late->name);
+      if (late && (late->type == "conv_2d" || late->type == "deconv_2d") && n_uses[late->name] == 1) add_tails.insert(late->name);
     }
     for (auto &op : parsed) {
       if (op.type != "conv_2d" || (op.dtype != "INT8" && op.dtype != "BF16") || op.in.empty()) continue;
