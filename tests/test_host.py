@@ -263,3 +263,61 @@ def test_kernels_are_set_up_on_every_device(tmp_path):
     src.write_text(KERNELS_READY)
     subprocess.run([b._nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "-O0", "-I", b.CSRC, str(src), "-o", exe], check=True)
     assert subprocess.run([exe], timeout=120).returncode == 0
+
+
+RESIDUAL_ADDS = r"""
+#include "module_text.h"
+#include <iostream>
+int main(int argc, char **argv) {
+  std::vector<tpucb::ParsedOp> ops;
+  std::map<std::string, const tpucb::ParsedOp *> by_name;
+  std::map<std::string, int> n_uses;
+  for (std::string line; std::getline(std::cin, line);) ops.push_back(tpucb::parse_line(line));
+  for (auto &op : ops) {
+    by_name[op.name] = &op;
+    for (auto &nm : op.in) n_uses[nm]++;
+  }
+  for (auto &name : tpucb::residual_add_tails(ops, by_name, n_uses, atoi(argv[1]), atoi(argv[2]))) std::cout << name << std::endl;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def add_tails(tmp_path_factory):
+    import subprocess
+    from tpu_compiler_b200 import build as b
+    d = tmp_path_factory.mktemp("add_tails")
+    (d / "t.cu").write_text(RESIDUAL_ADDS)
+    subprocess.run([b._nvcc(), "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "-I", b.CSRC, str(d / "t.cu"), "-o", str(d / "t")], check=True)
+
+    def run(text, fuse=2, batch=1):
+        return subprocess.run([str(d / "t"), str(fuse), str(batch)], input=text, text=True, check=True, capture_output=True).stdout.split()
+    return run
+
+
+def _residual(dtype="BF16", n=32, ic=64, oc=256, hw=28, conv="", add="do_relu=1", add_in="r,c", extra="", res="input"):
+    s = "shape=%d,%%d,%d,%d dtype=%s" % (n, hw, hw, dtype)
+    tail = ",-,-,ar,am" if dtype == "INT8" else ""
+    return ("input name=x " + s % ic + "\n%s name=r%s " % (res, "" if res == "input" else " in=x") + s % oc + "\nconv_2d name=c in=x,f,b " + s % oc +
+            " kh=1 kw=1 sh=1 sw=1 %s\neltwise_add name=s in=%s%s " % (conv, add_in, tail) + s % oc + " %s\n%s" % (add, extra))
+
+
+@pytest.mark.parametrize("case,kept", [
+    (dict(), True), (dict(add_in="c,r"), True), (dict(add="do_relu=1 coeff=1.0,1"), True),
+    (dict(add="do_relu=0"), False), (dict(add="do_relu=1 coeff=1.0,0.5"), False),   # the epilogue's BF16 add has a ReLU and no coefficients
+    (dict(conv="do_relu=1"), False), (dict(conv="g=2"), False), (dict(add_in="c,c"), False), (dict(add_in="r,c,x"), False),
+    (dict(extra="relu name=q in=c shape=32,256,28,28 dtype=BF16\n"), False),      # a second reader of the convolution
+    (dict(res="reshape"), False), (dict(add_in="r,w"), False),
+    (dict(n=1, hw=50), False), (dict(n=2, hw=51), True),                           # 1.22 and 2.54 MiB
+    (dict(ic=256, n=10, hw=28), True), (dict(ic=256, n=11, hw=28), False)])        # 3.83 and 4.21 MiB of a layer that does not widen
+def test_layers_give_up_large_tiles_only_for_an_add_they_take(add_tails, case, kept):
+    assert add_tails(_residual(**case)) == (["c"] if kept else [])
+
+
+def test_layers_that_give_up_large_tiles_by_option(add_tails):
+    assert add_tails(_residual(), fuse=0) == []
+    assert add_tails(_residual(n=1, hw=50), fuse=1) == ["c"]            # every add
+    assert add_tails(_residual(n=1, hw=50), fuse=2, batch=3) == ["c"]   # the size is that of all batch slots
+    assert add_tails(_residual("INT8"), fuse=1) == ["c"]
+    assert add_tails(_residual("INT8"), fuse=2) == []
+    assert add_tails(_residual("FP32"), fuse=1) == []

@@ -12,6 +12,7 @@
 #include "f32_kernels.cuh"
 #include "calib_kernels.cuh"
 #include "extra_kernels.cuh"
+#include "module_text.h"
 
 #include <algorithm>
 #include <cmath>
@@ -19,39 +20,6 @@
 #include <sstream>
 
 namespace tpucb {
-
-using Attrs = std::map<std::string, std::string>;
-
-struct ParsedOp {
-  std::string type, name;
-  std::vector<std::string> in;
-  std::vector<int64_t> shape;
-  std::string dtype = "FP32";
-  Attrs attrs;
-  std::string line; // the text the op was parsed from
-  int geti(const char *k, int def = 0) const {
-    auto it = attrs.find(k);
-    return it == attrs.end() ? def : atoi(it->second.c_str());
-  }
-  double getf(const char *k, double def = 0) const {
-    auto it = attrs.find(k);
-    return it == attrs.end() ? def : atof(it->second.c_str());
-  }
-  std::string gets(const char *k, const char *def = "") const {
-    auto it = attrs.find(k);
-    return it == attrs.end() ? std::string(def) : it->second;
-  }
-  // comma-separated integer list attribute (I32ArrayAttr in the reference's op definitions)
-  std::vector<int> getl(const char *k) const {
-    std::vector<int> v;
-    auto it = attrs.find(k);
-    if (it == attrs.end()) return v;
-    std::stringstream ss(it->second);
-    std::string tok;
-    while (std::getline(ss, tok, ',')) v.push_back(atoi(tok.c_str()));
-    return v;
-  }
-};
 
 class Interpreter;
 
@@ -165,9 +133,7 @@ public:
     int cp = 0, wl = 0, wphys = 0;
   };
   std::map<std::string, RowLayout> layout_requests;
-  // Convolutions whose result goes to one residual add only (load_module), planned without the large tiles, whose epilogue has no
-  // add: BF16 ones, and INT8 ones when every add is to be fused (by size, an INT8 layer that takes the large tiles keeps them).
-  std::set<std::string> add_tails;
+  std::set<std::string> add_tails; // convolutions planned so that the add behind them can be fused (residual_add_tails)
 
   TensorPtr make_tensor(const std::string &name, const std::vector<int64_t> &shape, int dtype) {
     auto t = std::make_shared<DevTensor>();
@@ -1908,35 +1874,6 @@ private:
 
 // ====================================================================== Interpreter bodies
 
-inline std::vector<std::string> split(const std::string &s, char sep) {
-  std::vector<std::string> out;
-  std::stringstream ss(s);
-  std::string tok;
-  while (std::getline(ss, tok, sep)) out.push_back(tok);
-  return out;
-}
-
-inline ParsedOp parse_line(const std::string &line) {
-  ParsedOp op;
-  op.line = line;
-  std::stringstream ss(line);
-  std::string tok;
-  ss >> op.type;
-  while (ss >> tok) {
-    auto eq = tok.find('=');
-    TPUCB_CHECK(eq != std::string::npos, "module text: token '%s' is not key=value", tok.c_str());
-    std::string k = tok.substr(0, eq), v = tok.substr(eq + 1);
-    if (k == "name") op.name = v;
-    else if (k == "in") op.in = split(v, ',');
-    else if (k == "shape") {
-      for (auto &d : split(v, ',')) op.shape.push_back(atoll(d.c_str()));
-    } else if (k == "dtype") op.dtype = v;
-    else op.attrs[k] = v;
-  }
-  TPUCB_CHECK(!op.name.empty(), "module text: op '%s' has no name", op.type.c_str());
-  return op;
-}
-
 // Who writes the remainder operand (x minus the upper 19 bits of x) of the fp32 tensors that TF32 x 3 convolutions read:
 // the kernel that produces the tensor when it can (an fp32 eltwise add or another TF32 x 3 convolution: 4 more bytes
 // written per value, no separate pass), else the split pass of the FIRST convolution that reads it; later readers of
@@ -2014,15 +1951,7 @@ inline void Interpreter::fuse_activation_chains(const std::map<std::string, int>
     const int self = pos[0] > pos[1] ? 0 : 1, other = 1 - self;
     auto *cv = dynamic_cast<Conv2DOp *>(kernels[pos[self]].get());
     if (!cv || !cv->can_fuse_add() || !single_use(cv->name)) continue;
-    // By size: layers that widen their input, results of 2.5 MiB and more. The launch that goes and the operand that is not read
-    // again count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
-    // modules in flight, none fused -> by this rule: INT8 batch 8 332 / 166 -> 319 / 158, 19 421 / 257 -> 393 / 236, 64 740 / 627 ->
-    // 693 / 573, 256 2423 / 2280 -> 2210 / 2011; smaller results gain too, a little (every add fused: batch 3 278 / 117 -> 272 /
-    // 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 499 / 233 -> 486 / 213, 32 803 / 602 -> 776 / 525, 128 2231 / 2174 ->
-    // 2088 / 1791. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
-    // fused: batch 1 182 / 65 -> 167 / 62, 7 217 / 104 -> 203 / 103, 32 357 / 235 -> 338 / 234, but 128 864 / 713 -> 851 / 719).
-    const bool widens = cv->out()->cp > cv->in()->cp;
-    if (fuse_residual_add == 2 && (widens ? cv->out()->bytes() < 5u << 19 : cv->out()->bytes() > 4u << 20)) continue;
+    if (fuse_residual_add == 2 && !add_fused_by_size(cv->out()->cp > cv->in()->cp, cv->out()->bytes())) continue;
     const TensorPtr &a = cv->out(), &r = ins[other], &o = ad->out();
     if (a->cp != r->cp || a->cp != o->cp || a->bytes() != r->bytes() || a->bytes() != o->bytes() || a->padded_rows() ||
         r->padded_rows() || o->padded_rows() || a->cp % 16 != 0)
@@ -2299,16 +2228,7 @@ inline void Interpreter::load_module(const std::string &text) {
       by_name[op.name] = &op;
       for (auto &nm : op.in) n_uses[nm]++;
     }
-    for (auto &op : parsed) {
-      if (!fuse_activations || !fuse_residual_add || op.type != "eltwise_add" || op.in.size() < 2) continue;
-      if (!(op.dtype == "BF16" || (op.dtype == "INT8" && fuse_residual_add == 1))) continue;
-      const ParsedOp *late = nullptr;
-      for (int k = 0; k < 2; ++k) {
-        auto it = by_name.find(op.in[k]);
-        if (it != by_name.end() && (!late || it->second > late)) late = it->second;
-      }
-      if (late && (late->type == "conv_2d" || late->type == "deconv_2d") && n_uses[late->name] == 1) add_tails.insert(late->name);
-    }
+    if (fuse_activations) add_tails = residual_add_tails(parsed, by_name, n_uses, fuse_residual_add, max_batch);
     for (auto &op : parsed) {
       if (op.type != "conv_2d" || (op.dtype != "INT8" && op.dtype != "BF16") || op.in.empty()) continue;
       auto it = by_name.find(op.in[0]);

@@ -1,0 +1,120 @@
+// The module text: its ops, and what is decided from the ops alone before any of them is built.
+#pragma once
+#include "host_common.h"
+
+#include <algorithm>
+#include <cstdlib>
+#include <sstream>
+
+namespace tpucb {
+
+using Attrs = std::map<std::string, std::string>;
+
+struct ParsedOp {
+  std::string type, name;
+  std::vector<std::string> in;
+  std::vector<int64_t> shape;
+  std::string dtype = "FP32";
+  Attrs attrs;
+  std::string line; // the text the op was parsed from
+  int geti(const char *k, int def = 0) const {
+    auto it = attrs.find(k);
+    return it == attrs.end() ? def : atoi(it->second.c_str());
+  }
+  double getf(const char *k, double def = 0) const {
+    auto it = attrs.find(k);
+    return it == attrs.end() ? def : atof(it->second.c_str());
+  }
+  std::string gets(const char *k, const char *def = "") const {
+    auto it = attrs.find(k);
+    return it == attrs.end() ? std::string(def) : it->second;
+  }
+  // comma-separated integer list attribute (I32ArrayAttr in the reference's op definitions)
+  std::vector<int> getl(const char *k) const {
+    std::vector<int> v;
+    auto it = attrs.find(k);
+    if (it == attrs.end()) return v;
+    std::stringstream ss(it->second);
+    std::string tok;
+    while (std::getline(ss, tok, ',')) v.push_back(atoi(tok.c_str()));
+    return v;
+  }
+};
+
+inline std::vector<std::string> split(const std::string &s, char sep) {
+  std::vector<std::string> out;
+  std::stringstream ss(s);
+  std::string tok;
+  while (std::getline(ss, tok, sep)) out.push_back(tok);
+  return out;
+}
+
+inline ParsedOp parse_line(const std::string &line) {
+  ParsedOp op;
+  op.line = line;
+  std::stringstream ss(line);
+  std::string tok;
+  ss >> op.type;
+  while (ss >> tok) {
+    auto eq = tok.find('=');
+    TPUCB_CHECK(eq != std::string::npos, "module text: token '%s' is not key=value", tok.c_str());
+    std::string k = tok.substr(0, eq), v = tok.substr(eq + 1);
+    if (k == "name") op.name = v;
+    else if (k == "in") op.in = split(v, ',');
+    else if (k == "shape") {
+      for (auto &d : split(v, ',')) op.shape.push_back(atoll(d.c_str()));
+    } else if (k == "dtype") op.dtype = v;
+    else op.attrs[k] = v;
+  }
+  TPUCB_CHECK(!op.name.empty(), "module text: op '%s' has no name", op.type.c_str());
+  return op;
+}
+
+// Which residual adds run in the epilogue of the convolution that produces their later operand (fuse_residual_add = 2): those
+// behind layers that widen their input, results of 2.5 MiB and more. The launch that goes and the operand that is not read again
+// count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
+// modules in flight, none fused -> by this rule: INT8 batch 8 332 / 166 -> 319 / 158, 19 421 / 257 -> 393 / 236, 64 740 / 627 ->
+// 693 / 573, 256 2423 / 2280 -> 2210 / 2011; smaller results gain too, a little (every add fused: batch 3 278 / 117 -> 272 /
+// 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 499 / 233 -> 486 / 213, 32 803 / 602 -> 776 / 525, 128 2231 / 2174 ->
+// 2088 / 1791. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
+// fused: batch 1 182 / 65 -> 167 / 62, 7 217 / 104 -> 203 / 103, 32 357 / 235 -> 338 / 234, but 128 864 / 713 -> 851 / 719).
+inline bool add_fused_by_size(bool widens, size_t result_bytes) { return widens ? result_bytes >= 5u << 19 : result_bytes <= 4u << 20; }
+
+// The convolutions whose result goes to one residual add only, an add that their epilogue is going to take. They are planned
+// without the large tiles of conv_big.cuh, whose epilogue has no add: BF16 ones, and INT8 ones when every add is to be fused (by
+// size, an INT8 layer that takes the large tiles keeps them). The conditions are those of fuse_activation_chains, as far as the
+// ops tell: a layer kept off the large tiles for an add that then runs by itself would have neither.
+inline std::set<std::string> residual_add_tails(const std::vector<ParsedOp> &ops, const std::map<std::string, const ParsedOp *> &by_name,
+                                                const std::map<std::string, int> &n_uses, int fuse, int max_batch) {
+  std::set<std::string> tails;
+  for (const ParsedOp &add : ops) {
+    const bool bf16 = add.dtype == "BF16";
+    if (fuse == 0 || add.type != "eltwise_add" || !(bf16 || (add.dtype == "INT8" && fuse == 1))) continue;
+    std::vector<const ParsedOp *> from; // the operands that are results
+    for (auto &nm : add.in) {
+      auto it = by_name.find(nm);
+      if (it != by_name.end() && it->second < &add) from.push_back(it->second);
+    }
+    if (from.size() != 2 || from[0] == from[1]) continue;
+    const ParsedOp &conv = *std::max(from[0], from[1]), &other = *std::min(from[0], from[1]);
+    if (conv.type != "conv_2d" && conv.type != "deconv_2d") continue;
+    if (other.type == "reshape" || conv.geti("g", 1) != 1 || conv.geti("do_relu", 0) || n_uses.at(conv.name) != 1) continue;
+    if (conv.dtype != add.dtype || other.dtype != add.dtype || conv.shape != add.shape || other.shape != add.shape) continue;
+    bool ones = true;
+    std::stringstream coeffs(add.gets("coeff"));
+    for (std::string c; std::getline(coeffs, c, ',');) ones = ones && atof(c.c_str()) == 1.0;
+    if (bf16 && !(add.geti("do_relu", 0) && ones)) continue;
+    if (fuse == 2) {
+      auto src = conv.in.empty() ? by_name.end() : by_name.find(conv.in[0]);
+      if (src == by_name.end()) continue;
+      auto extent = [](const ParsedOp &op, size_t k) { return k < op.shape.size() ? op.shape[k] : (int64_t)1; };
+      const int pitch = round_up((int)extent(conv, 1), 16);
+      const size_t pixels = (size_t)extent(conv, 0) * max_batch * extent(conv, 2) * extent(conv, 3);
+      if (!add_fused_by_size(pitch > round_up((int)extent(*src->second, 1), 16), pixels * pitch * (bf16 ? 2 : 1))) continue;
+    }
+    tails.insert(conv.name);
+  }
+  return tails;
+}
+
+} // namespace tpucb
