@@ -223,12 +223,13 @@ def test_residual_add_with_prefetch(case):
     m.close()
 
 
-@pytest.mark.parametrize("case", [  # n, ic, oc, hw, big_tiles: by size (196 tiles of 256 pixels, 9 K blocks) and forced on a small one
-    (16, 64, 128, 56, 1), (2, 96, 136, 13, 1256), (2, 96, 136, 13, 2192)])
-def test_every_add_is_fused_when_asked(case):
-    """fuse_residual_add = 1 on layers that would run large tiles: the add launches nothing, both tensors keep their bits."""
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, big_tiles, fuse_residual_add
+    (16, 64, 128, 56, 1, 1), (2, 96, 136, 13, 1256, 1), (2, 96, 136, 13, 2192, 1),   # every add: large tiles by size, and forced on a small layer
+    (32, 64, 128, 56, 1, 2), (97, 256, 512, 14, 1, 2)])                             # by size: 9 and 18 K blocks of a layer that widens
+def test_adds_behind_layers_that_fill_the_gpu(case):
+    """Layers that would run large tiles do not when their add is fused: it launches nothing, both tensors keep their bits."""
     from tpu_compiler_b200 import module
-    n, ic, oc, hw, big = case
+    n, ic, oc, hw, big, mode = case
     model = graphs.single_conv_i8(1, ic, oc, hw, 3, 1, 1, relu=False, seed=78)
     w = dict(model.weights, ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
     shape = "shape=%d,%d,%d,%d dtype=INT8" % (n, oc, hw, hw)
@@ -237,7 +238,7 @@ def test_every_add_is_fused_when_asked(case):
     rng = np.random.default_rng(oc)
     x = {"x": rng.integers(-128, 128, (n, ic, hw, hw)).astype(np.float32), "res": rng.integers(-128, 128, (n, oc, hw, hw)).astype(np.float32)}
     got = []
-    for fuse in (0, 1):
+    for fuse in (0, mode):
         m = module(0)
         m.set_option("fuse_residual_add", fuse)
         m.set_option("big_tiles", big)

@@ -319,5 +319,10 @@ def test_layers_that_give_up_large_tiles_by_option(add_tails):
     assert add_tails(_residual(n=1, hw=50), fuse=1) == ["c"]            # every add
     assert add_tails(_residual(n=1, hw=50), fuse=2, batch=3) == ["c"]   # the size is that of all batch slots
     assert add_tails(_residual("INT8"), fuse=1) == ["c"]
-    assert add_tails(_residual("INT8"), fuse=2) == []
+    assert add_tails(_residual("INT8", n=100, ic=1536, oc=2048), fuse=2) == ["c"]                 # 12 K blocks, 153 MiB
+    k3 = "kh=3 kw=3 pt=1 pb=1 pl=1 pr=1"
+    assert add_tails(_residual("INT8", n=26, ic=256, oc=512, conv=k3), fuse=2) == ["c"]           # 18 blocks, 9.95 MiB
+    assert add_tails(_residual("INT8", n=27, ic=256, oc=512, conv=k3), fuse=2) == []              # 10.3 MiB: the loop counts, not the add
+    assert add_tails(_residual("INT8", n=10, ic=257, oc=512, conv=k3), fuse=2) == []              # 27
+    assert add_tails(_residual("INT8", n=27, ic=257, oc=512, conv=k3), fuse=1) == ["c"]
     assert add_tails(_residual("FP32"), fuse=1) == []

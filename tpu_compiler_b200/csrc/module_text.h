@@ -81,15 +81,24 @@ inline ParsedOp parse_line(const std::string &line) {
 inline bool add_fused_by_size(bool widens, size_t result_bytes) { return widens ? result_bytes >= 5u << 19 : result_bytes <= 4u << 20; }
 
 // The convolutions whose result goes to one residual add only, an add that their epilogue is going to take. They are planned
-// without the large tiles of conv_big.cuh, whose epilogue has no add: BF16 ones, and INT8 ones when every add is to be fused (by
-// size, an INT8 layer that takes the large tiles keeps them). The conditions are those of fuse_activation_chains, as far as the
-// ops tell: a layer kept off the large tiles for an add that then runs by itself would have neither.
+// without the large tiles of conv_big.cuh, whose epilogue has no add. The conditions are those of fuse_activation_chains, as far
+// as the ops tell: a layer kept off the large tiles for an add that then runs by itself would have neither.
+// INT8 layers whose time is the loop's keep the large tiles and leave the add to a launch of its own (unless every add is to be
+// fused): those of more than 12 K blocks, up to 10 MiB those of 24 and more. Layer and add, us alone / with three modules in
+// flight, large tiles and add -> fused:
+//   8 blocks (1x1 1024 -> 2048, 7x7) 12 MiB 22.2 / 18.0 -> 18.5 / 18.1, 24 MiB 35.1 / 34.2 -> 34.8 / 33.6; 9 (3x3 64 -> 128, 56x56) 6 MiB 16.6 /
+//   10.8 -> 12.0 / 9.8, 12 MiB 22.5 / 17.9 -> 17.4 / 16.5, 24 MiB 37.0 / 33.2 -> 31.2 / 28.9; (128 -> 256, 28x28) 49 MiB 71.5 / 72.7 ->
+//   71.0 / 68.9; 12 (1x1 1536 -> 2048) 12 MiB 24.7 / 22.2 -> 22.1 / 22.3;
+//   18 blocks, 3x3 at 14x14: 256 -> 512 6 MiB 22.7 / 15.1 -> 19.3 / 14.7, 192 -> 384 9 MiB 30.6 / 25.1 -> 23.3 / 22.5, 256 -> 512 9 MiB
+//   24.8 / 21.9 -> 20.9 / 21.8;
+//   not: 256 -> 512 12 MiB 31.0 / 27.1 against 28.8 / 28.8, 24 MiB 53.5 / 51.3 against 57.2 / 55.5; 15 blocks (1x1 1900 -> 2048) 24 MiB
+//   61.8 / 57.5 against 62.3 / 59.7; 27 (3x3 320 -> 512) 6 MiB 28.5 / 19.2 against 25.2 / 20.6, 12 MiB 39.1 / 34.3 against 40.0 / 40.2.
 inline std::set<std::string> residual_add_tails(const std::vector<ParsedOp> &ops, const std::map<std::string, const ParsedOp *> &by_name,
                                                 const std::map<std::string, int> &n_uses, int fuse, int max_batch) {
   std::set<std::string> tails;
   for (const ParsedOp &add : ops) {
     const bool bf16 = add.dtype == "BF16";
-    if (fuse == 0 || add.type != "eltwise_add" || !(bf16 || (add.dtype == "INT8" && fuse == 1))) continue;
+    if (fuse == 0 || add.type != "eltwise_add" || !(bf16 || add.dtype == "INT8")) continue;
     std::vector<const ParsedOp *> from; // the operands that are results
     for (auto &nm : add.in) {
       auto it = by_name.find(nm);
@@ -108,9 +117,11 @@ inline std::set<std::string> residual_add_tails(const std::vector<ParsedOp> &ops
       auto src = conv.in.empty() ? by_name.end() : by_name.find(conv.in[0]);
       if (src == by_name.end()) continue;
       auto extent = [](const ParsedOp &op, size_t k) { return k < op.shape.size() ? op.shape[k] : (int64_t)1; };
-      const int pitch = round_up((int)extent(conv, 1), 16);
-      const size_t pixels = (size_t)extent(conv, 0) * max_batch * extent(conv, 2) * extent(conv, 3);
-      if (!add_fused_by_size(pitch > round_up((int)extent(*src->second, 1), 16), pixels * pitch * (bf16 ? 2 : 1))) continue;
+      const int pitch = round_up((int)extent(conv, 1), 16), in_pitch = round_up((int)extent(*src->second, 1), 16);
+      const size_t bytes = (size_t)extent(conv, 0) * max_batch * extent(conv, 2) * extent(conv, 3) * pitch * (bf16 ? 2 : 1);
+      if (!add_fused_by_size(pitch > in_pitch, bytes)) continue;
+      const int k_blocks = conv.geti("kh", 1) * conv.geti("kw", 1) * ((in_pitch + 127) / 128);
+      if (!bf16 && k_blocks > 12 && (k_blocks >= 24 || bytes > 10u << 20)) continue;
     }
     tails.insert(conv.name);
   }
