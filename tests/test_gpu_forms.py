@@ -408,3 +408,60 @@ def test_float_requantisation_past_its_range(relu, shape):
         text = "input name=x shape=%d,%d,%d,%d dtype=INT8\n" % (n, ic, hw, hw) + conv_text("INT8", n, ic, oc, hw, k, 1, k // 2, 1, int(relu), True)
         got, ref = run_model(text, {"f": f, "b": b, "r": np.where(r < top, r, 9), "m": m}, {"x": x}, ["c"])["c"]
         assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("form", [1256, 1096, 2256, 2192, 2032])  # 1000 CTAs per tile + pixels per tile
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, k, stride; shifts: the floating-point requantisation, the integer one
+    (3, 64, 256, 20, 1, 1, (11, 17)), (2, 96, 136, 13, 3, 1, (11, 15)), (2, 96, 136, 13, 3, 1, (11, 17)),
+    (5, 160, 300, 9, 3, 2, (11, 17)), (1, 1040, 520, 5, 1, 1, (11, 15)), (23, 80, 144, 41, 3, 1, (11, 15)), (23, 80, 144, 41, 3, 1, (11, 17))])
+def test_big_tiles_with_leaky_relu(form, case):
+    """Two stores per column group, the plain result and the activated one: several tiles per CTA, ragged tiles and channel tiles.
+    Shifts of 15 and 16 do not saturate the ends of the floating-point form's range, which K of 720 and more weights reaches."""
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, k, s, shifts = case
+    model = graphs.single_conv_i8(n, ic, oc, hw, k, s, k // 2, relu=False, seed=6300 + ic + k, rshift_range=shifts)
+    o = (hw + 2 * (k // 2) - k) // s + 1
+    text = model.text + ("leaky_relu name=lk in=conv,-,-,-,-,rp,mp,rn,mn shape=%d,%d,%d,%d dtype=INT8 negative_slope=0.1\n" % (n, oc, o, o))
+    got = []
+    for pos in ((4, 13), (0, 0)):  # the positive side rescaled, and as it is
+        w = dict(model.weights, **{nm: np.array([v], np.float32) for nm, v in zip(("rp", "mp", "rn", "mn"), pos + (7, 12))})
+        for mode in (0, form):
+            m = module(0)
+            m.set_option("big_tiles", mode)
+            m.load_text(text, w)
+            assert m.kernel_count() == 1
+            m.set_tensor("x", model.meta["x"])
+            for _ in range(2):
+                m.invoke()
+            got.append([m.get_tensor("conv"), m.get_tensor("lk")])
+            m.close()
+        if n < 23:
+            ref = graph_runner.run(text, w, {"x": model.meta["x"]})
+            assert all(np.array_equal(g, ref[nm]) for g, nm in zip(got[-1], ("conv", "lk")))
+    assert len(np.unique(got[0][0])) > 100  # live values
+    for a, b in ((0, 1), (2, 3)):
+        assert np.array_equal(got[a][0], got[b][0]) and np.array_equal(got[a][1], got[b][1])
+
+
+@pytest.mark.parametrize("scale,fused", [(0.03, True), (9.9e29, True), (-9.9e29, True), (1e30, False), (-1e30, False), (3e36, False), (3.3e38, False)])
+def test_activation_chain_up_to_its_largest_scale(scale, fused):
+    """The fused chain rounds its products without a check for overflow, so scales from 1e30 on keep the three ops: every byte
+    value, the three tensors of the default against those of the ops by themselves."""
+    from tpu_compiler_b200 import module
+    base, slope = graphs.lut_slope_tables("mish")
+    w = {"t0": np.tile(base, 4), "t1": np.tile(slope, 4)}
+    shape = "shape=1,32,4,8"
+    text = ("input name=x %s dtype=INT8\nquant name=d in=x %s dtype=BF16 from=INT8 to=BF16 scale=%r\nmish name=a in=d,t0,t1 %s dtype=BF16\n"
+            "quant name=q in=a %s dtype=INT8 from=BF16 to=INT8 scale=32.0\n" % (shape, shape, scale, shape, shape))
+    x = np.arange(1024, dtype=np.float32).reshape(1, 32, 4, 8) % 256 - 128
+    got = []
+    for on in (0, 1):
+        m = module(0)
+        m.set_option("fuse_activations", on)
+        m.load_text(text, w)
+        m.set_tensor("x", x)
+        m.invoke()
+        got.append([m.get_tensor(nm) for nm in "daq"] + [m.kernel_count()])
+        m.close()
+    assert got[0][3] == 3 and got[1][3] == (1 if fused else 3)
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(got[0][:3], got[1][:3]))

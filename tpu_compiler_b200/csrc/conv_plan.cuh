@@ -450,11 +450,15 @@ inline void finish_plan(ConvPlan &pl, int rows, int taps, int k_inner, int oc_pa
   const int k_iters = taps * p.c_chunks;
   const int n_tiles = (oc_pad + bn - 1) / bn;
   // A launch of few tiles takes half tiles: twice the CTAs, each with half the epilogue and three quarters of the bytes per K
-  // block (us alone and with three modules in flight: ResNet-50 batch 1 313 / 128 -> 292 / 116, BF16 batch 8 657 / 295 -> 594 /
-  // 285, YOLOv4-style batch 1 1069 / 446 -> 905 / 397; 8 x 14 x 14, 256 channels, 26 tiles: 9.3 / 4.7 -> 8.7 / 4.1). Up to a
-  // third of the SMs: with more, launches of other streams that would have run beside this one no longer fit (half tiles
-  // throughout: ResNet-50 batch 19 465 / 330 against 458 / 274, BF16 batch 8 582 / 319; 19 x 14 x 14, 256 channels, 60 tiles:
-  // 9.0 us against 10.2 alone, but 4.4 against 4.2). Quarter tiles gained nothing more.
+  // block. Up to a third of the SMs; us alone / with three modules in flight, no half tiles -> by this rule: ResNet-50 INT8 batch 1
+  // 260.0 / 110.8 -> 240.0 / 98.4, 4 319.6 / 131.7 -> 285.5 / 122.5, 8 354.2 / 159.1 -> 315.2 / 155.7, 19 398.7 / 232.6 -> 385.4 / 229.0, BF16 batch
+  // 2 514.4 / 191.2 -> 435.0 / 162.2, 8 550.0 / 230.1 -> 486.0 / 212.1, YOLOv4-style batch 1 855.5 / 357.1 -> 740.1 / 322.9. With more, launches
+  // of other streams that would have run beside this one no longer fit. Up to half of the SMs: alone faster, in flight level or
+  // slower: INT8 batch 4 285.0 / 123.1, 8 312.8 / 156.0, 19 374.8 / 230.4, BF16 batch 8 483.3 / 215.7, 32 771.0 / 526.5 -> 743.4 / 530.1 (a layer by
+  // itself, 7 x 23 x 23, 5x5 of 72 -> 200 channels, 58 tiles, 15.1 / 5.2 -> 10.9 / 4.8). All that have the SMs for it: 4 284.4 / 128.1, 8 311.4 /
+  // 164.3, 19 373.0 / 247.3, BF16 8 465.5 / 227.4, 32 717.4 / 548.5. fp32 runs alone and has nothing to gain from another line: batch
+  // 4 1449 (none 1488, half of the SMs 1441, all 1446), 16 1945 (1954, 1937, 1964), 30 2627 (2629, 2627, 2678), 64 4500 (4502, 4503,
+  // 4544). Quarter tiles gained nothing more.
   p.m_tile = p.dual ? 256 : 128;
   if (!p.dual && (rows + 127) / 128 * n_tiles * 3 <= sm_count) p.m_tile = 64;
   const int m_tiles = (rows + p.m_tile - 1) / p.m_tile;

@@ -70,14 +70,19 @@ inline ParsedOp parse_line(const std::string &line) {
   return op;
 }
 
-// Which residual adds run in the epilogue of the convolution that produces their later operand (fuse_residual_add = 2): those
-// behind layers that widen their input, results of 2.5 MiB and more. The launch that goes and the operand that is not read again
-// count; the epilogue has room for the add's 14 instructions per four values. ResNet-50, us per step alone / with three
-// modules in flight, none fused -> by this rule: INT8 batch 8 332 / 166 -> 319 / 158, 19 421 / 257 -> 393 / 236, 64 740 / 627 ->
-// 693 / 573, 256 2423 / 2280 -> 2210 / 2011; smaller results gain too, a little (every add fused: batch 3 278 / 117 -> 272 /
-// 109, 8 323 / 147); BF16 (two operands, ReLU): batch 8 499 / 233 -> 486 / 213, 32 803 / 602 -> 776 / 525, 128 2231 / 2174 ->
-// 2088 / 1791. Layers that narrow it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, every add
-// fused: batch 1 182 / 65 -> 167 / 62, 7 217 / 104 -> 203 / 103, 32 357 / 235 -> 338 / 234, but 128 864 / 713 -> 851 / 719).
+// Which residual adds run in the epilogue of the convolution that produces their later operand (fuse_residual_add = 2). The launch
+// that goes and the operand that is not read again count; the epilogue has room for the add's 14 instructions per four values.
+// Behind layers that widen their input: results of 2.5 MiB and more. ResNet-50, us per step alone / with three modules in flight,
+// none fused -> by this rule: INT8 batch 8 328.5 / 161.6 -> 314.3 / 155.3, 19 416.6 / 249.1 -> 385.9 / 230.3, 64 729.5 / 621.1 -> 689.7 /
+// 561.4, 256 2423 / 2280 -> 2210 / 2011; BF16 (two operands, ReLU) batch 8 498.9 / 233.7 -> 486.9 / 213.6, 32 800.7 / 601.5 -> 779.9 /
+// 527.2, 128 2231 / 2174 -> 2088 / 1791. The line is not where the two sides meet: it is that of the epilogue before this one, under
+// which smaller results lost 2 to 7 us alone. With this one they gain: every add fused, INT8 batch 1 (none by this rule) 240.4 / 97.8 ->
+// 230.7 / 91.7, 3 (none) 273.6 / 114.2 -> 265.0 / 105.7, 8 315.7 / 143.5, 12 340.5 / 187.2 -> 330.7 / 173.1, 19 385.4 / 225.5, 32 484.9 /
+// 329.8 against 484.3 / 329.2; BF16 batch 1 (none) 410.9 / 151.9 -> 404.8 / 146.6, 4 446.7 / 174.7 against 450.0 / 177.4. Calls at
+// small batches that want them set the option to 1.
+// Behind layers that do not widen it (a long K, a short result): up to 4 MiB, where the launch counts (MobileNet-v2, none -> by this
+// rule: batch 1 178.2 / 63.8 -> 162.3 / 60.3, 7 213.1 / 104.0 -> 200.3 / 102.1, 32 354.8 / 233.2 -> 335.6 / 234.3, 128 861.0 / 711.6 -> 845.8 /
+// 712.5, there every add fused 849.0 / 715.5).
 inline bool add_fused_by_size(bool widens, size_t result_bytes) { return widens ? result_bytes >= 5u << 19 : result_bytes <= 4u << 20; }
 
 // The convolutions whose result goes to one residual add only, an add that their epilogue is going to take. They are planned
