@@ -156,7 +156,7 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          self-test of the error path. Every wait inside the tensor-core kernels is bounded (1024 rounds of 1024
  *          polls); when one runs out the kernel records a code in the interpreter's device error word, drains its
  *          copies, frees its tensor memory and returns, and the next tpucb_interp_sync / invoke reports it as an
- *          error status while the interpreter stays usable. With this option the INT8 convolutions of the next
+ *          error status while the interpreter stays usable. With this option the tensor-core convolutions of the next
  *          module never hand their accumulator back and wait only `rounds` rounds, so that exactly this happens.
  *          "fuse_residual_add" (0 never, 1 always, 2 = default: by size; read by the next load_module; needs fuse_activations): an INT8
  *          two-input eltwise add (or a BF16 one with ReLU) whose later-produced operand is a tensor-core convolution that feeds nothing else

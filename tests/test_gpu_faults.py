@@ -71,17 +71,30 @@ def test_malformed_modules_are_refused_with_a_status():
     m.close()
 
 
-@pytest.mark.parametrize("form", ["big_tiles 1256", "big_tiles 2256", "fused add"])
-def test_bounded_wait_runs_out_in_the_other_forms(form):
-    """The kernels whose epilogue warps meet at barriers: after the MMA issuer's wait and then theirs have run out, every warp (and
-    both CTAs of a pair) still leaves, and the interpreter stays usable."""
+@pytest.mark.parametrize("form,dtype", [
+    ("big_tiles 1256", "INT8"), ("big_tiles 2256", "INT8"), ("fused add", "INT8"), ("small tiles", "BF16"), ("big_tiles 1256", "BF16"),
+    ("big_tiles 2256", "BF16"), ("fused add", "BF16"), ("small tiles", "FP32"), ("big_tiles 1256", "FP32"), ("big_tiles 2256", "FP32"),
+    ("stem", "FP32")])
+def test_bounded_wait_runs_out_in_the_other_forms(form, dtype):
+    """The kernels whose epilogue warps meet at barriers, and the image stem: after the MMA issuer's wait and then theirs have run
+    out, every warp (and both CTAs of a pair) still leaves, and the interpreter stays usable."""
     from tpu_compiler_b200 import TpucbError, module
-    k, hw = (1, 56) if form == "fused add" else (3, 28)
-    model = graphs.single_conv_i8(64, 64, 256, hw, k, 1, k // 2, relu=False, seed=37)  # more than two tiles per CTA
-    text, w, x, names = model.text, dict(model.weights), {"x": model.meta["x"]}, ["conv"]
+    n, ic, oc = (16, 3, 64) if form == "stem" else (64, 64, 256)
+    k, hw = (1, 56) if form == "fused add" else ((3, 56) if form == "stem" else (3, 28))  # more than two tiles per CTA
+    if dtype == "INT8":
+        model = graphs.single_conv_i8(n, ic, oc, hw, k, 1, k // 2, relu=False, seed=37)
+        text, w, x = model.text, dict(model.weights), {"x": model.meta["x"]}
+    else:
+        rng = np.random.default_rng(37)
+        cut = graphs._bf16_np if dtype == "BF16" else (lambda v: np.asarray(v, np.float32))
+        w = {"f": cut(rng.normal(0, 0.1, (oc, ic, k, k))), "b": rng.normal(0, 0.2, oc).astype(np.float32)}
+        x = {"x": cut(rng.normal(0, 1, (n, ic, hw, hw)))}
+        text = ("input name=x shape=%d,%d,%d,%d dtype=%s\nconv_2d name=conv in=x,f,b shape=%d,%d,%d,%d dtype=%s kh=%d kw=%d sh=1 sw=1 pt=%d "
+                "pb=%d pl=%d pr=%d dh=1 dw=1 g=1 do_relu=0 with_bias=1\n" % ((n, ic, hw, hw, dtype, n, oc, hw, hw, dtype, k, k) + (k // 2,) * 4))
+    names = ["conv"]
     if form == "fused add":
-        shape = "shape=64,256,%d,%d dtype=INT8" % (hw, hw)
-        text = "input name=res %s\n" % shape + text + "eltwise_add name=s in=res,conv,-,-,ar,am %s do_relu=1\n" % shape
+        shape = "shape=64,256,%d,%d dtype=%s" % (hw, hw, dtype)
+        text = "input name=res %s\n" % shape + text + "eltwise_add name=s in=res,conv%s %s do_relu=1\n" % (",-,-,ar,am" if dtype == "INT8" else "", shape)
         w.update(ar=np.array([7.0], np.float32), am=np.array([70.0, 60.0], np.float32))
         x["res"], names = np.random.default_rng(3).integers(-128, 128, (64, 256, hw, hw)).astype(np.float32), ["conv", "s"]
     got = []
@@ -91,7 +104,7 @@ def test_bounded_wait_runs_out_in_the_other_forms(form):
         if form == "fused add":
             m.set_option("fuse_residual_add", 1 if rounds else 0)
         else:
-            m.set_option("big_tiles", int(form.split()[1]) if rounds else 0)
+            m.set_option("big_tiles", int(form.split()[1]) if rounds and form.startswith("big") else 0)
         m.load_text(text, w)
         for name, v in x.items():
             m.set_tensor(name, v)
@@ -103,7 +116,7 @@ def test_bounded_wait_runs_out_in_the_other_forms(form):
             m.invoke()
             got.append([m.get_tensor(n) for n in names])
     m.set_option("fuse_residual_add", 1)
-    m.set_option("big_tiles", 1 if form == "fused add" else int(form.split()[1]))
+    m.set_option("big_tiles", int(form.split()[1]) if form.startswith("big") else 1)
     m.load_text(text, w)
     for name, v in x.items():
         m.set_tensor(name, v)

@@ -45,9 +45,11 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
   const uint32_t wgt = base + kStemHeader, act = wgt + 2 * part; // wh, wl; xl, xh
 
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int tiles = (p.M_total + kStemPx - 1) / kStemPx;
+  int tiles = (p.M_total + kStemPx - 1) / kStemPx;
+  const int wait_rounds = p.wait_rounds > 0 ? p.wait_rounds : 1024;
   pdl_trigger();
   if (threadIdx.x == 0) {
+    const int gave_up = *reinterpret_cast<volatile int *>(p.err); // as in conv_gemm_body
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(bar_full + 8 * i, 8);
       ptx::mbar_init(bar_empty + 8 * i, 1);
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
     }
     ptx::mbar_init(bar_w, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    *abort_flag = *reinterpret_cast<volatile int *>(p.err);
+    *abort_flag = gave_up;
     ptx::mbar_expect_tx(bar_w, 2 * part); // written at load time only: the copy need not wait for the previous kernel
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(wgt), "l"(a.w),
                  "r"(2 * part), "r"(bar_w) : "memory");
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if (*abort_flag != 0) tiles = 0;
   auto gave_up = [&](int code) {
     if (lane == 0 && !*abort_flag) report_error(p.err, code);
     *abort_flag = 1;
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
       bool ok = true;
 #pragma unroll
       for (int h = 0; h < 2; ++h) { // the remainders, then the high parts: the tensor core reads the upper 19 bits of the value itself
-        if (t > 0 && !ptx::mbar_wait_warp(bar_empty + 8 * h, (uint32_t)((t - 1) & 1), abort_flag, 1024)) {
+        if (t > 0 && !ptx::mbar_wait_warp(bar_empty + 8 * h, (uint32_t)((t - 1) & 1), abort_flag, wait_rounds)) {
           gave_up(kErrEmptyWait);
           ok = false;
           break;
@@ -130,19 +133,19 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
     // unswizzled operand: 8 rows x 16 bytes lie together, the next 8 rows 128 bytes on, the next 16 bytes of K 1024
     const uint32_t hi = (128u >> 4) | (1u << 14), lbo = (1024u >> 4) << 16;
     const uint32_t wh = wgt >> 4 | lbo, wl = (wgt + part) >> 4 | lbo, xl = act >> 4 | lbo, xh = (act + part) >> 4 | lbo;
-    bool ok = ptx::mbar_wait_warp(bar_w, 0u, abort_flag, 1024);
+    bool ok = ptx::mbar_wait_warp(bar_w, 0u, abort_flag, wait_rounds);
     if (!ok) gave_up(kErrFullWait);
     int t = 0;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++t) {
       const int buf = t & 1;
-      if (t >= 2 && !ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, 1024)) {
+      if (t >= 2 && !ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
         gave_up(kErrAccWait);
         break;
       }
       const uint32_t d = tmem_base + (uint32_t)buf * kStemPx;
       for (int term = 0; term < 3 && ok; ++term) {
         if (term < 2) {
-          ok = ptx::mbar_wait_warp(bar_full + 8 * term, (uint32_t)(t & 1), abort_flag, 1024);
+          ok = ptx::mbar_wait_warp(bar_full + 8 * term, (uint32_t)(t & 1), abort_flag, wait_rounds);
           if (!ok) {
             gave_up(kErrFullWait);
             break;
@@ -171,7 +174,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
     int t = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
       const int buf = t & 1, m0 = tile * kStemPx;
-      if (!ptx::mbar_wait_warp(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, 1024)) {
+      if (!ptx::mbar_wait_warp(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds)) {
         gave_up(kErrAccWait);
         break;
       }
@@ -180,7 +183,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
       epilogue_channels_f32<RELU>(p, tmem_base + (uint32_t)buf * kStemPx + ((uint32_t)(quarter * 32) << 16), out, ch_ok, m0, half, 2, bias, kStemPx);
       ptx::tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty + 8 * buf) : "memory");
+      if (lane == 0 && !p.lose_arrival) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_acc_empty + 8 * buf) : "memory");
     }
   }
 

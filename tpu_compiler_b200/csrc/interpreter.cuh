@@ -222,10 +222,14 @@ public:
   // then take their SMs in the order the predecessor's CTAs leave instead of evenly.
   int use_pdl = 1;
   void capture_graph();
-  // Self-test (option "selftest_lost_arrival", read by the next load_module): > 0 makes every INT8 tensor-core
+  // Self-test (option "selftest_lost_arrival", read by the next load_module): > 0 makes every tensor-core
   // convolution built from then on lose its accumulator hand-back and wait only that many rounds of 1024 polls
   // (ConvGemmParams::wait_rounds / lose_arrival), so that a launch ends with a bounded-wait error status.
   int selftest_lost_arrival = 0;
+  void selftest_waits(ConvGemmParams &p) const {
+    p.wait_rounds = selftest_lost_arrival;
+    p.lose_arrival = selftest_lost_arrival > 0;
+  }
   bool split_k = true; // set before load_module: launches with few tiles and a long K share each tile among CTAs
   // partial-sum workspaces of the split-K plans (zero between launches; cleared again after a failed launch)
   std::vector<std::pair<void *, size_t>> split_ws;
@@ -605,10 +609,7 @@ public:
         encode_matrix_map(&pl.tmA, pl.patch_buf, rows, a.kp, a.kp, p.BK, p.m_tile);
         encode_weight_map(&pl.tmB, d_w, ocg_pad, 1, a.kp, p.BK, p.dual ? 192 : p.BN);
       }
-      if (I.selftest_lost_arrival > 0) {
-        pl.p.wait_rounds = I.selftest_lost_arrival;
-        pl.p.lose_arrival = 1;
-      }
+      I.selftest_waits(p);
       I.attach_split_ws(pl);
       conv_kernel_ready(pl);
       plans_.push_back(pl);
@@ -635,6 +636,7 @@ public:
     p.err = &I.ss.d_err->code;
     p.out = (int8_t *)out_->dev;
     p.ldc = out_cp * 4; // bytes
+    I.selftest_waits(p);
     std::vector<int32_t> bias_bits(out_cp, 0);
     for (int o = 0; o < g.oc; ++o) bias_bits[o] = (int32_t)f32_bits(bias[o]);
     p.bias = p.mult = p.rshift = I.upload(bias_bits);
@@ -714,6 +716,7 @@ public:
     p.err = &I.ss.d_err->code;
     p.out = (int8_t *)out_->dev;
     p.ldc = d.out_cp * es;
+    I.selftest_waits(p);
     if (kind == 0) {
       p.fastq = requant_fast_flags(rshift, bias, (long long)g_.ic * g_.kh * g_.kw);
       p.bias = I.upload(to_i32(d.bias, d.out_cp));
@@ -721,10 +724,6 @@ public:
       p.rshift = I.upload(to_i32(d.rshift, d.out_cp, true));
       const std::vector<FloatRequant> fq = float_requant(d.w, (size_t)g.ic * g.kh * g.kw, d.bias, d.mult, d.rshift, do_relu_ != 0, d.out_cp);
       if (!fq.empty()) p.fq = I.upload(fq);
-      if (I.selftest_lost_arrival > 0) {
-        p.wait_rounds = I.selftest_lost_arrival;
-        p.lose_arrival = 1;
-      }
     } else {
       std::vector<int32_t> bias_bits(d.out_cp, 0);
       for (size_t o = 0; o < d.bias.size(); ++o) bias_bits[o] = (int32_t)f32_bits(d.bias[o]);
