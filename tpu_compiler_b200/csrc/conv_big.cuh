@@ -169,10 +169,6 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
   }
   // barriers of the pair's first CTA, which counts the copies of both and issues the MMAs
   const uint32_t lead_full = CTAS == 1 ? bar_full : ptx::map_cluster(bar_full, 0);
-  auto gave_up = [&](int code) {
-    if (!*abort_flag) report_error(p.err, code);
-    *abort_flag = 1;
-  };
 
   if (warp <= 1) {
     // ------------------------------------------------------------ copies: warp 0 the activations, warp 1 the weights
@@ -199,7 +195,7 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
         int tap = 0, tr = 0, ts = 0, chunk = 0, term = 0;
         for (int kit = 0; kit < kTerms * k_iters; ++kit, ++it) {
           if (it >= p.stages && !ptx::mbar_wait_warp(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
-            if (lane == 0) gave_up(kErrEmptyWait);
+            wait_expired(p.err, abort_flag, kErrEmptyWait);
             ok = false;
             break;
           }
@@ -259,7 +255,7 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
         const int buf = t & 1;
         if (t >= 2) {
           if (!ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
-            if (lane == 0) gave_up(kErrAccWait);
+            wait_expired(p.err, abort_flag, kErrAccWait);
             break;
           }
           ptx::tcgen05_fence_after();
@@ -269,7 +265,7 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
         auto k_loop = [&](auto whole) {
           for (int kit = 0; kit < kTerms * k_iters; ++kit) {
             if (!ptx::mbar_wait_warp(m_full, mph, abort_flag, wait_rounds)) {
-              if (lane == 0) gave_up(kErrFullWait);
+              wait_expired(p.err, abort_flag, kErrFullWait);
               ok = false;
               break;
             }
@@ -342,7 +338,7 @@ __device__ __forceinline__ void conv_big_body(const CUtensorMap &tmA, const CUte
       bool ok = *abort_flag == 0;
       if (ok) ok = ptx::mbar_wait_bounded(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok && lane == 0) gave_up(kErrAccWait);
+      if (!ok) wait_expired(p.err, abort_flag, kErrAccWait);
       // After an expired wait a warp does no more work, but it comes to every barrier of its group.
       ptx::tcgen05_fence_after();
       const int cols = min(nt, p.M_total - m0); // this tile's pixels

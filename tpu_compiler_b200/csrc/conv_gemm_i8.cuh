@@ -336,6 +336,14 @@ __device__ __forceinline__ void report_error(int *err, int code) {
 
 enum ConvErr { kErrFullWait = 1, kErrEmptyWait = 2, kErrAccWait = 3 };
 
+// A warp's wait has run out: the host is told, unless another role of the CTA has done so, and then the other roles. (The flag is
+// raised behind the read by the lane that reports: a lane that came first would have hidden the error.)
+__device__ __forceinline__ void wait_expired(int *err, volatile int *abort_flag, int code) {
+  if ((threadIdx.x & 31) == 0 && !*abort_flag) report_error(err, code);
+  __syncwarp();
+  *abort_flag = 1;
+}
+
 // Per-channel requantisation constants, held in registers by the thread that owns the channel.
 // The reference computes, for s = acc + bias and multiplier M in [0, 2^31),
 //   hi = SaturatingRoundingDoublingHighMul(s, M) = floor((s * M + 2^30) / 2^31)
@@ -1044,8 +1052,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
           const CUtensorMap *mapA = (TF32 && term == 0) ? &tmA2 : &tmA;
           const CUtensorMap *mapB = (TF32 && term == 1) ? &tmB2 : &tmB;
           if (it >= p.stages && !ptx::mbar_wait_warp(bar_empty + 8 * ps, pph ^ 1u, abort_flag, wait_rounds)) {
-            if (lane == 0 && !*abort_flag) report_error(p.err, kErrEmptyWait);
-            *abort_flag = 1;
+            wait_expired(p.err, abort_flag, kErrEmptyWait);
             ok = false;
             break;
           }
@@ -1121,8 +1128,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
       const int ksteps = p.ksteps;
       if (p.w_resident && (int)blockIdx.x < total_tiles) {
         if (!ptx::mbar_wait_warp(bar_w, 0u, abort_flag, wait_rounds)) {
-          if (lane == 0 && !*abort_flag) report_error(p.err, kErrFullWait);
-          *abort_flag = 1;
+          wait_expired(p.err, abort_flag, kErrFullWait);
           ok = false;
         }
       }
@@ -1136,8 +1142,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         if (t >= 2) {
           // the epilogue must have drained this accumulator buffer (its previous use)
           if (!ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
-            if (lane == 0 && !*abort_flag) report_error(p.err, kErrAccWait);
-            *abort_flag = 1;
+            wait_expired(p.err, abort_flag, kErrAccWait);
             ok = false;
             break;
           }
@@ -1151,8 +1156,7 @@ __device__ __forceinline__ void conv_gemm_body(const CUtensorMap &tmA, const CUt
         auto k_loop = [&](auto whole) {
           for (int kit = k_begin; kit < k_end; ++kit, ++it) {
             if (!ptx::mbar_wait_warp(m_full, mph, abort_flag, wait_rounds)) {
-              if (lane == 0 && !*abort_flag) report_error(p.err, kErrFullWait);
-              *abort_flag = 1;
+              wait_expired(p.err, abort_flag, kErrFullWait);
               ok = false;
               break;
             }

@@ -74,10 +74,6 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   if (*abort_flag != 0) tiles = 0;
-  auto gave_up = [&](int code) {
-    if (lane == 0 && !*abort_flag) report_error(p.err, code);
-    *abort_flag = 1;
-  };
 
   if (warp < 8) {
     // ------------------------------------------------------------------------------------------------------- patches
@@ -108,7 +104,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
 #pragma unroll
       for (int h = 0; h < 2; ++h) { // the remainders, then the high parts: the tensor core reads the upper 19 bits of the value itself
         if (t > 0 && !ptx::mbar_wait_warp(bar_empty + 8 * h, (uint32_t)((t - 1) & 1), abort_flag, wait_rounds)) {
-          gave_up(kErrEmptyWait);
+          wait_expired(p.err, abort_flag, kErrEmptyWait);
           ok = false;
           break;
         }
@@ -134,12 +130,12 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
     const uint32_t hi = (128u >> 4) | (1u << 14), lbo = (1024u >> 4) << 16;
     const uint32_t wh = wgt >> 4 | lbo, wl = (wgt + part) >> 4 | lbo, xl = act >> 4 | lbo, xh = (act + part) >> 4 | lbo;
     bool ok = ptx::mbar_wait_warp(bar_w, 0u, abort_flag, wait_rounds);
-    if (!ok) gave_up(kErrFullWait);
+    if (!ok) wait_expired(p.err, abort_flag, kErrFullWait);
     int t = 0;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++t) {
       const int buf = t & 1;
       if (t >= 2 && !ptx::mbar_wait_warp(bar_acc_empty + 8 * buf, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, wait_rounds)) {
-        gave_up(kErrAccWait);
+        wait_expired(p.err, abort_flag, kErrAccWait);
         break;
       }
       const uint32_t d = tmem_base + (uint32_t)buf * kStemPx;
@@ -147,7 +143,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
         if (term < 2) {
           ok = ptx::mbar_wait_warp(bar_full + 8 * term, (uint32_t)(t & 1), abort_flag, wait_rounds);
           if (!ok) {
-            gave_up(kErrFullWait);
+            wait_expired(p.err, abort_flag, kErrFullWait);
             break;
           }
           ptx::tcgen05_fence_after();
@@ -175,7 +171,7 @@ __global__ void __launch_bounds__(kStemThreads, 1) conv_stem_tf32x3_kernel(const
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
       const int buf = t & 1, m0 = tile * kStemPx;
       if (!ptx::mbar_wait_warp(bar_acc_full + 8 * buf, (uint32_t)((t >> 1) & 1), abort_flag, wait_rounds)) {
-        gave_up(kErrAccWait);
+        wait_expired(p.err, abort_flag, kErrAccWait);
         break;
       }
       ptx::tcgen05_fence_after();
