@@ -135,6 +135,10 @@ int tpucb_interp_get_all_tensor_names(tpucb_interp *it, char *out, size_t cap, s
 int tpucb_interp_get_details(tpucb_interp *it, int outputs, char *out, size_t cap, size_t *needed);
 /* op_info of pymlir (bindings/python/pymlir.cpp:62-97): "name\ttype\tdtype\tshape" lines */
 int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *needed);
+/* How the rules by size, type and value range run a convolution or an inner product (no reference counterpart), as "key=value" words:
+ * tiles (small, big, stem; depthwise; direct), and for the tensor-core forms ctas and pixels per tile, split_k (CTAs that share a
+ * tile's K), requant (float, integer: a high multiply, wide: 64-bit; none outside INT8). Empty for other ops. */
+int tpucb_interp_get_op_form(tpucb_interp *it, const char *name, char *out, size_t cap, size_t *needed);
 
 /* Options: "cuda_graph" (0/1, default 1): replay the op list as one CUDA graph.
  *          "pdl" (0 off, 1 = default, 2 every kernel): programmatic dependent launch. A kernel launched with the
@@ -144,8 +148,8 @@ int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *ne
  *          launches too small to fill the chip, which measured faster than none and than all (on large memory-bound
  *          kernels it costs 1-5%).
  *          "split_k" (0/1, default 1; read by the next load_module): INT8 convolutions and inner products with at most
- *          half as many tiles as SMs and a K that is long enough to pay for the exchange (from about 24 K blocks for
- *          a few tiles to 48 for many) share each tile among several CTAs (exact: int32 partial sums).
+ *          half as many tiles as SMs and a K that is long enough to pay for the exchange (from about 26 K blocks for
+ *          a few tiles to 52 for many, 74 for many tiles of 128 pixels) share each tile among several CTAs (exact: int32 partial sums).
  *          "big_tiles" (0 never, 1 = default: by size, else 1000 * CTAs (1, 2) + pixels (32 .. 256, a multiple of 32): every
  *          layer that can, in this form; read by the next load_module): tensor-core convolutions that fill the GPU and have a
  *          long K run tiles of up to 256 pixels, one CTA per SM, or two SMs per tile.

@@ -106,6 +106,9 @@ def test_bounded_wait_runs_out_in_the_other_forms(form, dtype):
         else:
             m.set_option("big_tiles", int(form.split()[1]) if rounds and form.startswith("big") else 0)
         m.load_text(text, w)
+        if rounds:
+            assert m.op_form("conv")["tiles"] == {"big": "big", "ste": "stem"}.get(form[:3], "small")
+            assert m.kernel_count() == (2 if dtype == "FP32" and form != "stem" else 1)  # fp32: the pass that forms the remainder
         for name, v in x.items():
             m.set_tensor(name, v)
         if rounds:

@@ -8,10 +8,16 @@ from tpu_compiler_b200 import graphs
 pytestmark = pytest.mark.gpu
 
 
-def run_model(text, weights, inputs, names):
+def has_form(m, name, **words):
+    form = m.op_form(name)
+    return all(form.get(k) == v for k, v in words.items())
+
+
+def run_model(text, weights, inputs, names, **form):
     from tpu_compiler_b200 import module
     m = module(0)
     m.load_text(text, weights)
+    assert has_form(m, names[0], **form), m.op_form(names[0])
     for k, v in inputs.items():
         m.set_tensor(k, v)
     m.invoke()
@@ -44,7 +50,7 @@ def test_float_requantisation_edges(relu, mults):
     b[:23] = rng.integers(-3, 4, 23)  # small sums around zero at every shift
     text = "input name=x shape=2,%d,%d,%d dtype=INT8\n" % (ic, hw, hw) + conv_text("INT8", 2, ic, oc, hw, 1, 1, 0, 1, int(relu), True)
     x = rng.integers(-128, 128, (2, ic, hw, hw)).astype(np.float32)
-    got, ref = run_model(text, {"f": f, "b": b, "r": r, "m": m}, {"x": x}, ["c"])["c"]
+    got, ref = run_model(text, {"f": f, "b": b, "r": r, "m": m}, {"x": x}, ["c"], requant="float")["c"]
     assert np.array_equal(got, ref)
 
 
@@ -192,11 +198,11 @@ def test_depthwise_rows_and_requantisation(relu, case, wide):
     w = {"f": rng.integers(-127, 128, (c, 1, 3, 3)).astype(np.float32), "b": rng.integers(-5000, 5000, c).astype(np.float32),
          "r": rng.integers(6, 11, c).astype(np.float32), "m": (rng.integers(2 ** 23, 2 ** 24, c) * 128).astype(np.float32)}
     if wide:
-        w["b"][3] = 2.0 ** 24
+        w["b"][3], w["r"][3] = 2.0 ** 24, 18  # sums past its range, and a shift whose results there are not all saturated
     x = rng.integers(-128, 128, (n, c, hw, hw)).astype(np.float32)
     text = ("input name=x shape=%d,%d,%d,%d dtype=INT8\nconv_2d name=c in=x,f,b,-,-,r,m shape=%d,%d,%d,%d dtype=INT8 kh=3 kw=3 sh=%d sw=%d "
             "pt=1 pb=1 pl=1 pr=1 dh=1 dw=1 g=%d do_relu=%d with_bias=1\n" % (n, c, hw, hw, n, c, o, o, s, s, c, relu))
-    got, ref = run_model(text, w, {"x": x}, ["c"])["c"]
+    got, ref = run_model(text, w, {"x": x}, ["c"], tiles="depthwise", requant="integer" if wide else "float")["c"]
     assert np.array_equal(got, ref)
 
 
@@ -215,6 +221,7 @@ def test_residual_add_with_prefetch(case):
     m = module(0)
     m.set_option("fuse_residual_add", mode)
     m.load_text(text, w)
+    assert m.kernel_count() == 1
     for name, v in x.items():
         m.set_tensor(name, v)
     for _ in range(2):
@@ -269,17 +276,21 @@ def test_download_forms(dtype, shape):
     m.close()
 
 
-@pytest.mark.parametrize("case", [  # n, ic, oc, hw, k: most tiles that are still split in three, in two, and fewest that are not
-    (12, 512, 512, 7, 3), (8, 128, 512, 10, 7), (1, 64, 128, 33, 5), (16, 512, 512, 7, 3)])
+@pytest.mark.parametrize("case", [  # n, ic, oc, hw, k, pixels per tile, parts (148 SMs)
+    (11, 512, 512, 7, 3, 64, 4), (12, 512, 512, 7, 3, 64, 1),  # 36 K blocks: the most tiles that are still split, the fewest that are not
+    (15, 1024, 512, 7, 3, 64, 3), (23, 1024, 512, 7, 3, 64, 2), (24, 1024, 512, 7, 3, 64, 1),  # 72: in three, in two, not
+    (8, 512, 512, 7, 3, 64, 5), (3, 330, 520, 8, 5, 64, 9), (1, 330, 200, 6, 5, 64, 11),        # a last part of fewer K blocks
+    (25, 330, 512, 8, 5, 128, 2), (36, 330, 512, 8, 5, 128, 2), (37, 330, 512, 8, 5, 128, 1)])  # 75: tiles of 128 pixels, whose blocks are shared, too
 def test_split_rule_edges(case):
     from tpu_compiler_b200 import module
-    n, ic, oc, hw, k = case
+    n, ic, oc, hw, k, pixels, parts = case
     model = graphs.single_conv_i8(n, ic, oc, hw, k, 1, k // 2, seed=3300 + k)
     got = []
     for split in (1, 0):
         m = module(0)
         m.set_option("split_k", split)
         m.load_text(model.text, model.weights)
+        assert has_form(m, "conv", tiles="small", pixels=pixels, split_k=parts if split else 1), m.op_form("conv")
         m.set_tensor("x", model.meta["x"])
         for _ in range(2):
             m.invoke()
@@ -316,6 +327,8 @@ def test_bf16_results_past_the_largest_finite(relu):
 def test_big_tiles(dtype, form, case):
     from tpu_compiler_b200 import module
     n, ic, oc, hw, k, s, p, d, relu = case
+    if dtype == "FP32":
+        oc = (oc + 15) // 16 * 16  # (their channels are padded to 4 only, and large tiles take whole sixteens)
     if dtype == "INT8":
         model = graphs.single_conv_i8(n, ic, oc, hw, k, s, p, d, relu=bool(relu), seed=6200 + ic + k)
         text, w, x, name = model.text, model.weights, model.meta["x"], "conv"
@@ -330,6 +343,7 @@ def test_big_tiles(dtype, form, case):
         m = module(0)
         m.set_option("big_tiles", mode)
         m.load_text(text, w)
+        assert has_form(m, name, **(dict(tiles="big", ctas=form // 1000, pixels=form % 1000) if mode else dict(tiles="small"))), m.op_form(name)
         m.set_tensor("x", x)
         for _ in range(2):
             m.invoke()
@@ -396,7 +410,8 @@ def test_float_requantisation_past_its_range(relu, shape):
     f = rng.integers(-127, 128, (oc, ic, k, k)).astype(np.float32)
     f[::3] = np.sign(f[::3]) * 127          # the largest sums
     f[1::3] = np.where(rng.random(f[1::3].shape) < 0.03, f[1::3], 0)
-    r = (np.arange(oc) % 16).astype(np.float32)
+    past = 17 if relu else 16  # from this less one on the integer form, where sums are large
+    r = (np.arange(oc) % past).astype(np.float32)
     r[oc // 2:] = rng.integers(7, 14, oc - oc // 2)
     m = (rng.integers(2 ** 23, 2 ** 24, oc) * 128).astype(np.float32)
     m[::7], m[3::7] = 2.0 ** 30, 2.0 ** 31 - 128
@@ -404,9 +419,10 @@ def test_float_requantisation_past_its_range(relu, shape):
     b[::11] = rng.choice([-1, 1], b[::11].shape) * np.float32(2.0) ** 27
     x = rng.integers(-128, 128, (n, ic, hw, hw)).astype(np.float32)
     x[0, :, : hw // 2] = np.sign(f[0, :, :1, :1] + 0.5) * 127  # in step with the first filter
-    for top in (16, 14):  # with a shift that keeps the layer on the integer form, and without
+    for top in (past, past - 1):  # with a shift that keeps the layer on the integer form, and without
         text = "input name=x shape=%d,%d,%d,%d dtype=INT8\n" % (n, ic, hw, hw) + conv_text("INT8", n, ic, oc, hw, k, 1, k // 2, 1, int(relu), True)
-        got, ref = run_model(text, {"f": f, "b": b, "r": np.where(r < top, r, 9), "m": m}, {"x": x}, ["c"])["c"]
+        got, ref = run_model(text, {"f": f, "b": b, "r": np.where(r < top, r, 9), "m": m}, {"x": x}, ["c"],
+                             requant="integer" if top == past else "float")["c"]
         assert np.array_equal(got, ref)
 
 
@@ -430,6 +446,8 @@ def test_big_tiles_with_leaky_relu(form, case):
             m.set_option("big_tiles", mode)
             m.load_text(text, w)
             assert m.kernel_count() == 1
+            requant = "integer" if shifts[1] == 17 and ic * k * k >= 720 else "float"
+            assert has_form(m, "conv", tiles="big" if mode else "small", requant=requant), m.op_form("conv")
             m.set_tensor("x", model.meta["x"])
             for _ in range(2):
                 m.invoke()
@@ -441,6 +459,33 @@ def test_big_tiles_with_leaky_relu(form, case):
     assert len(np.unique(got[0][0])) > 100  # live values
     for a, b in ((0, 1), (2, 3)):
         assert np.array_equal(got[a][0], got[b][0]) and np.array_equal(got[a][1], got[b][1])
+
+
+@pytest.mark.parametrize("form", [1256, 1096, 2256, 2192, 2032])
+@pytest.mark.parametrize("case", [(2, 48, 144, 13, 3), (23, 16, 144, 41, 1)])  # n, ic, oc, hw, k
+def test_big_tiles_write_remainders(form, case):
+    """An fp32 convolution that another one reads stores its remainder operand from the same buffer, behind its result."""
+    from tpu_compiler_b200 import module
+    n, ic, oc, hw, k = case
+    rng = np.random.default_rng(51 + oc + k)
+    w = {"f": rng.normal(0, 0.1, (oc, ic, k, k)).astype(np.float32), "b": rng.normal(0, 0.2, oc).astype(np.float32),
+         "g": rng.normal(0, 0.1, (64, oc, 1, 1)).astype(np.float32), "h": rng.normal(0, 0.2, 64).astype(np.float32)}
+    x = rng.normal(0, 1, (n, ic, hw, hw)).astype(np.float32)
+    text = ("input name=x shape=%d,%d,%d,%d dtype=FP32\n" % (n, ic, hw, hw) + conv_text("FP32", n, ic, oc, hw, k, 1, k // 2, 1, 1) +
+            conv_text("FP32", n, oc, 64, hw, 1, 1, 0, 1, 0).replace("name=c in=x,f,b", "name=d in=c,g,h"))
+    got = []
+    for mode in (0, form):
+        m = module(0)
+        m.set_option("big_tiles", mode)
+        m.load_text(text, w)
+        assert m.kernel_count() == 3  # the pass that forms the remainder is that of x
+        assert all(has_form(m, nm, tiles="big" if mode else "small") for nm in "cd")
+        m.set_tensor("x", x)
+        for _ in range(2):
+            m.invoke()
+        got.append([m.get_tensor(nm) for nm in "cd"])
+        m.close()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
 
 
 @pytest.mark.parametrize("scale,fused", [(0.03, True), (9.9e29, True), (-9.9e29, True), (1e30, False), (-1e30, False), (3e36, False), (3.3e38, False)])

@@ -55,6 +55,7 @@ def _declare(lib):
         "tpucb_interp_get_all_tensor_names": [vp, cp, sz, szp],
         "tpucb_interp_get_details": [vp, C.c_int, cp, sz, szp],
         "tpucb_interp_get_op_info": [vp, cp, sz, szp],
+        "tpucb_interp_get_op_form": [vp, cp, cp, sz, szp],
         "tpucb_interp_set_option": [vp, cp, C.c_int],
         "tpucb_interp_profile": [vp, fp, C.c_int, ip],
         "tpucb_interp_time_launches": [vp, C.c_int, fp],

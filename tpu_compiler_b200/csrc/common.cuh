@@ -260,7 +260,6 @@ __device__ __forceinline__ unsigned long long pack_b32x2(uint32_t lo, uint32_t h
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
   return d;
 }
-__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) { return pack_b32x2(__float_as_uint(lo), __float_as_uint(hi)); }
 // Two values of one channel: the packed multiply-adds round each half as the single ones do and take one issue slot for two.
 // The constants are held as pairs whose making the compiler may not repeat (it did, before some uses).
 __device__ __forceinline__ unsigned long long hold_pair(float v) {

@@ -591,6 +591,15 @@ inline void pair_layer(DenseLayer &d) {
   d.paired = true;
 }
 
+// How a plan runs, in words (tpucb_interp_get_op_form).
+inline std::string conv_form(const ConvPlan &pl) {
+  const ConvGemmParams &p = pl.p;
+  const bool floating = p.fq && p.split_k <= 1;
+  return std::string("tiles=") + (pl.stem ? "stem" : (pl.ctas > 0 ? "big" : "small")) + " ctas=" + std::to_string(std::max(1, pl.ctas)) +
+         " pixels=" + std::to_string(pl.stem ? kStemPx : p.m_tile) + " split_k=" + std::to_string(std::max(1, p.split_k)) +
+         " requant=" + (pl.bf16 || pl.tf32 ? "none" : (floating ? "float" : (p.fastq & 1 ? "integer" : "wide")));
+}
+
 // The tensor-core kernel of a plan, as a constant that `use` gets.
 template <auto K> struct KernelConstant {
   static constexpr auto value = K;

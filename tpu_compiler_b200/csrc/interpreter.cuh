@@ -34,6 +34,7 @@ public:
     if (!disabled) invoke(s);
   }
   virtual int kernel_launches() const { return 1; }
+  virtual std::string form() const { return ""; } // of a convolution or an inner product: how it runs
   bool disabled = false;
   std::string name, op_type;
   std::vector<int64_t> shape;
@@ -893,6 +894,10 @@ public:
     for (auto &pl : plans_) k += 1 + (pl.use_patch || pl.use_repack || pl.split_src ? 1 : 0);
     return k;
   }
+  std::string form() const override {
+    if (dw_) return std::string("tiles=depthwise requant=") + (!dw_wt_ ? "wide" : (dwargs_.fq ? "float" : "integer"));
+    return plans_.empty() ? std::string("tiles=direct") : conv_form(plans_[0]);
+  }
   bool is_tensor_core() const { return !f32_ && !dw_ && !bf16g_; }
   std::vector<ConvPlan> plans_;
 
@@ -1069,6 +1074,7 @@ public:
     } else if (f32_) launch_fc_f32((const float *)in_->dev, f32_w_, f32_b_, (float *)out_->dev, m_, kdev_, n_, out_->cp, do_relu_, s);
     else launch_conv_plan(plan_, s, I_.sm_count);
   }
+  std::string form() const override { return is_batched() || f32_ ? std::string("tiles=direct") : conv_form(plan_); }
   bool is_batched() const { return batch_ > 0; }
   ConvPlan plan_;
 

@@ -344,6 +344,17 @@ int tpucb_interp_get_details(tpucb_interp *it, int outputs, char *out, size_t ca
   TPUCB_API_END
 }
 
+int tpucb_interp_get_op_form(tpucb_interp *it, const char *name, char *out, size_t cap, size_t *needed) {
+  TPUCB_API_BEGIN
+  TPUCB_CHECK(it && name, "tpucb_interp_get_op_form: bad argument");
+  const OpKernel *op = nullptr;
+  for (auto &k : it->impl.kernels)
+    if (k->name == name) op = k.get();
+  TPUCB_CHECK(op, "tpucb_interp_get_op_form: no op '%s'", name);
+  copy_out(op->form(), out, cap, needed);
+  TPUCB_API_END
+}
+
 int tpucb_interp_get_op_info(tpucb_interp *it, char *out, size_t cap, size_t *needed) {
   TPUCB_API_BEGIN
   TPUCB_CHECK(it, "tpucb_interp_get_op_info: bad argument");

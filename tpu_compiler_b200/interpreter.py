@@ -133,6 +133,11 @@ class module:
                                  "shape": [int(s) for s in shape.split(",") if s],
                                  "ops": float(ops), "bytes": float(nbytes), "bound": bound})
 
+    def op_form(self, name):
+        """How the library runs a convolution or an inner product (tpucb_interp_get_op_form): a dict of words and numbers."""
+        words = (w.split("=") for w in _text(self._lib.tpucb_interp_get_op_form, self._h, name.encode()).split())
+        return {k: int(v) if v.isdigit() else v for k, v in words}
+
     def get_weight_file_path(self):
         return self._weight_file
 
