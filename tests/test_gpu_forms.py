@@ -34,23 +34,29 @@ def conv_text(dtype, n, ic, oc, hw, k, s, p, d, relu, int8=False, extra=""):
 
 
 @pytest.mark.parametrize("relu", [False, True])
-@pytest.mark.parametrize("mults", ["random", "power_of_two", "small"])
+@pytest.mark.parametrize("mults", ["normalised", "large_powers", "random", "power_of_two", "small"])
 def test_float_requantisation_edges(relu, mults):
-    """Every shift of the floating-point form's range, multipliers that make exact ties in the first rounding (powers of
-    two) or few significant bits, zero multipliers; sums close to both ends of the range."""
+    """Every shift of the floating-point form's range, normalised multipliers and those that make exact ties in the first rounding
+    (powers of two); with zero multipliers or ones of few significant bits, whose addend is no float, the same layers on the integer
+    form (with ReLU) and the 64-bit one (shifts of 30 and 31)."""
     rng = np.random.default_rng(5 + relu)
     ic, oc, hw = 32, 96, 12
     f = rng.integers(-20, 21, (oc, ic, 1, 1)).astype(np.float32)
     r = (np.arange(oc) % (23 if relu else 32)).astype(np.float32)
     m = {"random": (rng.integers(2 ** 23, 2 ** 24, oc) * 128).astype(np.float32),
          "power_of_two": np.float32(2.0) ** rng.integers(7, 31, oc).astype(np.float32),
-         "small": (rng.integers(0, 64, oc) * 2 ** 20).astype(np.float32)}[mults]
-    m[::17] = 0
+         "small": (rng.integers(0, 64, oc) * 2 ** 20).astype(np.float32),
+         "normalised": (rng.integers(2 ** 23, 2 ** 24, oc) * 128).astype(np.float32),
+         "large_powers": np.float32(2.0) ** np.where(r < 22, rng.integers(29, 31, oc), 30).astype(np.float32)}[mults]
+    floating = mults in ("normalised", "large_powers")
+    if not floating:
+        m[::17] = 0
     b = rng.integers(-2 ** 18, 2 ** 18, oc).astype(np.float32)
     b[:23] = rng.integers(-3, 4, 23)  # small sums around zero at every shift
     text = "input name=x shape=2,%d,%d,%d dtype=INT8\n" % (ic, hw, hw) + conv_text("INT8", 2, ic, oc, hw, 1, 1, 0, 1, int(relu), True)
     x = rng.integers(-128, 128, (2, ic, hw, hw)).astype(np.float32)
-    got, ref = run_model(text, {"f": f, "b": b, "r": r, "m": m}, {"x": x}, ["c"], requant="float")["c"]
+    got, ref = run_model(text, {"f": f, "b": b, "r": r, "m": m}, {"x": x}, ["c"],
+                         requant="float" if floating else ("integer" if relu else "wide"))["c"]
     assert np.array_equal(got, ref)
 
 
