@@ -50,6 +50,20 @@ def new_module(device):
     return m
 
 
+def conv_kernels(m):
+    """Which kernels the module's convolutions and inner products run on, with their launches: conv_gemm (tiles of up to 128 pixels,
+    conv_gemm_i8.cuh) and conv_big (256 pixels, on one or two SMs, conv_big.cuh), by form of the requantisation."""
+    count = {}
+    for info in m.op_info:
+        if info["bound"] == "tensor":
+            f = m.op_form(info["name"])
+            kernel = "conv_big on %d SM%s" % (f["ctas"], "s" * (f["ctas"] > 1)) if f.get("tiles") == "big" else "conv_gemm"
+            kernel += {"float": ", floating-point requantisation", "integer": ", integer requantisation",
+                       "wide": ", 64-bit requantisation"}.get(f.get("requant"), "") + (", split K" if f.get("split_k", 1) > 1 else "")
+            count[kernel] = count.get(kernel, 0) + 1
+    return "; ".join("%d %s" % (n, k) for k, n in sorted(count.items(), key=lambda e: -e[1]))
+
+
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -723,7 +737,7 @@ def main():
         i8_tops = C.c_double(0.0)  # this library's own tcgen05 kind::i8 issue microbenchmark, live on this GPU
         check(L.tpucb_measure_i8_mma_peak(local_rank, 128, C.byref(i8_tops)))
         # DRAM traffic per launch: not captured in this run (a profiler capture of this size is out of bounds). The read
-        # side is the ncu figure of a whole step at batch 64 (profiles/launch_lists.md: 16.66 MB of dram__bytes_read per
+        # side is the ncu figure of a whole step at batch 64 (16.66 MB of dram__bytes_read per
         # tensor-core launch, residuals of the fused adds among them) scaled by the images per launch; ncu attributes no write-back to these kernels (their outputs
         # are still dirty in L2 when they end), so the write side is the algorithmic output bytes. Null for the workloads
         # that have no capture.
@@ -736,8 +750,7 @@ def main():
             # BF16 graph: the same pipeline with kind::f16 MMAs; the denominator is the measured bf16 rate itself
             roofline = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
                         "frac": achieved / peaks["bf16_tflops_sustained"], "traffic": None,
-                        "kernel": "conv_gemm_bf16_kernel (tcgen05 kind::f16 implicit GEMM on BF16 operands, %d launches "
-                                  "per step)" % n_conv,
+                        "kernel": "tcgen05 kind::f16 implicit GEMM on BF16 operands, %d launches per step: %s" % (n_conv, conv_kernels(m)),
                         "peak_source": "bf16_tflops_sustained of %s peaks" % peaks["source"],
                         "avg_launch_us": conv_ms * 1e3 / max(n_conv, 1)}
         else:
@@ -749,9 +762,7 @@ def main():
                                         "batch / 64, plus the algorithmic output bytes (ncu attributes no write-back to "
                                         "the kernel); not captured in this run. Algorithmic bytes per launch: %.1f MB"
                                         % (conv_bytes / max(n_conv, 1) / 1e6),
-                        "kernel": "conv_gemm_i8_fq_kernel<0> / <1> and conv_gemm_i8_kernel: the tcgen05 kind::i8 implicit GEMM "
-                                  "of conv_gemm_i8.cuh with the floating-point and the integer requantisation, %d launches "
-                                  "per step" % n_conv,
+                        "kernel": "tcgen05 kind::i8 implicit GEMM, %d launches per step: %s" % (n_conv, conv_kernels(m)),
                         "peak_source": "2 x bf16_tflops_sustained of %s peaks (no INT8 figure is measured; the 8-bit "
                                        "rate of the same tensor pipe is twice the 16-bit rate)" % peaks["source"],
                         "avg_launch_us": conv_ms * 1e3 / max(n_conv, 1),

@@ -168,8 +168,10 @@ int tpucb_interp_get_op_form(tpucb_interp *it, const char *name, char *out, size
  *          operand and writes both the convolution's tensor and the sum; the add launches nothing. Same bits.
  *          Always: whatever "big_tiles" says of that convolution, but not in the forms whose epilogue has no add: tiles that are
  *          split ("split_k"), image stems as row windows, layers of at most 64 channels on pairs of pixel tiles.
- *          By size: results of 2.5 MiB and more of layers that widen their input (INT8 ResNet-50 at batch 19:
- *          6% fewer us, at batch 256 3% alone and 7% with three modules in flight; BF16 at batch 128 3% and 12%).
+ *          By size: behind layers that widen their input, results of 2.5 MiB and more; behind others, up to 4 MiB. INT8 layers
+ *          of more than 12 K blocks that fill the GPU keep their large tiles and an add of its own, up to 10 MiB those of 24 and more.
+ *          Fewer us than with no add fused, alone / with three modules in flight: INT8 ResNet-50 batch 19 7 / 8%, batch 256
+ *          9 / 12%, BF16 batch 128 6 / 18%, MobileNet-v2 batch 7 6 / 2%. At small batches 1 gains a little more (batch 3 3 / 7%).
  *          "fp32_tensor_cores" (0/1, default 1; read by the next load_module): fp32 convolutions with a
  *          multiple of 8 input channels run on the tensor cores as three TF32 products with fp32 accumulation
  *          (about 5e-6 of a tensor's range per layer against a double-accumulated sum, 6e-5 at the end of an
