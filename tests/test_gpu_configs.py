@@ -77,7 +77,7 @@ def test_conv_sweep_point_full_rshift_range(relu):
     _conv_against_oracle(graphs.single_conv_i8(8, 128, 128, 28, 3, 1, 1, relu=relu, rshift_range=(0, 32), seed=2999))
 
 
-@pytest.mark.parametrize("n,c,hw,relu", [(1, 512, 7, True), (2, 1024, 5, False), (3, 384, 9, True)])
+@pytest.mark.parametrize("n,c,hw,relu", [(1, 512, 7, True), (2, 1024, 5, False), (3, 512, 9, True)])
 def test_split_k_layers(n, c, hw, relu):
     """Launches with few tiles and a long K share each tile among several CTAs (int32 partial sums added in
     global memory, the CTA that completes a tile runs the epilogue). Exact against the oracle, equal to the unsplit
@@ -90,6 +90,7 @@ def test_split_k_layers(n, c, hw, relu):
         m = module(0)
         m.set_option("split_k", split)
         m.load_text(model.text, model.weights)
+        assert (m.op_form("conv")["split_k"] > 1) == bool(split)
         m.set_tensor("x", model.meta["x"])
         for _ in range(4):
             m.invoke()

@@ -290,7 +290,7 @@ def test_download_forms(dtype, shape):
 def test_split_rule_edges(case):
     from tpu_compiler_b200 import module
     n, ic, oc, hw, k, pixels, parts = case
-    model = graphs.single_conv_i8(n, ic, oc, hw, k, 1, k // 2, seed=3300 + k)
+    model = graphs.single_conv_i8(n, ic, oc, hw, k, 1, k // 2, relu=parts % 2 == 0, seed=3300 + k)
     got = []
     for split in (1, 0):
         m = module(0)

@@ -313,12 +313,18 @@ def test_softmax_bf16(cfg, do_log):
 
 
 @pytest.mark.parametrize("relu", [False, True])
-@pytest.mark.parametrize("rshift_range", [(0, 4), (8, 30), (28, 32)])
-def test_conv_i8_requant_forms(relu, rshift_range):
-    """Both forms of the tensor-core requantisation against the oracle: shifts up to 29 take the multiply-high
-    form, a layer with a larger shift the 64-bit multiply-add form; small shifts saturate most outputs."""
+@pytest.mark.parametrize("rshift_range,form", [((0, 4), "float"), ((0, 24), "integer"), ((8, 30), "integer"), ((28, 32), "wide")])
+def test_conv_i8_requant_forms(relu, rshift_range, form):
+    """The forms of the tensor-core requantisation against the oracle: layers whose results are saturated where sums leave its
+    exact range take the floating-point form, others with shifts up to 29 the multiply-high form, with a larger shift the 64-bit
+    multiply-add form; small shifts saturate most outputs."""
+    from tpu_compiler_b200 import module
     model = graphs.single_conv_i8(n=2, c_in=64, c_out=160, hw=12, k=3, pad=1, relu=relu, seed=4100 + rshift_range[0],
                                   rshift_range=rshift_range)
+    m = module(0)
+    m.load_text(model.text, model.weights)
+    assert m.op_form("conv")["requant"] == form
+    m.close()
     assert_exact(run_both(model.text, model.weights, model.meta, ["conv"]))
 
 
